@@ -278,35 +278,34 @@ __device__ __forceinline__ int monotonize_r(const CurveGeom &g, bool visible, fl
 }
 
 // Crossing of coordinate P(t) = c on [tmin, tmax].
-__device__ __forceinline__ float solve_crossing(const CurveGeom &g, const float *P, float c, float tmin, float tmax) {
-    if (g.type == kLinear) {
+__device__ __forceinline__ float solve_crossing(int type, float w, const float *P, float c, float tmin, float tmax) {
+    if (type == kLinear) {
         float t = (c - P[0]) * safe_rcp(P[1] - P[0]);
         t = t > tmin ? t : tmin;
         return t < tmax ? t : tmax;
     }
-    if (g.type == kQuad) return solve_quad_bezier(P[0], P[1], P[2], c, tmin, tmax);
-    if (g.type == kRational) return solve_quad_bezier(P[0] - c, (P[1] - c) * g.w, P[2] - c, 0.f, tmin, tmax);
+    if (type == kQuad) return solve_quad_bezier(P[0], P[1], P[2], c, tmin, tmax);
+    if (type == kRational) return solve_quad_bezier(P[0] - c, (P[1] - c) * w, P[2] - c, 0.f, tmin, tmax);
+    // 24 bisection steps.  The sign of the coordinate's offset from c at the
+    // bracket's start never changes (a step replaces the start only by a point
+    // of the same sign), so it is taken once; both next midpoints are formed
+    // while the point is evaluated, which takes them off the serial chain.
     float t0 = tmin, t1 = tmax;
-    float vt0 = cubic_coord(P, t0);
-    float ts = t0;
-    if (vt0 != c) {
-        float raw_t0 = t0;
-        float last = 0.f;
+    const float vt0 = cubic_coord(P, t0);
+    if (vt0 == c) return t0;
+    const bool s0 = (int32_t)fbits(vt0 - c) < 0;
+    float tm = (t0 + t1) * .5f, ts = tm, last = 0.f;
 #pragma unroll 4
-        for (int it = 0; it < 24; ++it) {
-            float tm = (t0 + t1) * .5f;
-            float vtm = cubic_coord(P, tm);
-            ts = tm;
-            last = vtm;
-            if ((int32_t)(fbits(vtm - c) ^ fbits(vt0 - c)) >= 0) {
-                t0 = tm;
-                vt0 = vtm;
-            } else {
-                t1 = tm;
-            }
-        }
-        if (fabsf(last - c) > 1.f) ts = raw_t0;
+    for (int it = 0; it < 24; ++it) {
+        ts = tm;
+        last = cubic_coord(P, tm);
+        const float ta = (tm + t1) * .5f, tb = (t0 + tm) * .5f;
+        const bool same = ((int32_t)fbits(last - c) < 0) == s0;
+        t0 = same ? tm : t0;
+        t1 = same ? t1 : tm;
+        tm = same ? ta : tb;
     }
+    if (fabsf(last - c) > 1.f) ts = tmin;
     return ts;
 }
 

@@ -204,8 +204,8 @@ int launch_emit_keys(const FrameArgs &a, const uint32_t *counts, uint32_t *key, 
 // The kernels below read the frame's sizes from the counters (ctr); their
 // grids are sized for the buffers' capacities (cap_*).
 int launch_curve_emit(const FrameArgs &a, const float2 *tvert, const uint8_t *path_visible,
-                      const uint32_t *offsets, const uint32_t *order, int2 *entries, const FrameCounters *ctr,
-                      cudaStream_t s);
+                      const uint32_t *offsets, const uint32_t *order, float *scratch, int2 *entries,
+                      const FrameCounters *ctr, cudaStream_t s);
 int launch_fragment(const FrameArgs &a, const float2 *tvert, const int2 *entries, int64_t cap_nf,
                     const FrameCounters *ctr, int32_t *key, uint32_t *pidw, int8_t *wn, uint32_t *mask,
                     uint64_t *sort_key, uint32_t *sort_val, cudaStream_t s);

@@ -162,10 +162,9 @@ __global__ void k_curve_count(FrameArgs a, const float2 *__restrict__ tv, const 
 // Entries of one curve in t order: each monotone piece emits its start and
 // every crossing with a vertical (x = even) or horizontal (y = even) cell
 // line, the two crossing chains merged by t; equal t values OR their flags.
-// Emission order: curves grouped by type (cubics, whose crossings are
-// bisections, first) and within a type by decreasing entry count, so that
-// the curves of a warp run the same solver the same number of times and
-// the longest start first.  16-bit key, ascending.
+// Emission order (a tuning choice, off by default): curves grouped by type
+// (cubics, whose crossings are bisections, first) and within a type by
+// decreasing entry count.  16-bit key, ascending.
 __global__ void k_emit_keys(FrameArgs a, const uint32_t *__restrict__ counts, uint32_t *__restrict__ key,
                             uint32_t *__restrict__ val) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -176,197 +175,304 @@ __global__ void k_emit_keys(FrameArgs a, const uint32_t *__restrict__ counts, ui
     val[c] = (uint32_t)c;
 }
 
-// Entries of one monotone piece, whose chain starts from the piece's own
-// t0 and is solved crossing by crossing (k_make_intersection_impl_1,
-// ras_cut.h:837-1241): every piece is an independent work item.
-struct PieceState {
-    CurveGeom g;
-    int2 *out;
-    int cid, p, i, n_loop, nx, ny;
-    float x, y, dx, dy, slot0, slot1, t1_ms;
-    uint32_t last;
+// Entries of one monotone piece (k_make_intersection_impl_1,
+// ras_cut.h:837-1241): its start and its crossings with vertical and
+// horizontal cell lines.  The reference solves the crossings one by one in
+// merged t order, each from the parameter of the previous crossing with a
+// line of the same direction: the two directions are independent chains, and
+// the merge takes the nearer of their current crossings, the vertical one on
+// ties (CurveChain below solves a chain, merge_piece merges two).
+constexpr int kEmitThreads = 256;
+constexpr int kEmitCurves = 128;   // curves of a block, at most
+constexpr int kEmitLocal = 4096;   // crossings of a block's curves held in shared memory (else in global scratch)
+constexpr int kMergeSerial = 24;   // entries of a piece merged by one lane (longer pieces: by a warp)
+constexpr int kChainClasses = 24;  // solver (cubic, quadratic, line) x length octave
+
+// A block's curves, their monotone pieces' end parameters (flags in the low
+// bits), the pieces' first entries within the curve, and per piece and
+// direction the crossings: first line (13 bits) | falling << 13 | count << 14.
+struct EmitBlock {
+    float px[4][kEmitCurves], py[4][kEmitCurves], w[kEmitCurves], tq[5][kEmitCurves];
+    uint32_t chain[2][5][kEmitCurves];
+    uint32_t rel[5][kEmitCurves];
+    uint32_t type[kEmitCurves], cid[kEmitCurves];
+    uint32_t off[kEmitCurves];  // the curve's first entry
+    uint32_t tof[kEmitCurves];  // its first solved parameter
+    uint32_t cls[32], warp_pieces[8], warp_entries[8], next_chain;
+    uint16_t item[2 * 5 * kEmitCurves];  // chains in the order they are solved: curve | piece << 7 | direction << 10
+    uint16_t piece[5 * kEmitCurves];     // the pieces: curve | piece << 7
+    float t[kEmitLocal];
 };
 
-// Sets up piece ms of a curve (v0, v1: its end points; t0_ms: the previous
-// piece's end parameter with its flags, 0 for the first).
-__device__ __forceinline__ void piece_begin(PieceState &st, const Dim &dm, float t0_ms, float traw, float v0x,
-                                            float v0y, float v1x, float v1y) {
-    const uint32_t tb = fbits(traw) & 0xFFFFFFFCu;
-    st.t1_ms = (floorf(v1x) == v1x) ? ffrom(tb | 2u) : ffrom(tb | 3u);
-    const CutRange cr = cut_range(v0x, v0y, v1x, v1y, dm.W, dm.H);
-    st.nx = cr.nx;
-    st.ny = cr.ny;
-    st.n_loop = cr.nx + cr.ny + 1;
-    st.x = (float)(cr.dx < 0.f ? cr.xe : cr.xb);
-    st.y = (float)(cr.dy < 0.f ? cr.ye : cr.yb);
-    st.dx = cr.dx;
-    st.dy = cr.dy;
-    st.slot0 = st.slot1 = t0_ms;
-    st.last = fbits(-1.f);
-    st.p = 0;
-    st.i = -1;
+__device__ __forceinline__ float piece_t0(const EmitBlock &S, int L, int ms) { return ms > 0 ? S.tq[ms - 1][L] : 0.f; }
+
+// Class of a chain: solver, then length octaves from the longest.
+__device__ __forceinline__ uint32_t chain_class(int type, uint32_t n) {
+    return (type == kCubic ? 0u : (type == kLinear ? 16u : 8u)) + 7u - (uint32_t)min(31 - __clz((int)n), 7);
 }
 
-// One step of a piece: the entry at the nearer of the two chains' current
-// crossings (the piece start first), then the next crossing of that chain.
-// Returns false once the piece is done.
-__device__ __forceinline__ bool piece_step(PieceState &st) {
-    float t_solve = 0.f, c = 0.f, t_min;
-    int side = 0;
-    if (st.i == -1) {
-        t_min = st.slot0;
-        if (st.nx == 0) {
-            side = 0;
-            t_solve = 2.f;
-        } else if (st.ny == 0) {
-            side = 1;
-            t_solve = 2.f;
-        } else {
-            side = 0;
-            st.nx--;
-            c = st.x;
-            st.x += st.dx;
-        }
-    } else if (st.slot0 <= st.slot1) {
-        t_min = st.slot0;
-        side = 0;
-        if (st.nx > 0) {
-            st.nx--;
-            c = st.x;
-            st.x += st.dx;
-        } else {
-            t_solve = 2.f;
-        }
+// Entries of a piece from its solved chains, X[nx] and Y[ny], by one lane:
+// the heads of the two chains compared as the reference does.  Coincident
+// parameters: both entries get both flags.
+__device__ __forceinline__ void merge_piece(const float *X, int nx, const float *Y, int ny, float t0, int cid,
+                                            int2 *__restrict__ out) {
+    const float none0 = 2.f, none1 = ffrom(fbits(2.f) | 1u);
+    int ix = 0, iy = 0;
+    float h0, h1;
+    if (nx == 0) {
+        h0 = none0;
+        h1 = t0;
+    } else if (ny == 0) {
+        h0 = t0;
+        h1 = none1;
     } else {
-        t_min = st.slot1;
-        side = 1;
-        if (st.ny > 0) {
-            st.ny--;
-            c = st.y;
-            st.y += st.dy;
+        h0 = X[ix++];
+        h1 = t0;
+    }
+    uint32_t last = fbits(-1.f);
+    const int n = nx + ny + 1;
+    for (int p = 0; p < n; ++p) {
+        uint32_t ob;
+        if (h0 <= h1) {
+            ob = fbits(h0);
+            h0 = ix < nx ? X[ix++] : none0;
         } else {
-            t_solve = 2.f;
+            ob = fbits(h1);
+            h1 = iy < ny ? Y[iy++] : none1;
         }
-    }
-    if (st.i >= 0) {
-        uint32_t ob = fbits(t_min);
-        if ((ob & 0xFFFFFFFCu) == (st.last & 0xFFFFFFFCu)) {  // coincident t: both entries get both flags
-            ob |= st.last;
-            st.out[st.p - 1] = make_int2(st.cid, (int)ob);
+        if ((ob & 0xFFFFFFFCu) == (last & 0xFFFFFFFCu)) {
+            ob |= last;
+            out[p - 1] = make_int2(cid, (int)ob);
         }
-        st.out[st.p] = make_int2(st.cid, (int)ob);
-        st.last = ob;
-        st.p++;
+        out[p] = make_int2(cid, (int)ob);
+        last = ob;
     }
-    if (t_solve < 2.f) t_solve = solve_crossing(st.g, side ? st.g.py : st.g.px, c, t_min, st.t1_ms);
-    const float sv = ffrom((fbits(t_solve) & 0xFFFFFFFCu) | (uint32_t)side);
-    if (side) st.slot1 = sv;
-    else st.slot0 = sv;
-    return ++st.i < st.n_loop;
 }
 
-// Per warp: its 32 curves (in emission order), their monotone cut points
-// and the output position of every piece.
-constexpr int kEmitWarps = 4;
-struct EmitStash {
-    float px[4][32], py[4][32], w[32], q[5][32];
-    uint32_t type[32], cid[32], poff[5][32];
-    uint32_t item[5 * 32];  // warp item k: lane | piece << 8
-};
+// The same by the whole warp, 32 entries at a time: entry p's split between
+// the chains by a binary search on the merge diagonal.  X ascends; Y, with
+// the piece start before it, ascends but for crossings whose flag bits order
+// them just before the start: the search compares the running maximum, which
+// gives the head comparison's order.  A run of coincident parameters
+// accumulates its flags in order (an entry gets those up to its successor).
+__device__ __forceinline__ void merge_piece_warp(const float *X, int nx, const float *Y, int ny, float t0, int cid,
+                                                 int2 *__restrict__ out, int lane) {
+    const int n = nx + ny + 1;
+    uint32_t carry_t = 0xFFFFFFFFu, carry_f = 0u;
+    for (int base = 0; base < n; base += 32) {
+        const int p = base + lane;
+        const bool live = p < n;
+        float e = 0.f;
+        if (live) {
+            if (nx == 0 || ny == 0) {
+                e = p == 0 ? t0 : (nx == 0 ? Y[p - 1] : X[p - 1]);
+            } else {
+                const int b = ny + 1;  // the start, then Y
+                int lo = max(0, p - b), hi = min(p, nx);
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1, j = p - 1 - mid;
+                    const float y = j == 0 ? t0 : fmaxf(t0, Y[j - 1]);
+                    if (X[mid] <= y) lo = mid + 1;
+                    else hi = mid;
+                }
+                const int j = p - lo;
+                const float y = j == 0 ? t0 : (j < b ? Y[j - 1] : 2.f);
+                e = lo < nx && (j >= b || X[lo] <= fmaxf(t0, y)) ? X[lo] : y;
+            }
+        }
+        const uint32_t tb = live ? fbits(e) & 0xFFFFFFFCu : 0xFFFFFFF8u, f = live ? fbits(e) & 3u : 0u;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, tb, 1);
+        if (lane == 0) prev = carry_t;
+        const uint32_t eq = __ballot_sync(0xffffffffu, live && tb == prev);
+        const uint32_t b0 = __ballot_sync(0xffffffffu, f & 1u), b1 = __ballot_sync(0xffffffffu, f & 2u);
+        const uint32_t le = 0xFFFFFFFFu >> (31 - lane);
+        const uint32_t heads = ~eq & le;  // this lane's run: from its last head (or from the previous window)
+        const uint32_t run = heads ? le & ~((1u << (31 - __clz(heads))) - 1u) : le;
+        const uint32_t nx1 = lane < 31 ? (eq >> (lane + 1)) & 1u : 0u;  // the next entry is in the run
+        const uint32_t upto = run | (nx1 << (lane < 31 ? lane + 1 : 0));
+        const uint32_t in = heads ? 0u : carry_f;
+        const uint32_t own = in | ((b0 & run) ? 1u : 0u) | ((b1 & run) ? 2u : 0u);
+        const uint32_t full = in | ((b0 & upto) ? 1u : 0u) | ((b1 & upto) ? 2u : 0u);
+        if (live) out[p] = make_int2(cid, (int)(tb | full));
+        if (lane == 0 && (eq & 1u)) out[p - 1] = make_int2(cid, (int)(tb | own));  // (written by the last window)
+        carry_t = __shfl_sync(0xffffffffu, tb, 31);
+        carry_f = __shfl_sync(0xffffffffu, own, 31);
+        __syncwarp();
+    }
+}
 
-// One warp per 32 curves.  Each lane expands its curve into its monotone
-// pieces; the warp's pieces form one list, and a lane whose piece is done
-// takes the next one (a ballot ranks the lanes asking), so the lanes stay
-// busy until the list runs out instead of waiting for the curve with the
-// most crossings.  Curves come in emission order (grouped by type), so a
-// warp's pieces mostly run the same solver.
-__global__ void __launch_bounds__(kEmitWarps * 32) k_curve_emit(FrameArgs a, const float2 *__restrict__ tv,
-                                                                const uint8_t *__restrict__ vis,
-                                                                const uint32_t *__restrict__ offsets,
-                                                                const uint32_t *__restrict__ order,
-                                                                int2 *__restrict__ entries,
-                                                                const FrameCounters *__restrict__ ctr) {
-    __shared__ EmitStash stash[kEmitWarps];
+// One block per `per_block` curves.  Each thread expands one curve into its
+// monotone pieces; the crossings of a piece are two independent chains (see
+// above), and every chain is one work item of a lane: the longest serial
+// sequence is the crossings of one curve with the lines of one direction.
+// The block's chains are solved grouped by solver (cubics, whose crossings are
+// bisections, first) and by decreasing length, a lane whose chain is done
+// taking the block's next one, so that the lanes of a warp run the same solver
+// and stay busy until the list runs out.  Then the pieces are merged, short
+// ones one per lane and long ones by a warp.  Bound by the latency of a
+// chain's bisections (about 0.9 us a crossing) where curves are few and by
+// issue (420 thread instructions an entry, 19 lanes active) where they are
+// many.  With one lane solving both directions of a piece, 32 curves to a
+// warp in a device-wide order by type and length, emission + fragments took
+// 620 us on 64 paths over 512 x 512, 533 us on 2,500 paths over 1917 x 1079
+// and 787 us on the 20,000-path 2048 x 2048 scene; here 304, 280 and 783.
+__global__ void __launch_bounds__(kEmitThreads)
+    k_curve_emit(FrameArgs a, int per_block, const float2 *__restrict__ tv, const uint8_t *__restrict__ vis,
+                 const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ order, float *scratch,
+                 int2 *__restrict__ entries, const FrameCounters *__restrict__ ctr) {
+    __shared__ EmitBlock S;
     // entries not admitted (the buffers are too small), or the offsets not
     // to be trusted (a scan gave up waiting): nothing is written
     if (ctr->status != 0u || ctr->nf != ctr->need_nf) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    EmitStash &S = stash[warp];
-    const int i = (blockIdx.x * kEmitWarps + warp) * 32 + lane;
-    int np = 0;
-    if (i < a.C) {
-        const int cid = order != nullptr ? (int)order[i] : i;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t i = (int64_t)blockIdx.x * per_block + tid;
+    int np = 0, type = 0;
+    uint32_t n_ent = 0;
+    if (tid < 32) S.cls[tid] = 0u;
+    if (tid == 0) S.next_chain = 0u;
+    __syncthreads();
+    if (tid < per_block && i < a.C) {
+        const int cid = order != nullptr ? (int)order[i] : (int)i;
         const CurveDesc d = a.curves[cid];
         CurveGeom g;
         load_geom(d, tv, g);
+        type = g.type;
         float q[5];
         np = monotonize_r(g, vis[d.pid] != 0, q);
         const Dim dm = dim_of(a, d.pid);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) S.px[k][lane] = g.px[k], S.py[k][lane] = g.py[k];
-        S.w[lane] = g.w;
-        S.type[lane] = (uint32_t)g.type;
-        S.cid[lane] = (uint32_t)cid;
-        uint32_t run = offsets[cid];
+        for (int k = 0; k < 4; ++k) S.px[k][tid] = g.px[k], S.py[k][tid] = g.py[k];
+        S.w[tid] = g.w;
+        S.type[tid] = (uint32_t)type;
+        S.cid[tid] = (uint32_t)cid;
+        S.off[tid] = offsets[cid];
         float v0x = g.px[0], v0y = g.py[0];
 #pragma unroll
         for (int ms = 0; ms < 5; ++ms) {
-            S.q[ms][lane] = q[ms];
-            S.poff[ms][lane] = run;
             if (ms < np) {
                 const float v1x = curve_coord(g.type, g.w, g.px, q[ms]), v1y = curve_coord(g.type, g.w, g.py, q[ms]);
                 const CutRange cr = cut_range(v0x, v0y, v1x, v1y, dm.W, dm.H);
-                run += 1 + cr.nx + cr.ny;
+                const uint32_t tb = fbits(q[ms]) & 0xFFFFFFFCu;
+                S.tq[ms][tid] = (floorf(v1x) == v1x) ? ffrom(tb | 2u) : ffrom(tb | 3u);
+                S.rel[ms][tid] = n_ent;
+                const int bx = cr.dx < 0.f ? cr.xe : cr.xb, by = cr.dy < 0.f ? cr.ye : cr.yb;
+                S.chain[0][ms][tid] = ((uint32_t)bx & 0x1FFFu) | (cr.dx < 0.f ? 0x2000u : 0u) | ((uint32_t)cr.nx << 14);
+                S.chain[1][ms][tid] = ((uint32_t)by & 0x1FFFu) | (cr.dy < 0.f ? 0x2000u : 0u) | ((uint32_t)cr.ny << 14);
+                if (cr.nx) atomicAdd(&S.cls[chain_class(type, (uint32_t)cr.nx)], 1u);
+                if (cr.ny) atomicAdd(&S.cls[chain_class(type, (uint32_t)cr.ny)], 1u);
+                n_ent += 1 + cr.nx + cr.ny;
                 v0x = v1x;
                 v0y = v1y;
             }
         }
     }
-    // the warp's piece list
-    uint32_t pre = (uint32_t)np;
+    // the block's pieces and entries; the chains placed by class
+    uint32_t pre = (uint32_t)np, lpre = n_ent;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
-        if (lane >= o) pre += v;
+        const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o), u = __shfl_up_sync(0xffffffffu, lpre, o);
+        if (lane >= o) pre += v, lpre += u;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
-    pre -= (uint32_t)np;
-    for (int ms = 0; ms < np; ++ms) S.item[pre + ms] = (uint32_t)lane | ((uint32_t)ms << 8);
-    __syncwarp();
-    PieceState st;
-    bool active = false;
-    uint32_t next = 0;
-    for (;;) {
-        const uint32_t want = __ballot_sync(0xffffffffu, !active);
-        if (!active) {
-            const uint32_t k = next + __popc(want & ((1u << lane) - 1u));
-            if (k < total) {
-                const uint32_t it = S.item[k];
-                const int L = (int)(it & 0xFFu), ms = (int)(it >> 8);
-                st.g.type = (int)S.type[L];
-                st.g.w = S.w[L];
+    if (lane == 31) S.warp_pieces[warp] = pre, S.warp_entries[warp] = lpre;
+    __syncthreads();
+    uint32_t n_pieces = 0, n_total = 0, wp = 0, we = 0;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) st.g.px[c] = S.px[c][L], st.g.py[c] = S.py[c][L];
-                st.cid = (int)S.cid[L];
-                st.out = entries + S.poff[ms][L];
-                const float tq = S.q[ms][L];
-                const float v1x = curve_coord(st.g.type, st.g.w, st.g.px, tq),
-                            v1y = curve_coord(st.g.type, st.g.w, st.g.py, tq);
-                float t0_ms = 0.f, v0x = st.g.px[0], v0y = st.g.py[0];
-                if (ms > 0) {  // the previous piece's end: its parameter with its flags
-                    const float tp = S.q[ms - 1][L];
-                    v0x = curve_coord(st.g.type, st.g.w, st.g.px, tp);
-                    v0y = curve_coord(st.g.type, st.g.w, st.g.py, tp);
-                    const uint32_t tb = fbits(tp) & 0xFFFFFFFCu;
-                    t0_ms = (floorf(v0x) == v0x) ? ffrom(tb | 2u) : ffrom(tb | 3u);
-                }
-                piece_begin(st, dim_of(a, a.curves[st.cid].pid), t0_ms, tq, v0x, v0y, v1x, v1y);
-                active = true;
+    for (int k = 0; k < kEmitThreads / 32; ++k) {
+        if (k == warp) wp = n_pieces, we = n_total;
+        n_pieces += S.warp_pieces[k];
+        n_total += S.warp_entries[k];
+    }
+    pre += wp - (uint32_t)np;
+    lpre += we - n_ent;
+    const bool local = n_total <= (uint32_t)kEmitLocal;
+    // every warp scans the class counts (the same values); one keeps them as cursors
+    uint32_t cls = lane < kChainClasses ? S.cls[lane] : 0u;
+    const uint32_t cls_n = cls;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, cls, o);
+        if (lane >= o) cls += v;
+    }
+    const uint32_t n_chains = __shfl_sync(0xffffffffu, cls, 31);
+    __syncthreads();
+    if (warp == 0) S.cls[lane] = cls - cls_n;
+    __syncthreads();
+    if (np > 0) {
+        S.tof[tid] = local ? lpre : S.off[tid];
+        for (int ms = 0; ms < np; ++ms) {
+            S.piece[pre + ms] = (uint16_t)(tid | (ms << 7));
+            for (int ax = 0; ax < 2; ++ax) {
+                const uint32_t n = S.chain[ax][ms][tid] >> 14;
+                if (n) S.item[atomicAdd(&S.cls[chain_class(type, n)], 1u)] = (uint16_t)(tid | (ms << 7) | (ax << 10));
             }
         }
-        next += __popc(want);
-        if (!__any_sync(0xffffffffu, active)) break;
-        if (active) active = piece_step(st);
+    }
+    __syncthreads();
+    float *const tbuf = local ? S.t : scratch;
+    // chains: crossing k of a piece's vertical lines at t[1 + k] of the piece,
+    // of its horizontal ones past them
+    {
+        int ctype = 0, rem = 0, ax = 0;
+        float P[4] = {0.f, 0.f, 0.f, 0.f}, w = 0.f, c = 0.f, dc = 0.f, t = 0.f, t1 = 0.f;
+        float *out = nullptr;
+        bool more = true;
+        for (;;) {
+            const uint32_t want = __ballot_sync(0xffffffffu, rem == 0);
+            if (more && want) {
+                uint32_t next = 0;
+                if (lane == 0) next = atomicAdd(&S.next_chain, (uint32_t)__popc(want));
+                next = __shfl_sync(0xffffffffu, next, 0);
+                more = next + __popc(want) < n_chains;
+                const uint32_t k = next + __popc(want & ((1u << lane) - 1u));
+                if (rem == 0 && k < n_chains) {
+                    const uint32_t it = S.item[k];
+                    const int L = (int)(it & 127u), ms = (int)(it >> 7) & 7;
+                    ax = (int)(it >> 10);
+                    ctype = (int)S.type[L];
+                    w = S.w[L];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) P[j] = ax ? S.py[j][L] : S.px[j][L];
+                    const uint32_t ch = S.chain[ax][ms][L];
+                    rem = (int)(ch >> 14);
+                    c = (float)(ch & 0x1FFFu);
+                    dc = (ch & 0x2000u) ? -2.f : 2.f;
+                    t = piece_t0(S, L, ms);
+                    t1 = S.tq[ms][L];
+                    out = tbuf + S.tof[L] + S.rel[ms][L] + 1 + (ax ? S.chain[0][ms][L] >> 14 : 0u);
+                }
+            }
+            if (!__any_sync(0xffffffffu, rem > 0)) break;
+            if (rem > 0) {
+                t = ffrom((fbits(solve_crossing(ctype, w, P, c, t, t1)) & 0xFFFFFFFCu) | (uint32_t)ax);
+                *out++ = t;
+                c += dc;
+                --rem;
+            }
+        }
+    }
+    __syncthreads();
+    for (uint32_t base = warp * 32; base < n_pieces; base += kEmitThreads) {
+        const uint32_t k = base + lane;
+        int L = 0, ms = 0, nx = 0, ny = 0;
+        if (k < n_pieces) {
+            L = S.piece[k] & 127;
+            ms = S.piece[k] >> 7;
+            nx = (int)(S.chain[0][ms][L] >> 14);
+            ny = (int)(S.chain[1][ms][L] >> 14);
+        }
+        const bool lng = nx + ny + 1 > kMergeSerial;
+        if (k < n_pieces && !lng) {
+            const float *X = tbuf + S.tof[L] + S.rel[ms][L] + 1;
+            merge_piece(X, nx, X + nx, ny, piece_t0(S, L, ms), (int)S.cid[L], entries + S.off[L] + S.rel[ms][L]);
+        }
+        for (uint32_t m = __ballot_sync(0xffffffffu, lng); m; m &= m - 1u) {
+            const int src = __ffs(m) - 1;
+            const int qL = __shfl_sync(0xffffffffu, L, src), qm = __shfl_sync(0xffffffffu, ms, src);
+            const int qx = __shfl_sync(0xffffffffu, nx, src), qy = __shfl_sync(0xffffffffu, ny, src);
+            const float *X = tbuf + S.tof[qL] + S.rel[qm][qL] + 1;
+            merge_piece_warp(X, qx, X + qx, qy, piece_t0(S, qL, qm), (int)S.cid[qL], entries + S.off[qL] + S.rel[qm][qL],
+                             lane);
+        }
     }
 }
 
@@ -1885,6 +1991,17 @@ int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, ui
     return n;
 }
 
+// Curves a block of k_curve_emit takes: about 5 blocks per SM, so that few
+// curves still reach every SM, up to the 128 that a block holds, which pack
+// their chains best.  Emission + fragments of the measured scenes, us at
+// 8 / 32 / 128 curves: 1,378 curves 304 / 309 / 395, 24 k 288 / 167 / 169,
+// 158 k 386 / 167 / 118, 1.74 M 3972 / 1488 / 783.
+static int emit_curves(int C) {
+    int n = 8;
+    while (n < kEmitCurves && n * 768 < C) n *= 2;
+    return n;
+}
+
 int launch_curve_count(const FrameArgs &a, const float2 *tvert, const uint8_t *vis, uint32_t *counts, cudaStream_t s) {
     if (a.C <= 0) return 0;
     k_curve_count<<<grid_for(a.C), kThreads, 0, s>>>(a, tvert, vis, counts);
@@ -1898,10 +2015,12 @@ int launch_emit_keys(const FrameArgs &a, const uint32_t *counts, uint32_t *key, 
 }
 
 int launch_curve_emit(const FrameArgs &a, const float2 *tvert, const uint8_t *vis, const uint32_t *offsets,
-                       const uint32_t *order, int2 *entries, const FrameCounters *ctr, cudaStream_t s) {
+                       const uint32_t *order, float *scratch, int2 *entries, const FrameCounters *ctr,
+                       cudaStream_t s) {
     if (a.C <= 0) return 0;
-    k_curve_emit<<<grid_for(a.C, kEmitWarps * 32), kEmitWarps * 32, 0, s>>>(a, tvert, vis, offsets, order, entries,
-                                                                           ctr);
+    const int per_block = emit_curves(a.C);
+    k_curve_emit<<<grid_for(a.C, per_block), kEmitThreads, 0, s>>>(a, per_block, tvert, vis, offsets, order, scratch,
+                                                                   entries, ctr);
     return 1;
 }
 

@@ -194,7 +194,7 @@ int spr_set_gradients(spr_handle *h, const uint32_t *table, uint32_t n_entries, 
  * band height; 64 x 1, 32 x 2, 16 x 4 or 8 x 8 cells of 2 x 2 pixels, 32
  * cells: one per lane of the warp that resolves the tile).  -1 / 0 select
  * the built-in rule (segment sort for frames of at least 1,024 paths
- * averaging at most 2,048 entries; emission order from 4,096 curves; 4
+ * averaging at most 2,048 entries; no emission order; 4
  * blocks per SM; tiles of 16 x 4 cells when the spans of the handle's last
  * sized frame covered at most 8 pixels per draw item, else 64 x 1: narrow
  * tiles cut long spans into many more resolve pairs).  Differentiable
