@@ -135,7 +135,9 @@ struct spr_handle {
     // gradient paints: table entries and ramp texels on the device, and the
     // reverse transform (pixel -> scene) of their coordinates
     DevBuf grad_table, grad_ramp;
-    DevBuf path_start;  // first curve of every path (the per-path segment sort)
+    DevBuf path_start;  // first curve of every path (the per-path segment sort; written with the scene)
+    DevBuf seg_list;    // the paths whose segments blocks sort
+    int64_t longest = 0;  // entries of the longest path in the last sized frame
     // launch choices (spr_autotune; -1 / 0 = the built-in rule): fragment
     // sort (0 device-wide radix, 1 per-path segments), curve-emission order
     // (0 off, 1 on), resolve blocks per SM
@@ -220,7 +222,7 @@ std::vector<DevBuf *> handle_bufs(spr_handle *h) {
                       &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->tape_rec,
                       &h->grad_tvert, &h->vmap, &h->bitems, &h->vmask, &h->chain, &h->ekey[0], &h->ekey[1], &h->eval[0],
                       &h->eval[1], &h->sc_vpos, &h->sc_type, &h->sc_pid, &h->sc_w, &h->scene_flags,
-                      &h->sums, &h->gfill_pass, &h->gtvert_total, &h->grad_table, &h->grad_ramp, &h->path_start,
+                      &h->sums, &h->gfill_pass, &h->gtvert_total, &h->grad_table, &h->grad_ramp, &h->path_start, &h->seg_list,
                       &h->output, &h->lb_mark, &h->lb_pair};
 }
 
@@ -536,6 +538,8 @@ int set_scene_host(spr_handle *h, const spr_scene_view *v) {
     if ((st = upload(h->fill, v->path_fill_rgba, P))) return st;
     h->has_affine = v->path_affine != nullptr;
     if (h->has_affine && (st = upload(h->affine, v->path_affine, 6 * (size_t)P))) return st;
+    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), nullptr);
+    if (cudaStreamSynchronize(nullptr) != cudaSuccess) return cuda_status();
     h->P = P;
     h->C = C;
     h->V = V;
@@ -570,7 +574,7 @@ int spr_set_scene(spr_handle *h, const spr_scene_view *v) {
         (st = ensure(h->sc_vpos, 4 * (size_t)C)) || (st = ensure(h->sc_type, (size_t)C)) ||
         (st = ensure(h->sc_pid, 4 * (size_t)C)) || (st = ensure(h->sc_w, 4 * (size_t)C)) ||
         (st = ensure(h->rule, (size_t)P)) || (st = ensure(h->fill, 4 * (size_t)P)) ||
-        (st = ensure(h->scene_flags, 4)) || (v->path_affine && (st = ensure(h->affine, 24 * (size_t)P))))
+        (st = ensure(h->scene_flags, 4)) || (st = ensure(h->path_start, 4 * ((size_t)P + 1))) || (v->path_affine && (st = ensure(h->affine, 24 * (size_t)P))))
         return st;
     cudaStream_t s = nullptr;
     auto put = [&](DevBuf &b, const void *src, size_t bytes) {
@@ -590,6 +594,8 @@ int spr_set_scene(spr_handle *h, const spr_scene_view *v) {
                          v->curve_arc_w ? h->sc_w.as<float>() : nullptr, C, V, P, h->vertex.as<float2>(),
                          h->vpid.as<uint32_t>(), h->vmap.as<uint32_t>(), h->curves.as<CurveDesc>(),
                          h->scene_flags.as<uint32_t>(), s);
+    // (of an invalid scene: entries past P are never written)
+    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), s);
     cudaMemcpyAsync(h->h_u32, h->scene_flags.p, 4, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
     if ((st = cuda_status())) return st;
@@ -813,11 +819,15 @@ void supersede(spr_handle *h) {
     cudaGetLastError();  // (cudaErrorNotReady)
 }
 
-// Fragment sort choice: one block per path needs enough paths to fill the
-// GPU and segments short enough for shared memory (longer ones are sorted by
-// a single block, chunk by chunk).
-constexpr int64_t kSegmentSortMinPaths = 1024;
-constexpr int64_t kSegmentSortMaxMean = 2048;  // mean entries per path
+// Fragment sort choice: per-path segments unless one path is so long that the
+// block sorting it alone outlasts the device-wide radix sort.  Measured: a
+// block takes 4.1 us per 1,000 entries of the longest path (43 k: 193 us, 179 k:
+// 762), the radix sort 90 us and 5.2 us per 100,000 entries of the frame
+// (0.18 M: 94 us, 5.7 M: 370).
+bool per_path_sort(const spr_handle *h) {
+    if (h->tune_sort >= 0) return h->tune_sort == 1;
+    return 15.0 + 4.2e-3 * (double)h->longest <= 88.0 + 5.2e-5 * (double)h->cap_nf;
+}
 
 // One frame.  Sized (differentiable frames, and the first frame after a
 // change of scene, viewport or sample count): the entry count and then the
@@ -870,12 +880,15 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     L += scan_lookback_u32(h->counts.as<uint32_t>(), h->offsets.as<uint32_t>(), nullptr, h->C, h->lb_off.as<uint64_t>(),
                            &ctr->tiles[0], h->lb_spin_cap, &ctr->status, &ctr->need_nf, s, h->lb_hold_tile);
     if (sized) {
+        L += launch_longest_path(h->path_start.as<uint32_t>(), h->offsets.as<uint32_t>(), h->P, &ctr->longest, s);
         cudaMemcpyAsync(h->h_u32, &ctr->need_nf, 4, cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(h->h_u32 + 1, &ctr->longest, 4, cudaMemcpyDeviceToHost, s);
         ++h->host_syncs;
         if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
         if ((st = cuda_status())) return st;
         const int64_t need = h->h_u32[0];
         if (need > INT32_MAX) return SPR_ERR_CAPACITY_EXCEEDED;
+        h->longest = h->h_u32[1];
         h->cap_nf = dc ? std::max<int64_t>(need, 1) : with_headroom(need);
         h->cap_items = 2 * h->cap_nf;
     }
@@ -933,18 +946,15 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
                          h->skey[0].as<uint64_t>(), h->sval[0].as<uint32_t>(), s);
     rec(h, 3, s);
     // stage 8: stable sort by (path, cell key).  The entries arrive grouped by
-    // path, so with enough paths to fill the GPU each path's segment is
-    // sorted on its own by one block; frames of few (hence long) paths take
-    // the device-wide LSD radix sort, whose work does not depend on them.
+    // path, so each path's segment is sorted on its own; a frame with a very
+    // long path takes the device-wide LSD radix sort, whose work does not
+    // depend on the paths.
     int rl = 0;
-    const bool segment_sort = h->tune_sort >= 0 ? h->tune_sort == 1
-                                                : h->P >= kSegmentSortMinPaths &&
-                                                      cap_nf / std::max<int64_t>(h->P, 1) <= kSegmentSortMaxMean;
-    if (segment_sort && h->P > 0) {
-        if ((st = ensure(h->path_start, 4 * ((size_t)h->P + 1)))) return st;
-        L += launch_segment_sort(h->curves.as<CurveDesc>(), h->C, h->P, h->offsets.as<uint32_t>(),
-                                 h->skey[0].as<uint64_t>(), h->sval[0].as<uint32_t>(), h->skey[1].as<uint64_t>(),
-                                 h->sval[1].as<uint32_t>(), h->path_start.as<uint32_t>(), ctr, s);
+    if (per_path_sort(h) && h->P > 0) {
+        if ((st = ensure(h->seg_list, 12 * (size_t)h->P))) return st;
+        L += launch_segment_sort(h->P, cap_nf, h->offsets.as<uint32_t>(), h->skey[0].as<uint64_t>(),
+                                 h->sval[0].as<uint32_t>(), h->skey[1].as<uint64_t>(), h->sval[1].as<uint32_t>(),
+                                 h->path_start.as<uint32_t>(), h->seg_list.as<uint32_t>(), ctr, s);
         h->skey_sorted = h->skey[1].as<uint64_t>();
         h->perm_sorted = h->sval[1].as<uint32_t>();
     } else {

@@ -51,6 +51,8 @@ struct FrameCounters {
     uint32_t n_items;      // n_merged + n_span
     uint32_t tiles[3];     // look-back tile counters: entry offsets, scan-mark, pair offsets
     uint32_t diff_status;  // differentiable frames: bit 0 tape too short, bit 1 chain too short
+    uint32_t n_seg[3], q_seg[3];  // segment sort: listed segments by size class, and those taken
+    uint32_t longest;            // entries of the longest path (sized frames)
     uint32_t pairs_alt;          // resolve pairs in the other built-in tile (FrameArgs::alt_shift)
     unsigned long long span_px;  // the spans' pixels (sum of their widths)
 };
@@ -123,9 +125,9 @@ int scan_exclusive_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *t
 int scan_tiles_inplace(uint32_t *a, int64_t n, cudaStream_t s);
 int64_t radix_tiles(int64_t n);
 // Stable sort of the fragment entries by (path, 24-bit cell key), given that
-// they arrive grouped by path: every path's segment sorted by one block.
-// Reads keys (values are the positions), writes keys_out / vals_out; keys and
-// vals serve as scratch for long segments.  path_start: P + 1 words.
+// they arrive grouped by path: every path's segment sorted by one warp or
+// block.  Reads keys (values are the positions), writes keys_out / vals_out;
+// keys and vals serve as scratch for long segments.
 // Nothing is sorted when the frame's entries were not admitted (ctr->nf 0).
 // Sort key of a fragment: path << 24 | cell key within the path (24 bits),
 // with the fragment's scan winding swn and change sign chg (each -1, 0 or
@@ -138,9 +140,15 @@ __host__ __device__ __forceinline__ uint32_t pack_fw(int swn, int chg) {
 }
 __host__ __device__ __forceinline__ int fw_swn(uint32_t b) { return (int)(b << 30) >> 30; }
 __host__ __device__ __forceinline__ int fw_chg(uint32_t b) { return (int)(b << 28) >> 30; }
-int launch_segment_sort(const CurveDesc *curves, uint32_t C, uint32_t P, const uint32_t *offsets, uint64_t *keys,
-                        uint32_t *vals, uint64_t *keys_out, uint32_t *vals_out, uint32_t *path_start,
-                        const FrameCounters *ctr, cudaStream_t s);
+// list: 3 P words (the segments that blocks sort, by size class).  cap_nf: the entries' capacity.
+int launch_segment_sort(uint32_t P, int64_t cap_nf, const uint32_t *offsets, uint64_t *keys, uint32_t *vals,
+                        uint64_t *keys_out, uint32_t *vals_out, const uint32_t *path_start, uint32_t *list,
+                        FrameCounters *ctr, cudaStream_t s);
+// First curve of every path (P + 1 words; curves ascend by path), and the
+// entries of the longest path.
+int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, cudaStream_t s);
+int launch_longest_path(const uint32_t *path_start, const uint32_t *offsets, uint32_t P, uint32_t *longest,
+                        cudaStream_t s);
 int64_t radix_tmp_words(int64_t n);
 // Stable LSD sort on bits [0, key_bits); returns true when the result is in
 // the *_alt buffers.

@@ -240,37 +240,57 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const K *__rest
 // ---- per-path segment sort ---------------------------------------------------
 // The fragment entries arrive grouped by path (curves are in path order and
 // each curve's entries are contiguous), so the stable sort by (path, cell
-// key) is a stable sort of every path's segment by its 24-bit cell key.  One
-// block per path: segments of up to kSegTile entries are sorted in shared
-// memory (three 8-bit passes, a pass skipped when its digit is constant) and
-// written once; longer ones make the same passes over the segment in global
-// memory, chunk by chunk, ping-ponging through the input keys' own range.
+// key) is a stable sort of every path's segment by its 24-bit cell key.  A
+// path covers few of the cells of the viewport, so its keys are first packed
+// into the bits that its own rows and columns need (a 60 x 60 pixel glyph: 10
+// bits instead of 24), then sorted by that many bits in balanced digits of at
+// most 8.  Segments of up to kWarpSeg entries are sorted by one warp, up to
+// kSegTile0 and kSegTile1 by blocks of 256 and 512 threads and longer ones by
+// a block of 1,024 (up to kSegTile2 in shared memory, beyond that chunk by
+// chunk through global memory, ping-ponging through the input keys' own
+// range).  The warps list the longer segments by size class for the blocks,
+// which take them from the lists.
 // Ranking inside a chunk is the scatter's (per-warp digit counters, lanes in
-// input order), so equal keys keep their input order.  Inside a segment the
-// keys' path bits are the path's own, so only the 24-bit cell keys move.
+// input order), so equal keys keep their input order.  Bound by the latency of
+// the ranking's shared-memory chain.  Sort step, us, against the device-wide
+// radix sort that frames of fewer than 1,024 paths took before: 64 paths of
+// 4,800 entries 127 -> 35, 256 paths of 660 entries 127 -> 41, 8 paths of 175
+// entries 97 -> 15; against three 8-bit passes over unpacked keys and one block
+// size: 20,000 paths of 17 M entries 409 -> 332, 40,000 paths of 50 M entries
+// 1095 -> 927.
 
-constexpr int kSegThreads = 256;
-constexpr int kSegWarps = kSegThreads / 32;
-constexpr int kSegItems = 8;
-constexpr int kSegTile = kSegThreads * kSegItems;
-constexpr int kSegWarpSpan = 32 * kSegItems;
+constexpr int kWarpSeg = 512;
+constexpr int kSmallWarps = 4;
+constexpr int kSegThreads0 = 256, kSegItems0 = 8, kSegTile0 = kSegThreads0 * kSegItems0;
+constexpr int kSegThreads1 = 512, kSegItems1 = 8, kSegTile1 = kSegThreads1 * kSegItems1;
+constexpr int kSegThreads2 = 1024, kSegItems2 = 16, kSegTile2 = kSegThreads2 * kSegItems2;
 
-struct SegSmem {
-    uint32_t key[kSegTile];
-    uint32_t val[kSegTile];
-    uint32_t whist[kSegWarps][256];
-    uint32_t lstart[256];  // first position of each digit in the staged chunk
-    uint32_t dstart[256];  // next output position of each digit in the segment (long segments)
-    uint32_t wsum[kSegWarps + 1];
+// Shared-memory form of a sort key: the packed cell key in bits 0-23, key
+// bits 60-63 in bits 24-27.  Cell keys are (row rank << 12) | column.
+struct CellRange {
+    uint32_t row, col;  // the segment's lowest row rank and column
+    int cb, bits;       // bits of the column, and of the packed key
 };
-
-// Shared-memory form of a sort key within its path: the 24-bit cell key
-// and, in bits 24-27, key bits 60-63 (the digit passes read bits 0-23).
-__device__ __forceinline__ uint32_t sk_pack(uint64_t k) {
+__device__ __forceinline__ uint32_t sk_raw(uint64_t k) {
     return ((uint32_t)k & 0xFFFFFFu) | ((uint32_t)(k >> kFwShift) << 24);
 }
-__device__ __forceinline__ uint64_t sk_unpack(uint64_t hi, uint32_t k) {
-    return hi | (uint64_t)(k & 0xFFFFFFu) | ((uint64_t)(k >> 24) << kFwShift);
+__device__ __forceinline__ CellRange cell_range(uint32_t rmin, uint32_t rmax, uint32_t cmin, uint32_t cmax) {
+    CellRange c{rmin, cmin, 32 - __clz((int)(cmax - cmin)), 0};
+    c.bits = c.cb + 32 - __clz((int)(rmax - rmin));
+    return c;
+}
+__device__ __forceinline__ uint32_t sk_pack(uint32_t raw, const CellRange &c) {
+    return (raw & 0xFF000000u) | ((((raw >> 12) & 0xFFFu) - c.row) << c.cb) | ((raw & 0xFFFu) - c.col);
+}
+__device__ __forceinline__ uint64_t sk_unpack(uint64_t hi, uint32_t k, const CellRange &c) {
+    const uint32_t ck = k & 0xFFFFFFu;
+    return hi | (uint64_t)((((ck >> c.cb) + c.row) << 12) | ((ck & ((1u << c.cb) - 1u)) + c.col)) |
+           ((uint64_t)(k >> 24) << kFwShift);
+}
+// Digit width: the packed bits in as few passes as 8-bit digits need, balanced.
+__device__ __forceinline__ int digit_bits(int bits) {
+    const int passes = (bits + 7) / 8;
+    return passes > 0 ? (bits + passes - 1) / passes : 0;
 }
 
 // First curve of every path (curves ascending by path); start[P] = C.
@@ -282,118 +302,50 @@ __global__ void k_path_starts(const CurveDesc *__restrict__ curves, uint32_t C, 
     for (uint32_t q = lo; q <= hi && q <= P; ++q) start[q] = (uint32_t)c;
 }
 
-// Ranks one chunk (kk[], count cnt, input order = warp-major, then item,
-// then lane) by digit `shift` and stages it in shared memory ordered by
-// digit; sm.lstart gets each digit's first staged position, the return value
-// through `tot` the per-digit counts of thread d (d = threadIdx.x).
-__device__ __forceinline__ void seg_stage_chunk(SegSmem &sm, const uint32_t (&kk)[kSegItems],
-                                                const uint32_t (&vv)[kSegItems], int cnt, int shift, uint32_t *tot) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kSegWarps * 256; i += kSegThreads) (&sm.whist[0][0])[i] = 0;
-    __syncthreads();
-    uint32_t rank[kSegItems];
-#pragma unroll
-    for (int r = 0; r < kSegItems; ++r) {
-        if (warp * kSegWarpSpan + r * 32 >= cnt) break;  // the warp's remaining items are past the end
-        const int li = warp * kSegWarpSpan + r * 32 + lane;
-        const bool valid = li < cnt;
-        const uint32_t d = valid ? ((kk[r] >> shift) & 0xFFu) : (256u + lane);
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const uint32_t before = __popc(peers & ((1u << lane) - 1u));
-        const uint32_t cur = valid ? sm.whist[warp][d] : 0u;
-        __syncwarp();
-        if (valid && before == 0) sm.whist[warp][d] = cur + __popc(peers);
-        __syncwarp();
-        rank[r] = cur + before;
-    }
-    __syncthreads();
-    {
-        // one digit per thread of the first 256: its count and per-warp offsets
-        const int d = threadIdx.x;
-        const bool dig = d < 256;
-        uint32_t t = 0;
-        if (dig) {
-#pragma unroll
-            for (int w = 0; w < kSegWarps; ++w) {
-                const uint32_t c = sm.whist[w][d];
-                sm.whist[w][d] = t;
-                t += c;
-            }
-        }
-        uint32_t inc = t;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        if (lane == 31 && dig) sm.wsum[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {  // the 8 digit warps' totals
-            const uint32_t x = lane < 8 ? sm.wsum[lane] : 0u;
-            uint32_t xi = x;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, xi, o);
-                if (lane >= o) xi += v;
-            }
-            if (lane < 8) sm.wsum[lane] = xi - x;
-        }
-        __syncthreads();
-        if (dig) {
-            const uint32_t ls = sm.wsum[warp] + inc - t;
-            sm.lstart[d] = ls;
-#pragma unroll
-            for (int w = 0; w < kSegWarps; ++w) sm.whist[w][d] += ls;
-        }
-        *tot = t;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < kSegItems; ++r) {
-        if (warp * kSegWarpSpan + r * 32 >= cnt) break;
-        const int li = warp * kSegWarpSpan + r * 32 + lane;
-        if (li < cnt) {
-            const uint32_t d = (kk[r] >> shift) & 0xFFu;
-            const uint32_t lp = sm.whist[warp][d] + rank[r];
-            sm.key[lp] = kk[r];
-            sm.val[lp] = vv[r];
-        }
-    }
-    __syncthreads();
+// Entries of the longest path.
+__global__ void k_longest_path(const uint32_t *__restrict__ start, const uint32_t *__restrict__ offsets, uint32_t P,
+                               uint32_t *__restrict__ longest) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n = p < P ? offsets[start[p + 1]] - offsets[start[p]] : 0u;
+    const uint32_t m = __reduce_max_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) atomicMax(longest, m);
 }
 
-// Segments of up to kWarpSeg entries: one warp each, three 8-bit passes in
-// the warp's own shared memory (no block barriers).  Lane l ranks entry
-// 32c + l of every chunk c; the warp's digit counters make the ranks stable.
-constexpr int kWarpSeg = 512;
-constexpr int kSmallWarps = 4;
-
-__global__ void __launch_bounds__(kSmallWarps * 32) k_segment_sort_small(const uint64_t *__restrict__ keys_in,
-                                                                        const uint32_t *__restrict__ start,
-                                                                        const uint32_t *__restrict__ offsets,
-                                                                        uint32_t P, uint64_t *__restrict__ keys_out,
-                                                                        uint32_t *__restrict__ vals_out,
-                                                                        const FrameCounters *__restrict__ ctr) {
+__global__ void __launch_bounds__(kSmallWarps * 32)
+    k_segment_sort_small(const uint64_t *__restrict__ keys_in, const uint32_t *__restrict__ start,
+                         const uint32_t *__restrict__ offsets, uint32_t P, uint64_t *__restrict__ keys_out,
+                         uint32_t *__restrict__ vals_out, uint32_t *__restrict__ list, int one_class,
+                         FrameCounters *__restrict__ ctr) {
     __shared__ uint32_t skey[kSmallWarps][2][kWarpSeg], sval[kSmallWarps][2][kWarpSeg], shist[kSmallWarps][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t p = blockIdx.x * kSmallWarps + w;
     if (p >= P || ctr->status != 0u || ctr->nf != ctr->need_nf) return;  // (entries not admitted: nothing to sort)
     const uint32_t b = offsets[start[p]], e = offsets[start[p + 1]];
-    if (e <= b || e - b > (uint32_t)kWarpSeg) return;
+    if (e <= b) return;
+    if (e - b > (uint32_t)kWarpSeg) {  // a block's: listed by size class
+        if (lane == 0) {
+            const int cls = one_class ? 2 : e - b <= (uint32_t)kSegTile0 ? 0 : (e - b <= (uint32_t)kSegTile1 ? 1 : 2);
+            list[(size_t)cls * P + atomicAdd(&ctr->n_seg[cls], 1u)] = p;
+        }
+        return;
+    }
     const int n = (int)(e - b);
     const uint64_t hi = (uint64_t)p << 24;
+    uint32_t rmin = 0xFFFu, rmax = 0u, cmin = 0xFFFu, cmax = 0u;
     for (int i = lane; i < n; i += 32) {
-        skey[w][0][i] = sk_pack(keys_in[b + i]);
+        const uint32_t k = sk_raw(keys_in[b + i]), r = (k >> 12) & 0xFFFu, c = k & 0xFFFu;
+        skey[w][0][i] = k;
         sval[w][0][i] = b + (uint32_t)i;
+        rmin = min(rmin, r), rmax = max(rmax, r), cmin = min(cmin, c), cmax = max(cmax, c);
     }
+    const CellRange cr = cell_range(__reduce_min_sync(0xffffffffu, rmin), __reduce_max_sync(0xffffffffu, rmax),
+                                    __reduce_min_sync(0xffffffffu, cmin), __reduce_max_sync(0xffffffffu, cmax));
+    for (int i = lane; i < n; i += 32) skey[w][0][i] = sk_pack(skey[w][0][i], cr);
     __syncwarp();
     int cur = 0;
-    const int nch = (n + 31) >> 5;
-    for (int shift = 0; shift < 24; shift += 8) {
-        const uint32_t d0 = (skey[w][cur][0] >> shift) & 0xFFu;
-        bool diff = false;
-        for (int i = lane; i < n; i += 32) diff |= ((skey[w][cur][i] >> shift) & 0xFFu) != d0;
-        if (!__any_sync(0xffffffffu, diff)) continue;  // one digit throughout
+    const int nch = (n + 31) >> 5, db = digit_bits(cr.bits);
+    const uint32_t dmask = (1u << db) - 1u;
+    for (int shift = 0; shift < cr.bits; shift += db) {
         for (int i = lane; i < 256; i += 32) shist[w][i] = 0u;
         __syncwarp();
         uint32_t rk[kWarpSeg / 32];
@@ -402,7 +354,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_segment_sort_small(const u
             if (c >= nch) break;
             const int i = c * 32 + lane;
             const bool valid = i < n;
-            const uint32_t d = valid ? (skey[w][cur][i] >> shift) & 0xFFu : 256u + lane;
+            const uint32_t d = valid ? (skey[w][cur][i] >> shift) & dmask : 256u + lane;
             const uint32_t peers = __match_any_sync(0xffffffffu, d);
             const uint32_t before = __popc(peers & ((1u << lane) - 1u));
             const uint32_t old = valid ? shist[w][d] : 0u;
@@ -434,7 +386,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_segment_sort_small(const u
             const int i = c * 32 + lane;
             if (i < n) {
                 const uint32_t k = skey[w][cur][i];
-                const uint32_t pos = shist[w][(k >> shift) & 0xFFu] + rk[c];
+                const uint32_t pos = shist[w][(k >> shift) & dmask] + rk[c];
                 skey[w][cur ^ 1][pos] = k;
                 sval[w][cur ^ 1][pos] = sval[w][cur][i];
             }
@@ -443,166 +395,292 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_segment_sort_small(const u
         cur ^= 1;
     }
     for (int i = lane; i < n; i += 32) {
-        keys_out[b + i] = sk_unpack(hi, skey[w][cur][i]);
+        keys_out[b + i] = sk_unpack(hi, skey[w][cur][i], cr);
         vals_out[b + i] = sval[w][cur][i];
     }
 }
 
-__global__ void __launch_bounds__(kSegThreads, 5) k_segment_sort(const uint64_t *__restrict__ keys_in,
-                                                               const uint32_t *__restrict__ start,
-                                                               const uint32_t *__restrict__ offsets,
-                                                               uint64_t *__restrict__ keys_out,
-                                                               uint32_t *__restrict__ vals_out, uint64_t *keys_tmp,
-                                                               uint32_t *vals_tmp, const FrameCounters *__restrict__ ctr) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SegSmem &sm = *reinterpret_cast<SegSmem *>(smem_raw);
+// Staged keys, and their positions in the chunk before the pass.
+template <int T, int ITEMS>
+struct SegSmem {
+    static constexpr int kTile = T * ITEMS;
+    uint32_t key[kTile];
+    uint16_t pos[kTile];
+    uint32_t whist[T / 32][256];
+    uint32_t lstart[256];  // first position of each digit in the staged chunk
+    uint32_t dstart[256];  // next output position of each digit in the segment (long segments)
+    uint32_t wsum[8];
+    uint32_t range[4];  // lowest and highest row rank and column
+    uint32_t seg;       // the segment taken from the list
+};
+
+// Exclusive scan of one value per digit (thread d < 256 holds digit d's).
+template <int T, int ITEMS>
+__device__ __forceinline__ uint32_t digit_scan(SegSmem<T, ITEMS> &sm, uint32_t t) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t p = blockIdx.x;
-    if (ctr->status != 0u || ctr->nf != ctr->need_nf) return;  // entries not admitted: nothing to sort
-    const uint32_t b = offsets[start[p]], e = offsets[start[p + 1]];
-    if (e - b <= (uint32_t)kWarpSeg) return;  // empty, or a warp's (k_segment_sort_small)
-    const uint32_t n = e - b;
-    const uint64_t hi = (uint64_t)p << 24;  // the segment's path bits
-    if (n <= (uint32_t)kSegTile) {
-        uint32_t kk[kSegItems];
-        uint32_t vv[kSegItems];
+    const uint32_t inc = warp_incl_scan(t);
+    if (lane == 31 && warp < 8) sm.wsum[warp] = inc;
+    __syncthreads();
+    uint32_t base = 0;
 #pragma unroll
-        for (int r = 0; r < kSegItems; ++r) {
-            const uint32_t li = (uint32_t)(warp * kSegWarpSpan + r * 32 + lane);
-            kk[r] = li < n ? sk_pack(keys_in[b + li]) : 0u;
-            vv[r] = b + li;
+    for (int w = 0; w < 8; ++w)
+        if (w < warp) base += sm.wsum[w];
+    return base + inc - t;
+}
+
+// Ranks one chunk (keys kk[] and positions ix[], count cnt, ipl items per
+// lane, input order = warp-major, then item, then lane) by the digit of mask
+// dmask at `shift` and stages it in shared memory ordered by digit; sm.lstart
+// gets each digit's first staged position, the return value is the count of
+// digit threadIdx.x.  ix is consumed.
+template <int T, int ITEMS>
+__device__ __forceinline__ uint32_t seg_stage_chunk(SegSmem<T, ITEMS> &sm, const uint32_t (&kk)[ITEMS],
+                                                    uint32_t (&ix)[ITEMS], int cnt, int ipl, int shift,
+                                                    uint32_t dmask) {
+    constexpr int W = T / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nd = (int)dmask + 1;
+    for (int d = lane; d < nd; d += 32) sm.whist[warp][d] = 0u;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        if (r >= ipl || (warp * ipl + r) * 32 >= cnt) break;  // the warp's remaining items are past the end
+        const bool valid = (warp * ipl + r) * 32 + lane < cnt;
+        const uint32_t d = valid ? ((kk[r] >> shift) & dmask) : (256u + lane);
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = __popc(peers & ((1u << lane) - 1u));
+        const uint32_t cur = valid ? sm.whist[warp][d] : 0u;
+        __syncwarp();
+        if (valid && before == 0) sm.whist[warp][d] = cur + __popc(peers);
+        __syncwarp();
+        ix[r] |= (cur + before) << 16;
+    }
+    __syncthreads();
+    // one digit per thread: its count and per-warp offsets
+    const int d = threadIdx.x;
+    uint32_t t = 0;
+    if (d < nd) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            const uint32_t c = sm.whist[w][d];
+            sm.whist[w][d] = t;
+            t += c;
         }
-        bool staged = false;  // the current order is in shared memory
-        for (int shift = 0; shift < 24; shift += 8) {
-            const uint32_t d0 = (__shfl_sync(0xffffffffu, kk[0], 0) >> shift) & 0xFFu;
-            bool diff = false;
+    }
+    const uint32_t ls = digit_scan(sm, t);
+    if (d < nd) sm.lstart[d] = ls;
+    __syncthreads();
 #pragma unroll
-            for (int r = 0; r < kSegItems; ++r) {
-                const uint32_t li = (uint32_t)(warp * kSegWarpSpan + r * 32 + lane);
-                diff |= li < n && ((kk[r] >> shift) & 0xFFu) != d0;
+    for (int r = 0; r < ITEMS; ++r) {
+        if (r >= ipl) break;
+        if ((warp * ipl + r) * 32 + lane < cnt) {
+            const uint32_t dg = (kk[r] >> shift) & dmask;
+            const uint32_t lp = sm.lstart[dg] + sm.whist[warp][dg] + (ix[r] >> 16);
+            sm.key[lp] = kk[r];
+            sm.pos[lp] = (uint16_t)ix[r];
+        }
+    }
+    __syncthreads();
+    return t;
+}
+
+// Lowest and highest row rank and column of the block's keys.
+template <int T, int ITEMS>
+__device__ __forceinline__ CellRange block_range(SegSmem<T, ITEMS> &sm, uint32_t rmin, uint32_t rmax, uint32_t cmin,
+                                                 uint32_t cmax) {
+    if (threadIdx.x < 4) sm.range[threadIdx.x] = (threadIdx.x & 1) ? 0u : 0xFFFu;
+    __syncthreads();
+    rmin = __reduce_min_sync(0xffffffffu, rmin), rmax = __reduce_max_sync(0xffffffffu, rmax);
+    cmin = __reduce_min_sync(0xffffffffu, cmin), cmax = __reduce_max_sync(0xffffffffu, cmax);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&sm.range[0], rmin);
+        atomicMax(&sm.range[1], rmax);
+        atomicMin(&sm.range[2], cmin);
+        atomicMax(&sm.range[3], cmax);
+    }
+    __syncthreads();
+    return cell_range(sm.range[0], sm.range[1], sm.range[2], sm.range[3]);
+}
+
+// Sorts the segment of path p, [b, b + n).
+template <int T, int ITEMS>
+__device__ __forceinline__ void sort_segment(SegSmem<T, ITEMS> &sm, uint32_t p, uint32_t b, uint32_t n,
+                                             const uint64_t *keys_in, uint64_t *__restrict__ keys_out,
+                                             uint32_t *__restrict__ vals_out, uint64_t *keys_tmp, uint32_t *vals_tmp) {
+    constexpr int TILE = T * ITEMS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t hi = (uint64_t)p << 24;  // the segment's path bits
+    uint32_t rmin = 0xFFFu, rmax = 0u, cmin = 0xFFFu, cmax = 0u;
+    uint32_t kk[ITEMS], ix[ITEMS];
+    if (n <= (uint32_t)TILE) {
+        const int ipl = (int)((n + T - 1) / T);
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            if (r >= ipl) break;
+            const uint32_t li = (uint32_t)((warp * ipl + r) * 32 + lane);
+            kk[r] = li < n ? sk_raw(keys_in[b + li]) : 0u;
+            ix[r] = li;
+            if (li < n) {
+                const uint32_t y = (kk[r] >> 12) & 0xFFFu, x = kk[r] & 0xFFFu;
+                rmin = min(rmin, y), rmax = max(rmax, y), cmin = min(cmin, x), cmax = max(cmax, x);
             }
-            // warp 0's first key stands for the block: compare across warps too
-            if (warp == 0 && lane == 0) sm.wsum[kSegWarps] = d0;
-            __syncthreads();
-            const uint32_t dblock = sm.wsum[kSegWarps];
-            diff = diff || (n > 0 && ((kk[0] >> shift) & 0xFFu) != dblock &&
-                            (uint32_t)(warp * kSegWarpSpan + lane) < n);
-            if (!__syncthreads_or(diff)) continue;  // one digit throughout: order unchanged
-            uint32_t tot;
-            seg_stage_chunk(sm, kk, vv, (int)n, shift, &tot);
-            staged = true;
+        }
+        const CellRange cr = block_range(sm, rmin, rmax, cmin, cmax);
 #pragma unroll
-            for (int r = 0; r < kSegItems; ++r) {
-                const uint32_t li = (uint32_t)(warp * kSegWarpSpan + r * 32 + lane);
+        for (int r = 0; r < ITEMS; ++r) kk[r] = sk_pack(kk[r], cr);
+        const int db = digit_bits(cr.bits);
+        for (int shift = 0; shift < cr.bits; shift += db) {
+            seg_stage_chunk(sm, kk, ix, (int)n, ipl, shift, (1u << db) - 1u);
+            if (shift + db >= cr.bits) {  // sorted: written as staged
+                for (uint32_t i = threadIdx.x; i < n; i += T) {
+                    keys_out[b + i] = sk_unpack(hi, sm.key[i], cr);
+                    vals_out[b + i] = b + sm.pos[i];
+                }
+                return;
+            }
+#pragma unroll
+            for (int r = 0; r < ITEMS; ++r) {
+                if (r >= ipl) break;
+                const uint32_t li = (uint32_t)((warp * ipl + r) * 32 + lane);
                 if (li < n) {
                     kk[r] = sm.key[li];
-                    vv[r] = sm.val[li];
+                    ix[r] = sm.pos[li];
                 }
             }
             __syncthreads();
         }
-        if (!staged) {  // already in order
-#pragma unroll
-            for (int r = 0; r < kSegItems; ++r) {
-                const uint32_t li = (uint32_t)(warp * kSegWarpSpan + r * 32 + lane);
-                if (li < n) {
-                    keys_out[b + li] = sk_unpack(hi, kk[r]);
-                    vals_out[b + li] = vv[r];
-                }
-            }
-            return;
-        }
-        for (uint32_t i = threadIdx.x; i < n; i += kSegThreads) {
-            keys_out[b + i] = sk_unpack(hi, sm.key[i]);
-            vals_out[b + i] = sm.val[i];
+        for (uint32_t i = threadIdx.x; i < n; i += T) {  // one cell throughout: already in order
+            keys_out[b + i] = keys_in[b + i];
+            vals_out[b + i] = b + i;
         }
         return;
     }
     // long segment: chunked passes through global memory
+    for (uint32_t i = threadIdx.x; i < n; i += T) {
+        const uint32_t k = sk_raw(keys_in[b + i]), y = (k >> 12) & 0xFFFu, x = k & 0xFFFu;
+        rmin = min(rmin, y), rmax = max(rmax, y), cmin = min(cmin, x), cmax = max(cmax, x);
+    }
+    const CellRange cr = block_range(sm, rmin, rmax, cmin, cmax);
+    const int db = digit_bits(cr.bits);
+    const uint32_t dmask = (1u << db) - 1u;
+    const bool dig = threadIdx.x < 256;
     int cur = 0;  // data in: 0 keys_in (values = positions), 1 *_out, 2 *_tmp
-    for (int shift = 0; shift < 24; shift += 8) {
+    for (int shift = 0; shift < cr.bits; shift += db) {
         const uint64_t *ksrc = cur == 0 ? keys_in : (cur == 1 ? keys_out : keys_tmp);
         const uint32_t *vsrc = cur == 1 ? vals_out : vals_tmp;
         uint64_t *kdst = cur == 1 ? keys_tmp : keys_out;
         uint32_t *vdst = cur == 1 ? vals_tmp : vals_out;
         // digit histogram of the segment
-        const bool dig = threadIdx.x < 256;
-        if (dig) sm.dstart[threadIdx.x] = 0;
+        if (dig) sm.dstart[threadIdx.x] = 0u;
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += kSegThreads)
-            atomicAdd(&sm.dstart[(uint32_t)(ksrc[b + i] >> shift) & 0xFFu], 1u);
+        for (uint32_t i = threadIdx.x; i < n; i += T)
+            atomicAdd(&sm.dstart[(sk_pack(sk_raw(ksrc[b + i]), cr) >> shift) & dmask], 1u);
         __syncthreads();
-        const uint32_t cnt_d = dig ? sm.dstart[threadIdx.x] : 0u;
-        if (__syncthreads_or(cnt_d == n)) continue;  // one digit throughout
-        {
-            uint32_t inc = cnt_d;
+        const uint32_t first = b + digit_scan(sm, dig ? sm.dstart[threadIdx.x] : 0u);
+        if (dig) sm.dstart[threadIdx.x] = first;
+        __syncthreads();
+        for (uint32_t c0 = 0; c0 < n; c0 += TILE) {
+            const int cnt = (int)min((uint32_t)TILE, n - c0);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
+            for (int r = 0; r < ITEMS; ++r) {
+                const int li = (warp * ITEMS + r) * 32 + lane;
+                kk[r] = li < cnt ? sk_pack(sk_raw(ksrc[b + c0 + li]), cr) : 0u;
+                ix[r] = (uint32_t)li;
             }
-            if (lane == 31 && dig) sm.wsum[warp] = inc;
-            __syncthreads();
-            if (warp == 0) {
-                const uint32_t x = lane < 8 ? sm.wsum[lane] : 0u;
-                uint32_t xi = x;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(0xffffffffu, xi, o);
-                    if (lane >= o) xi += v;
-                }
-                if (lane < 8) sm.wsum[lane] = xi - x;
-            }
-            __syncthreads();
-            if (dig) sm.dstart[threadIdx.x] = b + sm.wsum[warp] + inc - cnt_d;
-            __syncthreads();
-        }
-        for (uint32_t c0 = 0; c0 < n; c0 += kSegTile) {
-            const int cnt = (int)min((uint32_t)kSegTile, n - c0);
-            uint32_t kk[kSegItems];
-            uint32_t vv[kSegItems];
-#pragma unroll
-            for (int r = 0; r < kSegItems; ++r) {
-                const int li = warp * kSegWarpSpan + r * 32 + lane;
-                const bool valid = li < cnt;
-                kk[r] = valid ? sk_pack(ksrc[b + c0 + li]) : 0u;
-                vv[r] = valid ? (cur == 0 ? b + c0 + (uint32_t)li : vsrc[b + c0 + li]) : 0u;
-            }
-            uint32_t tot;
-            seg_stage_chunk(sm, kk, vv, cnt, shift, &tot);
-            for (int i = threadIdx.x; i < cnt; i += kSegThreads) {
-                const uint32_t k = sm.key[i];
-                const uint32_t d = (k >> shift) & 0xFFu;
+            const uint32_t tot = seg_stage_chunk(sm, kk, ix, cnt, ITEMS, shift, dmask);
+            for (int i = threadIdx.x; i < cnt; i += T) {
+                const uint32_t k = sm.key[i], src = b + c0 + sm.pos[i];
+                const uint32_t d = (k >> shift) & dmask;
                 const uint32_t pos = sm.dstart[d] + (uint32_t)i - sm.lstart[d];
-                kdst[pos] = sk_unpack(hi, k);
-                vdst[pos] = sm.val[i];
+                kdst[pos] = sk_unpack(hi, k, cr);
+                vdst[pos] = cur == 0 ? src : vsrc[src];
             }
             __syncthreads();
-            if (threadIdx.x < 256) sm.dstart[threadIdx.x] += tot;
+            if (dig) sm.dstart[threadIdx.x] += tot;
             __syncthreads();
         }
         cur = cur == 1 ? 2 : 1;
     }
     if (cur == 1) return;
-    for (uint32_t i = threadIdx.x; i < n; i += kSegThreads) {  // into the output arrays
+    for (uint32_t i = threadIdx.x; i < n; i += T) {  // into the output arrays
         keys_out[b + i] = cur == 0 ? keys_in[b + i] : keys_tmp[b + i];
         vals_out[b + i] = cur == 0 ? b + i : vals_tmp[b + i];
     }
 }
 
+// Blocks of T threads take the listed segments of class CLS until none is left.
+template <int T, int ITEMS, int CLS, int BPS>
+__global__ void __launch_bounds__(T, BPS)
+    k_segment_sort(const uint64_t *keys_in, const uint32_t *__restrict__ start, const uint32_t *__restrict__ offsets,
+                   uint32_t P, uint64_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint64_t *keys_tmp,
+                   uint32_t *vals_tmp, const uint32_t *__restrict__ list, FrameCounters *__restrict__ ctr) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SegSmem<T, ITEMS> &sm = *reinterpret_cast<SegSmem<T, ITEMS> *>(smem_raw);
+    // (entries not admitted: the lists are empty)
+    const uint32_t count = ctr->n_seg[CLS];
+    for (;;) {
+        if (threadIdx.x == 0) sm.seg = atomicAdd(&ctr->q_seg[CLS], 1u);
+        __syncthreads();
+        const uint32_t k = sm.seg;
+        if (k >= count) return;
+        const uint32_t p = list[(size_t)CLS * P + k];
+        const uint32_t b = offsets[start[p]], e = offsets[start[p + 1]];
+        sort_segment(sm, p, b, e - b, keys_in, keys_out, vals_out, keys_tmp, vals_tmp);
+        __syncthreads();
+    }
+}
+
+int sort_sms() {
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 152;
+    }
+    return n;
+}
+
 }  // namespace
 
-int launch_segment_sort(const CurveDesc *curves, uint32_t C, uint32_t P, const uint32_t *offsets, uint64_t *keys,
-                        uint32_t *vals, uint64_t *keys_out, uint32_t *vals_out, uint32_t *path_start,
-                        const FrameCounters *ctr, cudaStream_t s) {
-    if (P == 0) return 0;
+int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, cudaStream_t s) {
     k_path_starts<<<(unsigned)(((int64_t)C + 1 + 255) / 256), 256, 0, s>>>(curves, C, P, path_start);
-    cudaFuncSetAttribute(k_segment_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmem));
-    k_segment_sort_small<<<(P + kSmallWarps - 1) / kSmallWarps, kSmallWarps * 32, 0, s>>>(keys, path_start, offsets, P,
-                                                                                      keys_out, vals_out, ctr);
-    k_segment_sort<<<P, kSegThreads, sizeof(SegSmem), s>>>(keys, path_start, offsets, keys_out, vals_out, keys, vals,
-                                                           ctr);
-    return 3;
+    return 1;
+}
+
+int launch_longest_path(const uint32_t *path_start, const uint32_t *offsets, uint32_t P, uint32_t *longest,
+                        cudaStream_t s) {
+    if (P == 0) return 0;
+    k_longest_path<<<(P + 255) / 256, 256, 0, s>>>(path_start, offsets, P, longest);
+    return 1;
+}
+
+int launch_segment_sort(uint32_t P, int64_t cap_nf, const uint32_t *offsets, uint64_t *keys, uint32_t *vals,
+                        uint64_t *keys_out, uint32_t *vals_out, const uint32_t *path_start, uint32_t *list,
+                        FrameCounters *ctr, cudaStream_t s) {
+    if (P == 0) return 0;
+    int n = 1;
+    // with at least an SM for every path, all segments go to the largest
+    // blocks: one launch, each segment sorted as fast as one block can
+    const int one_class = P <= (uint32_t)sort_sms() ? 1 : 0;
+    k_segment_sort_small<<<(P + kSmallWarps - 1) / kSmallWarps, kSmallWarps * 32, 0, s>>>(
+        keys, path_start, offsets, P, keys_out, vals_out, list, one_class, ctr);
+    // (no more segments of a class than entries for them: small frames need no blocks)
+    auto blocks = [&](auto kern, int threads, size_t smem, int64_t shortest, int per_sm) {
+        const int64_t most = std::min<int64_t>(P, cap_nf / shortest);
+        if (most <= 0) return;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<(unsigned)std::min<int64_t>(most, (int64_t)per_sm * sort_sms()), threads, smem, s>>>(
+            keys, path_start, offsets, P, keys_out, vals_out, keys, vals, list, ctr);
+        ++n;
+    };
+    blocks(k_segment_sort<kSegThreads2, kSegItems2, 2, 1>, kSegThreads2, sizeof(SegSmem<kSegThreads2, kSegItems2>),
+           one_class ? kWarpSeg + 1 : kSegTile1 + 1, 1);
+    if (one_class) return n;
+    blocks(k_segment_sort<kSegThreads1, kSegItems1, 1, 2>, kSegThreads1, sizeof(SegSmem<kSegThreads1, kSegItems1>),
+           kSegTile0 + 1, 2);
+    blocks(k_segment_sort<kSegThreads0, kSegItems0, 0, 5>, kSegThreads0, sizeof(SegSmem<kSegThreads0, kSegItems0>),
+           kWarpSeg + 1, 5);
+    return n;
 }
 
 // ---- single-pass scans of frame sizes ------------------------------------------

@@ -188,13 +188,13 @@ int spr_set_gradients(spr_handle *h, const uint32_t *table, uint32_t n_entries, 
                       uint32_t n_texels);
 /* ---- launch tuning (an extension) --------------------------------------------
  * Launch choices that change speed, never results: the fragment sort (0 =
- * device-wide LSD radix, 1 = one block per path segment), the curve-emission
+ * device-wide LSD radix, 1 = per path segment, a warp or block each), the curve-emission
  * order by estimated cost (0 off, 1 on), the resolve's blocks per SM (1-4)
  * and its tile: bin_width pixel columns by 64 / bin_width cell rows (the
  * band height; 64 x 1, 32 x 2, 16 x 4 or 8 x 8 cells of 2 x 2 pixels, 32
  * cells: one per lane of the warp that resolves the tile).  -1 / 0 select
- * the built-in rule (segment sort for frames of at least 1,024 paths
- * averaging at most 2,048 entries; no emission order; 4
+ * the built-in rule (segment sort unless one path holds so many
+ * entries that its own sort would outlast the device-wide one; no emission order; 4
  * blocks per SM; tiles of 16 x 4 cells when the spans of the handle's last
  * sized frame covered at most 8 pixels per draw item, else 64 x 1: narrow
  * tiles cut long spans into many more resolve pairs).  Differentiable
