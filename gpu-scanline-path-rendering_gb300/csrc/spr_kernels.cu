@@ -1763,8 +1763,11 @@ __device__ __forceinline__ void resolve_persistent(const FrameArgs &a, const uin
                                                    const uint32_t *__restrict__ rec_m,
                                                    const uint32_t *__restrict__ bstart,
                                                    const uint32_t *__restrict__ bend, uint32_t *__restrict__ image,
-                                                   uint32_t *__restrict__ overflow, uint32_t *__restrict__ bin_queue) {
+                                                   uint32_t *__restrict__ overflow, FrameCounters *__restrict__ ctr) {
     constexpr int CAP = MS ? kCellCap : 1;
+    // sizes not admitted or a scan that gave up: the bin offsets run past the
+    // records, and the frame is rendered again or reported
+    if (ctr->status != 0u) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemTables &T = *reinterpret_cast<SmemTables *>(smem_raw);
     {
@@ -1784,7 +1787,7 @@ __device__ __forceinline__ void resolve_persistent(const FrameArgs &a, const uin
     uint32_t *gx = MS ? overflow + slot * (int64_t)(4 * S - CAP) * (S / 8 + 1) * 32 : nullptr;
     for (;;) {
         uint32_t b = 0;
-        if (lane == 0) b = atomicAdd(bin_queue, 1u);
+        if (lane == 0) b = atomicAdd(&ctr->bin_queue, 1u);
         b = __shfl_sync(0xffffffffu, b, 0);
         if ((int64_t)b >= a.n_bins) break;
         resolve_bin<S, MS, SRGB, CAP, GRAD>(a, rec_a, rec_m, bstart, bend, image, gx, T, w, lane, b);
@@ -1799,8 +1802,8 @@ __global__ void __launch_bounds__(kResolveWarps * 32, 4) k_resolve(FrameArgs a, 
                                                                  const uint32_t *__restrict__ bend,
                                                                  uint32_t *__restrict__ image,
                                                                  uint32_t *__restrict__ overflow,
-                                                                 uint32_t *__restrict__ bin_queue) {
-    resolve_persistent<S, MS, SRGB, false>(a, rec_a, rec_m, bstart, bend, image, overflow, bin_queue);
+                                                                 FrameCounters *__restrict__ ctr) {
+    resolve_persistent<S, MS, SRGB, false>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr);
 }
 
 // With gradient paints: registers capped so that two blocks stay resident
@@ -1810,8 +1813,8 @@ __global__ void __launch_bounds__(kResolveWarps * 32, 2)
     k_resolve_grad(FrameArgs a, const uint2 *__restrict__ rec_a, const uint32_t *__restrict__ rec_m,
                    const uint32_t *__restrict__ bstart,
                    const uint32_t *__restrict__ bend, uint32_t *__restrict__ image, uint32_t *__restrict__ overflow,
-                   uint32_t *__restrict__ bin_queue) {
-    resolve_persistent<S, MS, SRGB, true>(a, rec_a, rec_m, bstart, bend, image, overflow, bin_queue);
+                   FrameCounters *__restrict__ ctr) {
+    resolve_persistent<S, MS, SRGB, true>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr);
 }
 
 // The image of a 256-sample frame from its passes' fixed-point sample sums
@@ -1955,7 +1958,7 @@ int64_t resolve_blocks(const FrameArgs &a) {
 
 template <int S, bool MS, bool SRGB, bool GRAD>
 void resolve_variant_g(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
-                     uint32_t *queue, cudaStream_t s) {
+                     FrameCounters *ctr, cudaStream_t s) {
     constexpr int CAP = MS ? kCellCap : 1;
     const size_t smem = sizeof(SmemTables) + (size_t)kResolveWarps * sizeof(CellState<S / 8, CAP>);
     auto kern = GRAD ? k_resolve_grad<S, MS, SRGB> : k_resolve<S, MS, SRGB>;
@@ -1967,18 +1970,18 @@ void resolve_variant_g(const FrameArgs &a, const uint2 *rec_a, const uint32_t *r
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kResolveWarps * 32, smem) != cudaSuccess || fit < 1)
         fit = 1;
     const int64_t blocks = std::min<int64_t>(resolve_blocks(a), (int64_t)sm_count() * fit);
-    kern<<<(unsigned)blocks, kResolveWarps * 32, smem, s>>>(a, rec_a, rec_m, bstart, bend, image, overflow, queue);
+    kern<<<(unsigned)blocks, kResolveWarps * 32, smem, s>>>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr);
 }
 
 // Gradient paints get their own instantiations: the per-pixel paint costs
 // registers that plain frames should not pay for.
 template <int S, bool MS, bool SRGB>
 void resolve_variant(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
-                     uint32_t *queue, cudaStream_t s) {
+                     FrameCounters *ctr, cudaStream_t s) {
     if (a.grad_table != nullptr)
-        resolve_variant_g<S, MS, SRGB, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
+        resolve_variant_g<S, MS, SRGB, true>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr, s);
     else
-        resolve_variant_g<S, MS, SRGB, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
+        resolve_variant_g<S, MS, SRGB, false>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr, s);
 }
 
 }  // namespace
@@ -2099,24 +2102,23 @@ int launch_bin_sort(const uint32_t *bin_off, int64_t nbins, uint32_t *pval, cons
 int launch_resolve(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
                     FrameCounters *counters, cudaStream_t s) {
     if (a.n_bins <= 0) return 0;
-    uint32_t *queue = &counters->bin_queue;
-    cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
+    cudaMemsetAsync(&counters->bin_queue, 0, sizeof(uint32_t), s);
     const bool ms = a.ms_output != 0, srgb = a.srgb != 0;
     if (a.S == 8) {
-        if (ms && srgb) resolve_variant<8, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (ms) resolve_variant<8, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (srgb) resolve_variant<8, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else resolve_variant<8, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
+        if (ms && srgb) resolve_variant<8, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (ms) resolve_variant<8, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (srgb) resolve_variant<8, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else resolve_variant<8, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
     } else if (a.S == 16) {
-        if (ms && srgb) resolve_variant<16, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (ms) resolve_variant<16, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (srgb) resolve_variant<16, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else resolve_variant<16, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
+        if (ms && srgb) resolve_variant<16, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (ms) resolve_variant<16, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (srgb) resolve_variant<16, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else resolve_variant<16, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
     } else {
-        if (ms && srgb) resolve_variant<32, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (ms) resolve_variant<32, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else if (srgb) resolve_variant<32, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
-        else resolve_variant<32, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, queue, s);
+        if (ms && srgb) resolve_variant<32, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (ms) resolve_variant<32, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else if (srgb) resolve_variant<32, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
+        else resolve_variant<32, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
     }
     return 1;
 }

@@ -142,3 +142,30 @@ def test_same_structure_scene_keeps_capacities():
         ref = oracle.run(big, 320, 256, samples=32)
         assert np.array_equal(r.read_image().reshape(-1), ref["IMAGE"])
         assert r.element_number() == ref.counts
+
+
+@pytest.mark.parametrize("samples,ms", [(8, True), (32, False)])
+def test_more_resolve_pairs_than_the_records_hold(samples, ms):
+    # paths of two vertical lines, first 4 pixels apart, then far apart: the
+    # entries stay the same while the spans between them, and so the pairs,
+    # grow past the buffers; the frame is rendered again when it is read
+    n, h = 40, 200
+
+    def scene(gap):
+        x = 3.3 + 2.0 * np.arange(n)
+        pts = np.stack([np.stack([x, np.full(n, 4.5)], -1), np.stack([x, np.full(n, h + 0.5)], -1),
+                        np.stack([x + gap, np.full(n, 4.5)], -1), np.stack([x + gap, np.full(n, h + 0.5)], -1)], 1)
+        pid = np.repeat(np.arange(n), 2)
+        return spr.Scene(pts.reshape(-1, 2), np.repeat(pid, 2), 2 * np.arange(2 * n), np.full(2 * n, spr.CURVE_LINEAR),
+                         pid, np.zeros(2 * n), np.zeros(n), 0x80402010 + 3 * np.arange(n))
+
+    near, wide = scene(4.0), scene(900.0)
+    ref = oracle.run(wide, 1024, h + 10, samples=samples, ms_output=ms)
+    with spr.VGRasterizer(1024, h + 10, samples=samples, ms_output=ms) as r:
+        r.add_vg(near)
+        r.rasterize()
+        few = r.frame_stats()["resolve_pairs"]
+        r.update_vertices(wide.vertex.ctypes.data)
+        r.rasterize()
+        assert np.array_equal(r.read_image().reshape(-1), ref["IMAGE"])
+        assert r.frame_stats()["resolve_pairs"] > 4 * few
