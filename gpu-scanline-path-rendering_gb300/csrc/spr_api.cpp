@@ -155,10 +155,11 @@ struct spr_handle {
     bool scene_on_device = false, scene_has_arcw = false;
     int tape_depth = 128;
     // frame buffers
-    DevBuf tvert, pflags, pvis, counts, offsets, scan_tmp, entries, key, pidw, wn, mask, skey[2], sval[2], sort_tmp,
+    DevBuf tvert, pvis, counts, offsets, scan_tmp, entries, key, pidw, wn, mask, skey[2], sval[2], sort_tmp,
         wn_scan, draw, heads, merged, pval, rec_a, rec_m, bins, image, counters, dump_tmp, overflow;
-    // look-back tile words of the frame's scans: entry offsets, scan-mark, pair offsets
-    DevBuf lb_off, lb_mark, lb_pair;
+    // look-back tile words of the scan-mark pass, and of the pair-offset scan
+    // of a frame that changes its tile (the other zeroed words: ZeroedWords)
+    DevBuf lb_mark, lb_pair;
     uint64_t *skey_sorted = nullptr;
     uint32_t *perm_sorted = nullptr;
     const uint32_t *pv_sorted = nullptr;  // resolve pairs in bin order
@@ -213,10 +214,10 @@ namespace {
 // Every device buffer of a handle.
 std::vector<DevBuf *> handle_bufs(spr_handle *h) {
     return {&h->mask_table, &h->rtables, &h->vertex,   &h->vpid,      &h->curves,  &h->rule,
-                      &h->fill,       &h->affine,  &h->tvert,    &h->pflags,    &h->pvis,    &h->counts,
+                      &h->fill,       &h->affine,  &h->tvert,    &h->pvis,    &h->counts,
                       &h->offsets,    &h->scan_tmp, &h->entries, &h->key,       &h->pidw,    &h->wn,
                       &h->mask,       &h->skey[0], &h->skey[1],  &h->sval[0],   &h->sval[1], &h->sort_tmp,
-                      &h->wn_scan,    &h->draw,    &h->heads,    &h->lb_off,    &h->merged,  &h->pval,
+                      &h->wn_scan,    &h->draw,    &h->heads,    &h->merged,  &h->pval,
                       &h->rec_a,      &h->rec_m,   &h->bins,
                       &h->image,      &h->counters, &h->dump_tmp, &h->overflow, &h->scenes_d, &h->path_scene,
                       &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->tape_rec,
@@ -740,6 +741,21 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
 int64_t bin_stride(int64_t nbins) { return (nbins + 1 + 3) & ~int64_t(3); }
 int64_t bin_words(int64_t nbins) { return 3 * bin_stride(nbins); }
 
+// Offsets (in words) of the frame's zeroed arrays in the counters' buffer,
+// every one on a 16-byte boundary.
+struct ZeroedWords {
+    int64_t flags, lb_off, lb_pair, count, fill, total;
+    ZeroedWords(int64_t P, int64_t C, int64_t nbins) {
+        auto pad = [](int64_t n) { return (n + 3) & ~int64_t(3); };
+        flags = pad((int64_t)(sizeof(FrameCounters) + 3) / 4);
+        lb_off = flags + pad(P);
+        lb_pair = lb_off + pad(2 * lookback_words(C));
+        count = lb_pair + pad(2 * lookback_words(nbins));
+        fill = count + bin_stride(nbins);
+        total = fill + bin_stride(nbins);
+    }
+};
+
 // The batch scene table for bin geometry `shift` (tiles of 1 << shift
 // columns): every scene's tile and band counts and first bin, uploaded when
 // the geometry differs from the table's.
@@ -859,26 +875,28 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
         for (auto &e : h->ev)
             if (!e) cudaEventCreate(&e);
     }
-    FrameCounters *ctr = h->counters.as<FrameCounters>();
     int64_t nbins = a.n_bins;
+    // the frame's zeroed words in one buffer, cleared at once: counters, path
+    // flags, look-back words of the entry-offset and pair-offset scans, pair
+    // counts and fill counters of the bins
+    const ZeroedWords z(h->P, h->C, nbins);
+    if ((st = ensure(h->counters, 4 * (size_t)z.total))) return st;
+    FrameCounters *ctr = h->counters.as<FrameCounters>();
+    uint32_t *const zw = h->counters.as<uint32_t>();
     // stage 3: transform + visibility
-    if ((st = ensure(h->tvert, sizeof(float2) * h->V)) || (st = ensure(h->pflags, 4 * (size_t)h->P)) ||
-        (st = ensure(h->pvis, h->P)) || (st = ensure(h->counts, 4 * (size_t)h->C + 16)) ||
+    if ((st = ensure(h->tvert, sizeof(float2) * h->V)) || (st = ensure(h->pvis, h->P)) || (st = ensure(h->counts, 4 * (size_t)h->C + 16)) ||
         (st = ensure(h->offsets, 4 * ((size_t)h->C + 1) + 16)) ||
-        (st = ensure(h->lb_off, 8 * (size_t)lookback_words(h->C))) || (st = ensure(h->image, 4 * (size_t)npix)) ||
-        (st = ensure(h->bins, 4 * (size_t)bin_words(nbins))) ||
-        (st = ensure(h->lb_pair, 8 * (size_t)lookback_words(nbins))) ||
+        (st = ensure(h->image, 4 * (size_t)npix)) || (st = ensure(h->bins, 4 * (size_t)bin_stride(nbins))) ||
         (st = ensure(h->overflow, 4 * (size_t)std::max<int64_t>(resolve_overflow_words(a), 1))))
         return st;
-    cudaMemsetAsync(h->counters.p, 0, sizeof(FrameCounters), s);
+    cudaMemsetAsync(zw, 0, 4 * (size_t)z.total, s);
     rec(h, 0, s);
-    L += launch_transform(a, h->tvert.as<float2>(), h->pflags.as<uint32_t>(), h->pvis.as<uint8_t>(), s);
+    L += launch_transform(a, h->tvert.as<float2>(), zw + z.flags, s);
     rec(h, 1, s);
-    // stages 4-5: monotone pieces, entry counts, offsets (single-pass scan)
-    L += launch_curve_count(a, h->tvert.as<float2>(), h->pvis.as<uint8_t>(), h->counts.as<uint32_t>(), s);
-    cudaMemsetAsync(h->lb_off.p, 0, 8 * (size_t)lookback_words(h->C), s);
-    L += scan_lookback_u32(h->counts.as<uint32_t>(), h->offsets.as<uint32_t>(), nullptr, h->C, h->lb_off.as<uint64_t>(),
-                           &ctr->tiles[0], h->lb_spin_cap, &ctr->status, &ctr->need_nf, s, h->lb_hold_tile);
+    // stages 4-5: visible paths, monotone pieces, entry counts, offsets (single-pass scan)
+    L += launch_curve_count(a, h->tvert.as<float2>(), zw + z.flags, h->pvis.as<uint8_t>(), h->counts.as<uint32_t>(), s);
+    L += scan_lookback_u32(h->counts.as<uint32_t>(), h->offsets.as<uint32_t>(), nullptr, h->C,
+                           reinterpret_cast<uint64_t *>(zw + z.lb_off), &ctr->tiles[0], h->lb_spin_cap, &ctr->status, &ctr->need_nf, s, h->lb_hold_tile);
     if (sized) {
         L += launch_longest_path(h->path_start.as<uint32_t>(), h->offsets.as<uint32_t>(), h->P, &ctr->longest, s);
         cudaMemcpyAsync(h->h_u32, &ctr->need_nf, 4, cudaMemcpyDeviceToHost, s);
@@ -917,7 +935,6 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
         a.vmask = h->vmask.as<uint32_t>();
         a.item_path = h->item_path.as<uint32_t>();
     }
-    L += launch_admit(&ctr->need_nf, &ctr->nf, (uint32_t)std::min<int64_t>(cap_nf, INT32_MAX), &ctr->status, s);
     rec(h, 2, s);
     // emission order, on request: curves sorted by estimated cost (16-bit
     // keys, two passes).  Off by default: a block groups its own chains, and
@@ -940,10 +957,10 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     // (the sort's second value buffer, not yet in use, holds the crossings of
     // the warps with more than fit in shared memory)
     L += launch_curve_emit(a, h->tvert.as<float2>(), h->pvis.as<uint8_t>(), h->offsets.as<uint32_t>(), order,
-                           h->sval[1].as<float>(), h->entries.as<int2>(), ctr, s);
+                           h->sval[1].as<float>(), h->entries.as<int2>(), cap_nf, ctr, s);
     L += launch_fragment(a, h->tvert.as<float2>(), h->entries.as<int2>(), cap_nf, ctr, h->key.as<int32_t>(),
                          h->pidw.as<uint32_t>(), h->wn.as<int8_t>(), h->mask.as<uint32_t>(),
-                         h->skey[0].as<uint64_t>(), h->sval[0].as<uint32_t>(), s);
+                         h->skey[0].as<uint64_t>(), h->sval[0].as<uint32_t>(), h->lb_mark.as<uint64_t>(), s);
     rec(h, 3, s);
     // stage 8: stable sort by (path, cell key).  The entries arrive grouped by
     // path, so each path's segment is sorted on its own; a frame with a very
@@ -970,10 +987,7 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     rec(h, 4, s);
     // stages 9-12, 14: winding scan, marks, draw list (one look-back pass),
     // with the pairs of each resolve bin counted
-    uint32_t *bin_off = h->bins.as<uint32_t>(), *bin_count = bin_off + bin_stride(nbins),
-             *bin_fill = bin_count + bin_stride(nbins);
-    cudaMemsetAsync(bin_count, 0, 8 * (size_t)bin_stride(nbins), s);
-    cudaMemsetAsync(h->lb_mark.p, 0, 8 * (size_t)scan_mark_status_words(cap_nf), s);
+    uint32_t *bin_off = h->bins.as<uint32_t>(), *bin_count = zw + z.count, *bin_fill = zw + z.fill;
     L += launch_scan_mark(a, cap_nf, h->skey_sorted, h->wn_scan.as<int8_t>(),
                           h->draw.as<int4>(), h->heads.as<uint32_t>(), item_scene, bin_count, ctr,
                           h->lb_mark.as<uint64_t>(),
@@ -986,9 +1000,8 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     rec(h, 6, s);
     // stage 15: draw items binned by resolve tile (a band of cell rows x columns): bin offsets
     // from the counts, then the items placed and sorted per bin; resolve
-    cudaMemsetAsync(h->lb_pair.p, 0, 8 * (size_t)lookback_words(nbins), s);
-    L += scan_lookback_u32(bin_count, bin_off, nullptr, nbins, h->lb_pair.as<uint64_t>(), &ctr->tiles[2],
-                           h->lb_spin_cap, &ctr->status, &ctr->need_pairs, s);
+    L += scan_lookback_u32(bin_count, bin_off, nullptr, nbins, reinterpret_cast<uint64_t *>(zw + z.lb_pair),
+                           &ctr->tiles[2], h->lb_spin_cap, &ctr->status, &ctr->need_pairs, s);
     if (sized) {
         cudaMemcpyAsync(h->h_counters, h->counters.p, sizeof(FrameCounters), cudaMemcpyDeviceToHost, s);
         ++h->host_syncs;
@@ -1031,9 +1044,7 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     if (!dc && ((st = ensure(h->rec_a, 8 * (size_t)cap_pairs)) ||
                 (st = ensure(h->rec_m, 4 * (size_t)WORDS * cap_pairs))))
         return st;
-    L += launch_admit(&ctr->need_pairs, &ctr->n_pairs, (uint32_t)std::min<int64_t>(cap_pairs, INT32_MAX),
-                      &ctr->status, s);
-    L += launch_bin_scatter(a, h->draw.as<int4>(), item_scene, cap_items, ctr, bin_off, bin_fill,
+    L += launch_bin_scatter(a, h->draw.as<int4>(), item_scene, cap_items, cap_pairs, ctr, bin_off, bin_fill,
                             h->pval.as<uint32_t>(), s);
     L += launch_bin_sort(bin_off, nbins, h->pval.as<uint32_t>(), ctr, a.S, a.bin_shift, h->draw.as<int4>(),
                          h->merged.as<uint32_t>(), dc ? nullptr : h->rec_a.as<uint2>(),

@@ -35,7 +35,7 @@ constexpr uint32_t kLbSpinCap = 1u << 24;
 
 // Frame-level sizes and flags written by the kernels (device memory): a
 // frame's kernels read their sizes here, so no size has to come back to the
-// host.  A size is "admitted" once it is known to fit its buffers; one that
+// host.  A size is "admitted" (by the first kernel that uses it) once it is known to fit its buffers; one that
 // does not fit is admitted as 0 (the rest of the frame then does nothing)
 // and sets kStatusOverflow, and the frame is rendered again with larger
 // buffers before anything reads it.
@@ -115,14 +115,8 @@ int64_t lookback_words(int64_t n);
 int scan_lookback_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, int64_t n_cap, uint64_t *tile_status,
                       uint32_t *tile_ctr, uint32_t spin_cap, uint32_t *frame_status, uint32_t *total_out,
                       cudaStream_t s, int64_t hold_tile = -1);
-// Admits a size: *admitted = *need if *need <= cap, else 0 and
-// kStatusOverflow in *status; 0 as well after a timeout (the size may be
-// wrong then).
-int launch_admit(const uint32_t *need, uint32_t *admitted, uint32_t cap, uint32_t *status, cudaStream_t s);
 // out[0..n) = exclusive prefix sums of in, out[n] = total.
 int scan_exclusive_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tmp, cudaStream_t s);
-// In-place exclusive scan of a short array by one block; a[n] = total.
-int scan_tiles_inplace(uint32_t *a, int64_t n, cudaStream_t s);
 int64_t radix_tiles(int64_t n);
 // Stable sort of the fragment entries by (path, 24-bit cell key), given that
 // they arrive grouped by path: every path's segment sorted by one warp or
@@ -202,22 +196,22 @@ struct FrameArgs {
     int resolve_bps;  // resolve blocks per SM (1..4; 0 = the default 4)
 };
 
-int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, uint8_t *path_visible,
-                      cudaStream_t s);
-int launch_curve_count(const FrameArgs &a, const float2 *tvert, const uint8_t *path_visible, uint32_t *counts,
-                        cudaStream_t s);
+// path_flags: P words, zero before.
+int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, cudaStream_t s);
+int launch_curve_count(const FrameArgs &a, const float2 *tvert, const uint32_t *path_flags, uint8_t *path_visible,
+                       uint32_t *counts, cudaStream_t s);
 // Sort keys of the emission order (curves by decreasing estimated cost).
 int launch_emit_keys(const FrameArgs &a, const uint32_t *counts, uint32_t *key, uint32_t *val, cudaStream_t s);
 // order: curve processed by thread i (null = identity); outputs do not depend on it.
 // The kernels below read the frame's sizes from the counters (ctr); their
 // grids are sized for the buffers' capacities (cap_*).
 int launch_curve_emit(const FrameArgs &a, const float2 *tvert, const uint8_t *path_visible,
-                      const uint32_t *offsets, const uint32_t *order, float *scratch, int2 *entries,
-                      const FrameCounters *ctr, cudaStream_t s);
+                      const uint32_t *offsets, const uint32_t *order, float *scratch, int2 *entries, int64_t cap_nf,
+                      FrameCounters *ctr, cudaStream_t s);
 int launch_fragment(const FrameArgs &a, const float2 *tvert, const int2 *entries, int64_t cap_nf,
                     const FrameCounters *ctr, int32_t *key, uint32_t *pidw, int8_t *wn, uint32_t *mask,
-                    uint64_t *sort_key, uint32_t *sort_val, cudaStream_t s);
-// Look-back words of launch_scan_mark (zero before the launch).
+                    uint64_t *sort_key, uint32_t *sort_val, uint64_t *mark_words, cudaStream_t s);
+// Look-back words of launch_scan_mark (cleared by launch_fragment).
 int64_t scan_mark_status_words(int64_t cap_nf);
 // Winding scan, merged-fragment / span marks, draw list and merged heads in
 // one pass (decoupled look-back); writes the item counts to the counters
@@ -236,7 +230,7 @@ int launch_stencil(const FrameArgs &a, int64_t cap_nf, FrameCounters *ctr, const
 // pval[bin_off[b] .. bin_off[b + 1]) (bin_off: the exclusive scan of the
 // bin counts; bin_fill: n_bins words, zero before).
 int launch_bin_scatter(const FrameArgs &a, const int4 *draw, const uint32_t *item_scene, int64_t cap_items,
-                       const FrameCounters *ctr, const uint32_t *bin_off, uint32_t *bin_fill, uint32_t *pval,
+                       int64_t cap_pairs, FrameCounters *ctr, const uint32_t *bin_off, uint32_t *bin_fill, uint32_t *pval,
                        cudaStream_t s);
 // Pairs of every bin counted from the draw list into bin_count (zero before).
 int launch_bin_count(const FrameArgs &a, const int4 *draw, const uint32_t *item_scene, int64_t cap_items,
@@ -249,7 +243,7 @@ int launch_bin_sort(const uint32_t *bin_off, int64_t nbins, uint32_t *pval, cons
                     int bin_shift, const int4 *draw, const uint32_t *merged, uint2 *rec_a, uint32_t *rec_m,
                     cudaStream_t s);
 // The resolve is persistent: resolve_warps(a) warps take bins from
-// counters->bin_queue (zeroed by launch_resolve).  overflow:
+// counters->bin_queue (zero before).  overflow:
 // resolve_overflow_words(a) words, the cell entries past the ones each warp
 // keeps in shared memory (multisample modes; unused otherwise).
 int64_t resolve_warps(const FrameArgs &a);

@@ -31,6 +31,7 @@ namespace {
 
 constexpr int kThreads = 256;
 
+inline uint32_t cap32(int64_t cap) { return (uint32_t)std::min<int64_t>(cap, INT32_MAX); }
 inline unsigned grid_for(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
 // Viewport of the scene that path pid belongs to.
@@ -41,6 +42,20 @@ __device__ __forceinline__ Dim dim_of(const FrameArgs &a, uint32_t pid) {
     if (a.path_scene == nullptr) return Dim{a.W, a.H};
     const SceneInfo *sc = a.scenes + __ldg(a.path_scene + pid);
     return Dim{sc->W, sc->H};
+}
+
+// Admission of a size by the first kernel that uses it: *admitted = *need if
+// it fits cap and no scan gave up before, else 0 and kStatusOverflow.  Every
+// block takes the same decision (the timeout bit was set by earlier kernels
+// only) and block 0 records it.
+__device__ __forceinline__ bool admit(const uint32_t *need, uint32_t *admitted, uint32_t cap, uint32_t *status) {
+    const uint32_t n = *need, st = *status & kStatusTimeout;
+    const bool ok = n <= cap && st == 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *admitted = ok ? n : 0u;
+        if (!ok) atomicOr(status, kStatusOverflow);
+    }
+    return ok;
 }
 
 __device__ __forceinline__ void load_geom(const CurveDesc &d, const float2 *__restrict__ tv, CurveGeom &g) {
@@ -126,23 +141,22 @@ __global__ void k_transform(FrameArgs a, float2 *__restrict__ tvert, uint32_t *_
 }
 
 // PATH_VISIBLE (ras_define.h:113-127): not entirely on one side of the viewport.
-__global__ void k_path_visible(int P, const uint32_t *__restrict__ flags, uint8_t *__restrict__ vis) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P) return;
-    const uint32_t f = flags[p];
-    vis[p] = ((f & 0xF8u) && (f & 0x6Bu) && (f & 0x1Fu) && (f & 0xD6u)) ? 1 : 0;
+__device__ __forceinline__ bool path_visible(uint32_t f) {
+    return (f & 0xF8u) && (f & 0x6Bu) && (f & 0x1Fu) && (f & 0xD6u);
 }
 
 // ------------------------------------------------------ intersections --
-__global__ void k_curve_count(FrameArgs a, const float2 *__restrict__ tv, const uint8_t *__restrict__ vis,
-                              uint32_t *__restrict__ counts) {
+// Thread i: path i's visibility, for the later stages, and curve i's entries.
+__global__ void k_curve_count(FrameArgs a, const float2 *__restrict__ tv, const uint32_t *__restrict__ flags,
+                              uint8_t *__restrict__ vis, uint32_t *__restrict__ counts) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < a.P) vis[c] = path_visible(flags[c]) ? 1 : 0;
     if (c >= a.C) return;
     const CurveDesc d = a.curves[c];
     CurveGeom g;
     load_geom(d, tv, g);
     float q[5];
-    const int np = monotonize_r(g, vis[d.pid] != 0, q);
+    const int np = monotonize_r(g, path_visible(flags[d.pid]), q);
     const Dim dm = dim_of(a, d.pid);
     float v0x = g.px[0], v0y = g.py[0];
     uint32_t p = 0;
@@ -319,11 +333,12 @@ __device__ __forceinline__ void merge_piece_warp(const float *X, int nx, const f
 __global__ void __launch_bounds__(kEmitThreads)
     k_curve_emit(FrameArgs a, int per_block, const float2 *__restrict__ tv, const uint8_t *__restrict__ vis,
                  const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ order, float *scratch,
-                 int2 *__restrict__ entries, const FrameCounters *__restrict__ ctr) {
+                 int2 *__restrict__ entries, uint32_t cap_nf, FrameCounters *ctr) {
     __shared__ EmitBlock S;
-    // entries not admitted (the buffers are too small), or the offsets not
-    // to be trusted (a scan gave up waiting): nothing is written
-    if (ctr->status != 0u || ctr->nf != ctr->need_nf) return;
+    // the entries admitted for the rest of the frame; too many for the buffers,
+    // or the offsets not to be trusted (a scan gave up waiting): none, and
+    // nothing is written
+    if (!admit(&ctr->need_nf, &ctr->nf, cap_nf, &ctr->status)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t i = (int64_t)blockIdx.x * per_block + tid;
     int np = 0, type = 0;
@@ -483,10 +498,12 @@ __global__ void __launch_bounds__(kThreads, 8) k_fragment(FrameArgs a, const flo
                                                        const FrameCounters *__restrict__ ctr,
                                                        int32_t *__restrict__ key_out, uint32_t *__restrict__ pid_out,
                                                        int8_t *__restrict__ wn_out, uint32_t *__restrict__ mask_out,
-                                                       uint64_t *__restrict__ sort_key, uint32_t *__restrict__ sort_val) {
+                                                       uint64_t *__restrict__ sort_key, uint32_t *__restrict__ sort_val,
+                                                       uint64_t *__restrict__ mark_words, int64_t n_mark) {
     constexpr int WORDS = S / 8;
     const int64_t nf = ctr->nf;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n_mark) mark_words[i] = 0ull;  // the scan-mark pass's look-back words, cleared on the way
     if (i >= nf) return;
     const int2 e0 = entries[i];
     const int2 e1 = (i + 1) != nf ? entries[i + 1] : make_int2(-1, 0x3f800000);
@@ -1147,12 +1164,13 @@ constexpr int kResolveMaxBlocksPerSM = 4;
 // k_scan_mark took) by warp-aggregated atomic slots, and every bin's range
 // is then sorted (item indices are the draw order).
 __global__ void k_bin_scatter(FrameArgs a, const int4 *__restrict__ draw, const uint32_t *__restrict__ item_scene,
-                              const FrameCounters *__restrict__ ctr, const uint32_t *__restrict__ bin_off,
-                              uint32_t *__restrict__ bin_fill, uint32_t *__restrict__ pval) {
+                              FrameCounters *ctr, const uint32_t *__restrict__ bin_off,
+                              uint32_t *__restrict__ bin_fill, uint32_t *__restrict__ pval, uint32_t cap_pairs) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    // (pairs not admitted: the pair buffer is too small; or a scan gave up)
-    const bool ok = ctr->status == 0u && ctr->n_pairs == ctr->need_pairs;
+    // (not admitted: the pair buffer is too small, or a scan gave up; entries
+    // not admitted: there are no items)
+    const bool ok = admit(&ctr->need_pairs, &ctr->n_pairs, cap_pairs, &ctr->status);
     int nb = 0;
     uint32_t b0 = 0;
     if (ok && i < (int64_t)ctr->n_items) {
@@ -1986,12 +2004,10 @@ void resolve_variant(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec
 
 }  // namespace
 
-int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, uint8_t *path_visible, cudaStream_t s) {
-    cudaMemsetAsync(path_flags, 0, sizeof(uint32_t) * (size_t)a.P, s);
-    int n = 0;
-    if (a.V > 0) k_transform<<<grid_for(a.V), kThreads, 0, s>>>(a, tvert, path_flags), ++n;
-    if (a.P > 0) k_path_visible<<<grid_for(a.P), kThreads, 0, s>>>(a.P, path_flags, path_visible), ++n;
-    return n;
+int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, cudaStream_t s) {
+    if (a.V <= 0) return 0;
+    k_transform<<<grid_for(a.V), kThreads, 0, s>>>(a, tvert, path_flags);
+    return 1;
 }
 
 // Curves a block of k_curve_emit takes: about 5 blocks per SM, so that few
@@ -2005,9 +2021,10 @@ static int emit_curves(int C) {
     return n;
 }
 
-int launch_curve_count(const FrameArgs &a, const float2 *tvert, const uint8_t *vis, uint32_t *counts, cudaStream_t s) {
-    if (a.C <= 0) return 0;
-    k_curve_count<<<grid_for(a.C), kThreads, 0, s>>>(a, tvert, vis, counts);
+int launch_curve_count(const FrameArgs &a, const float2 *tvert, const uint32_t *path_flags, uint8_t *vis,
+                       uint32_t *counts, cudaStream_t s) {
+    if (a.C <= 0 && a.P <= 0) return 0;
+    k_curve_count<<<grid_for(std::max(a.C, a.P)), kThreads, 0, s>>>(a, tvert, path_flags, vis, counts);
     return 1;
 }
 
@@ -2018,26 +2035,29 @@ int launch_emit_keys(const FrameArgs &a, const uint32_t *counts, uint32_t *key, 
 }
 
 int launch_curve_emit(const FrameArgs &a, const float2 *tvert, const uint8_t *vis, const uint32_t *offsets,
-                       const uint32_t *order, float *scratch, int2 *entries, const FrameCounters *ctr,
+                       const uint32_t *order, float *scratch, int2 *entries, int64_t cap_nf, FrameCounters *ctr,
                        cudaStream_t s) {
     if (a.C <= 0) return 0;
     const int per_block = emit_curves(a.C);
     k_curve_emit<<<grid_for(a.C, per_block), kEmitThreads, 0, s>>>(a, per_block, tvert, vis, offsets, order, scratch,
-                                                                   entries, ctr);
+                                                                   entries, cap32(cap_nf), ctr);
     return 1;
 }
 
 int launch_fragment(const FrameArgs &a, const float2 *tvert, const int2 *entries, int64_t cap_nf,
                     const FrameCounters *ctr, int32_t *key, uint32_t *pidw, int8_t *wn, uint32_t *mask,
-                    uint64_t *sort_key, uint32_t *sort_val, cudaStream_t s) {
-    if (cap_nf <= 0) return 0;
-    const unsigned g = grid_for(cap_nf);
+                    uint64_t *sort_key, uint32_t *sort_val, uint64_t *mark_words, cudaStream_t s) {
+    const int64_t n_mark = scan_mark_status_words(cap_nf);
+    const unsigned g = grid_for(std::max(cap_nf, n_mark));
     if (a.S == 8)
-        k_fragment<8><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val);
+        k_fragment<8><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val,
+                                            mark_words, n_mark);
     else if (a.S == 16)
-        k_fragment<16><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val);
+        k_fragment<16><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val,
+                                            mark_words, n_mark);
     else
-        k_fragment<32><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val);
+        k_fragment<32><<<g, kThreads, 0, s>>>(a, tvert, entries, ctr, key, pidw, wn, mask, sort_key, sort_val,
+                                            mark_words, n_mark);
     return 1;
 }
 
@@ -2067,10 +2087,11 @@ int launch_stencil(const FrameArgs &a, int64_t cap_nf, FrameCounters *ctr, const
 }
 
 int launch_bin_scatter(const FrameArgs &a, const int4 *draw, const uint32_t *item_scene, int64_t cap_items,
-                       const FrameCounters *ctr, const uint32_t *bin_off, uint32_t *bin_fill, uint32_t *pval,
+                       int64_t cap_pairs, FrameCounters *ctr, const uint32_t *bin_off, uint32_t *bin_fill, uint32_t *pval,
                        cudaStream_t s) {
     if (cap_items <= 0) return 0;
-    k_bin_scatter<<<grid_for(cap_items), kThreads, 0, s>>>(a, draw, item_scene, ctr, bin_off, bin_fill, pval);
+    k_bin_scatter<<<grid_for(cap_items), kThreads, 0, s>>>(a, draw, item_scene, ctr, bin_off, bin_fill, pval,
+                                                         cap32(cap_pairs));
     return 1;
 }
 
@@ -2102,7 +2123,6 @@ int launch_bin_sort(const uint32_t *bin_off, int64_t nbins, uint32_t *pval, cons
 int launch_resolve(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
                     FrameCounters *counters, cudaStream_t s) {
     if (a.n_bins <= 0) return 0;
-    cudaMemsetAsync(&counters->bin_queue, 0, sizeof(uint32_t), s);
     const bool ms = a.ms_output != 0, srgb = a.srgb != 0;
     if (a.S == 8) {
         if (ms && srgb) resolve_variant<8, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);

@@ -752,17 +752,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lb(const uint32_t *__rest
     }
 }
 
-__global__ void k_admit(const uint32_t *__restrict__ need, uint32_t *__restrict__ admitted, uint32_t cap,
-                        uint32_t *__restrict__ status) {
-    const uint32_t v = *need;
-    if (v <= cap && !(*status & kStatusTimeout)) {  // (after a timeout the size itself may be wrong)
-        *admitted = v;
-    } else {
-        *admitted = 0u;
-        atomicOr(status, kStatusOverflow);
-    }
-}
-
 int64_t scan_tmp_words(int64_t n) { return (n + kScanTile - 1) / kScanTile + 2; }
 
 int64_t lookback_words(int64_t n) { return std::max<int64_t>(1, (n + kScanTile - 1) / kScanTile); }
@@ -772,11 +761,6 @@ int scan_lookback_u32(const uint32_t *in, uint32_t *out, const uint32_t *n_dev, 
                       cudaStream_t s, int64_t hold_tile) {
     k_scan_lb<<<(unsigned)lookback_words(n_cap), kScanThreads, 0, s>>>(in, out, n_dev, n_cap, tile_status, tile_ctr,
                                                                      spin_cap, frame_status, total_out, hold_tile);
-    return 1;
-}
-
-int launch_admit(const uint32_t *need, uint32_t *admitted, uint32_t cap, uint32_t *status, cudaStream_t s) {
-    k_admit<<<1, 1, 0, s>>>(need, admitted, cap, status);
     return 1;
 }
 
@@ -790,11 +774,6 @@ int scan_exclusive_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *t
     k_scan_tiles<<<1, 1024, 0, s>>>(tmp, ntiles);
     k_scan_down<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, out, n, tmp, ntiles);
     return 3;
-}
-
-int scan_tiles_inplace(uint32_t *a, int64_t n, cudaStream_t s) {
-    k_scan_tiles<<<1, 1024, 0, s>>>(a, n);
-    return 1;
 }
 
 int64_t radix_tiles(int64_t n) { return (n + kRadixTile - 1) / kRadixTile; }
