@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "spr_device.cuh"
 #include "spr_internal.h"
@@ -1311,36 +1312,48 @@ __global__ void __launch_bounds__(kBinSortWarps * 32)
     }
 }
 
+// Under sRGB blending the resolve carries linear colour values times 4096: a
+// power of two changes no rounding, and the encode's bin is then the value's
+// integer part.
+constexpr float kLinScale = 4096.f;
+
 // Shared-memory tables of the resolve.  The sRGB decode table is replicated
 // twice (entry k of lane l at k * 2 + l % 2), which measures as fast as more
 // replicas and leaves the room for 4 resolve blocks per SM.
 struct SmemTables {
-    float dec8r[256 * 2];
-    float th[256];
-    uint8_t bin[4096];  // number of thresholds <= b / 4096
+    float dec8r[256 * 2];  // x kLinScale
+    float th[256];         // x kLinScale; th[255] is infinite
+    uint8_t bin[4112];     // number of thresholds <= b / 4096; 255 at b = 4096
 };
 
-__device__ __forceinline__ float lin8(uint32_t k) { return (float)k * (1.f / 255.f); }
-
-// Blend results are finite and never -0 (products and sums of non-negative
-// values), so the hardware min/max give the same clamp as fmin_r/fmax_r.
-__device__ __forceinline__ float clamp01(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
-
-__device__ __forceinline__ uint32_t enc_lin(float v) {
-    const float c = clamp01(v);
-    return (uint32_t)cvt_rzi(c * 255.f + 0.5f);
+template <bool DECODE>
+__device__ __forceinline__ void load_tables(SmemTables &T, const ResolveTables *rt) {
+    if constexpr (DECODE)
+        for (int i = threadIdx.x; i < 256 * 2; i += blockDim.x) T.dec8r[i] = rt->srgb_dec[i >> 1] * kLinScale;
+    for (int i = threadIdx.x; i < 256; i += blockDim.x)
+        T.th[i] = i < 255 ? rt->threshold[i] * kLinScale : __uint_as_float(0x7F800000u);
+    for (int i = threadIdx.x; i < 1028; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(T.bin)[i] =
+            i < 1024 ? reinterpret_cast<const uint32_t *>(rt->bin)[i] : 0xFFFFFFFFu;
 }
 
-// sRGB encode: the number of thresholds t[k] (the linear value at which the
-// 8-bit code steps from k to k+1) that are <= v.  The thresholds are at
-// least 3.0e-4 apart, wider than the 1/4096 bins of `bin`, so a bin holds at
-// most one of them: the count is the bin's base plus one comparison.
+// Float of an 8-bit value (the exponent trick: one add instead of a conversion).
+__device__ __forceinline__ float u8f(uint32_t k) { return ffrom(0x4B000000u | k) - 8388608.f; }
+__device__ __forceinline__ float lin8(uint32_t k) { return u8f(k) * (1.f / 255.f); }
+// Integer part of v in [0, 8191].
+__device__ __forceinline__ uint32_t floor_u13(float v) { return fbits(__fadd_rd(v, 8388608.f)) & 0x1FFFu; }
+
+// 8-bit code of a linear value in [0, 1] (a hair above 1 allowed).
+__device__ __forceinline__ uint32_t enc_lin(float v) { return floor_u13(v * 255.f + 0.5f); }
+
+// sRGB encode of v = value x kLinScale, value in [0, 1] (a hair above 1
+// allowed): the number of thresholds t[k] (the linear value at which the
+// 8-bit code steps from k to k+1) that are <= the value.  The thresholds are
+// at least 3.0e-4 apart, wider than the 1/4096 bins of `bin`, so a bin holds
+// at most one of them: the count is the bin's base plus one comparison.
 __device__ __forceinline__ uint32_t enc_srgb(const SmemTables &t, float v) {
-    const float c = clamp01(v);
-    const int b = min(cvt_rzi(c * 4096.f), 4095);
-    uint32_t k = t.bin[b];
-    if (k < 255u && c >= t.th[k]) ++k;
-    return k;
+    const uint32_t k = t.bin[floor_u13(v)];
+    return k + (v >= t.th[k] ? 1u : 0u);
 }
 
 template <bool SRGB>
@@ -1355,16 +1368,39 @@ __device__ __forceinline__ uint32_t enc8(const SmemTables &t, float v) {
     else return enc_lin(v);
 }
 
+// An item's colour as its blends use it: premultiplied by alpha (linear,
+// x kLinScale under sRGB), alpha squared and 1 - alpha.
+struct Source {
+    float r, g, b, aa, om;
+};
+__device__ __forceinline__ Source make_source(float r, float g, float b, float a) {
+    return Source{r * a, g * a, b * a, a * a, 1.f - a};
+}
 template <bool SRGB>
-__device__ __forceinline__ uint32_t blend_sample(const SmemTables &t, int lane, uint32_t dv, float sr, float sg,
-                                                 float sb, float a, float om) {
+__device__ __forceinline__ Source solid_source(const SmemTables &T, int lane, uint32_t c) {
+    return make_source(dec8<SRGB>(T, c & 0xFF, lane), dec8<SRGB>(T, (c >> 8) & 0xFF, lane),
+                       dec8<SRGB>(T, (c >> 16) & 0xFF, lane), lin8(c >> 24));
+}
+
+// Blend results are finite, never negative and at most a rounding above 1
+// (sums of products of values in [0, 1] with weights a and 1 - a), except of
+// paints whose map is not finite: CLAMP takes those to [0, 1], NaN to 0.
+template <bool SRGB, bool CLAMP>
+__device__ __forceinline__ uint32_t blend_sample(const SmemTables &t, int lane, uint32_t dv, const Source &s) {
     const float dr = dec8<SRGB>(t, dv & 0xFF, lane), dg = dec8<SRGB>(t, (dv >> 8) & 0xFF, lane),
                 db = dec8<SRGB>(t, (dv >> 16) & 0xFF, lane);
     const float da = lin8(dv >> 24);
-    const float orr = sr * a + dr * om;
-    const float og = sg * a + dg * om;
-    const float ob = sb * a + db * om;
-    const float oa = a * a + da * om;
+    float orr = s.r + dr * s.om;
+    float og = s.g + dg * s.om;
+    float ob = s.b + db * s.om;
+    float oa = s.aa + da * s.om;
+    if constexpr (CLAMP) {
+        constexpr float one = SRGB ? kLinScale : 1.f;
+        orr = fminf(fmaxf(orr, 0.f), one);
+        og = fminf(fmaxf(og, 0.f), one);
+        ob = fminf(fmaxf(ob, 0.f), one);
+        oa = fminf(fmaxf(oa, 0.f), 1.f);
+    }
     return enc8<SRGB>(t, orr) | (enc8<SRGB>(t, og) << 8) | (enc8<SRGB>(t, ob) << 16) | (enc_lin(oa) << 24);
 }
 
@@ -1413,36 +1449,62 @@ __device__ __forceinline__ float4 gradient_colour(const FrameArgs &a, const Smem
 }
 
 // ---- resolve state -------------------------------------------------------
-// A bin is one cell row (2 pixel rows) x 64 pixel columns = 32 cells of 2x2
-// pixels; lane l of the warp resolving the bin owns cell l.  Every draw item
-// covers whole cells, and the 4 pixels of a cell see the same items in the
-// same order, so a cell keeps its 4 x S samples (pixel k = px.x * 2 + px.y,
-// the merged masks' layout: bits [k S, (k + 1) S) of the cell's mask words)
-// as a short list of (sample mask, RGBA8 colour) entries whose masks
-// partition the samples.  An item blends each entry it touches once,
-// splitting the entries it covers in part, and entries of equal colour are
-// merged after every item: a cell typically holds 1-4 entries, and an entry
-// often spans several pixels, so one blend serves many samples.  Entries
+// A bin is a tile of 32 cells of 2x2 pixels; lane l of the warp resolving the
+// bin owns cell l.  Every draw item covers whole cells, and the 4 pixels of a
+// cell see the same items in the same order, so a cell keeps its 4 x S samples
+// (pixel k = px.x * 2 + px.y, the merged masks' layout: bits [k S, (k + 1) S)
+// of the cell's mask words) as a short list of (sample mask, RGBA8 colour)
+// entries whose masks partition the samples.  An item blends each entry it
+// touches once, splitting the entries it covers in part, and covered parts of
+// equal colour become one entry: a cell typically holds 1-4 entries, and an
+// entry often spans several pixels, so one blend serves many samples.  Entries
 // 0..kCellCap-1 live in shared memory; a cell that needs more (rare: up to
 // one per sample) keeps the rest in a global area owned by its warp and
-// lane, with the same layout.  Every sample gets exactly the value the
-// per-sample rule gives.
+// lane.  Every sample gets exactly the value the per-sample rule gives.
 constexpr int kCellCap = 8;
 
-// Draw items per window: kWin batches of 32.
-constexpr int kWin = 8;
+// Draw items per window: kWin batches of 32.  (Resolve of the three scenes
+// measured above: 2 batches 1807 / 209 / 5143, 4 batches 1832 / 209 / 5190, 8
+// batches 1895 / 223 / 5433 us; on 64 paths 133, 121 and 127.)
+constexpr int kWin = 4;
 
 template <int MW, int CAP>
 struct CellState {
-    uint32_t ent[CAP][MW + 1][32];  // entry j of lane l's cell: mask words k < MW, colour at k = MW
-    uint32_t mine[kWin][32];        // per batch, the window's items covering lane l's cell
+    using MV = typename MaskVec<MW>::T;
+    // entry j of lane l's cell, in column (l + j) % 32 (which puts the entries
+    // of one cell into different banks)
+    MV mask[CAP][32];
+    uint32_t colour[CAP][32];
+    uint32_t mine[kWin][32];  // per batch, the window's items covering lane l's cell
+    uint32_t owner[32];       // a round's runs: the lane whose cell the run at a start belongs to
 };
 
-// Entry j of lane `lane`'s cell: its first word; word k is at [k * 32].
-template <int MW, int CAP>
-__device__ __forceinline__ uint32_t *entry(CellState<MW, CAP> &w, uint32_t *gx, int j, int lane) {
-    return j < CAP ? &w.ent[j][0][lane] : gx + (size_t)(j - CAP) * (MW + 1) * 32 + lane;
+// Mask and colour of entry j of lane `lane`'s cell.  gx: the warp's global area
+// of the entries past CAP (S the samples per pixel: up to 4 S entries); with
+// LOCAL the entry is known to be among the first CAP.
+template <int S, bool LOCAL, int CAP>
+__device__ __forceinline__ typename MaskVec<S / 8>::T *entry_mask(CellState<S / 8, CAP> &w, uint32_t *gx, int j,
+                                                                 int lane) {
+    using MV = typename MaskVec<S / 8>::T;
+    return LOCAL || j < CAP ? &w.mask[j][(lane + j) & 31] : reinterpret_cast<MV *>(gx) + (j - CAP) * 32 + lane;
 }
+template <int S, bool LOCAL, int CAP>
+__device__ __forceinline__ uint32_t *entry_colour(CellState<S / 8, CAP> &w, uint32_t *gx, int j, int lane) {
+    return LOCAL || j < CAP ? &w.colour[j][(lane + j) & 31]
+                            : gx + ((4 * S - CAP) * (S / 8) + (j - CAP)) * 32 + lane;
+}
+__device__ __forceinline__ void get_mask(const uint32_t *p, uint32_t (&m)[1]) { m[0] = *p; }
+__device__ __forceinline__ void get_mask(const uint2 *p, uint32_t (&m)[2]) {
+    const uint2 v = *p;
+    m[0] = v.x, m[1] = v.y;
+}
+__device__ __forceinline__ void get_mask(const uint4 *p, uint32_t (&m)[4]) {
+    const uint4 v = *p;
+    m[0] = v.x, m[1] = v.y, m[2] = v.z, m[3] = v.w;
+}
+__device__ __forceinline__ void put_mask(uint32_t *p, const uint32_t (&m)[1]) { *p = m[0]; }
+__device__ __forceinline__ void put_mask(uint2 *p, const uint32_t (&m)[2]) { *p = make_uint2(m[0], m[1]); }
+__device__ __forceinline__ void put_mask(uint4 *p, const uint32_t (&m)[4]) { *p = make_uint4(m[0], m[1], m[2], m[3]); }
 
 // Cells [c0, c1) of cell row `ro` of a bin whose rows hold cpr cells (lane
 // ro * cpr + c holds cell c of row ro) as a lane mask.
@@ -1462,81 +1524,145 @@ __device__ __forceinline__ uint32_t pixel_word_bits(int wd, int k) {
     else return 0xFFu << (8 * k);
 }
 
-// Merges entries of equal colour.
-template <int MW, int CAP>
-__device__ __forceinline__ void cell_dedup(CellState<MW, CAP> &w, uint32_t *gx, int lane, int &n) {
-    for (int j = 1; j < n; ++j) {
-        uint32_t *ej = entry(w, gx, j, lane);
-        const uint32_t cj = ej[MW * 32];
-        for (int i = 0; i < j; ++i) {
-            uint32_t *ei = entry(w, gx, i, lane);
-            if (ei[MW * 32] == cj) {
-                --n;
-                uint32_t *en = entry(w, gx, n, lane);
-#pragma unroll
-                for (int k = 0; k < MW; ++k) {
-                    ei[k * 32] |= ej[k * 32];
-                    ej[k * 32] = en[k * 32];
-                }
-                ej[MW * 32] = en[MW * 32];
-                --j;
-                break;
-            }
-        }
-    }
-}
-
-// One item (source colour sr, sg, sb with alpha sa) over the samples of mask
-// m of lane `lane`'s cell, in the multisample modes.
-template <int S, bool SRGB, int CAP>
-__device__ __forceinline__ void cell_apply(CellState<S / 8, CAP> &w, uint32_t *gx, int lane, int &n,
-                                           const uint32_t (&m)[S / 8], const SmemTables &T, float sr, float sg,
-                                           float sb, float sa) {
+// One item per lane (source src over the samples of mask m of the lane's
+// cell; none if !have) in the multisample modes, called by the whole warp.
+// The cells' entries differ in number (2.9 on average, 6 to 7 in the longest
+// cell of a warp), so they are listed over the warp and blended in rounds of
+// 32, one pair (cell, entry) per lane whoever owns the cell.  An entry keeps
+// what the item does not cover and gives the covered samples, blended, to an
+// entry of their colour: the covered parts of one cell that come out equal are
+// found by a match over the round and become one entry.  The cell's entries
+// are written back without gaps.  A cell whose pairs fall into two rounds is
+// not merged this time: covered parts of split entries go past its last one.
+//
+// Bound by issue (73% of the schedulers' slots, 25 of 32 lanes active).  With
+// a lane blending its own cell's entries one after the other and comparing all
+// pairs of them for merges (10 lanes active), the resolve took 3430 us on the
+// 20,000-path 2048 x 2048 scene, 390 us on a 3,300-path 1024 x 1024 page and
+// 8350 us on a batch of 48 scenes; here 1832, 209 and 5190.  Sharing only the
+// entries past the first took 2833, 287 and 6710; lanes as independent state
+// machines 4340, 479 and 8966.
+template <int S, bool SRGB, bool CLAMP, int CAP>
+__device__ __forceinline__ void warp_apply(CellState<S / 8, CAP> &w, uint32_t *gx, int lane, int &n, bool have,
+                                           const uint32_t (&m)[S / 8], const SmemTables &T, const Source &src) {
     constexpr int MW = S / 8;
-    const float om = 1.f - sa;
-    uint32_t full = 0xFFFFFFFFu;
-#pragma unroll
-    for (int k = 0; k < MW; ++k) full &= m[k];
-    if (sa == 1.f && full == 0xFFFFFFFFu) {
-        // opaque over every sample: src * 1 + dst * 0 is the source whatever
-        // dst holds, so one entry stands for all (the per-sample blends and
-        // the merge give the same)
-        uint32_t *e0 = &w.ent[0][0][lane];
-        e0[MW * 32] = blend_sample<SRGB>(T, lane, 0u, sr, sg, sb, sa, om);
-#pragma unroll
-        for (int k = 0; k < MW; ++k) e0[k * 32] = 0xFFFFFFFFu;
-        n = 1;
-        return;
-    }
-    const int n0 = n;
-    bool changed = false;
-    for (int j = 0; j < n0; ++j) {
-        uint32_t *ej = entry(w, gx, j, lane);
-        uint32_t em[MW], in[MW], any = 0u, part = 0u;
-#pragma unroll
-        for (int k = 0; k < MW; ++k) {
-            em[k] = ej[k * 32];
-            in[k] = em[k] & m[k];
-            any |= in[k];
-            part |= em[k] & ~m[k];
-        }
-        if (!any) continue;
-        const uint32_t r = blend_sample<SRGB>(T, lane, ej[MW * 32], sr, sg, sb, sa, om);
-        changed = true;
-        if (!part) {
-            ej[MW * 32] = r;
-        } else {
-            uint32_t *en = entry(w, gx, n, lane);
+    const int cnt = have ? n : 0;
+    if (!__any_sync(0xffffffffu, cnt > 1)) {
+        // every cell has one entry (open background, flat areas): its own lane
+        // blends it, with nothing to merge but a colour that stays the same
+        if (cnt == 1) {
+            uint32_t em[MW], in[MW], rest[MW], any = 0u, part = 0u;
+            get_mask(&w.mask[0][lane], em);
+            const uint32_t old = w.colour[0][lane];
 #pragma unroll
             for (int k = 0; k < MW; ++k) {
-                ej[k * 32] = em[k] & ~m[k];
-                en[k * 32] = in[k];
+                in[k] = em[k] & m[k];
+                rest[k] = em[k] & ~m[k];
+                any |= in[k];
+                part |= rest[k];
             }
-            en[MW * 32] = r;
-            ++n;
+            const uint32_t r = blend_sample<SRGB, CLAMP>(T, lane, old, src);
+            if (any && !part) {
+                w.colour[0][lane] = r;
+            } else if (any && r != old) {
+                put_mask(&w.mask[0][lane], rest);
+                put_mask(entry_mask<S, (CAP > 1)>(w, gx, 1, lane), in);
+                *entry_colour<S, (CAP > 1)>(w, gx, 1, lane) = r;
+                n = 2;
+            }
         }
+        __syncwarp();
+        return;
     }
-    if (changed && n > 1) cell_dedup<MW, CAP>(w, gx, lane, n);
+    const int incl = (int)warp_incl_scan((uint32_t)cnt), first = incl - cnt;
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int base = 0; base < total; base += 32) {
+        // this cell's pairs of the round: lanes [lo, hi)
+        const int lo = min(max(first - base, 0), 32), hi = min(max(incl - base, 0), 32);
+        const bool mine = hi > lo, whole = mine && hi - lo == cnt;
+        if (mine) w.owner[lo] = (uint32_t)lane;
+        const uint32_t starts = __reduce_or_sync(0xffffffffu, mine ? 1u << lo : 0u);
+        __syncwarp();
+        const bool act = base + lane < total;
+        const uint32_t lt = (1u << lane) - 1u;
+        const int run = 31 - __clz((int)(starts & (lt | (1u << lane))));
+        const int L = (int)w.owner[run];
+        // the owner's first pair, entries and whether it is whole
+        const uint32_t info = __shfl_sync(0xffffffffu, (uint32_t)first | ((uint32_t)n << 16) | (whole ? 1u << 31 : 0u), L);
+        uint32_t mL[MW];
+#pragma unroll
+        for (int k = 0; k < MW; ++k) mL[k] = __shfl_sync(0xffffffffu, m[k], L);
+        Source sL;
+        sL.r = __shfl_sync(0xffffffffu, src.r, L);
+        sL.g = __shfl_sync(0xffffffffu, src.g, L);
+        sL.b = __shfl_sync(0xffffffffu, src.b, L);
+        sL.aa = __shfl_sync(0xffffffffu, src.aa, L);
+        sL.om = __shfl_sync(0xffffffffu, src.om, L);
+        const int j = act ? base + lane - (int)(info & 0xFFFFu) : 0;
+        const bool merge = (info >> 31) != 0u;
+        uint32_t em[MW], rest = 0u, any = 0u;
+        uint32_t old;
+        if (!__any_sync(0xffffffffu, j >= CAP)) {
+            get_mask(entry_mask<S, true>(w, gx, j, L), em);
+            old = *entry_colour<S, true>(w, gx, j, L);
+        } else {
+            get_mask(entry_mask<S, false>(w, gx, j, L), em);
+            old = *entry_colour<S, false>(w, gx, j, L);
+        }
+#pragma unroll
+        for (int k = 0; k < MW; ++k) {
+            any |= em[k] & mL[k];
+            rest |= em[k] & ~mL[k];
+        }
+        const bool hit = act && any, keep = act && rest;
+        const uint32_t r = blend_sample<SRGB, CLAMP>(T, lane, old, sL);
+        // lanes of this cell, and among those before this one
+        const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+        const uint32_t later = starts & ~(lt | (1u << lane));
+        const uint32_t seg = (later ? (later & (0u - later)) - 1u : 0xFFFFFFFFu) & ~((1u << run) - 1u);
+        const uint32_t same = __match_any_sync(0xffffffffu, r) & seg & hits;
+        const int lead = merge ? __ffs(same) - 1 : lane;
+        const bool put = hit && lead == lane;
+        const uint32_t keeps = __ballot_sync(0xffffffffu, keep), puts = __ballot_sync(0xffffffffu, put);
+        const uint32_t before = seg & lt;
+        // the rest's and the covered part's places
+        const int at = merge ? __popc(keeps & before) + __popc(puts & before) : j;
+        const int slot = merge ? at + (keep ? 1 : 0)
+                               : (keep ? (int)((info >> 16) & 0x7FFFu) + __popc(keeps & hits & before) : j);
+        const bool move = keep && (hit || merge);
+        uint32_t rm[MW], cm[MW];
+#pragma unroll
+        for (int k = 0; k < MW; ++k) {
+            rm[k] = em[k] & ~mL[k];
+            cm[k] = em[k] & mL[k];
+        }
+        const int to = __shfl_sync(0xffffffffu, slot, lead & 31);
+        __syncwarp();  // (every pair is read: the cells' entries may be overwritten)
+        auto write = [&](auto local) {
+            constexpr bool LOCAL = decltype(local)::value;
+            if (move) {
+                put_mask(entry_mask<S, LOCAL>(w, gx, at, L), rm);
+                *entry_colour<S, LOCAL>(w, gx, at, L) = old;
+            }
+            if (put) {
+                put_mask(entry_mask<S, LOCAL>(w, gx, slot, L), cm);
+                *entry_colour<S, LOCAL>(w, gx, slot, L) = r;
+            }
+            __syncwarp();
+            if (hit && !put) {
+                uint32_t *const d = reinterpret_cast<uint32_t *>(entry_mask<S, LOCAL>(w, gx, to, L));
+#pragma unroll
+                for (int k = 0; k < MW; ++k) atomicOr(d + k, cm[k]);
+            }
+        };
+        if (!__any_sync(0xffffffffu, max(at, slot) >= CAP)) write(std::true_type{});
+        else write(std::false_type{});
+        if (mine) {
+            const uint32_t range = (hi < 32 ? (1u << hi) - 1u : 0xFFFFFFFFu) & ~((1u << lo) - 1u);
+            n = whole ? __popc(keeps & range) + __popc(puts & range) : n + __popc(keeps & hits & range);
+        }
+        __syncwarp();
+    }
 }
 
 // Sample mask m (MW words) of resolve record p.
@@ -1560,25 +1686,102 @@ struct PixelSum {
 };
 template <bool SRGB>
 __device__ __forceinline__ void add_sample(PixelSum &p, const SmemTables &T, int lane, uint32_t v, int weight) {
-    p.r += (long long)weight * (long long)(dec8<SRGB>(T, v & 0xFF, lane) * 68719476736.0f);
-    p.g += (long long)weight * (long long)(dec8<SRGB>(T, (v >> 8) & 0xFF, lane) * 68719476736.0f);
-    p.b += (long long)weight * (long long)(dec8<SRGB>(T, (v >> 16) & 0xFF, lane) * 68719476736.0f);
+    constexpr float unit = SRGB ? 68719476736.0f / kLinScale : 68719476736.0f;
+    p.r += (long long)weight * (long long)(dec8<SRGB>(T, v & 0xFF, lane) * unit);
+    p.g += (long long)weight * (long long)(dec8<SRGB>(T, (v >> 8) & 0xFF, lane) * unit);
+    p.b += (long long)weight * (long long)(dec8<SRGB>(T, (v >> 16) & 0xFF, lane) * unit);
     p.a += (long long)weight * (long long)(lin8(v >> 24) * 68719476736.0f);
 }
 
 template <bool SRGB>
 __device__ __forceinline__ uint32_t encode_mean(const SmemTables &T, const PixelSum &p, double scale) {
-    const float ar = (float)((double)p.r * scale), ag = (float)((double)p.g * scale);
-    const float ab = (float)((double)p.b * scale), aa = (float)((double)p.a * scale);
+    constexpr float k = SRGB ? kLinScale : 1.f;
+    const float ar = (float)((double)p.r * scale) * k, ag = (float)((double)p.g * scale) * k;
+    const float ab = (float)((double)p.b * scale) * k, aa = (float)((double)p.a * scale);
     return enc8<SRGB>(T, ar) | (enc8<SRGB>(T, ag) << 8) | (enc8<SRGB>(T, ab) << 16) | (enc_lin(aa) << 24);
+}
+
+// Applies the window's items to the warp's cells, every lane its own cell's
+// items in order, in the multisample modes.
+template <int S, bool SRGB, int CAP, bool GRAD, class NextItem>
+__device__ __forceinline__ void apply_items(const FrameArgs &a, CellState<S / 8, CAP> &w, uint32_t *gx, int lane,
+                                            int &n_io, const SmemTables &T, const uint2 *__restrict__ rec_a,
+                                            const uint32_t *__restrict__ rec_m, uint32_t base, int X0, int y0,
+                                            NextItem &&next_item) {
+    constexpr int MW = S / 8;
+    int n = n_io;
+    int q = next_item();
+    uint32_t m[MW];
+    uint2 r = make_uint2(0u, 0u);
+    if (q >= 0) {
+        r = __ldg(rec_a + base + q);
+        load_mask<MW>(rec_m, base + q, m);
+    }
+    while (__any_sync(0xffffffffu, q >= 0)) {
+        const int qn = next_item();  // the next item, loaded while the current one is applied
+        uint32_t mn[MW];
+        uint2 rn = make_uint2(0u, 0u);
+        if (qn >= 0) {
+            rn = __ldg(rec_a + base + qn);
+            load_mask<MW>(rec_m, base + qn, mn);
+        }
+        bool have = q >= 0;
+        const bool paint = GRAD && have && r.x - 1u < a.n_grad;
+        Source src{};
+        if (have && !paint) {
+            uint32_t full = 0xFFFFFFFFu;
+#pragma unroll
+            for (int k = 0; k < MW; ++k) full &= m[k];
+            if ((r.x >> 24) == 255u && full == 0xFFFFFFFFu) {
+                // opaque over every sample: src * 1 + dst * 0 is the source
+                // whatever dst holds, and its code is the source's own, so one
+                // entry stands for all (the per-sample blends and the merge
+                // give the same)
+                w.mask[0][lane] = MaskVec<MW>::all();
+                w.colour[0][lane] = r.x;
+                n = 1;
+                have = false;
+            } else {
+                src = solid_source<SRGB>(T, lane, r.x);
+            }
+        }
+        if constexpr (!GRAD) {
+            warp_apply<S, SRGB, false, CAP>(w, gx, lane, n, have, m, T, src);
+        } else {
+            // a paint has a colour per pixel: one application per pixel
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                uint32_t mk[MW], any = 0u;
+#pragma unroll
+                for (int wd = 0; wd < MW; ++wd) {
+                    mk[wd] = paint ? m[wd] & pixel_word_bits<S>(wd, k) : m[wd];
+                    any |= mk[wd];
+                }
+                const bool hk = have && any && (paint || k == 0);
+                if (!__any_sync(0xffffffffu, hk)) continue;
+                if (hk && paint) {
+                    const float4 gc = gradient_colour<SRGB>(a, T, r.x - 1u, (int)(int16_t)(r.y & 0xFFFFu),
+                                                            (int)((r.y >> 16) & 0x1FFFu), X0 + (k >> 1), y0 + (k & 1),
+                                                            lane);
+                    src = make_source(gc.x, gc.y, gc.z, gc.w);
+                }
+                warp_apply<S, SRGB, true, CAP>(w, gx, lane, n, hk, mk, T, src);
+            }
+        }
+        q = qn;
+        r = rn;
+#pragma unroll
+        for (int k = 0; k < MW; ++k) m[k] = mn[k];
+    }
+    n_io = n;
 }
 
 // One warp per bin.  The bin's resolve records (merged fragments and spans
 // in draw-list order: colour, columns, sample mask) are taken kWin x 32 at a
 // time; a 32 x 32 ballot transpose of each batch's cell sets gives every
-// lane the window's items covering its cell, which it applies in order,
-// independently of the other lanes until the window ends (a lane's work is
-// the items over its own cell, not the most any lane has in each batch).
+// lane the window's items covering its cell, which are applied in order, the
+// k-th of every lane together (a warp's steps are the most items over one of
+// its cells in the window, not in each batch).
 // The record of the lane's next item is loaded while it applies the current
 // one.  Then every pixel is averaged over its samples.
 template <int S, bool MS, bool SRGB, int CAP, bool GRAD>
@@ -1620,8 +1823,8 @@ __device__ __forceinline__ void resolve_bin(const FrameArgs &a, const uint2 *__r
     int n = 1;
     uint32_t pc[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
     if constexpr (MS) {
-#pragma unroll
-        for (int k = 0; k <= MW; ++k) w.ent[0][k][lane] = 0xFFFFFFFFu;
+        w.mask[0][lane] = MaskVec<MW>::all();
+        w.colour[0][lane] = 0xFFFFFFFFu;
     }
     const uint32_t beg = bstart[b], fin = bend[b];
     for (uint32_t base = beg; base < fin; base += kWin * 32) {
@@ -1665,67 +1868,51 @@ __device__ __forceinline__ void resolve_bin(const FrameArgs &a, const uint2 *__r
             bits &= bits - 1u;
             return q;
         };
-        int q = next_item();
-        uint32_t m[MW];
-        uint2 r = make_uint2(0u, 0u);
-        if (q >= 0) {
-            r = __ldg(rec_a + base + q);
-            load_mask<MW>(rec_m, base + q, m);
-        }
-        while (q >= 0) {
-            const int qn = next_item();
-            uint32_t mn[MW];
-            uint2 rn = make_uint2(0u, 0u);
-            if (qn >= 0) {
-                rn = __ldg(rec_a + base + qn);
-                load_mask<MW>(rec_m, base + qn, mn);
+        if constexpr (MS) {
+            apply_items<S, SRGB, CAP, GRAD>(a, w, gx, lane, n, T, rec_a, rec_m, base, X0, y0, next_item);
+        } else {
+            // single-sample output: alpha x coverage per pixel, the next
+            // item's record loaded while the current one is applied
+            int q = next_item();
+            uint32_t m[MW];
+            uint2 r = make_uint2(0u, 0u);
+            if (q >= 0) {
+                r = __ldg(rec_a + base + q);
+                load_mask<MW>(rec_m, base + q, m);
             }
-            const uint32_t c = r.x;
-            if (!GRAD || c - 1u >= a.n_grad) {  // a solid colour (else a gradient paint)
-                const float sr = dec8<SRGB>(T, c & 0xFF, lane), sg = dec8<SRGB>(T, (c >> 8) & 0xFF, lane),
-                            sb = dec8<SRGB>(T, (c >> 16) & 0xFF, lane), sa = lin8(c >> 24);
-                if constexpr (MS) {
-                    cell_apply<S, SRGB, CAP>(w, gx, lane, n, m, T, sr, sg, sb, sa);
-                } else {
-                    // single-sample output: alpha x coverage per pixel
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        int cov = 0;
-#pragma unroll
-                        for (int wd = 0; wd < MW; ++wd) cov += __popc(m[wd] & pixel_word_bits<S>(wd, k));
-                        if (cov == 0) continue;
-                        const float ak = sa * ((float)cov / (float)S);
-                        pc[k] = blend_sample<SRGB>(T, lane, pc[k], sr, sg, sb, ak, 1.f - ak);
-                    }
+            while (q >= 0) {
+                const int qn = next_item();
+                uint32_t mn[MW];
+                uint2 rn = make_uint2(0u, 0u);
+                if (qn >= 0) {
+                    rn = __ldg(rec_a + base + qn);
+                    load_mask<MW>(rec_m, base + qn, mn);
                 }
-            } else if constexpr (GRAD) {
-                // a colour per pixel: one application per pixel
-                const uint32_t xw = r.y;
+                const uint32_t c = r.x;
+                const bool paint = GRAD && c - 1u < a.n_grad;
+                float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (!paint)
+                    col = make_float4(dec8<SRGB>(T, c & 0xFF, lane), dec8<SRGB>(T, (c >> 8) & 0xFF, lane),
+                                      dec8<SRGB>(T, (c >> 16) & 0xFF, lane), lin8(c >> 24));
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const int X = X0 + (k >> 1), Y = y0 + (k & 1);
-                    uint32_t mk[MW];
                     int cov = 0;
 #pragma unroll
-                    for (int wd = 0; wd < MW; ++wd) {
-                        mk[wd] = m[wd] & pixel_word_bits<S>(wd, k);
-                        cov += __popc(mk[wd]);
-                    }
+                    for (int wd = 0; wd < MW; ++wd) cov += __popc(m[wd] & pixel_word_bits<S>(wd, k));
                     if (cov == 0) continue;
-                    const float4 gc = gradient_colour<SRGB>(a, T, c - 1u, (int)(int16_t)(xw & 0xFFFFu), (int)((xw >> 16) & 0x1FFFu),
-                                                            X, Y, lane);
-                    if constexpr (MS) {
-                        cell_apply<S, SRGB, CAP>(w, gx, lane, n, mk, T, gc.x, gc.y, gc.z, gc.w);
-                    } else {
-                        const float ak = gc.w * ((float)cov / (float)S);
-                        pc[k] = blend_sample<SRGB>(T, lane, pc[k], gc.x, gc.y, gc.z, ak, 1.f - ak);
+                    if constexpr (GRAD) {
+                        if (paint)
+                            col = gradient_colour<SRGB>(a, T, c - 1u, (int)(int16_t)(r.y & 0xFFFFu),
+                                                        (int)((r.y >> 16) & 0x1FFFu), X0 + (k >> 1), y0 + (k & 1), lane);
                     }
+                    const float ak = col.w * ((float)cov / (float)S);
+                    pc[k] = blend_sample<SRGB, GRAD>(T, lane, pc[k], make_source(col.x, col.y, col.z, ak));
                 }
-            }
-            q = qn;
-            r = rn;
+                q = qn;
+                r = rn;
 #pragma unroll
-            for (int k = 0; k < MW; ++k) m[k] = mn[k];
+                for (int k = 0; k < MW; ++k) m[k] = mn[k];
+            }
         }
     }
     __syncwarp();
@@ -1737,12 +1924,17 @@ __device__ __forceinline__ void resolve_bin(const FrameArgs &a, const uint2 *__r
     for (int k = 0; k < 4; ++k) {
         PixelSum p;
         if constexpr (MS) {
+            if (n == 1 && a.sums == nullptr) {  // one colour: its mean encodes to its own code
+                out[k] = w.colour[0][lane];
+                continue;
+            }
             for (int j = 0; j < n; ++j) {
-                const uint32_t *ej = entry(w, gx, j, lane);
+                uint32_t em[MW];
+                get_mask(entry_mask<S, false>(w, gx, j, lane), em);
                 int cov = 0;
 #pragma unroll
-                for (int wd = 0; wd < MW; ++wd) cov += __popc(ej[wd * 32] & pixel_word_bits<S>(wd, k));
-                if (cov) add_sample<SRGB>(p, T, lane, ej[MW * 32], cov);
+                for (int wd = 0; wd < MW; ++wd) cov += __popc(em[wd] & pixel_word_bits<S>(wd, k));
+                if (cov) add_sample<SRGB>(p, T, lane, *entry_colour<S, false>(w, gx, j, lane), cov);
             }
         } else {
             add_sample<SRGB>(p, T, lane, pc[k], 1);
@@ -1788,15 +1980,7 @@ __device__ __forceinline__ void resolve_persistent(const FrameArgs &a, const uin
     if (ctr->status != 0u) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemTables &T = *reinterpret_cast<SmemTables *>(smem_raw);
-    {
-        const ResolveTables *rt = a.rtables;
-        if constexpr (SRGB)
-            for (int i = threadIdx.x; i < 256 * 2; i += blockDim.x) T.dec8r[i] = rt->srgb_dec[i >> 1];
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) T.th[i] = rt->threshold[i];
-        if constexpr (SRGB)
-            for (int i = threadIdx.x; i < 1024; i += blockDim.x)
-                reinterpret_cast<uint32_t *>(T.bin)[i] = reinterpret_cast<const uint32_t *>(rt->bin)[i];
-    }
+    load_tables<SRGB>(T, a.rtables);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     CellState<S / 8, CAP> &w = reinterpret_cast<CellState<S / 8, CAP> *>(smem_raw + sizeof(SmemTables))[warp];
@@ -1813,8 +1997,10 @@ __device__ __forceinline__ void resolve_persistent(const FrameArgs &a, const uin
     }
 }
 
+// 3 blocks per SM where cells keep entries (76 registers; 4 blocks spill: 2080
+// against 1832 us), 4 where they keep a colour per pixel.
 template <int S, bool MS, bool SRGB>
-__global__ void __launch_bounds__(kResolveWarps * 32, 4) k_resolve(FrameArgs a, const uint2 *__restrict__ rec_a,
+__global__ void __launch_bounds__(kResolveWarps * 32, MS ? 3 : 4) k_resolve(FrameArgs a, const uint2 *__restrict__ rec_a,
                                                                  const uint32_t *__restrict__ rec_m,
                                                                  const uint32_t *__restrict__ bstart,
                                                                  const uint32_t *__restrict__ bend,
@@ -1841,21 +2027,15 @@ template <bool SRGB>
 __global__ void k_encode_sums(FrameArgs a, const long long *__restrict__ sums, uint32_t *__restrict__ image,
                               int64_t npix) {
     __shared__ SmemTables T;
-    {
-        const ResolveTables *rt = a.rtables;
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) T.th[i] = rt->threshold[i];
-        if constexpr (SRGB)
-            for (int i = threadIdx.x; i < 1024; i += blockDim.x)
-                reinterpret_cast<uint32_t *>(T.bin)[i] = reinterpret_cast<const uint32_t *>(rt->bin)[i];
-    }
+    load_tables<false>(T, a.rtables);
     __syncthreads();
     const double scale = 1.0 / (68719476736.0 * 256.0);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += (int64_t)gridDim.x * blockDim.x) {
         const longlong2 q0 = reinterpret_cast<const longlong2 *>(sums)[2 * i];
         const longlong2 q1 = reinterpret_cast<const longlong2 *>(sums)[2 * i + 1];
-        const float ar = (float)((double)q0.x * scale), ag = (float)((double)q0.y * scale);
-        const float ab = (float)((double)q1.x * scale), aa = (float)((double)q1.y * scale);
-        image[i] = enc8<SRGB>(T, ar) | (enc8<SRGB>(T, ag) << 8) | (enc8<SRGB>(T, ab) << 16) | (enc_lin(aa) << 24);
+        PixelSum p;
+        p.r = q0.x, p.g = q0.y, p.b = q1.x, p.a = q1.y;
+        image[i] = encode_mean<SRGB>(T, p, scale);
     }
 }
 
@@ -1865,21 +2045,20 @@ __global__ void k_encode_sums(FrameArgs a, const long long *__restrict__ sums, u
 __global__ void k_selftest_encode(const ResolveTables *__restrict__ rt, uint32_t lo, uint32_t hi,
                                   unsigned long long *__restrict__ bad) {
     __shared__ SmemTables T;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) T.th[i] = rt->threshold[i];
-    for (int i = threadIdx.x; i < 4096; i += blockDim.x) T.bin[i] = rt->bin[i];
+    load_tables<false>(T, rt);
     __syncthreads();
     unsigned long long local = 0;
     for (uint64_t u = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < hi;
          u += (uint64_t)gridDim.x * blockDim.x) {
-        const float v = __uint_as_float((uint32_t)u);
-        const float c = fmin_r(fmax_r(v, 0.f), 1.f);
+        const float v = fmax_r(__uint_as_float((uint32_t)u), 0.f);
+        const float c = fmin_r(v, 1.f);
         int a = 0, b = 255;  // thresholds th[0..254] ascending: count those <= c
         while (a < b) {
             const int m = (a + b) >> 1;
-            if (T.th[m] <= c) a = m + 1;
+            if (rt->threshold[m] <= c) a = m + 1;
             else b = m;
         }
-        if (enc_srgb(T, v) != (uint32_t)a) ++local;
+        if (enc_srgb(T, v * kLinScale) != (uint32_t)a) ++local;
     }
     if (local) atomicAdd(bad, local);
 }
@@ -1959,7 +2138,7 @@ int sm_count() {
 // Shared memory of a resolve block: the tables and one cell state per warp.
 size_t resolve_smem(int S, bool ms) {
     const int MW = S / 8, CAP = ms ? kCellCap : 1;
-    return sizeof(SmemTables) + (size_t)kResolveWarps * ((size_t)CAP * (MW + 1) * 32 * 4 + (size_t)kWin * 32 * 4);
+    return sizeof(SmemTables) + (size_t)kResolveWarps * ((size_t)CAP * (MW + 1) * 32 * 4 + (size_t)(kWin + 1) * 32 * 4);
 }
 
 // Resolve blocks per SM: as many as fit in shared memory (at most 4), or

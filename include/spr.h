@@ -194,8 +194,8 @@ int spr_set_gradients(spr_handle *h, const uint32_t *table, uint32_t n_entries, 
  * band height; 64 x 1, 32 x 2, 16 x 4 or 8 x 8 cells of 2 x 2 pixels, 32
  * cells: one per lane of the warp that resolves the tile).  -1 / 0 select
  * the built-in rule (segment sort unless one path holds so many
- * entries that its own sort would outlast the device-wide one; no emission order; 4
- * blocks per SM; tiles of 16 x 4 cells when the spans of the handle's last
+ * entries that its own sort would outlast the device-wide one; no emission order; as
+ * many blocks per SM as fit; tiles of 16 x 4 cells when the spans of the handle's last
  * sized frame covered at most 8 pixels per draw item, else 64 x 1: narrow
  * tiles cut long spans into many more resolve pairs).  Differentiable
  * frames use 64 x 1 tiles.  spr_autotune times `frames` frames of the
