@@ -688,7 +688,7 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
     }
     int st = ensure(h->grad_tvert, 8 * (size_t)std::max<uint32_t>(h->V, 1));
     if (st) return st;
-    if ((st = ensure(h->chain, 16 * (size_t)std::max<int64_t>(h->nf, 1) + 16))) return st;
+    if ((st = ensure(h->chain, 8 * (size_t)std::max<int64_t>(h->nf, 1)))) return st;
     d.grad_tvert = h->grad_tvert.as<float2>();
     const bool multi = dc.passes > 1;  // the pass's gradients go to staging buffers first
     if (multi) {
@@ -697,8 +697,7 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
             return st;
         d.grad_fill = h->gfill_pass.as<float4>();
     }
-    d.chain = h->chain.as<float4>() + 1;
-    d.n_chain = reinterpret_cast<uint32_t *>(h->chain.p);
+    d.chain = h->chain.as<float2>();
     for (int depth = h->tape_depth;; depth *= 2) {
         const int64_t words = diff_tape_words(a, depth);
         if ((st = ensure(h->tape, 16 * (size_t)words)) ||
@@ -710,7 +709,7 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         cudaMemsetAsync(d.grad_fill, 0, 16 * (size_t)h->P, s);
         cudaMemsetAsync(h->grad_tvert.p, 0, 8 * (size_t)h->V, s);
         cudaMemsetAsync(&ctr->diff_status, 0, 4, s);
-        cudaMemsetAsync(d.n_chain, 0, 4, s);
+        cudaMemsetAsync(d.chain, 0, 8 * (size_t)h->nf, s);
         *L += launch_diff_backward(a, d, s);
         cudaMemcpyAsync(h->h_u32, &ctr->diff_status, 4, cudaMemcpyDeviceToHost, s);
         ++h->host_syncs;

@@ -36,8 +36,7 @@ namespace spr {
 namespace {
 
 constexpr int kDiffThreads = 256;    // 8 warps, each working on its own cells
-constexpr int kDiffPathAcc = 4096;   // paths with shared-memory fill-gradient accumulators (backward)
-constexpr int kDiffCacheSlots = 256; // else: slots of each warp's path-gradient cache
+constexpr int kDiffItemAcc = 128;    // items of a bin whose fill gradients a warp gathers in shared memory (backward)
 constexpr int kTileW = kBinW;  // columns of a resolve bin
 
 __device__ __forceinline__ uint32_t pixel_mask(const uint4 &mm, int S, int k) {
@@ -46,21 +45,17 @@ __device__ __forceinline__ uint32_t pixel_mask(const uint4 &mm, int S, int k) {
     return (mm.x >> (8 * k)) & 0xFFu;
 }
 
-// Bit r of the 2S stacked sample rows of cell column px in a vertical-mask
-// word layout (vertical_mask / vertical_mask2).  The word is picked by
-// selects: px and r vary by lane, and a lane-dependent array index would
-// put the fragment's masks in local memory.
+// Words of a vertical row mask (vertical_mask / vertical_mask2) that hold the 2S
+// stacked sample rows of a cell: the masks repeat them for both pixel columns.
 template <int S>
-__device__ __forceinline__ uint32_t row_bit(const uint32_t *m, int px, int r) {
-    if constexpr (S == 32) {
-        const int i = 2 * px + (r >> 5);
-        const uint32_t w = i < 2 ? (i == 0 ? m[0] : m[1]) : (i == 2 ? m[2] : m[3]);
-        return (w >> (r & 31)) & 1u;
-    } else if constexpr (S == 16) {
-        return ((px ? m[1] : m[0]) >> r) & 1u;
-    } else {
-        return (m[0] >> r) & 1u;
-    }
+constexpr int kRowWords = S == 32 ? 2 : 1;
+
+// Bit r of the rows.  The word is picked by a select: r varies by lane, and a
+// lane-dependent array index would put the masks in local memory.
+template <int S>
+__device__ __forceinline__ uint32_t row_bit(const uint32_t (&m)[kRowWords<S>], int r) {
+    if constexpr (S == 32) return ((r < 32 ? m[0] : m[1]) >> (r & 31)) & 1u;
+    else return (m[0] >> r) & 1u;
 }
 
 // Curve basis at t: P(t) = sum_j B[j] P_j, and P'(t).
@@ -179,42 +174,25 @@ __device__ __forceinline__ float4 warp_sum4(float4 x, int lane) {
 // One fragment of a merged group, held by one lane of the cell's warp.
 template <int S>
 struct GroupFrag {
-    float4 q;          // chord in cell units: x0, y0, slope dx/dy (0 when horizontal), y1
-    uint32_t vm[S / 8];  // rows between the chord's end points
-    uint32_t lm[S / 8];  // left mask
-    int chg;           // winding change (0: no contribution)
+    float4 q;                    // chord in cell units: x0, y0, slope dx/dy (0 when horizontal), y1
+    uint32_t vm[kRowWords<S>];   // rows between the chord's end points
+    uint32_t lm[kRowWords<S>];   // left mask
+    int chg;                     // winding change (0: no contribution)
     uint32_t raw;
 };
 
 template <int S>
-__device__ __forceinline__ void load_group_frag(const DiffArgs &d, int64_t j, GroupFrag<S> &f) {
+__device__ __forceinline__ void load_group_frag(const DiffArgs &d, uint32_t raw, GroupFrag<S> &f) {
     constexpr int WORDS = S / 8;
-    f.raw = d.perm[j];
-    f.chg = (int32_t)d.pidw[f.raw] >> 30;
-    const float4 c = d.chord[f.raw];
+    f.raw = raw;
+    f.chg = (int32_t)d.pidw[raw] >> 30;
+    const float4 c = d.chord[raw];
+#pragma unroll
+    for (int w = 0; w < kRowWords<S>; ++w) {
+        f.vm[w] = d.vmask[(size_t)raw * WORDS + w];
+        f.lm[w] = d.lmask[(size_t)raw * WORDS + w];
+    }
     f.q = make_float4(c.x, c.y, c.w != c.y ? (c.z - c.x) / (c.w - c.y) : 0.f, c.w);
-#pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-        f.vm[w] = d.vmask[(size_t)f.raw * WORDS + w];
-        f.lm[w] = d.lmask[(size_t)f.raw * WORDS + w];
-    }
-}
-
-template <int S>
-__device__ __forceinline__ GroupFrag<S> shfl_frag(const GroupFrag<S> &f, int src) {
-    GroupFrag<S> o;
-    o.q.x = __shfl_sync(0xffffffffu, f.q.x, src);
-    o.q.y = __shfl_sync(0xffffffffu, f.q.y, src);
-    o.q.z = __shfl_sync(0xffffffffu, f.q.z, src);
-    o.q.w = __shfl_sync(0xffffffffu, f.q.w, src);
-#pragma unroll
-    for (int w = 0; w < S / 8; ++w) {
-        o.vm[w] = __shfl_sync(0xffffffffu, f.vm[w], src);
-        o.lm[w] = __shfl_sync(0xffffffffu, f.lm[w], src);
-    }
-    o.chg = __shfl_sync(0xffffffffu, f.chg, src);
-    o.raw = __shfl_sync(0xffffffffu, f.raw, src);
-    return o;
 }
 
 // Chain of one fragment's crossings to its curve's control points: the
@@ -243,18 +221,22 @@ __device__ void fragment_chain(const FrameArgs &a, const DiffArgs &d, uint32_t r
     }
 }
 
-// Edge-sampling adjoint of one merged group (a path's chords in one cell)
-// for the cell's warp.  Lane l holds samples sub + 8k of cell pixel k4 =
-// l >> 3 and J[k] = lambda . (blend(c) - c) of the path at those samples.
-// Groups are loaded 32 fragments at a time, one per lane, and broadcast by
-// shuffles; every shuffle is executed by the whole warp.
+// Edge-sampling adjoint of one merged group (a path's chords in one cell,
+// sorted positions from h) for the cell's warp.  Lane l holds samples sub + 8k
+// of cell pixel k4 = l >> 3 and J[k] = lambda . (blend(c) - c) of the path at
+// those samples.  A chord crosses a sample row in one of the cell's two pixel
+// columns, so lane l works on rows l (and l + 32 at 32 samples) of the cell and
+// takes J at the crossing's pixel from the lane that holds it.  Groups are
+// loaded 32 fragments at a time, one per lane, and broadcast by shuffles; every
+// shuffle is executed by the whole warp.  Every fragment is in one group, so
+// its sums have a place of their own (d.chain).
 template <int S>
-__device__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, int rule, const float *J, int lane) {
-    constexpr int SPT = S / 8;
-    const int k4 = lane >> 3, sub = lane & 7, px = k4 >> 1, py = k4 & 1;
+__device__ __forceinline__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, int rule, const float *J, int lane) {
+    constexpr int SPT = S / 8, ROWS = 2 * S, RPL = (ROWS + 31) / 32;
     const int w0 = (int)d.wn_scan[h];
-    // group size: the run of equal keys from h, 32 keys per step
+    // the first 32 fragments, and the group's size: the run of equal keys from h
     const uint64_t kh = d.skey[h] & kKeyMask;
+    uint32_t raw = h + lane < d.nf ? d.perm[h + lane] : 0u;
     int gs = 0;
     for (;;) {
         const int64_t j = h + gs + lane;
@@ -265,44 +247,65 @@ __device__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, 
         }
         gs += 32;
     }
+    float yr[RPL];
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) yr[i] = ((float)(lane + 32 * i) + 0.5f) / (float)ROWS;
     for (int base = 0; base < gs; base += 32) {
         const int nw = min(32, gs - base);
-        GroupFrag<S> mine;
-        if (lane < nw) load_group_frag<S>(d, h + base + lane, mine);
-        else mine = GroupFrag<S>{};
+        GroupFrag<S> mine{};
+        if (lane < nw) {
+            if (base > 0) raw = d.perm[h + base + lane];
+            load_group_frag<S>(d, raw, mine);
+        }
         for (int j = 0; j < nw; ++j) {
-            const GroupFrag<S> f = shfl_frag<S>(mine, j);
-            if (f.chg == 0 || f.q.y == f.q.w) continue;  // uniform
-            const float slope = f.q.z;
-            bool cand[SPT];
-            float xc[SPT], yr[SPT];
-            int W[SPT];
+            const int chg = __shfl_sync(0xffffffffu, mine.chg, j);
+            const float y0 = __shfl_sync(0xffffffffu, mine.q.y, j), y1 = __shfl_sync(0xffffffffu, mine.q.w, j);
+            if (chg == 0 || y0 == y1) continue;  // uniform
+            const float x0 = __shfl_sync(0xffffffffu, mine.q.x, j), slope = __shfl_sync(0xffffffffu, mine.q.z, j);
+            uint32_t vm[kRowWords<S>];
+#pragma unroll
+            for (int w = 0; w < kRowWords<S>; ++w) vm[w] = __shfl_sync(0xffffffffu, mine.vm[w], j);
+            float xc[RPL], Jr[RPL];
+            int W[RPL];
             bool any = false;
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) {
-                const int r = py * S + sub + 8 * k;
-                yr[k] = ((float)r + 0.5f) / (float)(2 * S);
-                xc[k] = f.q.x + (yr[k] - f.q.y) * slope;
-                const int pc = min(max((int)floorf(xc[k] * 2.f), 0), 1);
-                cand[k] = J[k] != 0.f && row_bit<S>(f.vm, px, r) && pc == px;
-                W[k] = w0;
-                any |= cand[k];
-            }
-            if (!__any_sync(0xffffffffu, any)) continue;
-            // winding just left of each candidate crossing: this window by shuffles ...
-            for (int j2 = 0; j2 < nw; ++j2) {
-                const GroupFrag<S> f2 = shfl_frag<S>(mine, j2);
-                if (f2.chg == 0) continue;  // uniform
+            for (int i = 0; i < RPL; ++i) {
+                const int r = lane + 32 * i, py = r / S, s = r % S;  // row s of pixel row py
+                xc[i] = x0 + (yr[i] - y0) * slope;
+                const int pc = xc[i] * 2.f >= 1.f ? 1 : 0;  // the crossing's pixel column
+                const int src = ((pc * 2 + py) & 3) * 8 + (s & 7);
+                float v = 0.f;
 #pragma unroll
                 for (int k = 0; k < SPT; ++k) {
-                    const int r = py * S + sub + 8 * k;
-                    uint32_t bit = 0u;
-                    if (j2 != j && row_bit<S>(f2.vm, px, r)) {
-                        const float x2 = f2.q.x + (yr[k] - f2.q.y) * f2.q.z;
-                        bit = xc[k] > x2 ? 1u : 0u;
-                    }
-                    bit ^= row_bit<S>(f2.lm, px, r);
-                    W[k] += f2.chg * (int)bit;
+                    const float t = __shfl_sync(0xffffffffu, J[k], src);
+                    v = (s >> 3) == k ? t : v;
+                }
+                Jr[i] = r < ROWS && row_bit<S>(vm, r & (ROWS - 1)) ? v : 0.f;
+                W[i] = w0;
+                any |= Jr[i] != 0.f;
+            }
+            if (!__any_sync(0xffffffffu, any)) continue;
+            // winding just left of each crossing: this window by shuffles ...
+            for (int j2 = 0; j2 < nw; ++j2) {
+                const int chg2 = nw == 1 ? chg : __shfl_sync(0xffffffffu, mine.chg, j2);
+                if (chg2 == 0) continue;  // uniform
+                uint32_t vm2[kRowWords<S>], lm2[kRowWords<S>];
+#pragma unroll
+                for (int w = 0; w < kRowWords<S>; ++w) lm2[w] = __shfl_sync(0xffffffffu, mine.lm[w], j2);
+                float x2 = 0.f, y2 = 0.f, s2 = 0.f;
+                if (j2 != j) {  // uniform
+                    x2 = __shfl_sync(0xffffffffu, mine.q.x, j2);
+                    y2 = __shfl_sync(0xffffffffu, mine.q.y, j2);
+                    s2 = __shfl_sync(0xffffffffu, mine.q.z, j2);
+#pragma unroll
+                    for (int w = 0; w < kRowWords<S>; ++w) vm2[w] = __shfl_sync(0xffffffffu, mine.vm[w], j2);
+                }
+#pragma unroll
+                for (int i = 0; i < RPL; ++i) {
+                    const int r = (lane + 32 * i) & (ROWS - 1);
+                    uint32_t bit = row_bit<S>(lm2, r);
+                    if (j2 != j && row_bit<S>(vm2, r)) bit ^= xc[i] > x2 + (yr[i] - y2) * s2 ? 1u : 0u;
+                    W[i] += chg2 * (int)bit;
                 }
             }
             // ... and the other windows of a group of more than 32 fragments from memory
@@ -310,41 +313,29 @@ __device__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, 
                 for (int j2 = 0; j2 < gs; ++j2) {
                     if (j2 >= base && j2 < base + nw) continue;
                     GroupFrag<S> f2;
-                    load_group_frag<S>(d, h + j2, f2);
+                    load_group_frag<S>(d, d.perm[h + j2], f2);
                     if (f2.chg == 0) continue;
 #pragma unroll
-                    for (int k = 0; k < SPT; ++k) {
-                        const int r = py * S + sub + 8 * k;
-                        uint32_t bit = 0u;
-                        if (row_bit<S>(f2.vm, px, r)) {
-                            const float x2 = f2.q.x + (yr[k] - f2.q.y) * f2.q.z;
-                            bit = xc[k] > x2 ? 1u : 0u;
-                        }
-                        bit ^= row_bit<S>(f2.lm, px, r);
-                        W[k] += f2.chg * (int)bit;
+                    for (int i = 0; i < RPL; ++i) {
+                        const int r = (lane + 32 * i) & (ROWS - 1);
+                        uint32_t bit = row_bit<S>(f2.lm, r);
+                        if (row_bit<S>(f2.vm, r)) bit ^= xc[i] > f2.q.x + (yr[i] - f2.q.y) * f2.q.z ? 1u : 0u;
+                        W[i] += f2.chg * (int)bit;
                     }
                 }
             }
-            float sA = 0.f, sB = 0.f;
+            float sAB[2] = {0.f, 0.f};
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) {
-                if (!cand[k]) continue;
-                const bool cl = filled(W[k], rule), cr = filled(W[k] + f.chg, rule);
-                if (cl == cr) continue;
-                const float g = cl ? J[k] : -J[k];
-                const float lam = (yr[k] - f.q.y) / (f.q.w - f.q.y);
-                sA += g * (1.f - lam);
-                sB += g * lam;
+            for (int i = 0; i < RPL; ++i) {
+                const bool cl = filled(W[i], rule), cr = filled(W[i] + chg, rule);
+                if (Jr[i] == 0.f || cl == cr) continue;
+                const float g = cl ? Jr[i] : -Jr[i];
+                const float lam = (yr[i] - y0) / (y1 - y0);
+                sAB[0] += g * (1.f - lam);
+                sAB[1] += g * lam;
             }
-            float sAB[2] = {sA, sB};
             warp_sums<2>(sAB, lane);
-            sA = sAB[0];
-            sB = sAB[1];
-            if (lane == 0 && (sA != 0.f || sB != 0.f)) {
-                const uint32_t n = atomicAdd(d.n_chain, 1u);
-                if ((int64_t)n < d.nf) d.chain[n] = make_float4(__uint_as_float(f.raw), slope, sA, sB);
-                else atomicOr(d.status, 2u);
-            }
+            if (lane == j) d.chain[mine.raw] = make_float2(sAB[0], sAB[1]);
         }
     }
 }
@@ -365,35 +356,56 @@ __device__ __forceinline__ void global_fill_grad(const DiffArgs &d, uint32_t pat
     atomicAdd(&d.grad_fill[path].w, g.w);
 }
 
-// A fill gradient (lane 0 of the warp): into the block's per-path
-// accumulators (acc) when every path has one; else into the warp's
-// direct-mapped cache (slot = path mod kDiffCacheSlots, tag = path), whose
-// evicted entries go to the global gradient.  Neighbouring cells share most
-// of their paths, so the cache turns most global atomics into register adds.
-__device__ __forceinline__ void add_fill_grad(const DiffArgs &d, float4 *acc, float4 *cache, uint32_t *tag,
-                                              uint32_t path, float4 g) {
-    if (cache != nullptr) {
-        const uint32_t slot = path & (kDiffCacheSlots - 1);
-        const uint32_t t = tag[slot];
-        if (t == path) {
-            float4 &v = cache[slot];
-            v.x += g.x;
-            v.y += g.y;
-            v.z += g.z;
-            v.w += g.w;
-        } else {
-            if (t != 0xFFFFFFFFu) global_fill_grad(d, t, cache[slot]);
-            cache[slot] = g;
-            tag[slot] = path;
-        }
-    } else if (acc != nullptr) {
-        atomicAdd(&acc[path].x, g.x);
-        atomicAdd(&acc[path].y, g.y);
-        atomicAdd(&acc[path].z, g.z);
-        atomicAdd(&acc[path].w, g.w);
+// c -> a * c + b per channel, and maps composed: `first`, then `t`.
+struct Affine {
+    float a;
+    float4 b;
+};
+__device__ __forceinline__ Affine after(const Affine &first, const Affine &t) {
+    return Affine{t.a * first.a, make_float4(t.a * first.b.x + t.b.x, t.a * first.b.y + t.b.y, t.a * first.b.z + t.b.z,
+                                             t.a * first.b.w + t.b.w)};
+}
+// From `o` lanes below (UP), or from lane o.
+template <bool UP>
+__device__ __forceinline__ Affine shfl_affine(const Affine &t, int o) {
+    auto get = [&](float v) { return UP ? __shfl_up_sync(0xffffffffu, v, o) : __shfl_sync(0xffffffffu, v, o); };
+    return Affine{get(t.a), make_float4(get(t.b.x), get(t.b.y), get(t.b.z), get(t.b.w))};
+}
+
+// A fill gradient of item `idx` of the warp's bin (lanes that call it together
+// have different items): into the item's accumulator, or, past those, straight
+// to the global gradient.
+__device__ __forceinline__ void add_fill_grad(const DiffArgs &d, float4 *acc, uint32_t idx, uint32_t path, float4 g) {
+    if (idx < (uint32_t)kDiffItemAcc) {
+        float4 v = acc[idx];
+        v.x += g.x;
+        v.y += g.y;
+        v.z += g.z;
+        v.w += g.w;
+        acc[idx] = v;
     } else {
         global_fill_grad(d, path, g);
     }
+}
+
+// The accumulators of a bin's items [beg, fin) added to their paths' gradients
+// and cleared.
+__device__ __forceinline__ void flush_fill_grads(const DiffArgs &d, float4 *acc, uint32_t beg, uint32_t fin, int lane) {
+    __syncwarp();
+    for (uint32_t i = lane; i < min(fin - beg, (uint32_t)kDiffItemAcc); i += 32) {
+        const float4 v = acc[i];
+        if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
+            global_fill_grad(d, d.bitem[beg + i].w, v);
+            acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __syncwarp();
+}
+
+// Tape slot (at most 65,536) and item of a record in one word; items past the
+// accumulators need no number of their own.
+__device__ __forceinline__ float slot_and_item(int slot, uint32_t item) {
+    return __uint_as_float((uint32_t)slot | (min(item, 0xFFFFu) << 16));
 }
 
 // The scene of resolve bin b: viewport, the bin index within the scene and
@@ -428,7 +440,8 @@ __global__ void k_diff_gather(DiffArgs d, int words) {
     const uint32_t idx = d.pval[p];
     const int4 it = d.draw[idx];
     const uint32_t path = d.item_path[idx];
-    d.bitem[p] = make_uint4((uint32_t)it.x, (uint32_t)it.y, (uint32_t)it.w, path);
+    // (a fragment is one cell wide: its length's place holds its group's first sorted position)
+    d.bitem[p] = make_uint4((uint32_t)it.x, it.w != 0 ? d.heads[it.w - 1] : (uint32_t)it.y, (uint32_t)it.w, path);
     d.bfill[p] = d.fill[path];
     d.bmm[p] = it.w != 0 ? load_merged(d.merged, words, (uint32_t)it.w - 1u) : make_uint4(0u, 0u, 0u, 0u);
 }
@@ -436,55 +449,74 @@ __global__ void k_diff_gather(DiffArgs d, int words) {
 // The crossing sums of every fragment chained to its curve's control points.
 __global__ void k_diff_chain(FrameArgs a, DiffArgs d) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)min((uint64_t)*d.n_chain, (uint64_t)d.nf)) return;
-    const float4 r = d.chain[i];
-    fragment_chain(a, d, __float_as_uint(r.x), r.y, r.z, r.w);
+    if (i >= d.nf) return;
+    const float2 r = d.chain[i];
+    if (r.x == 0.f && r.y == 0.f) return;
+    const float4 c = d.chord[i];
+    fragment_chain(a, d, (uint32_t)i, (c.z - c.x) / (c.w - c.y), r.x, r.y);
 }
 
-// Persistent warps over (bin, cell) units from a queue: warp = one cell of a
-// bin, lane l = pixel k4 = l >> 3 of the cell (k4 = px * 2 + py), samples
+// Persistent warps over units from a queue, 1 << unit_shift consecutive cells of
+// a bin each: warp = one cell of a bin at a time, lane l = pixel k4 = l >> 3 of the cell (k4 = px * 2 + py), samples
 // (l & 7) + 8k.  Every item touching a cell touches all its pixels, so the
 // walk over the bin's items is warp-uniform; the items are read 32 at a time
 // (one per lane), the touching ones found by a ballot and broadcast.  Warps
 // never wait for one another.
-template <int S, bool BWD, bool CACHE>
-__global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs d) {
+template <int S, bool BWD>
+__global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs d, int unit_shift) {
     constexpr int SPT = S / 8;
     constexpr int WORDS = S / 8;
-    extern __shared__ float4 s_acc[];  // fill-gradient accumulators (backward)
+    // fill-gradient accumulators of the warp's bin items: a warp's cells of one
+    // bin share them, so a path costs one set of global atomics a unit
+    __shared__ float4 s_acc[BWD ? kDiffThreads / 32 : 1][BWD ? kDiffItemAcc : 1];
+    // the reverse sweep's next 32 records of each warp (held in registers they
+    // would spill others)
+    __shared__ float4 s_rec[BWD ? kDiffThreads / 32 : 1][BWD ? 3 : 1][BWD ? 32 : 1];
     const int lane = threadIdx.x & 31;
     const int k4 = lane >> 3, sub = lane & 7;
     const int px_in = k4 >> 1, py_in = k4 & 1;
     const size_t wslot = (size_t)blockIdx.x * (kDiffThreads / 32) + (threadIdx.x >> 5);
-    // fill-gradient accumulators: per path for the block (few paths), else
-    // (CACHE) a path cache per warp: values, then tags
-    float4 *acc = (BWD && !CACHE) ? s_acc : nullptr;
-    float4 *cache = (BWD && CACHE) ? s_acc + (threadIdx.x >> 5) * kDiffCacheSlots : nullptr;
-    uint32_t *tag = (BWD && CACHE) ? reinterpret_cast<uint32_t *>(s_acc + (kDiffThreads / 32) * kDiffCacheSlots) +
-                                         (threadIdx.x >> 5) * kDiffCacheSlots
-                                   : nullptr;
-    if (acc)
-        for (int i = threadIdx.x; i < a.P; i += kDiffThreads) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tag)
-        for (int i = lane; i < kDiffCacheSlots; i += 32) tag[i] = 0xFFFFFFFFu;
-    if (BWD) __syncthreads();
-    const int64_t n_units = a.n_bins * (kTileW / 2);
+    float4 *const acc = s_acc[BWD ? threadIdx.x >> 5 : 0];
+    if (BWD) {
+        for (int i = lane; i < kDiffItemAcc; i += 32) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+    }
+    const int64_t n_units = a.n_bins * (kTileW / 2) >> unit_shift;
+    // the unit's bin and the next cell of it
+    BinScene bs{};
+    int tile = 0, crow = 0, cw = 0, end = 0;
+    uint32_t beg = 0, fin = 0;
+    // the bin's items, 32 at a time (lane l holds item base + l); in the forward
+    // a bin of one such chunk keeps it from cell to cell (the backward's reverse
+    // sweep needs the registers)
+    uint4 it = make_uint4(0u, 0u, 0u, 0u), my_mm = it;
+    float4 my_fill = make_float4(0.f, 0.f, 0.f, 0.f);
     for (;;) {
-        uint32_t u = 0;
-        if (lane == 0) u = atomicAdd(d.queue, 1u);
-        u = __shfl_sync(0xffffffffu, u, 0);
-        if ((int64_t)u >= n_units) break;
-        const uint32_t b = u / (kTileW / 2);
-        const int cw = (int)(u % (kTileW / 2));
-        const BinScene bs = bin_scene(a, b);
-        const int ntx = (bs.W + kTileW - 1) / kTileW;
-        const int tile = (int)(bs.lb % ntx), crow = (int)(bs.lb / ntx);
-        const int cellx = tile * kTileW + 2 * cw;
-        if (cellx >= bs.W) continue;
+        bool load = BWD || fin - beg > 32;
+        if (cw == end) {
+            if (BWD) flush_fill_grads(d, acc, beg, fin, lane);
+            uint32_t u = 0;
+            if (lane == 0) u = atomicAdd(d.queue, 1u);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if ((int64_t)u >= n_units) break;
+            const uint32_t b = (u << unit_shift) / (kTileW / 2);
+            bs = bin_scene(a, b);
+            const int ntx = (bs.W + kTileW - 1) / kTileW;
+            tile = (int)(bs.lb % ntx), crow = (int)(bs.lb / ntx);
+            cw = (int)((u << unit_shift) % (kTileW / 2));
+            end = min(cw + (1 << unit_shift), (bs.W - tile * kTileW + 1) / 2);  // (cells within the viewport)
+            beg = fin = 0;
+            if (cw >= end) {
+                cw = end;
+                continue;
+            }
+            beg = d.bstart[b], fin = d.bend[b];
+            load = true;
+        }
+        const int cellx = tile * kTileW + 2 * cw++;
         const int X = cellx + px_in, Y = crow * 2 + py_in;
         const bool valid = X < bs.W && Y < bs.H;
         const int64_t pix = bs.image_off + (int64_t)Y * bs.W + X;
-        const uint32_t beg = d.bstart[b], fin = d.bend[b];
         float4 c[SPT];
 #pragma unroll
         for (int k = 0; k < SPT; ++k) c[k] = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -494,22 +526,11 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
         float ralpha = 1.f;
         float4 rbeta = make_float4(0.f, 0.f, 0.f, 0.f);
         const size_t rbase = wslot * (size_t)d.tape_depth;
-        // the bin's items, 32 at a time (lane l holds item base + l), the next
-        // chunk loaded while the current one is applied
-        uint4 it = make_uint4(0u, 0u, 0u, 0u), my_mm = it;
-        float4 my_fill = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (beg + lane < fin) {
-            it = d.bitem[beg + lane];
-            my_fill = d.bfill[beg + lane];
-            my_mm = d.bmm[beg + lane];
-        }
         for (uint32_t base = beg; base < fin; base += 32) {
-            uint4 nit = make_uint4(0u, 0u, 0u, 0u), nmm = nit;
-            float4 nfill = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (base + 32 + lane < fin) {
-                nit = d.bitem[base + 32 + lane];
-                nfill = d.bfill[base + 32 + lane];
-                nmm = d.bmm[base + 32 + lane];
+            if ((load || base != beg) && base + lane < fin) {
+                it = d.bitem[base + lane];
+                my_fill = d.bfill[base + lane];
+                my_mm = d.bmm[base + lane];
             }
             bool touch = false;
             if (base + lane < fin) {
@@ -517,85 +538,111 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
                 touch = it.z != 0u ? x == cellx : (cellx >= x && cellx < x + (int)it.y);
             }
             uint32_t tm = __ballot_sync(0xffffffffu, touch);
+            const uint32_t frags = __ballot_sync(0xffffffffu, touch && it.z != 0u);
             while (tm) {
                 const int q = __ffs(tm) - 1;
+                const uint32_t later = frags & tm;  // the touching fragments ahead
+                if (!((frags >> q) & 1u)) {
+                    // The spans up to the next fragment.  A span covers every
+                    // sample of the cell, so a run of them is an affine map c =
+                    // ralpha * c_run + rbeta of the samples' state c_run where
+                    // the run starts; the maps are composed over the lanes that
+                    // hold the spans, each lane getting the map before its own.
+                    const uint32_t run = later ? tm & ((later & (0u - later)) - 1u) : tm;
+                    tm &= ~run;
+                    if (run_slot < 0) {
+                        run_slot = nsl++;
+                        ralpha = 1.f;
+                        rbeta = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (BWD && run_slot < d.tape_depth) {
+                            const size_t e = rbase + run_slot;
+#pragma unroll
+                            for (int k = 0; k < SPT; ++k) d.tape[(e * SPT + k) * 32 + lane] = c[k];
+                        }
+                    }
+                    const bool mine = (run >> lane) & 1u;
+                    Affine t = mine ? Affine{1.f - my_fill.w, make_float4(my_fill.x * my_fill.w, my_fill.y * my_fill.w,
+                                                                         my_fill.z * my_fill.w, my_fill.w * my_fill.w)}
+                                    : Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const Affine up = shfl_affine<true>(t, o);
+                        if (lane >= o) t = after(up, t);
+                    }
+                    if (BWD) {
+                        Affine ex = shfl_affine<true>(t, 1);
+                        if (lane == 0) ex = Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+                        ex = after(Affine{ralpha, rbeta}, ex);
+                        const int e = ne + __popc(run & ((1u << lane) - 1u));
+                        if (mine && e < d.tape_depth) {
+                            float4 *rec = d.tape_rec + (rbase + e) * 3;
+                            rec[0] = my_fill;
+                            rec[1] = ex.b;
+                            rec[2] = make_float4(ex.a, __uint_as_float(it.w), __uint_as_float(0u),
+                                                 slot_and_item(run_slot, base - beg + lane));
+                        } else if (mine) {
+                            atomicOr(d.status, 1u);
+                        }
+                        ne += __popc(run);
+                    }
+                    const Affine all = after(Affine{ralpha, rbeta}, shfl_affine<false>(t, 31));
+                    ralpha = all.a;
+                    rbeta = all.b;
+                    continue;
+                }
                 tm &= tm - 1u;
-                const uint32_t w = __shfl_sync(0xffffffffu, it.z, q);
-                const uint32_t path = __shfl_sync(0xffffffffu, it.w, q);
                 float4 f;
                 f.x = __shfl_sync(0xffffffffu, my_fill.x, q);
                 f.y = __shfl_sync(0xffffffffu, my_fill.y, q);
                 f.z = __shfl_sync(0xffffffffu, my_fill.z, q);
                 f.w = __shfl_sync(0xffffffffu, my_fill.w, q);
-                const bool frag = w != 0;
-                uint32_t m = 0xFFFFFFFFu;
-                if (frag) {
-                    uint4 mm;
-                    mm.x = __shfl_sync(0xffffffffu, my_mm.x, q);
-                    mm.y = WORDS > 1 ? __shfl_sync(0xffffffffu, my_mm.y, q) : 0u;
-                    mm.z = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.z, q) : 0u;
-                    mm.w = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.w, q) : 0u;
-                    m = pixel_mask(mm, S, k4);
-                }
+                uint4 mm;
+                mm.x = __shfl_sync(0xffffffffu, my_mm.x, q);
+                mm.y = WORDS > 1 ? __shfl_sync(0xffffffffu, my_mm.y, q) : 0u;
+                mm.z = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.z, q) : 0u;
+                mm.w = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.w, q) : 0u;
+                const uint32_t m = pixel_mask(mm, S, k4);
                 const float om = 1.f - f.w;
-                // A run of spans (which cover every sample of the cell) is
-                // carried as c = ralpha * c_run + rbeta, c_run the samples'
-                // state where the run starts; states are materialized at
-                // fragments and at the end.
-                if (frag && run_slot >= 0) {
+                // the samples' states are materialized at fragments and at the end
+                if (run_slot >= 0) {
 #pragma unroll
                     for (int k = 0; k < SPT; ++k)
                         c[k] = make_float4(ralpha * c[k].x + rbeta.x, ralpha * c[k].y + rbeta.y,
                                            ralpha * c[k].z + rbeta.z, ralpha * c[k].w + rbeta.w);
                     run_slot = -1;
                 }
-                int sidx = run_slot;
-                if (frag || run_slot < 0) {
-                    sidx = nsl++;
-                    if (BWD && sidx < d.tape_depth) {
+                if (BWD) {
+                    const int sidx = nsl++;
+                    if (sidx < d.tape_depth) {
                         const size_t e = rbase + sidx;
 #pragma unroll
                         for (int k = 0; k < SPT; ++k) d.tape[(e * SPT + k) * 32 + lane] = c[k];
                     }
-                    if (!frag) {
-                        run_slot = sidx;
-                        ralpha = 1.f;
-                        rbeta = make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                }
-                if (BWD) {
-                    if (ne < d.tape_depth) {
-                        if (lane == 0) {
+                    if (lane == q) {  // (the lane that holds the item)
+                        if (ne < d.tape_depth) {
+                            // (a fragment needs no run state: its mask and its group's place)
                             float4 *rec = d.tape_rec + (rbase + ne) * 3;
-                            rec[0] = f;
-                            rec[1] = rbeta;
-                            rec[2] = make_float4(ralpha, __uint_as_float(path), __uint_as_float(w),
-                                                 __uint_as_float((uint32_t)sidx));
+                            rec[0] = my_fill;
+                            rec[1] = make_float4(__uint_as_float(my_mm.x), __uint_as_float(my_mm.y),
+                                                 __uint_as_float(my_mm.z), __uint_as_float(my_mm.w));
+                            rec[2] = make_float4(__uint_as_float(it.y), __uint_as_float(it.w), __uint_as_float(it.z),
+                                                 slot_and_item(sidx, base - beg + lane));
+                        } else {
+                            atomicOr(d.status, 1u);
                         }
-                    } else if (lane == 0) {
-                        atomicOr(d.status, 1u);
                     }
                     ++ne;
                 }
-                if (!frag) {  // the run's composition up to and including this span
-                    rbeta = make_float4(f.x * f.w + rbeta.x * om, f.y * f.w + rbeta.y * om, f.z * f.w + rbeta.z * om,
-                                        f.w * f.w + rbeta.w * om);
-                    ralpha *= om;
-                } else {
 #pragma unroll
-                    for (int k = 0; k < SPT; ++k) {
-                        if ((m >> (sub + 8 * k)) & 1u) {
-                            c[k].x = f.x * f.w + c[k].x * om;
-                            c[k].y = f.y * f.w + c[k].y * om;
-                            c[k].z = f.z * f.w + c[k].z * om;
-                            c[k].w = f.w * f.w + c[k].w * om;
-                        }
+                for (int k = 0; k < SPT; ++k) {
+                    if ((m >> (sub + 8 * k)) & 1u) {
+                        c[k].x = f.x * f.w + c[k].x * om;
+                        c[k].y = f.y * f.w + c[k].y * om;
+                        c[k].z = f.z * f.w + c[k].z * om;
+                        c[k].w = f.w * f.w + c[k].w * om;
                     }
                 }
             }
-            it = nit;
-            my_fill = nfill;
-            my_mm = nmm;
         }
         if (run_slot >= 0) {
 #pragma unroll
@@ -640,39 +687,30 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
         int cur_slot = -1;  // run being swept (its start slot), -1 outside runs
         float pi = 1.f;
         float4 Lsum = make_float4(0.f, 0.f, 0.f, 0.f), Ksum = Lsum;
-        float4 rf = make_float4(0.f, 0.f, 0.f, 0.f), rbb = rf, rr2 = rf;  // lane l: record e_hi - l
-        for (int e0 = ne - 1; e0 >= 0; --e0) {
-            const int jl = (ne - 1 - e0) & 31;
-            if (jl == 0) {  // the next 32 records, one per lane
+        float4(*const rec_s)[BWD ? 32 : 1] = s_rec[BWD ? threadIdx.x >> 5 : 0];  // record e_hi - l at l
+        __syncwarp();  // (records written by their items' lanes)
+        for (int e0 = ne - 1, e_hi = ne + 31; e0 >= 0;) {
+            if (e_hi - e0 >= 32) {  // the next 32 records
+                __syncwarp();
+                e_hi = e0;
                 if (e0 - lane >= 0) {
                     const float4 *rec = d.tape_rec + (rbase + e0 - lane) * 3;
-                    rf = rec[0];
-                    rbb = rec[1];
-                    rr2 = rec[2];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) rec_s[i][lane] = rec[i];
                 }
+                __syncwarp();
             }
-            float4 f, rb, r2;
-            f.x = __shfl_sync(0xffffffffu, rf.x, jl);
-            f.y = __shfl_sync(0xffffffffu, rf.y, jl);
-            f.z = __shfl_sync(0xffffffffu, rf.z, jl);
-            f.w = __shfl_sync(0xffffffffu, rf.w, jl);
-            rb.x = __shfl_sync(0xffffffffu, rbb.x, jl);
-            rb.y = __shfl_sync(0xffffffffu, rbb.y, jl);
-            rb.z = __shfl_sync(0xffffffffu, rbb.z, jl);
-            rb.w = __shfl_sync(0xffffffffu, rbb.w, jl);
-            r2.x = __shfl_sync(0xffffffffu, rr2.x, jl);
-            r2.y = __shfl_sync(0xffffffffu, rr2.y, jl);
-            r2.z = __shfl_sync(0xffffffffu, rr2.z, jl);
-            r2.w = __shfl_sync(0xffffffffu, rr2.w, jl);
-            const float ra = r2.x;
-            const uint32_t path = __float_as_uint(r2.y), w = __float_as_uint(r2.z);
-            const int sidx = (int)__float_as_uint(r2.w);
-            const float av = f.w, om = 1.f - av;
+            const int jl = e_hi - e0;
+            const float4 r2 = rec_s[2][jl];
+            const uint32_t w = __float_as_uint(r2.z), si = __float_as_uint(r2.w);
+            const int sidx = (int)(si & 0xFFFFu);
             if (w == 0u) {
-                // span: every sample covered; inside a run the samples' adjoints
-                // are the run end's times the scalar pi, so the fill gradient
-                // needs only the run's sums Lsum = sum lambda and Ksum = sum
-                // lambda * c_run (c before the span = ra * c_run + rb).
+                // A run of spans, in the lanes that hold them: every sample is
+                // covered, so inside the run the samples' adjoints are the run
+                // end's times the scalar pi (the product of 1 - a of the later
+                // spans), and the fill gradients need only the run's sums Lsum =
+                // sum lambda and Ksum = sum lambda * c_run (c before the span =
+                // ra * c_run + rb).
                 if (sidx != cur_slot) {
                     if (cur_slot >= 0) {
 #pragma unroll
@@ -700,16 +738,38 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
                     cur_slot = sidx;
                     pi = 1.f;
                 }
-                const float cx = ra * Ksum.x + rb.x * Lsum.x, cy = ra * Ksum.y + rb.y * Lsum.y;
-                const float cz = ra * Ksum.z + rb.z * Lsum.z, cw = ra * Ksum.w + rb.w * Lsum.w;
+                // the run's records among the loaded ones: lanes [jl, jl + R)
+                const float4 rf = rec_s[0][lane], rbb = rec_s[1][lane], rr2 = rec_s[2][lane];
+                const uint32_t of_run = __ballot_sync(0xffffffffu, e_hi - lane >= 0 && __float_as_uint(rr2.z) == 0u &&
+                                                                       (int)(__float_as_uint(rr2.w) & 0xFFFFu) == sidx) >>
+                                         jl;
+                const int R = of_run == 0xFFFFFFFFu ? 32 : __ffs((int)~of_run) - 1;
+                const bool mine = lane >= jl && lane < jl + R;
+                float p = mine ? 1.f - rf.w : 1.f;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const float up = __shfl_up_sync(0xffffffffu, p, o);
+                    if (lane >= o) p *= up;
+                }
+                float pl = __shfl_up_sync(0xffffffffu, p, 1);
+                pl = lane == 0 ? pi : pi * pl;
+                const float av = rf.w, ra = rr2.x;
+                const float cx = ra * Ksum.x + rbb.x * Lsum.x, cy = ra * Ksum.y + rbb.y * Lsum.y;
+                const float cz = ra * Ksum.z + rbb.z * Lsum.z, cw = ra * Ksum.w + rbb.w * Lsum.w;
                 const float4 gf = make_float4(
-                    pi * av * Lsum.x, pi * av * Lsum.y, pi * av * Lsum.z,
-                    pi * (Lsum.x * f.x - cx + Lsum.y * f.y - cy + Lsum.z * f.z - cz + 2.f * av * Lsum.w - cw));
-                if (lane == 0 && (gf.x != 0.f || gf.y != 0.f || gf.z != 0.f || gf.w != 0.f))
-                    add_fill_grad(d, acc, cache, tag, path, gf);
-                pi *= om;
+                    pl * av * Lsum.x, pl * av * Lsum.y, pl * av * Lsum.z,
+                    pl * (Lsum.x * rf.x - cx + Lsum.y * rf.y - cy + Lsum.z * rf.z - cz + 2.f * av * Lsum.w - cw));
+                if (mine && (gf.x != 0.f || gf.y != 0.f || gf.z != 0.f || gf.w != 0.f))
+                    add_fill_grad(d, acc, __float_as_uint(rr2.w) >> 16, __float_as_uint(rr2.y), gf);
+                __syncwarp();
+                pi *= __shfl_sync(0xffffffffu, p, 31);
+                e0 -= R;
                 continue;
             }
+            --e0;
+            const float4 f = rec_s[0][jl], rb = rec_s[1][jl];
+            const uint32_t head = __float_as_uint(r2.x), path = __float_as_uint(r2.y);
+            const float av = f.w, om = 1.f - av;
             // fragment: per-sample coverage; first close a pending run
             if (cur_slot >= 0) {
 #pragma unroll
@@ -717,7 +777,10 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
                     lam[k] = make_float4(lam[k].x * pi, lam[k].y * pi, lam[k].z * pi, lam[k].w * pi);
                 cur_slot = -1;
             }
-            const uint32_t m = pixel_mask(load_merged(d.merged, WORDS, w - 1u), S, k4);
+            Lsum = Ksum = make_float4(0.f, 0.f, 0.f, 0.f);  // (of the closed run: not kept)
+            const uint32_t m = pixel_mask(make_uint4(__float_as_uint(rb.x), __float_as_uint(rb.y), __float_as_uint(rb.z),
+                                                     __float_as_uint(rb.w)),
+                                          S, k4);
             const size_t es = rbase + sidx;
             float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
             float J[SPT];
@@ -735,27 +798,11 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs 
                     lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
                 }
             }
-            group_adjoint<S>(a, d, d.heads[w - 1], a.fill_rule[path], J, lane);
+            group_adjoint<S>(a, d, (int64_t)head, a.fill_rule[path], J, lane);
             gf = warp_sum4(gf, lane);
             if (lane == 0 && (gf.x != 0.f || gf.y != 0.f || gf.z != 0.f || gf.w != 0.f))
-                add_fill_grad(d, acc, cache, tag, path, gf);
-        }
-    }
-    if (tag) {  // the warp's cached gradients
-        __syncwarp();
-        for (int i = lane; i < kDiffCacheSlots; i += 32)
-            if (tag[i] != 0xFFFFFFFFu) global_fill_grad(d, tag[i], cache[i]);
-    }
-    if (acc) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < a.P; i += kDiffThreads) {
-            const float4 v = acc[i];
-            if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
-                atomicAdd(&d.grad_fill[i].x, v.x);
-                atomicAdd(&d.grad_fill[i].y, v.y);
-                atomicAdd(&d.grad_fill[i].z, v.z);
-                atomicAdd(&d.grad_fill[i].w, v.w);
-            }
+                add_fill_grad(d, acc, si >> 16, path, gf);
+            __syncwarp();
         }
     }
 }
@@ -839,12 +886,12 @@ int diff_sm_count() {
     return n;
 }
 
-template <int S, bool BWD, bool CACHE>
-void run_diff(const FrameArgs &a, const DiffArgs &d, unsigned grid, size_t smem, cudaStream_t s) {
-    if constexpr (BWD || !CACHE) {  // the forward pass accumulates nothing
-        cudaFuncSetAttribute(k_diff<S, BWD, CACHE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_diff<S, BWD, CACHE><<<grid, kDiffThreads, smem, s>>>(a, d);
-    }
+template <int S, bool BWD>
+void run_diff(const FrameArgs &a, const DiffArgs &d, unsigned grid, cudaStream_t s) {
+    // units of up to a bin's 32 cells, at least 4 for every warp
+    int shift = 5;
+    while (shift > 0 && (a.n_bins * (kTileW / 2) >> shift) < 4 * (int64_t)grid * (kDiffThreads / 32)) --shift;
+    k_diff<S, BWD><<<grid, kDiffThreads, 0, s>>>(a, d, shift);
 }
 
 template <bool BWD>
@@ -857,19 +904,9 @@ int launch_diff(const FrameArgs &a, const DiffArgs &d, cudaStream_t s) {
         k_diff_gather<<<(unsigned)((d.npairs + 255) / 256), 256, 0, s>>>(d, a.S / 8);
         ++n;
     }
-    // backward: block-wide per-path accumulators up to kDiffPathAcc paths,
-    // per-warp path caches beyond
-    const bool cache = BWD && a.P > kDiffPathAcc;
-    const size_t smem = !BWD  ? 0
-                        : cache ? (sizeof(float4) + sizeof(uint32_t)) * kDiffCacheSlots * (kDiffThreads / 32)
-                                : sizeof(float4) * (size_t)std::max(a.P, 1);
-    if (a.S == 8) {
-        cache ? run_diff<8, BWD, true>(a, d, grid, smem, s) : run_diff<8, BWD, false>(a, d, grid, smem, s);
-    } else if (a.S == 16) {
-        cache ? run_diff<16, BWD, true>(a, d, grid, smem, s) : run_diff<16, BWD, false>(a, d, grid, smem, s);
-    } else {
-        cache ? run_diff<32, BWD, true>(a, d, grid, smem, s) : run_diff<32, BWD, false>(a, d, grid, smem, s);
-    }
+    if (a.S == 8) run_diff<8, BWD>(a, d, grid, s);
+    else if (a.S == 16) run_diff<16, BWD>(a, d, grid, s);
+    else run_diff<32, BWD>(a, d, grid, s);
     if (BWD && d.nf > 0) {
         k_diff_chain<<<(unsigned)((d.nf + 255) / 256), 256, 0, s>>>(a, d);
         ++n;

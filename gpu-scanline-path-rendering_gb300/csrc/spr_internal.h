@@ -50,7 +50,7 @@ struct FrameCounters {
     uint32_t need_pairs;   // resolve pairs of the frame
     uint32_t n_items;      // n_merged + n_span
     uint32_t tiles[3];     // look-back tile counters: entry offsets, scan-mark, pair offsets
-    uint32_t diff_status;  // differentiable frames: bit 0 tape too short, bit 1 chain too short
+    uint32_t diff_status;  // differentiable frames: bit 0 tape too short
     uint32_t n_seg[3], q_seg[3];  // segment sort: listed segments by size class, and those taken
     uint32_t longest;            // entries of the longest path (sized frames)
     uint32_t pairs_alt;          // resolve pairs in the other built-in tile (FrameArgs::alt_shift)
@@ -281,17 +281,16 @@ struct DiffArgs {
     const uint32_t *merged;
     const uint32_t *pval, *bstart, *bend;
     int64_t npairs;
-    // the resolve pairs' items gathered in bin order: (pos, length, merged
-    // index + 1, path), the path's fill, the merged sample mask
+    // the resolve pairs' items gathered in bin order: (pos, length (of a
+    // fragment: its group's first sorted position), merged index + 1, path), the path's fill, the merged sample mask
     uint4 *bitem;
     float4 *bfill;
     uint4 *bmm;
     const float4 *chord;
     const uint32_t *lmask, *vmask, *pidw, *perm, *heads, *item_path;
-    // per fragment crossing sums (raw fragment, slope, sum dL/dx (1 - lam),
-    // sum dL/dx lam), chained to the control points by a second kernel
-    float4 *chain;
-    uint32_t *n_chain;
+    // per fragment (raw order) its crossing sums, sum dL/dx (1 - lam) and sum
+    // dL/dx lam (zero before), chained to the control points by a second kernel
+    float2 *chain;
     const uint64_t *skey;
     const int8_t *wn_scan;
     const int2 *entries;
@@ -301,7 +300,7 @@ struct DiffArgs {
     float4 *tape_rec;  // per block: warps x tape_depth x 3 (per-cell item records)
     int tape_depth;
     uint32_t *queue;     // bin queue (zeroed by the launchers)
-    uint32_t *status;    // bit 0: a tape overflowed (rerun with a deeper tape); bit 1: chain list full
+    uint32_t *status;    // bit 0: a tape overflowed (rerun with a deeper tape)
     // pixel = out_scale * (mean of the samples), added to the image when
     // accumulate (the passes of a 256-sample frame: 1/8 each); the backward
     // takes out_scale * dL/d(pixel) likewise
