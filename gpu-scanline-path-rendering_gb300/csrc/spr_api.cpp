@@ -127,7 +127,7 @@ struct spr_handle {
     // differentiable frames: per-fragment chords and left masks, per-item
     // paths, the per-block tapes, the transformed-vertex gradient and the
     // stored -> input vertex map
-    DevBuf chord, lmask, vmask, item_path, tape, tape_rec, grad_tvert, vmap, bitems, chain, ekey[2], eval[2];
+    DevBuf chord, lmask, vmask, item_path, tape, run_pi, bruns, dcells, grad_tvert, vmap, bitems, chain, ekey[2], eval[2];
     // 256-sample frames: the pass being rendered, the passes' fixed-point
     // sample sums, and a pass's fill gradient / the summed vertex gradient
     int pass = 0;
@@ -153,7 +153,7 @@ struct spr_handle {
     // raw curve arrays of the device-side scene upload (kept for vertex updates)
     DevBuf sc_vpos, sc_type, sc_pid, sc_w, scene_flags;
     bool scene_on_device = false, scene_has_arcw = false;
-    int tape_depth = 128;
+    int tape_depth = 64, pi_depth = 128;  // (grown by the backward as its frames need)
     // frame buffers
     DevBuf tvert, pvis, counts, offsets, scan_tmp, entries, key, pidw, wn, mask, skey[2], sval[2], sort_tmp,
         wn_scan, draw, heads, merged, pval, rec_a, rec_m, bins, image, counters, dump_tmp, overflow;
@@ -220,7 +220,7 @@ std::vector<DevBuf *> handle_bufs(spr_handle *h) {
                       &h->wn_scan,    &h->draw,    &h->heads,    &h->merged,  &h->pval,
                       &h->rec_a,      &h->rec_m,   &h->bins,
                       &h->image,      &h->counters, &h->dump_tmp, &h->overflow, &h->scenes_d, &h->path_scene,
-                      &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->tape_rec,
+                      &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->run_pi, &h->bruns, &h->dcells,
                       &h->grad_tvert, &h->vmap, &h->bitems, &h->vmask, &h->chain, &h->ekey[0], &h->ekey[1], &h->eval[0],
                       &h->eval[1], &h->sc_vpos, &h->sc_type, &h->sc_pid, &h->sc_w, &h->scene_flags,
                       &h->sums, &h->gfill_pass, &h->gtvert_total, &h->grad_table, &h->grad_ramp, &h->path_start, &h->seg_list,
@@ -664,6 +664,11 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.bitem = h->bitems.as<uint4>();
         d.bfill = reinterpret_cast<float4 *>(d.bitem + d.npairs);
         d.bmm = d.bitem + 2 * d.npairs;
+        // the runs' maps, and after them (backward) their sums
+        if ((st = ensure(h->bruns, (dc.backward ? 52 : 20) * (size_t)d.npairs))) return st;
+        d.run_b = h->bruns.as<float4>();
+        d.run_sum = d.run_b + d.npairs;
+        d.run_a = reinterpret_cast<float *>(d.run_b + (dc.backward ? 3 : 1) * d.npairs);
     }
     d.chord = h->chord.as<float4>();
     d.lmask = h->lmask.as<uint32_t>();
@@ -678,7 +683,19 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
     d.tvert = h->tvert.as<float2>();
     d.nf = h->nf;
     FrameCounters *ctr = h->counters.as<FrameCounters>();
-    d.queue = &ctr->bin_queue;
+    d.queue = ctr->diff_queue;
+    d.n_cells = d.queue + 1;
+    d.cell_queue = d.queue + 2;
+    // per cell of the bins: its place in the list, the run map and the adjoint sum
+    const int64_t cells = a.n_bins * 32;
+    {
+        int st = ensure(h->dcells, 40 * (size_t)std::max<int64_t>(cells, 1));
+        if (st) return st;
+        d.cell_b = h->dcells.as<float4>();
+        d.cell_sum = d.cell_b + cells;
+        d.cell_a = reinterpret_cast<float *>(d.cell_sum + cells);
+        d.cell = reinterpret_cast<uint32_t *>(d.cell_a + cells);
+    }
     d.status = &ctr->diff_status;
     d.out_scale = dc.scale;
     d.accumulate = dc.pass > 0 ? 1 : 0;
@@ -698,14 +715,16 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.grad_fill = h->gfill_pass.as<float4>();
     }
     d.chain = h->chain.as<float2>();
-    for (int depth = h->tape_depth;; depth *= 2) {
-        const int64_t words = diff_tape_words(a, depth);
-        if ((st = ensure(h->tape, 16 * (size_t)words)) ||
-            (st = ensure(h->tape_rec, 16 * (size_t)diff_tape_rec_words(a, depth))))
+    // (most bins hold fewer than four times the mean of items)
+    while (h->pi_depth < 4 * (d.npairs / std::max<int64_t>(a.n_bins, 1)) && h->pi_depth < (1 << 16)) h->pi_depth *= 2;
+    for (;;) {
+        if ((st = ensure(h->tape, 16 * (size_t)diff_tape_words(a, h->tape_depth))) ||
+            (st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, h->pi_depth))))
             return st;
         d.tape = h->tape.as<float4>();
-        d.tape_rec = h->tape_rec.as<float4>();
-        d.tape_depth = depth;
+        d.run_pi = h->run_pi.as<float>();
+        d.tape_depth = h->tape_depth;
+        d.pi_depth = h->pi_depth;
         cudaMemsetAsync(d.grad_fill, 0, 16 * (size_t)h->P, s);
         cudaMemsetAsync(h->grad_tvert.p, 0, 8 * (size_t)h->V, s);
         cudaMemsetAsync(&ctr->diff_status, 0, 4, s);
@@ -714,11 +733,10 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         cudaMemcpyAsync(h->h_u32, &ctr->diff_status, 4, cudaMemcpyDeviceToHost, s);
         ++h->host_syncs;
         if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
-        if (!(h->h_u32[0] & 1u)) {
-            h->tape_depth = depth;
-            break;
-        }
-        if (depth >= (1 << 16)) return SPR_ERR_CAPACITY_EXCEEDED;
+        const uint32_t status = h->h_u32[0];
+        if (status == 0u) break;
+        if ((status & 1u) && (h->tape_depth *= 2) > (1 << 17)) return SPR_ERR_CAPACITY_EXCEEDED;
+        if ((status & 2u) && (h->pi_depth *= 2) > (1 << 24)) return SPR_ERR_CAPACITY_EXCEEDED;
     }
     const float2 *gt = h->grad_tvert.as<float2>();
     if (multi) {

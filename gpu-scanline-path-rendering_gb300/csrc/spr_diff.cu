@@ -36,7 +36,6 @@ namespace spr {
 namespace {
 
 constexpr int kDiffThreads = 256;    // 8 warps, each working on its own cells
-constexpr int kDiffItemAcc = 128;    // items of a bin whose fill gradients a warp gathers in shared memory (backward)
 constexpr int kTileW = kBinW;  // columns of a resolve bin
 
 __device__ __forceinline__ uint32_t pixel_mask(const uint4 &mm, int S, int k) {
@@ -349,64 +348,11 @@ __device__ __forceinline__ uint4 load_merged(const uint32_t *merged, int words, 
     return make_uint4(merged[g], 0u, 0u, 0u);
 }
 
-__device__ __forceinline__ void global_fill_grad(const DiffArgs &d, uint32_t path, float4 g) {
-    atomicAdd(&d.grad_fill[path].x, g.x);
-    atomicAdd(&d.grad_fill[path].y, g.y);
-    atomicAdd(&d.grad_fill[path].z, g.z);
-    atomicAdd(&d.grad_fill[path].w, g.w);
-}
-
-// c -> a * c + b per channel, and maps composed: `first`, then `t`.
+// c -> a * c + b per channel.
 struct Affine {
     float a;
     float4 b;
 };
-__device__ __forceinline__ Affine after(const Affine &first, const Affine &t) {
-    return Affine{t.a * first.a, make_float4(t.a * first.b.x + t.b.x, t.a * first.b.y + t.b.y, t.a * first.b.z + t.b.z,
-                                             t.a * first.b.w + t.b.w)};
-}
-// From `o` lanes below (UP), or from lane o.
-template <bool UP>
-__device__ __forceinline__ Affine shfl_affine(const Affine &t, int o) {
-    auto get = [&](float v) { return UP ? __shfl_up_sync(0xffffffffu, v, o) : __shfl_sync(0xffffffffu, v, o); };
-    return Affine{get(t.a), make_float4(get(t.b.x), get(t.b.y), get(t.b.z), get(t.b.w))};
-}
-
-// A fill gradient of item `idx` of the warp's bin (lanes that call it together
-// have different items): into the item's accumulator, or, past those, straight
-// to the global gradient.
-__device__ __forceinline__ void add_fill_grad(const DiffArgs &d, float4 *acc, uint32_t idx, uint32_t path, float4 g) {
-    if (idx < (uint32_t)kDiffItemAcc) {
-        float4 v = acc[idx];
-        v.x += g.x;
-        v.y += g.y;
-        v.z += g.z;
-        v.w += g.w;
-        acc[idx] = v;
-    } else {
-        global_fill_grad(d, path, g);
-    }
-}
-
-// The accumulators of a bin's items [beg, fin) added to their paths' gradients
-// and cleared.
-__device__ __forceinline__ void flush_fill_grads(const DiffArgs &d, float4 *acc, uint32_t beg, uint32_t fin, int lane) {
-    __syncwarp();
-    for (uint32_t i = lane; i < min(fin - beg, (uint32_t)kDiffItemAcc); i += 32) {
-        const float4 v = acc[i];
-        if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) {
-            global_fill_grad(d, d.bitem[beg + i].w, v);
-            acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    }
-    __syncwarp();
-}
-
-// Tape slot (at most 65,536) and item of a record in one word; items past the
-// accumulators need no number of their own.
-__device__ __forceinline__ float slot_and_item(int slot, uint32_t item) {
-    return __uint_as_float((uint32_t)slot | (min(item, 0xFFFFu) << 16));
-}
 
 // The scene of resolve bin b: viewport, the bin index within the scene and
 // the scene's first pixel (batch frames; a single scene otherwise).
@@ -456,353 +402,463 @@ __global__ void k_diff_chain(FrameArgs a, DiffArgs d) {
     fragment_chain(a, d, (uint32_t)i, (c.z - c.x) / (c.w - c.y), r.x, r.y);
 }
 
-// Persistent warps over units from a queue, 1 << unit_shift consecutive cells of
-// a bin each: warp = one cell of a bin at a time, lane l = pixel k4 = l >> 3 of the cell (k4 = px * 2 + py), samples
-// (l & 7) + 8k.  Every item touching a cell touches all its pixels, so the
-// walk over the bin's items is warp-uniform; the items are read 32 at a time
-// (one per lane), the touching ones found by a ballot and broadcast.  Warps
-// never wait for one another.
-template <int S, bool BWD>
-__global__ void __launch_bounds__(kDiffThreads, 3) k_diff(FrameArgs a, DiffArgs d, int unit_shift) {
+// A bin of the passes with a lane per cell, taken by a warp from a queue.
+struct Unit {
+    BinScene bs;
+    uint32_t beg, fin;  // the bin's items
+    uint32_t cell0;     // the first cell's number (bin * cells of a bin + column)
+    int x0, y0, cells;  // its pixel; cells within the viewport
+};
+__device__ __forceinline__ bool next_unit(const FrameArgs &a, const DiffArgs &d, int lane, Unit &u) {
+    uint32_t b = 0;
+    if (lane == 0) b = atomicAdd(d.queue, 1u);
+    b = __shfl_sync(0xffffffffu, b, 0);
+    if ((int64_t)b >= a.n_bins) return false;
+    u.beg = d.bstart[b];
+    u.fin = d.bend[b];
+    u.bs = bin_scene(a, b);
+    const int ntx = (u.bs.W + kTileW - 1) / kTileW, tile = (int)(u.bs.lb % ntx);
+    u.cell0 = b * (kTileW / 2);
+    u.x0 = tile * kTileW;
+    u.y0 = (int)(u.bs.lb / ntx) * 2;
+    u.cells = min(kTileW / 2, (u.bs.W - u.x0 + 1) / 2);
+    return true;
+}
+
+// (The gathered items are read with __ldg: an earlier kernel wrote them, and the
+// stores to the runs' maps and factors between the loads would otherwise keep
+// them one after the other.)
+
+// Item `it` touches the cell at column x (a fragment covers one cell).
+__device__ __forceinline__ bool touches(const uint4 &it, int x) {
+    const int ix = (int)(it.x & 0xFFFFu);
+    return it.z != 0u ? ix == x : (x >= ix && x < ix + (int)it.y);
+}
+
+// 32 of a bin's items, one per lane, for the passes with a lane per cell, which
+// take them one by one through shuffles (a load at a time would leave a memory
+// latency between them).  Column | length << 16 (a fragment: 0).
+__device__ __forceinline__ uint32_t item_cols(const uint4 &it) {
+    return (it.x & 0xFFFFu) | (it.z != 0u ? 0u : min(it.y, 0xFFFFu) << 16);
+}
+__device__ __forceinline__ float4 shfl_fill(const float4 &f, int q) {
+    return make_float4(__shfl_sync(0xffffffffu, f.x, q), __shfl_sync(0xffffffffu, f.y, q),
+                       __shfl_sync(0xffffffffu, f.z, q), __shfl_sync(0xffffffffu, f.w, q));
+}
+__device__ __forceinline__ bool touches(uint32_t cols, int x) {
+    const int ix = (int)(cols & 0xFFFFu), len = (int)(cols >> 16);
+    return len == 0 ? ix == x : (x >= ix && x < ix + len);
+}
+
+// A span: c -> fill * alpha + c * (1 - alpha), after the map `run`.
+__device__ __forceinline__ void add_span(Affine &run, const float4 &f) {
+    const float om = 1.f - f.w;
+    run.b = make_float4(f.x * f.w + run.b.x * om, f.y * f.w + run.b.y * om, f.z * f.w + run.b.z * om,
+                        f.w * f.w + run.b.w * om);
+    run.a *= om;
+}
+constexpr float kNoSpans = -1.f;  // in place of a run's factor: the run holds no span
+
+// First pass over a unit's items, a lane per cell (at column x).  A span covers
+// every sample of a cell, so the spans between two fragments of a cell are one
+// affine map of its samples' state: the map before each fragment goes to
+// d.run_b / d.run_a at the fragment's place (a fragment is in one cell), the
+// map after the last one is returned (a = kNoSpans: no spans).
+__device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, int &n_frags) {
+    const Affine none{kNoSpans, make_float4(0.f, 0.f, 0.f, 0.f)};
+    const int lane = threadIdx.x & 31;
+    Affine run = none;
+    n_frags = 0;
+    for (uint32_t base = u.beg; base < u.fin; base += 32) {
+        const uint32_t mine = min(base + lane, u.fin - 1);
+        const uint32_t my_cols = item_cols(__ldg(&d.bitem[mine]));
+        const float4 my_fill = __ldg(&d.bfill[mine]);
+        const int n = (int)min(u.fin - base, 32u);
+        for (int q = 0; q < n; ++q) {
+            const uint32_t cols = __shfl_sync(0xffffffffu, my_cols, q);
+            const bool touch = active && touches(cols, x);
+            if (cols >> 16) {  // (uniform) a span
+                const float4 f = shfl_fill(my_fill, q);
+                if (touch) {
+                    if (run.a < 0.f) run.a = 1.f;
+                    add_span(run, f);
+                }
+            } else if (touch) {
+                d.run_b[base + q] = run.b;
+                d.run_a[base + q] = run.a;
+                run = none;
+                ++n_frags;
+            }
+        }
+    }
+    return run;
+}
+
+// The fragments of the cell at column x among items [base, base + 32).
+__device__ __forceinline__ uint32_t cell_fragments(const DiffArgs &d, uint32_t fin, uint32_t base, int x, int lane) {
+    bool touch = false;
+    if (base + lane < fin) {
+        const uint4 it = __ldg(&d.bitem[base + lane]);
+        touch = it.z != 0u && touches(it, x);
+    }
+    return __ballot_sync(0xffffffffu, touch);
+}
+
+template <int SPT>
+__device__ __forceinline__ void apply_run(float4 (&c)[SPT], float ra, const float4 &rb) {
+    if (ra < 0.f) return;  // (uniform: no spans)
+#pragma unroll
+    for (int k = 0; k < SPT; ++k)
+        c[k] = make_float4(ra * c[k].x + rb.x, ra * c[k].y + rb.y, ra * c[k].z + rb.z, ra * c[k].w + rb.w);
+}
+
+template <int S, int SPT>
+__device__ __forceinline__ void apply_fragment(float4 (&c)[SPT], const float4 &f, uint32_t m, int sub) {
+    const float om = 1.f - f.w;
+#pragma unroll
+    for (int k = 0; k < SPT; ++k) {
+        if ((m >> (sub + 8 * k)) & 1u) {
+            c[k].x = f.x * f.w + c[k].x * om;
+            c[k].y = f.y * f.w + c[k].y * om;
+            c[k].z = f.z * f.w + c[k].z * om;
+            c[k].w = f.w * f.w + c[k].w * om;
+        }
+    }
+}
+
+__device__ __forceinline__ void store_pixel(const DiffArgs &d, int64_t pix, float4 v) {
+    if (d.accumulate) {
+        const float4 o = d.image[pix];
+        v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+    }
+    d.image[pix] = v;
+}
+
+// First pass of the composite and of its adjoint: the spans of every cell, a
+// lane per cell (cell_runs).  Cells without fragments have one colour, which
+// the forward writes at once; the others are listed for the second pass, with
+// the map of their last run.
+template <bool FORWARD>
+__global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArgs d) {
+    const int lane = threadIdx.x & 31;
+    Unit u;
+    while (next_unit(a, d, lane, u)) {
+        const bool active = lane < u.cells;
+        const int x = u.x0 + 2 * lane;
+        int n_frags;
+        const Affine last = cell_runs(d, u, active, x, n_frags);
+        if (FORWARD && active && n_frags == 0) {
+            float4 c[1] = {make_float4(1.f, 1.f, 1.f, 1.f)};
+            apply_run(c, last.a, last.b);
+            const float s = d.out_scale;
+            const float4 v = make_float4(c[0].x * s, c[0].y * s, c[0].z * s, c[0].w * s);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int X = x + (k >> 1), Y = u.y0 + (k & 1);
+                if (X < u.bs.W && Y < u.bs.H) store_pixel(d, u.bs.image_off + (int64_t)Y * u.bs.W + X, v);
+            }
+        }
+        const uint32_t cells = __ballot_sync(0xffffffffu, n_frags > 0);
+        uint32_t base = 0;
+        if (lane == 0 && cells) base = atomicAdd(d.n_cells, (uint32_t)__popc(cells));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (n_frags > 0) {
+            d.cell[base + __popc(cells & ((1u << lane) - 1u))] = u.cell0 + lane;
+            d.cell_b[u.cell0 + lane] = last.b;
+            d.cell_a[u.cell0 + lane] = last.a;
+        }
+    }
+}
+
+// A cell of the second pass: warp = cell, lane l = pixel k4 = l >> 3 of the cell
+// (k4 = px * 2 + py), samples (l & 7) + 8k.  Warps take kCellBatch cells at a
+// time from the list.
+constexpr uint32_t kCellBatch = 8;
+struct Cell {
+    uint32_t id, beg, fin;
+    int x;        // its column
+    int64_t pix;  // this lane's pixel in the image
+    bool valid;   // ... is inside the viewport
+    uint32_t next, end;  // the warp's listed cells
+    BinScene bs;         // of the bin that beg and fin are of
+};
+__device__ __forceinline__ bool next_cell(const FrameArgs &a, const DiffArgs &d, uint32_t n_cells, int lane, Cell &c) {
+    if (c.next == c.end) {
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(d.cell_queue, kCellBatch);
+        c.next = __shfl_sync(0xffffffffu, k, 0);
+        if (c.next >= n_cells) return false;
+        c.end = min(c.next + kCellBatch, n_cells);
+    }
+    const uint32_t id = d.cell[c.next++], b = id / (kTileW / 2);
+    if (c.id / (kTileW / 2) != b) {  // (a bin's cells are listed together)
+        c.beg = d.bstart[b];
+        c.fin = d.bend[b];
+        c.bs = bin_scene(a, b);
+    }
+    c.id = id;
+    const int ntx = (c.bs.W + kTileW - 1) / kTileW;
+    c.x = (int)(c.bs.lb % ntx) * kTileW + 2 * (int)(id % (kTileW / 2));
+    const int X = c.x + (lane >> 4), Y = (int)(c.bs.lb / ntx) * 2 + ((lane >> 3) & 1);
+    c.pix = c.bs.image_off + (int64_t)Y * c.bs.W + X;
+    c.valid = X < c.bs.W && Y < c.bs.H;
+    return true;
+}
+
+// The composite of the cells with fragments, through their fragments only.  With
+// every cell walking all items of its bin, the spans composed over the lanes
+// that held them, the composite of a 1024 x 1024 scene of 256 paths took 151 us
+// and that of a batch of 16 scenes 1435; in these two passes 93 and 818.
+template <int S>
+__global__ void __launch_bounds__(kDiffThreads, 5) k_diff_forward(FrameArgs a, DiffArgs d) {
     constexpr int SPT = S / 8;
-    constexpr int WORDS = S / 8;
-    // fill-gradient accumulators of the warp's bin items: a warp's cells of one
-    // bin share them, so a path costs one set of global atomics a unit
-    __shared__ float4 s_acc[BWD ? kDiffThreads / 32 : 1][BWD ? kDiffItemAcc : 1];
-    // the reverse sweep's next 32 records of each warp (held in registers they
-    // would spill others)
-    __shared__ float4 s_rec[BWD ? kDiffThreads / 32 : 1][BWD ? 3 : 1][BWD ? 32 : 1];
     const int lane = threadIdx.x & 31;
     const int k4 = lane >> 3, sub = lane & 7;
-    const int px_in = k4 >> 1, py_in = k4 & 1;
-    const size_t wslot = (size_t)blockIdx.x * (kDiffThreads / 32) + (threadIdx.x >> 5);
-    float4 *const acc = s_acc[BWD ? threadIdx.x >> 5 : 0];
-    if (BWD) {
-        for (int i = lane; i < kDiffItemAcc; i += 32) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncwarp();
-    }
-    const int64_t n_units = a.n_bins * (kTileW / 2) >> unit_shift;
-    // the unit's bin and the next cell of it
-    BinScene bs{};
-    int tile = 0, crow = 0, cw = 0, end = 0;
-    uint32_t beg = 0, fin = 0;
-    // the bin's items, 32 at a time (lane l holds item base + l); in the forward
-    // a bin of one such chunk keeps it from cell to cell (the backward's reverse
-    // sweep needs the registers)
-    uint4 it = make_uint4(0u, 0u, 0u, 0u), my_mm = it;
-    float4 my_fill = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (;;) {
-        bool load = BWD || fin - beg > 32;
-        if (cw == end) {
-            if (BWD) flush_fill_grads(d, acc, beg, fin, lane);
-            uint32_t u = 0;
-            if (lane == 0) u = atomicAdd(d.queue, 1u);
-            u = __shfl_sync(0xffffffffu, u, 0);
-            if ((int64_t)u >= n_units) break;
-            const uint32_t b = (u << unit_shift) / (kTileW / 2);
-            bs = bin_scene(a, b);
-            const int ntx = (bs.W + kTileW - 1) / kTileW;
-            tile = (int)(bs.lb % ntx), crow = (int)(bs.lb / ntx);
-            cw = (int)((u << unit_shift) % (kTileW / 2));
-            end = min(cw + (1 << unit_shift), (bs.W - tile * kTileW + 1) / 2);  // (cells within the viewport)
-            beg = fin = 0;
-            if (cw >= end) {
-                cw = end;
-                continue;
-            }
-            beg = d.bstart[b], fin = d.bend[b];
-            load = true;
-        }
-        const int cellx = tile * kTileW + 2 * cw++;
-        const int X = cellx + px_in, Y = crow * 2 + py_in;
-        const bool valid = X < bs.W && Y < bs.H;
-        const int64_t pix = bs.image_off + (int64_t)Y * bs.W + X;
+    const uint32_t n_cells = *d.n_cells;
+    Cell cell{};
+    cell.id = 0xFFFFFFFFu;
+    while (next_cell(a, d, n_cells, lane, cell)) {
         float4 c[SPT];
 #pragma unroll
         for (int k = 0; k < SPT; ++k) c[k] = make_float4(1.f, 1.f, 1.f, 1.f);
-        // backward tape: ne item records; nsl sample-state slots (the state
-        // before every fragment and at the start of every run of spans)
-        int ne = 0, nsl = 0, run_slot = -1;
-        float ralpha = 1.f;
-        float4 rbeta = make_float4(0.f, 0.f, 0.f, 0.f);
-        const size_t rbase = wslot * (size_t)d.tape_depth;
-        for (uint32_t base = beg; base < fin; base += 32) {
-            if ((load || base != beg) && base + lane < fin) {
-                it = d.bitem[base + lane];
-                my_fill = d.bfill[base + lane];
-                my_mm = d.bmm[base + lane];
-            }
-            bool touch = false;
-            if (base + lane < fin) {
-                const int x = (int)(it.x & 0xFFFFu);
-                touch = it.z != 0u ? x == cellx : (cellx >= x && cellx < x + (int)it.y);
-            }
-            uint32_t tm = __ballot_sync(0xffffffffu, touch);
-            const uint32_t frags = __ballot_sync(0xffffffffu, touch && it.z != 0u);
-            while (tm) {
-                const int q = __ffs(tm) - 1;
-                const uint32_t later = frags & tm;  // the touching fragments ahead
-                if (!((frags >> q) & 1u)) {
-                    // The spans up to the next fragment.  A span covers every
-                    // sample of the cell, so a run of them is an affine map c =
-                    // ralpha * c_run + rbeta of the samples' state c_run where
-                    // the run starts; the maps are composed over the lanes that
-                    // hold the spans, each lane getting the map before its own.
-                    const uint32_t run = later ? tm & ((later & (0u - later)) - 1u) : tm;
-                    tm &= ~run;
-                    if (run_slot < 0) {
-                        run_slot = nsl++;
-                        ralpha = 1.f;
-                        rbeta = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (BWD && run_slot < d.tape_depth) {
-                            const size_t e = rbase + run_slot;
-#pragma unroll
-                            for (int k = 0; k < SPT; ++k) d.tape[(e * SPT + k) * 32 + lane] = c[k];
-                        }
-                    }
-                    const bool mine = (run >> lane) & 1u;
-                    Affine t = mine ? Affine{1.f - my_fill.w, make_float4(my_fill.x * my_fill.w, my_fill.y * my_fill.w,
-                                                                         my_fill.z * my_fill.w, my_fill.w * my_fill.w)}
-                                    : Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const Affine up = shfl_affine<true>(t, o);
-                        if (lane >= o) t = after(up, t);
-                    }
-                    if (BWD) {
-                        Affine ex = shfl_affine<true>(t, 1);
-                        if (lane == 0) ex = Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
-                        ex = after(Affine{ralpha, rbeta}, ex);
-                        const int e = ne + __popc(run & ((1u << lane) - 1u));
-                        if (mine && e < d.tape_depth) {
-                            float4 *rec = d.tape_rec + (rbase + e) * 3;
-                            rec[0] = my_fill;
-                            rec[1] = ex.b;
-                            rec[2] = make_float4(ex.a, __uint_as_float(it.w), __uint_as_float(0u),
-                                                 slot_and_item(run_slot, base - beg + lane));
-                        } else if (mine) {
-                            atomicOr(d.status, 1u);
-                        }
-                        ne += __popc(run);
-                    }
-                    const Affine all = after(Affine{ralpha, rbeta}, shfl_affine<false>(t, 31));
-                    ralpha = all.a;
-                    rbeta = all.b;
-                    continue;
-                }
-                tm &= tm - 1u;
-                float4 f;
-                f.x = __shfl_sync(0xffffffffu, my_fill.x, q);
-                f.y = __shfl_sync(0xffffffffu, my_fill.y, q);
-                f.z = __shfl_sync(0xffffffffu, my_fill.z, q);
-                f.w = __shfl_sync(0xffffffffu, my_fill.w, q);
-                uint4 mm;
-                mm.x = __shfl_sync(0xffffffffu, my_mm.x, q);
-                mm.y = WORDS > 1 ? __shfl_sync(0xffffffffu, my_mm.y, q) : 0u;
-                mm.z = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.z, q) : 0u;
-                mm.w = WORDS > 2 ? __shfl_sync(0xffffffffu, my_mm.w, q) : 0u;
-                const uint32_t m = pixel_mask(mm, S, k4);
-                const float om = 1.f - f.w;
-                // the samples' states are materialized at fragments and at the end
-                if (run_slot >= 0) {
-#pragma unroll
-                    for (int k = 0; k < SPT; ++k)
-                        c[k] = make_float4(ralpha * c[k].x + rbeta.x, ralpha * c[k].y + rbeta.y,
-                                           ralpha * c[k].z + rbeta.z, ralpha * c[k].w + rbeta.w);
-                    run_slot = -1;
-                }
-                if (BWD) {
-                    const int sidx = nsl++;
-                    if (sidx < d.tape_depth) {
-                        const size_t e = rbase + sidx;
-#pragma unroll
-                        for (int k = 0; k < SPT; ++k) d.tape[(e * SPT + k) * 32 + lane] = c[k];
-                    }
-                    if (lane == q) {  // (the lane that holds the item)
-                        if (ne < d.tape_depth) {
-                            // (a fragment needs no run state: its mask and its group's place)
-                            float4 *rec = d.tape_rec + (rbase + ne) * 3;
-                            rec[0] = my_fill;
-                            rec[1] = make_float4(__uint_as_float(my_mm.x), __uint_as_float(my_mm.y),
-                                                 __uint_as_float(my_mm.z), __uint_as_float(my_mm.w));
-                            rec[2] = make_float4(__uint_as_float(it.y), __uint_as_float(it.w), __uint_as_float(it.z),
-                                                 slot_and_item(sidx, base - beg + lane));
-                        } else {
-                            atomicOr(d.status, 1u);
-                        }
-                    }
-                    ++ne;
-                }
-#pragma unroll
-                for (int k = 0; k < SPT; ++k) {
-                    if ((m >> (sub + 8 * k)) & 1u) {
-                        c[k].x = f.x * f.w + c[k].x * om;
-                        c[k].y = f.y * f.w + c[k].y * om;
-                        c[k].z = f.z * f.w + c[k].z * om;
-                        c[k].w = f.w * f.w + c[k].w * om;
-                    }
-                }
+        for (uint32_t base = cell.beg; base < cell.fin; base += 32) {
+            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr; fr &= fr - 1u) {
+                const uint32_t p = base + __ffs(fr) - 1;
+                apply_run(c, d.run_a[p], d.run_b[p]);
+                apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
             }
         }
-        if (run_slot >= 0) {
+        apply_run(c, d.cell_a[cell.id], d.cell_b[cell.id]);
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < SPT; ++k)
-                c[k] = make_float4(ralpha * c[k].x + rbeta.x, ralpha * c[k].y + rbeta.y, ralpha * c[k].z + rbeta.z,
-                                   ralpha * c[k].w + rbeta.w);
+        for (int k = 0; k < SPT; ++k) {
+            sum.x += c[k].x;
+            sum.y += c[k].y;
+            sum.z += c[k].z;
+            sum.w += c[k].w;
         }
-        if (!BWD) {
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) {
-                sum.x += c[k].x;
-                sum.y += c[k].y;
-                sum.z += c[k].z;
-                sum.w += c[k].w;
-            }
+        for (int o = 1; o < 8; o <<= 1) {
+            sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+            sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
+            sum.z += __shfl_xor_sync(0xffffffffu, sum.z, o);
+            sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
+        }
+        if (sub == 0 && cell.valid) {
+            const float inv = d.out_scale / (float)S;
+            store_pixel(d, cell.pix, make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv));
+        }
+    }
+}
+
+// Adds a fill gradient that all lanes hold: one component per lane.
+__device__ __forceinline__ void add_fill_grad(const DiffArgs &d, uint32_t path, const float4 &g, int lane) {
+    const float v = lane == 0 ? g.x : (lane == 1 ? g.y : (lane == 2 ? g.z : g.w));
+    if (lane < 4 && v != 0.f) atomicAdd(reinterpret_cast<float *>(d.grad_fill + path) + lane, v);
+}
+
+// The adjoint of the cells with fragments: forward through the fragments, the
+// samples' states before each to the tape, and in reverse with the samples'
+// adjoints lambda, which gives the fragments' gradients and for every run of
+// spans Lsum = sum lambda and Ksum = sum lambda * c_run (c_run the state where
+// the run starts; of the first run, white, Lsum alone).  Bound by dependent
+// loads and arithmetic at 6 warps a scheduler.  The adjoint with every cell
+// walking all items of its bin twice took 505 us on a 1024 x 1024 scene of 256
+// paths and 5120 on a batch of 16 scenes; in three passes 350 and 3240.
+template <int S>
+__global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, DiffArgs d) {
+    constexpr int SPT = S / 8;
+    const int lane = threadIdx.x & 31;
+    const int k4 = lane >> 3, sub = lane & 7;
+    const size_t wslot = (size_t)blockIdx.x * (kDiffThreads / 32) + (threadIdx.x >> 5);
+    float4 *const tape = d.tape + wslot * (size_t)d.tape_depth * SPT * 32 + lane;  // slot e, k: [(e * SPT + k) * 32]
+    const float inv = d.out_scale / (float)S;
+    const uint32_t n_cells = *d.n_cells;
+    Cell cell{};
+    cell.id = 0xFFFFFFFFu;
+    while (next_cell(a, d, n_cells, lane, cell)) {
+        float4 c[SPT];
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
-                sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
-                sum.z += __shfl_xor_sync(0xffffffffu, sum.z, o);
-                sum.w += __shfl_xor_sync(0xffffffffu, sum.w, o);
-            }
-            if (valid && sub == 0) {
-                const float inv = d.out_scale / (float)S;
-                float4 v = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, sum.w * inv);
-                if (d.accumulate) {
-                    const float4 o = d.image[pix];
-                    v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
+        for (int k = 0; k < SPT; ++k) c[k] = make_float4(1.f, 1.f, 1.f, 1.f);
+        int slot = 0;
+        for (uint32_t base = cell.beg; base < cell.fin; base += 32) {
+            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr; fr &= fr - 1u) {
+                const uint32_t p = base + __ffs(fr) - 1;
+                apply_run(c, d.run_a[p], d.run_b[p]);
+                if (slot < d.tape_depth) {
+#pragma unroll
+                    for (int k = 0; k < SPT; ++k) tape[((size_t)slot * SPT + k) * 32] = c[k];
                 }
-                d.image[pix] = v;
+                ++slot;
+                apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
             }
+        }
+        if (slot > d.tape_depth) {
+            if (lane == 0) atomicOr(d.status, 1u);
             continue;
         }
-        // ---- reverse sweep (warp-uniform)
-        if (ne > d.tape_depth || nsl > d.tape_depth) continue;
-        const float inv = d.out_scale / (float)S;
-        const float4 G = valid ? d.grad_image[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 G = cell.valid ? d.grad_image[cell.pix] : make_float4(0.f, 0.f, 0.f, 0.f);
         float4 lam[SPT];
 #pragma unroll
         for (int k = 0; k < SPT; ++k) lam[k] = make_float4(G.x * inv, G.y * inv, G.z * inv, G.w * inv);
-        int cur_slot = -1;  // run being swept (its start slot), -1 outside runs
-        float pi = 1.f;
-        float4 Lsum = make_float4(0.f, 0.f, 0.f, 0.f), Ksum = Lsum;
-        float4(*const rec_s)[BWD ? 32 : 1] = s_rec[BWD ? threadIdx.x >> 5 : 0];  // record e_hi - l at l
-        __syncwarp();  // (records written by their items' lanes)
-        for (int e0 = ne - 1, e_hi = ne + 31; e0 >= 0;) {
-            if (e_hi - e0 >= 32) {  // the next 32 records
-                __syncwarp();
-                e_hi = e0;
-                if (e0 - lane >= 0) {
-                    const float4 *rec = d.tape_rec + (rbase + e0 - lane) * 3;
+        float ra = d.cell_a[cell.id];  // the run after the current fragment
+        for (uint32_t base = cell.beg + ((cell.fin - cell.beg - 1) & ~31u);; base -= 32) {
+            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr;) {
+                const int q = 31 - __clz((int)fr);
+                fr ^= 1u << q;
+                const uint32_t p = base + q;
+                const uint4 it = __ldg(&d.bitem[p]);
+                const float4 f = __ldg(&d.bfill[p]);
+                const float next_ra = d.run_a[p];
+                const uint32_t m = pixel_mask(__ldg(&d.bmm[p]), S, k4);
+                const float av = f.w, om = 1.f - av;
+                --slot;
+                float4 cb[SPT];
 #pragma unroll
-                    for (int i = 0; i < 3; ++i) rec_s[i][lane] = rec[i];
-                }
-                __syncwarp();
-            }
-            const int jl = e_hi - e0;
-            const float4 r2 = rec_s[2][jl];
-            const uint32_t w = __float_as_uint(r2.z), si = __float_as_uint(r2.w);
-            const int sidx = (int)(si & 0xFFFFu);
-            if (w == 0u) {
-                // A run of spans, in the lanes that hold them: every sample is
-                // covered, so inside the run the samples' adjoints are the run
-                // end's times the scalar pi (the product of 1 - a of the later
-                // spans), and the fill gradients need only the run's sums Lsum =
-                // sum lambda and Ksum = sum lambda * c_run (c before the span =
-                // ra * c_run + rb).
-                if (sidx != cur_slot) {
-                    if (cur_slot >= 0) {
+                for (int k = 0; k < SPT; ++k) cb[k] = tape[((size_t)slot * SPT + k) * 32];
+                if (ra >= 0.f) {  // (uniform) the run of spans that follows starts where the fragment ends
 #pragma unroll
-                        for (int k = 0; k < SPT; ++k)
-                            lam[k] = make_float4(lam[k].x * pi, lam[k].y * pi, lam[k].z * pi, lam[k].w * pi);
-                    }
-                    const size_t es = rbase + sidx;
-                    float4 ls = make_float4(0.f, 0.f, 0.f, 0.f), ks = ls;
+                    for (int k = 0; k < SPT; ++k) c[k] = cb[k];
+                    apply_fragment<S>(c, f, m, sub);
+                    float lk[8] = {};
 #pragma unroll
                     for (int k = 0; k < SPT; ++k) {
-                        const float4 cr = d.tape[(es * SPT + k) * 32 + lane];
-                        ls.x += lam[k].x;
-                        ls.y += lam[k].y;
-                        ls.z += lam[k].z;
-                        ls.w += lam[k].w;
-                        ks.x += lam[k].x * cr.x;
-                        ks.y += lam[k].y * cr.y;
-                        ks.z += lam[k].z * cr.z;
-                        ks.w += lam[k].w * cr.w;
+                        lk[0] += lam[k].x;
+                        lk[1] += lam[k].y;
+                        lk[2] += lam[k].z;
+                        lk[3] += lam[k].w;
+                        lk[4] += lam[k].x * c[k].x;
+                        lk[5] += lam[k].y * c[k].y;
+                        lk[6] += lam[k].z * c[k].z;
+                        lk[7] += lam[k].w * c[k].w;
+                        lam[k] = make_float4(lam[k].x * ra, lam[k].y * ra, lam[k].z * ra, lam[k].w * ra);
                     }
-                    float lk[8] = {ls.x, ls.y, ls.z, ls.w, ks.x, ks.y, ks.z, ks.w};
                     warp_sums<8>(lk, lane);
-                    Lsum = make_float4(lk[0], lk[1], lk[2], lk[3]);
-                    Ksum = make_float4(lk[4], lk[5], lk[6], lk[7]);
-                    cur_slot = sidx;
+                    if (lane == 0) {
+                        d.run_sum[2 * (size_t)p] = make_float4(lk[0], lk[1], lk[2], lk[3]);
+                        d.run_sum[2 * (size_t)p + 1] = make_float4(lk[4], lk[5], lk[6], lk[7]);
+                    }
+                }
+                float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
+                float J[SPT];
+#pragma unroll
+                for (int k = 0; k < SPT; ++k) {
+                    const float4 l = lam[k];
+                    J[k] = l.x * av * (f.x - cb[k].x) + l.y * av * (f.y - cb[k].y) + l.z * av * (f.z - cb[k].z) +
+                           l.w * av * (av - cb[k].w);
+                    if ((m >> (sub + 8 * k)) & 1u) {
+                        gf.x += l.x * av;
+                        gf.y += l.y * av;
+                        gf.z += l.z * av;
+                        gf.w += l.x * (f.x - cb[k].x) + l.y * (f.y - cb[k].y) + l.z * (f.z - cb[k].z) +
+                                l.w * (2.f * av - cb[k].w);
+                        lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
+                    }
+                }
+                group_adjoint<S>(a, d, (int64_t)it.y, a.fill_rule[it.w], J, lane);
+                add_fill_grad(d, it.w, warp_sum4(gf, lane), lane);
+                ra = next_ra;
+            }
+            if (base == cell.beg) break;
+        }
+        if (ra >= 0.f) {  // the first run
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < SPT; ++k) s = make_float4(s.x + lam[k].x, s.y + lam[k].y, s.z + lam[k].z, s.w + lam[k].w);
+            s = warp_sum4(s, lane);
+            if (lane == 0) d.cell_sum[cell.id] = s;
+        }
+    }
+}
+
+// Third pass of the adjoint: the spans' fill gradients, a lane per cell again.
+// The adjoint inside a run is its end's times pi, the product of 1 - alpha of
+// the run's later spans (found first, in reverse), so a span's gradient needs
+// only its run's sums (c before the span = ra * c_run + rb); it is summed over
+// the unit's cells before it goes to memory.
+__global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffArgs d) {
+    const int lane = threadIdx.x & 31;
+    const size_t wslot = (size_t)blockIdx.x * (kDiffThreads / 32) + (threadIdx.x >> 5);
+    float *const pis = d.run_pi + wslot * (size_t)d.pi_depth * 32 + lane;  // item i: [i * 32]
+    Unit u;
+    while (next_unit(a, d, lane, u)) {
+        if (u.fin == u.beg) continue;
+        if (u.fin - u.beg > (uint32_t)d.pi_depth) {
+            if (lane == 0) atomicOr(d.status, 2u);
+            continue;
+        }
+        const bool active = lane < u.cells;
+        const int x = u.x0 + 2 * lane;
+        float pi = 1.f;
+        bool frags = false;
+        for (uint32_t base = u.beg + ((u.fin - u.beg - 1) & ~31u);; base -= 32) {
+            const uint32_t mine = min(base + lane, u.fin - 1);
+            const uint32_t my_cols = item_cols(__ldg(&d.bitem[mine]));
+            const float my_a = __ldg(&d.bfill[mine].w);
+            for (int q = (int)min(u.fin - base, 32u) - 1; q >= 0; --q) {
+                const uint32_t cols = __shfl_sync(0xffffffffu, my_cols, q);
+                const float om = 1.f - __shfl_sync(0xffffffffu, my_a, q);
+                if (!active || !touches(cols, x)) continue;
+                if ((cols >> 16) == 0u) {
                     pi = 1.f;
-                }
-                // the run's records among the loaded ones: lanes [jl, jl + R)
-                const float4 rf = rec_s[0][lane], rbb = rec_s[1][lane], rr2 = rec_s[2][lane];
-                const uint32_t of_run = __ballot_sync(0xffffffffu, e_hi - lane >= 0 && __float_as_uint(rr2.z) == 0u &&
-                                                                       (int)(__float_as_uint(rr2.w) & 0xFFFFu) == sidx) >>
-                                         jl;
-                const int R = of_run == 0xFFFFFFFFu ? 32 : __ffs((int)~of_run) - 1;
-                const bool mine = lane >= jl && lane < jl + R;
-                float p = mine ? 1.f - rf.w : 1.f;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const float up = __shfl_up_sync(0xffffffffu, p, o);
-                    if (lane >= o) p *= up;
-                }
-                float pl = __shfl_up_sync(0xffffffffu, p, 1);
-                pl = lane == 0 ? pi : pi * pl;
-                const float av = rf.w, ra = rr2.x;
-                const float cx = ra * Ksum.x + rbb.x * Lsum.x, cy = ra * Ksum.y + rbb.y * Lsum.y;
-                const float cz = ra * Ksum.z + rbb.z * Lsum.z, cw = ra * Ksum.w + rbb.w * Lsum.w;
-                const float4 gf = make_float4(
-                    pl * av * Lsum.x, pl * av * Lsum.y, pl * av * Lsum.z,
-                    pl * (Lsum.x * rf.x - cx + Lsum.y * rf.y - cy + Lsum.z * rf.z - cz + 2.f * av * Lsum.w - cw));
-                if (mine && (gf.x != 0.f || gf.y != 0.f || gf.z != 0.f || gf.w != 0.f))
-                    add_fill_grad(d, acc, __float_as_uint(rr2.w) >> 16, __float_as_uint(rr2.y), gf);
-                __syncwarp();
-                pi *= __shfl_sync(0xffffffffu, p, 31);
-                e0 -= R;
-                continue;
-            }
-            --e0;
-            const float4 f = rec_s[0][jl], rb = rec_s[1][jl];
-            const uint32_t head = __float_as_uint(r2.x), path = __float_as_uint(r2.y);
-            const float av = f.w, om = 1.f - av;
-            // fragment: per-sample coverage; first close a pending run
-            if (cur_slot >= 0) {
-#pragma unroll
-                for (int k = 0; k < SPT; ++k)
-                    lam[k] = make_float4(lam[k].x * pi, lam[k].y * pi, lam[k].z * pi, lam[k].w * pi);
-                cur_slot = -1;
-            }
-            Lsum = Ksum = make_float4(0.f, 0.f, 0.f, 0.f);  // (of the closed run: not kept)
-            const uint32_t m = pixel_mask(make_uint4(__float_as_uint(rb.x), __float_as_uint(rb.y), __float_as_uint(rb.z),
-                                                     __float_as_uint(rb.w)),
-                                          S, k4);
-            const size_t es = rbase + sidx;
-            float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
-            float J[SPT];
-#pragma unroll
-            for (int k = 0; k < SPT; ++k) {
-                const float4 cb = d.tape[(es * SPT + k) * 32 + lane];
-                const float4 l = lam[k];
-                J[k] = l.x * av * (f.x - cb.x) + l.y * av * (f.y - cb.y) + l.z * av * (f.z - cb.z) +
-                       l.w * av * (av - cb.w);
-                if ((m >> (sub + 8 * k)) & 1u) {
-                    gf.x += l.x * av;
-                    gf.y += l.y * av;
-                    gf.z += l.z * av;
-                    gf.w += l.x * (f.x - cb.x) + l.y * (f.y - cb.y) + l.z * (f.z - cb.z) + l.w * (2.f * av - cb.w);
-                    lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
+                    frags = true;
+                } else {
+                    pis[(size_t)(base + q - u.beg) * 32] = pi;
+                    pi *= om;
                 }
             }
-            group_adjoint<S>(a, d, (int64_t)head, a.fill_rule[path], J, lane);
-            gf = warp_sum4(gf, lane);
-            if (lane == 0 && (gf.x != 0.f || gf.y != 0.f || gf.z != 0.f || gf.w != 0.f))
-                add_fill_grad(d, acc, si >> 16, path, gf);
-            __syncwarp();
+            if (base == u.beg) break;
+        }
+        // the sums of the cell's first run, whose samples start white (not
+        // used if that run is empty); of a cell without fragments: the pixels'
+        // adjoints
+        float4 Ls = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (frags) {
+            Ls = d.cell_sum[u.cell0 + lane];
+        } else if (active) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int X = x + (k >> 1), Y = u.y0 + (k & 1);
+                if (X < u.bs.W && Y < u.bs.H) {
+                    const float4 G = d.grad_image[u.bs.image_off + (int64_t)Y * u.bs.W + X];
+                    Ls = make_float4(Ls.x + G.x * d.out_scale, Ls.y + G.y * d.out_scale, Ls.z + G.z * d.out_scale,
+                                     Ls.w + G.w * d.out_scale);
+                }
+            }
+        }
+        float4 Ks = Ls;
+        Affine run{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        for (uint32_t base = u.beg; base < u.fin; base += 32) {
+            const uint32_t mine = min(base + lane, u.fin - 1);
+            const uint4 my_it = __ldg(&d.bitem[mine]);
+            const uint32_t my_cols = item_cols(my_it);
+            const float4 my_fill = __ldg(&d.bfill[mine]);
+            const int n = (int)min(u.fin - base, 32u);
+            for (int q = 0; q < n; ++q) {
+                const uint32_t cols = __shfl_sync(0xffffffffu, my_cols, q);
+                const bool touch = active && touches(cols, x);
+                const size_t p = base + q;
+                if ((cols >> 16) == 0u) {  // (uniform) a fragment
+                    if (touch) {           // (its sums are not used where no span follows)
+                        Ls = d.run_sum[2 * p];
+                        Ks = d.run_sum[2 * p + 1];
+                        run = Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+                    }
+                    continue;
+                }
+                if (!__any_sync(0xffffffffu, touch)) continue;
+                const float4 f = shfl_fill(my_fill, q);
+                float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (touch) {
+                    const float pl = pis[(p - u.beg) * 32], av = f.w;
+                    const float cx = run.a * Ks.x + run.b.x * Ls.x, cy = run.a * Ks.y + run.b.y * Ls.y;
+                    const float cz = run.a * Ks.z + run.b.z * Ls.z, cw = run.a * Ks.w + run.b.w * Ls.w;
+                    gf = make_float4(pl * av * Ls.x, pl * av * Ls.y, pl * av * Ls.z,
+                                     pl * (Ls.x * f.x - cx + Ls.y * f.y - cy + Ls.z * f.z - cz + 2.f * av * Ls.w - cw));
+                    add_span(run, f);
+                }
+                add_fill_grad(d, __shfl_sync(0xffffffffu, my_it.w, q), warp_sum4(gf, lane), lane);
+            }
         }
     }
 }
@@ -886,27 +942,32 @@ int diff_sm_count() {
     return n;
 }
 
-template <int S, bool BWD>
-void run_diff(const FrameArgs &a, const DiffArgs &d, unsigned grid, cudaStream_t s) {
-    // units of up to a bin's 32 cells, at least 4 for every warp
-    int shift = 5;
-    while (shift > 0 && (a.n_bins * (kTileW / 2) >> shift) < 4 * (int64_t)grid * (kDiffThreads / 32)) --shift;
-    k_diff<S, BWD><<<grid, kDiffThreads, 0, s>>>(a, d, shift);
-}
-
 template <bool BWD>
 int launch_diff(const FrameArgs &a, const DiffArgs &d, cudaStream_t s) {
     if (a.n_bins <= 0) return 0;
-    cudaMemsetAsync(d.queue, 0, sizeof(uint32_t), s);
+    cudaMemsetAsync(d.queue, 0, 3 * sizeof(uint32_t), s);  // (and the cell list's length and queue after it)
     const unsigned grid = (unsigned)diff_blocks(a);
-    int n = 1;
+    int n = 2;
     if (d.npairs > 0) {
         k_diff_gather<<<(unsigned)((d.npairs + 255) / 256), 256, 0, s>>>(d, a.S / 8);
         ++n;
     }
-    if (a.S == 8) run_diff<8, BWD>(a, d, grid, s);
-    else if (a.S == 16) run_diff<16, BWD>(a, d, grid, s);
-    else run_diff<32, BWD>(a, d, grid, s);
+    const unsigned bin_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((a.n_bins + 7) / 8, grid));
+    k_diff_runs<!BWD><<<bin_grid, kDiffThreads, 0, s>>>(a, d);
+    // (the forward has no tape of its own per warp: as many blocks as are resident)
+    const unsigned fwd_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(a.n_bins * 4, 5 * (int64_t)diff_sm_count()));
+    auto run = [&](auto fwd, auto bwd) {
+        if (BWD) bwd<<<grid, kDiffThreads, 0, s>>>(a, d);
+        else fwd<<<fwd_grid, kDiffThreads, 0, s>>>(a, d);
+    };
+    if (a.S == 8) run(k_diff_forward<8>, k_diff_backward<8>);
+    else if (a.S == 16) run(k_diff_forward<16>, k_diff_backward<16>);
+    else run(k_diff_forward<32>, k_diff_backward<32>);
+    if (BWD) {
+        cudaMemsetAsync(d.queue, 0, sizeof(uint32_t), s);
+        k_diff_spans<<<bin_grid, kDiffThreads, 0, s>>>(a, d);
+        ++n;
+    }
     if (BWD && d.nf > 0) {
         k_diff_chain<<<(unsigned)((d.nf + 255) / 256), 256, 0, s>>>(a, d);
         ++n;
@@ -926,9 +987,7 @@ int64_t diff_tape_words(const FrameArgs &a, int depth) {
     return diff_blocks(a) * (int64_t)depth * (a.S / 8) * kDiffThreads;
 }
 
-int64_t diff_tape_rec_words(const FrameArgs &a, int depth) {
-    return diff_blocks(a) * (int64_t)(kDiffThreads / 32) * depth * 3;
-}
+int64_t diff_pi_words(const FrameArgs &a, int depth) { return diff_blocks(a) * (int64_t)depth * kDiffThreads; }
 
 __global__ void k_accumulate(float *__restrict__ dst, const float *__restrict__ src, int64_t n, int first) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -50,7 +50,8 @@ struct FrameCounters {
     uint32_t need_pairs;   // resolve pairs of the frame
     uint32_t n_items;      // n_merged + n_span
     uint32_t tiles[3];     // look-back tile counters: entry offsets, scan-mark, pair offsets
-    uint32_t diff_status;  // differentiable frames: bit 0 tape too short
+    uint32_t diff_queue[3];  // differentiable frames: DiffArgs::queue
+    uint32_t diff_status;  // differentiable frames: DiffArgs::status
     uint32_t n_seg[3], q_seg[3];  // segment sort: listed segments by size class, and those taken
     uint32_t longest;            // entries of the longest path (sized frames)
     uint32_t pairs_alt;          // resolve pairs in the other built-in tile (FrameArgs::alt_shift)
@@ -296,11 +297,24 @@ struct DiffArgs {
     const int2 *entries;
     const float2 *tvert;
     int64_t nf;
-    float4 *tape;      // per block: tape_depth x (samples per thread) x block threads (sample states)
-    float4 *tape_rec;  // per block: warps x tape_depth x 3 (per-cell item records)
-    int tape_depth;
-    uint32_t *queue;     // bin queue (zeroed by the launchers)
-    uint32_t *status;    // bit 0: a tape overflowed (rerun with a deeper tape)
+    // per resolve pair that is a fragment: the affine map of the spans before it
+    // in its cell (c -> run_a c + run_b; run_a < 0: none) and, backward, the sums
+    // of the run after it (2 per pair)
+    float *run_a;
+    float4 *run_b, *run_sum;
+    // the cells with fragments (numbers bin * 32 + column), and per cell number
+    // the map of its last run (as run_a, run_b) and the adjoint sum of its first
+    uint32_t *cell;
+    float *cell_a;
+    float4 *cell_b, *cell_sum;
+    // per warp: tape_depth x (samples per thread) x 32 sample states, and pi_depth
+    // x 32 span factors (backward)
+    float4 *tape;
+    float *run_pi;
+    int tape_depth, pi_depth;
+    uint32_t *queue;     // unit queue; then the cell list's length and its queue (zeroed by the launchers)
+    uint32_t *n_cells, *cell_queue;
+    uint32_t *status;    // bit 0: a cell has more fragments than tape_depth, bit 1: a bin more items than pi_depth (rerun with more)
     // pixel = out_scale * (mean of the samples), added to the image when
     // accumulate (the passes of a 256-sample frame: 1/8 each); the backward
     // takes out_scale * dL/d(pixel) likewise
@@ -309,7 +323,7 @@ struct DiffArgs {
 };
 int64_t diff_blocks(const FrameArgs &a);
 int64_t diff_tape_words(const FrameArgs &a, int depth);      // float4 count of the sample-state tape
-int64_t diff_tape_rec_words(const FrameArgs &a, int depth);  // float4 count of the item records
+int64_t diff_pi_words(const FrameArgs &a, int depth);        // float count of the span factors
 int launch_diff_forward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 int launch_diff_backward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 // dL/d(stored vertex in transformed space) -> dL/d(input vertex), dL/d(path affine).
