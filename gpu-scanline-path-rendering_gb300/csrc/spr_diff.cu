@@ -571,8 +571,9 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArg
 }
 
 // A cell of the second pass: warp = cell, lane l = pixel k4 = l >> 3 of the cell
-// (k4 = px * 2 + py), samples (l & 7) + 8k.  Warps take kCellBatch cells at a
-// time from the list.
+// (k4 = px * 2 + py), samples (l & 7) + 8k.  Warps take up to kCellBatch cells
+// at a time from the list, fewer as long as every warp would get less than two
+// such lots.
 constexpr uint32_t kCellBatch = 8;
 struct Cell {
     uint32_t id, beg, fin;
@@ -584,11 +585,12 @@ struct Cell {
 };
 __device__ __forceinline__ bool next_cell(const FrameArgs &a, const DiffArgs &d, uint32_t n_cells, int lane, Cell &c) {
     if (c.next == c.end) {
+        const uint32_t lot = min(max(n_cells / (2u * gridDim.x * (kDiffThreads / 32)), 1u), kCellBatch);
         uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(d.cell_queue, kCellBatch);
+        if (lane == 0) k = atomicAdd(d.cell_queue, lot);
         c.next = __shfl_sync(0xffffffffu, k, 0);
         if (c.next >= n_cells) return false;
-        c.end = min(c.next + kCellBatch, n_cells);
+        c.end = min(c.next + lot, n_cells);
     }
     const uint32_t id = d.cell[c.next++], b = id / (kTileW / 2);
     if (c.id / (kTileW / 2) != b) {  // (a bin's cells are listed together)
@@ -834,30 +836,41 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
             const uint32_t my_cols = item_cols(my_it);
             const float4 my_fill = __ldg(&d.bfill[mine]);
             const int n = (int)min(u.fin - base, 32u);
-            for (int q = 0; q < n; ++q) {
-                const uint32_t cols = __shfl_sync(0xffffffffu, my_cols, q);
-                const bool touch = active && touches(cols, x);
-                const size_t p = base + q;
-                if ((cols >> 16) == 0u) {  // (uniform) a fragment
-                    if (touch) {           // (its sums are not used where no span follows)
-                        Ls = d.run_sum[2 * p];
-                        Ks = d.run_sum[2 * p + 1];
-                        run = Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+            for (int q0 = 0; q0 < n; q0 += 8) {  // 8 items' gradients of this cell, then summed over the cells together
+                float v[32];
+                bool any = false;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int q = q0 + j;
+                    const uint32_t cols = __shfl_sync(0xffffffffu, my_cols, q);
+                    const bool touch = active && q < n && touches(cols, x);
+                    const size_t p = base + q;
+                    v[4 * j] = v[4 * j + 1] = v[4 * j + 2] = v[4 * j + 3] = 0.f;
+                    if ((cols >> 16) == 0u) {  // (uniform) a fragment
+                        if (touch) {           // (its sums are not used where no span follows)
+                            Ls = d.run_sum[2 * p];
+                            Ks = d.run_sum[2 * p + 1];
+                            run = Affine{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+                        }
+                        continue;
                     }
-                    continue;
+                    const float4 f = shfl_fill(my_fill, q);
+                    if (touch) {
+                        any = true;
+                        const float pl = pis[(p - u.beg) * 32], av = f.w;
+                        const float cx = run.a * Ks.x + run.b.x * Ls.x, cy = run.a * Ks.y + run.b.y * Ls.y;
+                        const float cz = run.a * Ks.z + run.b.z * Ls.z, cw = run.a * Ks.w + run.b.w * Ls.w;
+                        v[4 * j] = pl * av * Ls.x;
+                        v[4 * j + 1] = pl * av * Ls.y;
+                        v[4 * j + 2] = pl * av * Ls.z;
+                        v[4 * j + 3] = pl * (Ls.x * f.x - cx + Ls.y * f.y - cy + Ls.z * f.z - cz + 2.f * av * Ls.w - cw);
+                        add_span(run, f);
+                    }
                 }
-                if (!__any_sync(0xffffffffu, touch)) continue;
-                const float4 f = shfl_fill(my_fill, q);
-                float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (touch) {
-                    const float pl = pis[(p - u.beg) * 32], av = f.w;
-                    const float cx = run.a * Ks.x + run.b.x * Ls.x, cy = run.a * Ks.y + run.b.y * Ls.y;
-                    const float cz = run.a * Ks.z + run.b.z * Ls.z, cw = run.a * Ks.w + run.b.w * Ls.w;
-                    gf = make_float4(pl * av * Ls.x, pl * av * Ls.y, pl * av * Ls.z,
-                                     pl * (Ls.x * f.x - cx + Ls.y * f.y - cy + Ls.z * f.z - cz + 2.f * av * Ls.w - cw));
-                    add_span(run, f);
-                }
-                add_fill_grad(d, __shfl_sync(0xffffffffu, my_it.w, q), warp_sum4(gf, lane), lane);
+                if (!__any_sync(0xffffffffu, any)) continue;
+                reduce_scatter<16, 16, 32>(v, lane);  // lane i: the sum of value i
+                const uint32_t path = __shfl_sync(0xffffffffu, my_it.w, min(q0 + (lane >> 2), 31));
+                if (v[0] != 0.f) atomicAdd(reinterpret_cast<float *>(d.grad_fill + path) + (lane & 3), v[0]);
             }
         }
     }
