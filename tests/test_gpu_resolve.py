@@ -57,3 +57,16 @@ def test_paints_between_solid_fills(samples, ms):
     scene.path_fill_rgba[::2] = 1 + np.arange(25) % 3
     scene.gradients = (table.reshape(-1), ramp)
     check(scene, 36, 26, samples=samples, ms_output=ms)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 1024, 1025, 1500])
+def test_items_per_bin(n):
+    # n paths, each a triangle inside the one cell of the viewport: n items in
+    # one bin, whose order decides the colours
+    rng = np.random.default_rng(n)
+    tri = rng.uniform(0.05, 1.95, (n, 3, 2))
+    pts = tri[:, [0, 1, 1, 2, 2, 0]].reshape(-1, 2)
+    pid = np.repeat(np.arange(n), 3)
+    scene = spr.Scene(pts, np.repeat(pid, 2), 2 * np.arange(3 * n), np.full(3 * n, spr.CURVE_LINEAR), pid,
+                      np.zeros(3 * n), np.zeros(n), rng.integers(0x10000000, 1 << 32, n).astype(np.uint32))
+    check(scene, 2, 2, samples=32)
