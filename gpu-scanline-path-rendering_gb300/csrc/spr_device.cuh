@@ -92,7 +92,7 @@ __device__ __forceinline__ void solve_quad_eq(float a, float b, float c, float *
         return;
     }
     float A = a;
-    float B = (float)((double)b * 0.5);
+    float B = b * 0.5f;
     float C = c;
     float tx, ty;
     float R = B * B - A * C;
@@ -277,33 +277,56 @@ __device__ __forceinline__ int monotonize_r(const CurveGeom &g, bool visible, fl
     return n + 1;
 }
 
-// Crossing of coordinate P(t) = c on [tmin, tmax].
+// Crossing of coordinate P(t) = c on [tmin, tmax].  AHEAD: a bisection's two
+// next midpoints are evaluated along with the current one, two steps at a time
+// (half the serial chain for half as many evaluations again).
+template <bool AHEAD>
 __device__ __forceinline__ float solve_crossing(int type, float w, const float *P, float c, float tmin, float tmax) {
     if (type == kLinear) {
         float t = (c - P[0]) * safe_rcp(P[1] - P[0]);
         t = t > tmin ? t : tmin;
         return t < tmax ? t : tmax;
     }
-    if (type == kQuad) return solve_quad_bezier(P[0], P[1], P[2], c, tmin, tmax);
-    if (type == kRational) return solve_quad_bezier(P[0] - c, (P[1] - c) * w, P[2] - c, 0.f, tmin, tmax);
-    // 24 bisection steps.  The sign of the coordinate's offset from c at the
-    // bracket's start never changes (a step replaces the start only by a point
-    // of the same sign), so it is taken once; both next midpoints are formed
-    // while the point is evaluated, which takes them off the serial chain.
+    if (type != kCubic) {
+        const bool q = type == kQuad;
+        return solve_quad_bezier(q ? P[0] : P[0] - c, q ? P[1] : (P[1] - c) * w, q ? P[2] : P[2] - c, q ? c : 0.f,
+                                 tmin, tmax);
+    }
+    // 24 bisection steps.  The side of c on which the bracket's start lies
+    // never changes (a step replaces the start only by a point of the same
+    // side), so it is taken once; the next midpoints are formed while a point
+    // is evaluated, which takes them off the serial chain.
     float t0 = tmin, t1 = tmax;
     const float vt0 = cubic_coord(P, t0);
     if (vt0 == c) return t0;
-    const bool s0 = (int32_t)fbits(vt0 - c) < 0;
+    const bool s0 = vt0 < c;
     float tm = (t0 + t1) * .5f, ts = tm, last = 0.f;
+    if constexpr (AHEAD) {
+#pragma unroll 2
+        for (int it = 0; it < 12; ++it) {
+            const float ta = (tm + t1) * .5f, tb = (t0 + tm) * .5f;
+            const float taa = (ta + t1) * .5f, tab = (tm + ta) * .5f, tba = (tb + tm) * .5f, tbb = (t0 + tb) * .5f;
+            const float fm = cubic_coord(P, tm), fa = cubic_coord(P, ta), fb = cubic_coord(P, tb);
+            const bool up = (fm < c) == s0, ua = (fa < c) == s0, ub = (fb < c) == s0;
+            const bool up2 = up ? ua : ub;
+            ts = up ? ta : tb;
+            last = up ? fa : fb;
+            const float m0 = up ? tm : t0, m1 = up ? t1 : tm;
+            t0 = up2 ? ts : m0;
+            t1 = up2 ? m1 : ts;
+            tm = up ? (ua ? taa : tab) : (ub ? tba : tbb);
+        }
+    } else {
 #pragma unroll 4
-    for (int it = 0; it < 24; ++it) {
-        ts = tm;
-        last = cubic_coord(P, tm);
-        const float ta = (tm + t1) * .5f, tb = (t0 + tm) * .5f;
-        const bool same = ((int32_t)fbits(last - c) < 0) == s0;
-        t0 = same ? tm : t0;
-        t1 = same ? t1 : tm;
-        tm = same ? ta : tb;
+        for (int it = 0; it < 24; ++it) {
+            ts = tm;
+            last = cubic_coord(P, tm);
+            const float ta = (tm + t1) * .5f, tb = (t0 + tm) * .5f;
+            const bool same = (last < c) == s0;
+            t0 = same ? tm : t0;
+            t1 = same ? t1 : tm;
+            tm = same ? ta : tb;
+        }
     }
     if (fabsf(last - c) > 1.f) ts = tmin;
     return ts;

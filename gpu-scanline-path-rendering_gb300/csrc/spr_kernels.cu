@@ -202,6 +202,7 @@ constexpr int kEmitCurves = 128;   // curves of a block, at most
 constexpr int kEmitLocal = 4096;   // crossings of a block's curves held in shared memory (else in global scratch)
 constexpr int kMergeSerial = 24;   // entries of a piece merged by one lane (longer pieces: by a warp)
 constexpr int kChainClasses = 24;  // solver (cubic, quadratic, line) x length octave
+constexpr uint32_t kNoChain = 0xFFFFu;
 
 // A block's curves, their monotone pieces' end parameters (flags in the low
 // bits), the pieces' first entries within the curve, and per piece and
@@ -214,7 +215,7 @@ struct EmitBlock {
     uint32_t off[kEmitCurves];  // the curve's first entry
     uint32_t tof[kEmitCurves];  // its first solved parameter
     uint32_t cls[32], warp_pieces[8], warp_entries[8], next_chain;
-    uint16_t item[2 * 5 * kEmitCurves];  // chains in the order they are solved: curve | piece << 7 | direction << 10
+    uint16_t item[2 * 5 * kEmitCurves + 64];  // chains in the order they are solved: curve | piece << 7 | direction << 10
     uint16_t piece[5 * kEmitCurves];     // the pieces: curve | piece << 7
     float t[kEmitLocal];
 };
@@ -321,16 +322,22 @@ __device__ __forceinline__ void merge_piece_warp(const float *X, int nx, const f
 // above), and every chain is one work item of a lane: the longest serial
 // sequence is the crossings of one curve with the lines of one direction.
 // The block's chains are solved grouped by solver (cubics, whose crossings are
-// bisections, first) and by decreasing length, a lane whose chain is done
-// taking the block's next one, so that the lanes of a warp run the same solver
-// and stay busy until the list runs out.  Then the pieces are merged, short
-// ones one per lane and long ones by a warp.  Bound by the latency of a
-// chain's bisections (about 0.9 us a crossing) where curves are few and by
-// issue (420 thread instructions an entry, 19 lanes active) where they are
-// many.  With one lane solving both directions of a piece, 32 curves to a
-// warp in a device-wide order by type and length, emission + fragments took
-// 620 us on 64 paths over 512 x 512, 533 us on 2,500 paths over 1917 x 1079
-// and 787 us on the 20,000-path 2048 x 2048 scene; here 304, 280 and 783.
+// bisections, first; each solver from a multiple of 32 on, so that the first
+// chains of a warp are of one solver) and by decreasing length, a lane whose
+// chain is done taking the block's next one, so that the lanes of a warp run the
+// same solver and stay busy until the list runs out.  Then the pieces are merged,
+// short ones one per lane and long ones by a warp.  Bound by the latency of a
+// chain's bisections (about 0.7 us a crossing) where curves are few and by
+// issue (400 thread instructions an entry, 19 lanes active) where they are
+// many.  Emission + fragments of 64 paths over 512 x 512, 2,500 paths over
+// 1917 x 1079, 20,000 paths over 2048 x 2048 and a batch of 48 scenes, us:
+//   620  533  787  2510  one lane per piece, 32 curves to a warp, ordered by
+//                        type and length over the whole frame
+//   304  282  783  2550  a lane per chain, solvers one after the other
+//   253  280  777  2580  each solver's chains in warps of their own
+//   234  280  759  2450  one comparison instead of a difference's sign
+//   216  272  760  2450  AHEAD for few curves
+template <bool AHEAD>
 __global__ void __launch_bounds__(kEmitThreads)
     k_curve_emit(FrameArgs a, int per_block, const float2 *__restrict__ tv, const uint8_t *__restrict__ vis,
                  const uint32_t *__restrict__ offsets, const uint32_t *__restrict__ order, float *scratch,
@@ -409,9 +416,16 @@ __global__ void __launch_bounds__(kEmitThreads)
         const uint32_t v = __shfl_up_sync(0xffffffffu, cls, o);
         if (lane >= o) cls += v;
     }
-    const uint32_t n_chains = __shfl_sync(0xffffffffu, cls, 31);
+    // each solver's chains from a multiple of 32 on, with places left empty
+    const uint32_t n_cubic = __shfl_sync(0xffffffffu, cls, 7), n_quad = __shfl_sync(0xffffffffu, cls, 15) - n_cubic;
+    const uint32_t quad0 = (n_cubic + 31u) & ~31u, line0 = (quad0 + n_quad + 31u) & ~31u;
+    const uint32_t n_chains = line0 + __shfl_sync(0xffffffffu, cls, 31) - n_cubic - n_quad;
     __syncthreads();
-    if (warp == 0) S.cls[lane] = cls - cls_n;
+    if (warp == 0) {
+        S.cls[lane] = cls - cls_n + (lane < 8 ? 0u : (lane < 16 ? quad0 - n_cubic : line0 - n_cubic - n_quad));
+        if (n_cubic + lane < quad0) S.item[n_cubic + lane] = kNoChain;
+        if (quad0 + n_quad + lane < line0) S.item[quad0 + n_quad + lane] = kNoChain;
+    }
     __syncthreads();
     if (np > 0) {
         S.tof[tid] = local ? lpre : S.off[tid];
@@ -440,8 +454,8 @@ __global__ void __launch_bounds__(kEmitThreads)
                 next = __shfl_sync(0xffffffffu, next, 0);
                 more = next + __popc(want) < n_chains;
                 const uint32_t k = next + __popc(want & ((1u << lane) - 1u));
-                if (rem == 0 && k < n_chains) {
-                    const uint32_t it = S.item[k];
+                const uint32_t it = rem == 0 && k < n_chains ? S.item[k] : kNoChain;
+                if (it != kNoChain) {
                     const int L = (int)(it & 127u), ms = (int)(it >> 7) & 7;
                     ax = (int)(it >> 10);
                     ctype = (int)S.type[L];
@@ -459,7 +473,7 @@ __global__ void __launch_bounds__(kEmitThreads)
             }
             if (!__any_sync(0xffffffffu, rem > 0)) break;
             if (rem > 0) {
-                t = ffrom((fbits(solve_crossing(ctype, w, P, c, t, t1)) & 0xFFFFFFFCu) | (uint32_t)ax);
+                t = ffrom((fbits(solve_crossing<AHEAD>(ctype, w, P, c, t, t1)) & 0xFFFFFFFCu) | (uint32_t)ax);
                 *out++ = t;
                 c += dc;
                 --rem;
@@ -2253,7 +2267,7 @@ int launch_transform(const FrameArgs &a, float2 *tvert, uint32_t *path_flags, cu
 // Curves a block of k_curve_emit takes: about 5 blocks per SM, so that few
 // curves still reach every SM, up to the 128 that a block holds, which pack
 // their chains best.  Emission + fragments of the measured scenes, us at
-// 8 / 32 / 128 curves: 1,378 curves 304 / 309 / 395, 24 k 288 / 167 / 169,
+// 8 / 32 / 128 curves (solvers still in one list): 1,378 curves 304 / 309 / 395, 24 k 288 / 167 / 169,
 // 158 k 386 / 167 / 118, 1.74 M 3972 / 1488 / 783.
 static int emit_curves(int C) {
     int n = 8;
@@ -2279,8 +2293,12 @@ int launch_curve_emit(const FrameArgs &a, const float2 *tvert, const uint8_t *vi
                        cudaStream_t s) {
     if (a.C <= 0) return 0;
     const int per_block = emit_curves(a.C);
-    k_curve_emit<<<grid_for(a.C, per_block), kEmitThreads, 0, s>>>(a, per_block, tvert, vis, offsets, order, scratch,
-                                                                   entries, cap32(cap_nf), ctr);
+    // few curves leave issue slots idle, which two bisection steps at a time use;
+    // with more of them they only cost (1,378 curves 234 -> 216 us, but 24 k
+    // 280 -> 288 and 1.74 M 759 -> 859)
+    const auto kernel = per_block <= 8 ? k_curve_emit<true> : k_curve_emit<false>;
+    kernel<<<grid_for(a.C, per_block), kEmitThreads, 0, s>>>(a, per_block, tvert, vis, offsets, order, scratch, entries,
+                                                             cap32(cap_nf), ctr);
     return 1;
 }
 

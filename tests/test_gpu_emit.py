@@ -46,6 +46,16 @@ def test_curve_counts_around_block_sizes(n):
     check_entries(scene_of(curves_of(n, size, size, n)), size, size)
 
 
+@pytest.mark.parametrize("kinds", range(1, 16))
+def test_mixes_of_solvers(kinds):
+    # every set of curve types: a block's lists of the three solvers empty,
+    # partly filled and longer than a warp
+    for n in (8, 64, 400):
+        mix = [c for c in curves_of(4 * n, 120, 90, 100 * n + kinds)
+               if kinds >> [spr.CURVE_LINEAR, spr.CURVE_QUADRATIC, spr.CURVE_CUBIC, spr.CURVE_RATIONAL].index(c[0]) & 1]
+        check_entries(scene_of(mix[:n]), 120, 90)
+
+
 @pytest.mark.parametrize("W,H", [(4096, 64), (64, 4096), (4095, 4093)])
 def test_long_pieces_and_spilled_blocks(W, H):
     # (40 curves of thousands of crossings to a block: past its shared-memory buffer)
