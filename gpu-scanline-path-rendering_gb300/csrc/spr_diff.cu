@@ -132,11 +132,11 @@ __device__ __forceinline__ void load_curve(const CurveDesc &d, const float2 *__r
     }
 }
 
-// Warp sums of N values (N = 2, 4, 8), returned to every lane: a
-// reduce-scatter in which a lane keeps, at the exchange across lane bit O, the
-// half of its partial sums that its side owns (M values), then plain
-// butterflies over the remaining lane bits and one broadcast per value; value
-// i ends in lane i * 32 / N.  2N + 4 - log2(N) shuffles instead of 5N.
+// Warp sums of N values (a power of two): a reduce-scatter in which a lane
+// keeps, at the exchange across lane bit O, the half of its partial sums that
+// its side owns (M values), then plain butterflies over the remaining lane
+// bits; value i ends in lane i * 32 / N, which stores it: there is no
+// broadcast.  N + 4 - log2(N) shuffles instead of 5N.
 template <int M, int O, int N>
 __device__ __forceinline__ void reduce_scatter(float (&t)[N], int lane) {
     if constexpr (M >= 1) {
@@ -154,20 +154,11 @@ __device__ __forceinline__ void reduce_scatter(float (&t)[N], int lane) {
     }
 }
 
+// Sum i of v over the warp, in the N lanes i * 32 / N (other lanes: no meaning).
 template <int N>
-__device__ __forceinline__ void warp_sums(float (&v)[N], int lane) {
-    float t[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) t[i] = v[i];
-    reduce_scatter<N / 2, 16, N>(t, lane);
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = __shfl_sync(0xffffffffu, t[0], i * (32 / N));
-}
-
-__device__ __forceinline__ float4 warp_sum4(float4 x, int lane) {
-    float v[4] = {x.x, x.y, x.z, x.w};
-    warp_sums<4>(v, lane);
-    return make_float4(v[0], v[1], v[2], v[3]);
+__device__ __forceinline__ float scattered_sums(float (&v)[N], int lane) {
+    reduce_scatter<N / 2, 16, N>(v, lane);
+    return v[0];
 }
 
 // One fragment of a merged group, held by one lane of the cell's warp.
@@ -192,6 +183,19 @@ __device__ __forceinline__ void load_group_frag(const DiffArgs &d, uint32_t raw,
         f.lm[w] = d.lmask[(size_t)raw * WORDS + w];
     }
     f.q = make_float4(c.x, c.y, c.w != c.y ? (c.z - c.x) / (c.w - c.y) : 0.f, c.w);
+}
+
+// What a warp reads of a merged group before its fragments: the winding before it,
+// and lane l's entry and key of sorted position h + l.
+struct GroupHead {
+    int w0;
+    uint32_t raw;
+    uint64_t key;  // (no key past the last position)
+};
+__device__ __forceinline__ GroupHead group_head(const DiffArgs &d, int64_t h, int lane) {
+    const bool in = h + lane < d.nf;
+    return GroupHead{(int)__ldg(&d.wn_scan[h]), in ? __ldg(&d.perm[h + lane]) : 0u,
+                     in ? __ldg(&d.skey[h + lane]) & kKeyMask : ~0ull};
 }
 
 // Chain of one fragment's crossings to its curve's control points: the
@@ -230,21 +234,23 @@ __device__ void fragment_chain(const FrameArgs &a, const DiffArgs &d, uint32_t r
 // shuffle is executed by the whole warp.  Every fragment is in one group, so
 // its sums have a place of their own (d.chain).
 template <int S>
-__device__ __forceinline__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, int rule, const float *J, int lane) {
+__device__ __forceinline__ void group_adjoint(const FrameArgs &a, const DiffArgs &d, int64_t h, const GroupHead &head,
+                                              int rule, const float *J, int lane) {
     constexpr int SPT = S / 8, ROWS = 2 * S, RPL = (ROWS + 31) / 32;
-    const int w0 = (int)d.wn_scan[h];
-    // the first 32 fragments, and the group's size: the run of equal keys from h
-    const uint64_t kh = d.skey[h] & kKeyMask;
-    uint32_t raw = h + lane < d.nf ? d.perm[h + lane] : 0u;
+    const int w0 = head.w0;
+    uint32_t raw = head.raw;
+    // the group's size: the run of equal keys from h
+    const uint64_t kh = __shfl_sync(0xffffffffu, head.key, 0);
+    uint64_t key = head.key;
     int gs = 0;
     for (;;) {
-        const int64_t j = h + gs + lane;
-        const uint32_t ends = __ballot_sync(0xffffffffu, j >= d.nf || (d.skey[j] & kKeyMask) != kh);
+        const uint32_t ends = __ballot_sync(0xffffffffu, key != kh);
         if (ends) {
             gs += __ffs(ends) - 1;
             break;
         }
         gs += 32;
+        key = h + gs + lane < d.nf ? d.skey[h + gs + lane] & kKeyMask : ~0ull;
     }
     float yr[RPL];
 #pragma unroll
@@ -333,8 +339,9 @@ __device__ __forceinline__ void group_adjoint(const FrameArgs &a, const DiffArgs
                 sAB[0] += g * (1.f - lam);
                 sAB[1] += g * lam;
             }
-            warp_sums<2>(sAB, lane);
-            if (lane == j) d.chain[mine.raw] = make_float2(sAB[0], sAB[1]);
+            const float sum = scattered_sums<2>(sAB, lane);
+            const uint32_t to = __shfl_sync(0xffffffffu, mine.raw, j);
+            if ((lane & 15) == 0) reinterpret_cast<float *>(d.chain + to)[lane >> 4] = sum;
         }
     }
 }
@@ -653,12 +660,6 @@ __global__ void __launch_bounds__(kDiffThreads, 5) k_diff_forward(FrameArgs a, D
     }
 }
 
-// Adds a fill gradient that all lanes hold: one component per lane.
-__device__ __forceinline__ void add_fill_grad(const DiffArgs &d, uint32_t path, const float4 &g, int lane) {
-    const float v = lane == 0 ? g.x : (lane == 1 ? g.y : (lane == 2 ? g.z : g.w));
-    if (lane < 4 && v != 0.f) atomicAdd(reinterpret_cast<float *>(d.grad_fill + path) + lane, v);
-}
-
 // The adjoint of the cells with fragments: forward through the fragments, the
 // samples' states before each to the tape, and in reverse with the samples'
 // adjoints lambda, which gives the fragments' gradients and for every run of
@@ -713,6 +714,8 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
                 const float4 f = __ldg(&d.bfill[p]);
                 const float next_ra = d.run_a[p];
                 const uint32_t m = pixel_mask(__ldg(&d.bmm[p]), S, k4);
+                // (the group's, on their way while the samples are worked on)
+                const GroupHead head = group_head(d, (int64_t)it.y, lane);
                 const float av = f.w, om = 1.f - av;
                 --slot;
                 float4 cb[SPT];
@@ -735,13 +738,10 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
                         lk[7] += lam[k].w * c[k].w;
                         lam[k] = make_float4(lam[k].x * ra, lam[k].y * ra, lam[k].z * ra, lam[k].w * ra);
                     }
-                    warp_sums<8>(lk, lane);
-                    if (lane == 0) {
-                        d.run_sum[2 * (size_t)p] = make_float4(lk[0], lk[1], lk[2], lk[3]);
-                        d.run_sum[2 * (size_t)p + 1] = make_float4(lk[4], lk[5], lk[6], lk[7]);
-                    }
+                    const float sum = scattered_sums<8>(lk, lane);
+                    if ((lane & 3) == 0) reinterpret_cast<float *>(d.run_sum + 2 * (size_t)p)[lane >> 2] = sum;
                 }
-                float4 gf = make_float4(0.f, 0.f, 0.f, 0.f);
+                float gf[4] = {0.f, 0.f, 0.f, 0.f};
                 float J[SPT];
 #pragma unroll
                 for (int k = 0; k < SPT; ++k) {
@@ -749,26 +749,33 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
                     J[k] = l.x * av * (f.x - cb[k].x) + l.y * av * (f.y - cb[k].y) + l.z * av * (f.z - cb[k].z) +
                            l.w * av * (av - cb[k].w);
                     if ((m >> (sub + 8 * k)) & 1u) {
-                        gf.x += l.x * av;
-                        gf.y += l.y * av;
-                        gf.z += l.z * av;
-                        gf.w += l.x * (f.x - cb[k].x) + l.y * (f.y - cb[k].y) + l.z * (f.z - cb[k].z) +
+                        gf[0] += l.x * av;
+                        gf[1] += l.y * av;
+                        gf[2] += l.z * av;
+                        gf[3] += l.x * (f.x - cb[k].x) + l.y * (f.y - cb[k].y) + l.z * (f.z - cb[k].z) +
                                 l.w * (2.f * av - cb[k].w);
                         lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
                     }
                 }
-                group_adjoint<S>(a, d, (int64_t)it.y, a.fill_rule[it.w], J, lane);
-                add_fill_grad(d, it.w, warp_sum4(gf, lane), lane);
+                group_adjoint<S>(a, d, (int64_t)it.y, head, a.fill_rule[it.w], J, lane);
+                const float sum = scattered_sums<4>(gf, lane);
+                if ((lane & 7) == 0 && sum != 0.f)
+                    atomicAdd(reinterpret_cast<float *>(d.grad_fill + it.w) + (lane >> 3), sum);
                 ra = next_ra;
             }
             if (base == cell.beg) break;
         }
         if (ra >= 0.f) {  // the first run
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int k = 0; k < SPT; ++k) s = make_float4(s.x + lam[k].x, s.y + lam[k].y, s.z + lam[k].z, s.w + lam[k].w);
-            s = warp_sum4(s, lane);
-            if (lane == 0) d.cell_sum[cell.id] = s;
+            for (int k = 0; k < SPT; ++k) {
+                s[0] += lam[k].x;
+                s[1] += lam[k].y;
+                s[2] += lam[k].z;
+                s[3] += lam[k].w;
+            }
+            const float sum = scattered_sums<4>(s, lane);
+            if ((lane & 7) == 0) reinterpret_cast<float *>(d.cell_sum + cell.id)[lane >> 3] = sum;
         }
     }
 }
