@@ -664,11 +664,13 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.bitem = h->bitems.as<uint4>();
         d.bfill = reinterpret_cast<float4 *>(d.bitem + d.npairs);
         d.bmm = d.bitem + 2 * d.npairs;
-        // the runs' maps, and after them (backward) their sums
-        if ((st = ensure(h->bruns, (dc.backward ? 52 : 20) * (size_t)d.npairs))) return st;
+        // the runs' maps, after them (backward) their sums, and the links
+        if ((st = ensure(h->bruns, (dc.backward ? 60 : 24) * (size_t)d.npairs))) return st;
         d.run_b = h->bruns.as<float4>();
         d.run_sum = d.run_b + d.npairs;
         d.run_a = reinterpret_cast<float *>(d.run_b + (dc.backward ? 3 : 1) * d.npairs);
+        d.run_next = reinterpret_cast<uint32_t *>(d.run_a + d.npairs);
+        d.run_prev = dc.backward ? d.run_next + d.npairs : nullptr;
     }
     d.chord = h->chord.as<float4>();
     d.lmask = h->lmask.as<uint32_t>();
@@ -686,14 +688,15 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
     d.queue = ctr->diff_queue;
     d.n_cells = d.queue + 1;
     d.cell_queue = d.queue + 2;
-    // per cell of the bins: its place in the list, the run map and the adjoint sum
+    // per cell of the bins: its place in the list, the run map, the adjoint sum and the first and last fragments
     const int64_t cells = a.n_bins * 32;
     {
-        int st = ensure(h->dcells, 40 * (size_t)std::max<int64_t>(cells, 1));
+        int st = ensure(h->dcells, 48 * (size_t)std::max<int64_t>(cells, 1));
         if (st) return st;
         d.cell_b = h->dcells.as<float4>();
         d.cell_sum = d.cell_b + cells;
-        d.cell_a = reinterpret_cast<float *>(d.cell_sum + cells);
+        d.cell_ends = reinterpret_cast<uint2 *>(d.cell_sum + cells);
+        d.cell_a = reinterpret_cast<float *>(d.cell_ends + cells);
         d.cell = reinterpret_cast<uint32_t *>(d.cell_a + cells);
     }
     d.status = &ctr->diff_status;

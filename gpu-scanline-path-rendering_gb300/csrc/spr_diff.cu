@@ -469,13 +469,17 @@ constexpr float kNoSpans = -1.f;  // in place of a run's factor: the run holds n
 // First pass over a unit's items, a lane per cell (at column x).  A span covers
 // every sample of a cell, so the spans between two fragments of a cell are one
 // affine map of its samples' state: the map before each fragment goes to
-// d.run_b / d.run_a at the fragment's place (a fragment is in one cell), the
-// map after the last one is returned (a = kNoSpans: no spans).
-__device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, int &n_frags) {
+// d.run_b / d.run_a at the fragment's place (a fragment is in one cell), with
+// the places of the cell's next and (backward) previous fragments, the map after
+// the last one is returned (a = kNoSpans: no spans).  ends: the cell's first and
+// last fragment, if it has n_frags > 0.
+__device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, int &n_frags,
+                                            uint2 &ends) {
     const Affine none{kNoSpans, make_float4(0.f, 0.f, 0.f, 0.f)};
     const int lane = threadIdx.x & 31;
     Affine run = none;
     n_frags = 0;
+    ends = make_uint2(0u, 0u);
     for (uint32_t base = u.beg; base < u.fin; base += 32) {
         const uint32_t mine = min(base + lane, u.fin - 1);
         const uint32_t my_cols = item_cols(__ldg(&d.bitem[mine]));
@@ -491,24 +495,21 @@ __device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bo
                     add_span(run, f);
                 }
             } else if (touch) {
-                d.run_b[base + q] = run.b;
-                d.run_a[base + q] = run.a;
+                const uint32_t p = base + q;
+                d.run_b[p] = run.b;
+                d.run_a[p] = run.a;
+                if (n_frags++ == 0) {
+                    ends.x = p;
+                } else {
+                    d.run_next[ends.y] = p;
+                    if (d.run_prev != nullptr) d.run_prev[p] = ends.y;
+                }
+                ends.y = p;
                 run = none;
-                ++n_frags;
             }
         }
     }
     return run;
-}
-
-// The fragments of the cell at column x among items [base, base + 32).
-__device__ __forceinline__ uint32_t cell_fragments(const DiffArgs &d, uint32_t fin, uint32_t base, int x, int lane) {
-    bool touch = false;
-    if (base + lane < fin) {
-        const uint4 it = __ldg(&d.bitem[base + lane]);
-        touch = it.z != 0u && touches(it, x);
-    }
-    return __ballot_sync(0xffffffffu, touch);
 }
 
 template <int SPT>
@@ -553,7 +554,8 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArg
         const bool active = lane < u.cells;
         const int x = u.x0 + 2 * lane;
         int n_frags;
-        const Affine last = cell_runs(d, u, active, x, n_frags);
+        uint2 ends;
+        const Affine last = cell_runs(d, u, active, x, n_frags, ends);
         if (FORWARD && active && n_frags == 0) {
             float4 c[1] = {make_float4(1.f, 1.f, 1.f, 1.f)};
             apply_run(c, last.a, last.b);
@@ -571,6 +573,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArg
         base = __shfl_sync(0xffffffffu, base, 0);
         if (n_frags > 0) {
             d.cell[base + __popc(cells & ((1u << lane) - 1u))] = u.cell0 + lane;
+            d.cell_ends[u.cell0 + lane] = ends;
             d.cell_b[u.cell0 + lane] = last.b;
             d.cell_a[u.cell0 + lane] = last.a;
         }
@@ -583,12 +586,11 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArg
 // such lots.
 constexpr uint32_t kCellBatch = 8;
 struct Cell {
-    uint32_t id, beg, fin;
-    int x;        // its column
+    uint32_t id, first, last;  // number, first and last fragment
     int64_t pix;  // this lane's pixel in the image
     bool valid;   // ... is inside the viewport
     uint32_t next, end;  // the warp's listed cells
-    BinScene bs;         // of the bin that beg and fin are of
+    BinScene bs;         // of its bin
 };
 __device__ __forceinline__ bool next_cell(const FrameArgs &a, const DiffArgs &d, uint32_t n_cells, int lane, Cell &c) {
     if (c.next == c.end) {
@@ -600,15 +602,14 @@ __device__ __forceinline__ bool next_cell(const FrameArgs &a, const DiffArgs &d,
         c.end = min(c.next + lot, n_cells);
     }
     const uint32_t id = d.cell[c.next++], b = id / (kTileW / 2);
-    if (c.id / (kTileW / 2) != b) {  // (a bin's cells are listed together)
-        c.beg = d.bstart[b];
-        c.fin = d.bend[b];
-        c.bs = bin_scene(a, b);
-    }
+    const uint2 ends = __ldg(&d.cell_ends[id]);
+    if (c.id / (kTileW / 2) != b) c.bs = bin_scene(a, b);  // (a bin's cells are listed together)
     c.id = id;
+    c.first = ends.x;
+    c.last = ends.y;
     const int ntx = (c.bs.W + kTileW - 1) / kTileW;
-    c.x = (int)(c.bs.lb % ntx) * kTileW + 2 * (int)(id % (kTileW / 2));
-    const int X = c.x + (lane >> 4), Y = (int)(c.bs.lb / ntx) * 2 + ((lane >> 3) & 1);
+    const int x = (int)(c.bs.lb % ntx) * kTileW + 2 * (int)(id % (kTileW / 2));  // its column
+    const int X = x + (lane >> 4), Y = (int)(c.bs.lb / ntx) * 2 + ((lane >> 3) & 1);
     c.pix = c.bs.image_off + (int64_t)Y * c.bs.W + X;
     c.valid = X < c.bs.W && Y < c.bs.H;
     return true;
@@ -630,12 +631,12 @@ __global__ void __launch_bounds__(kDiffThreads, 5) k_diff_forward(FrameArgs a, D
         float4 c[SPT];
 #pragma unroll
         for (int k = 0; k < SPT; ++k) c[k] = make_float4(1.f, 1.f, 1.f, 1.f);
-        for (uint32_t base = cell.beg; base < cell.fin; base += 32) {
-            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr; fr &= fr - 1u) {
-                const uint32_t p = base + __ffs(fr) - 1;
-                apply_run(c, d.run_a[p], d.run_b[p]);
-                apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
-            }
+        for (uint32_t p = cell.first;;) {
+            const uint32_t next = p != cell.last ? __ldg(&d.run_next[p]) : p;
+            apply_run(c, __ldg(&d.run_a[p]), __ldg(&d.run_b[p]));
+            apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
+            if (p == cell.last) break;
+            p = next;
         }
         apply_run(c, d.cell_a[cell.id], d.cell_b[cell.id]);
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -684,17 +685,17 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
 #pragma unroll
         for (int k = 0; k < SPT; ++k) c[k] = make_float4(1.f, 1.f, 1.f, 1.f);
         int slot = 0;
-        for (uint32_t base = cell.beg; base < cell.fin; base += 32) {
-            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr; fr &= fr - 1u) {
-                const uint32_t p = base + __ffs(fr) - 1;
-                apply_run(c, d.run_a[p], d.run_b[p]);
-                if (slot < d.tape_depth) {
+        for (uint32_t p = cell.first;;) {
+            const uint32_t next = p != cell.last ? __ldg(&d.run_next[p]) : p;
+            apply_run(c, __ldg(&d.run_a[p]), __ldg(&d.run_b[p]));
+            if (slot < d.tape_depth) {
 #pragma unroll
-                    for (int k = 0; k < SPT; ++k) tape[((size_t)slot * SPT + k) * 32] = c[k];
-                }
-                ++slot;
-                apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
+                for (int k = 0; k < SPT; ++k) tape[((size_t)slot * SPT + k) * 32] = c[k];
             }
+            ++slot;
+            apply_fragment<S>(c, __ldg(&d.bfill[p]), pixel_mask(__ldg(&d.bmm[p]), S, k4), sub);
+            if (p == cell.last) break;
+            p = next;
         }
         if (slot > d.tape_depth) {
             if (lane == 0) atomicOr(d.status, 1u);
@@ -705,65 +706,62 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
 #pragma unroll
         for (int k = 0; k < SPT; ++k) lam[k] = make_float4(G.x * inv, G.y * inv, G.z * inv, G.w * inv);
         float ra = d.cell_a[cell.id];  // the run after the current fragment
-        for (uint32_t base = cell.beg + ((cell.fin - cell.beg - 1) & ~31u);; base -= 32) {
-            for (uint32_t fr = cell_fragments(d, cell.fin, base, cell.x, lane); fr;) {
-                const int q = 31 - __clz((int)fr);
-                fr ^= 1u << q;
-                const uint32_t p = base + q;
-                const uint4 it = __ldg(&d.bitem[p]);
-                const float4 f = __ldg(&d.bfill[p]);
-                const float next_ra = d.run_a[p];
-                const uint32_t m = pixel_mask(__ldg(&d.bmm[p]), S, k4);
-                // (the group's, on their way while the samples are worked on)
-                const GroupHead head = group_head(d, (int64_t)it.y, lane);
-                const float av = f.w, om = 1.f - av;
-                --slot;
-                float4 cb[SPT];
+        for (uint32_t p = cell.last;;) {
+            const uint4 it = __ldg(&d.bitem[p]);
+            const float4 f = __ldg(&d.bfill[p]);
+            const float next_ra = __ldg(&d.run_a[p]);
+            const uint32_t prev = p != cell.first ? __ldg(&d.run_prev[p]) : p;
+            const uint32_t m = pixel_mask(__ldg(&d.bmm[p]), S, k4);
+            // (the group's, on their way while the samples are worked on)
+            const GroupHead head = group_head(d, (int64_t)it.y, lane);
+            const float av = f.w, om = 1.f - av;
+            --slot;
+            float4 cb[SPT];
 #pragma unroll
-                for (int k = 0; k < SPT; ++k) cb[k] = tape[((size_t)slot * SPT + k) * 32];
-                if (ra >= 0.f) {  // (uniform) the run of spans that follows starts where the fragment ends
+            for (int k = 0; k < SPT; ++k) cb[k] = tape[((size_t)slot * SPT + k) * 32];
+            if (ra >= 0.f) {  // (uniform) the run of spans that follows starts where the fragment ends
 #pragma unroll
-                    for (int k = 0; k < SPT; ++k) c[k] = cb[k];
-                    apply_fragment<S>(c, f, m, sub);
-                    float lk[8] = {};
-#pragma unroll
-                    for (int k = 0; k < SPT; ++k) {
-                        lk[0] += lam[k].x;
-                        lk[1] += lam[k].y;
-                        lk[2] += lam[k].z;
-                        lk[3] += lam[k].w;
-                        lk[4] += lam[k].x * c[k].x;
-                        lk[5] += lam[k].y * c[k].y;
-                        lk[6] += lam[k].z * c[k].z;
-                        lk[7] += lam[k].w * c[k].w;
-                        lam[k] = make_float4(lam[k].x * ra, lam[k].y * ra, lam[k].z * ra, lam[k].w * ra);
-                    }
-                    const float sum = scattered_sums<8>(lk, lane);
-                    if ((lane & 3) == 0) reinterpret_cast<float *>(d.run_sum + 2 * (size_t)p)[lane >> 2] = sum;
-                }
-                float gf[4] = {0.f, 0.f, 0.f, 0.f};
-                float J[SPT];
+                for (int k = 0; k < SPT; ++k) c[k] = cb[k];
+                apply_fragment<S>(c, f, m, sub);
+                float lk[8] = {};
 #pragma unroll
                 for (int k = 0; k < SPT; ++k) {
-                    const float4 l = lam[k];
-                    J[k] = l.x * av * (f.x - cb[k].x) + l.y * av * (f.y - cb[k].y) + l.z * av * (f.z - cb[k].z) +
-                           l.w * av * (av - cb[k].w);
-                    if ((m >> (sub + 8 * k)) & 1u) {
-                        gf[0] += l.x * av;
-                        gf[1] += l.y * av;
-                        gf[2] += l.z * av;
-                        gf[3] += l.x * (f.x - cb[k].x) + l.y * (f.y - cb[k].y) + l.z * (f.z - cb[k].z) +
-                                l.w * (2.f * av - cb[k].w);
-                        lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
-                    }
+                    lk[0] += lam[k].x;
+                    lk[1] += lam[k].y;
+                    lk[2] += lam[k].z;
+                    lk[3] += lam[k].w;
+                    lk[4] += lam[k].x * c[k].x;
+                    lk[5] += lam[k].y * c[k].y;
+                    lk[6] += lam[k].z * c[k].z;
+                    lk[7] += lam[k].w * c[k].w;
+                    lam[k] = make_float4(lam[k].x * ra, lam[k].y * ra, lam[k].z * ra, lam[k].w * ra);
                 }
-                group_adjoint<S>(a, d, (int64_t)it.y, head, a.fill_rule[it.w], J, lane);
-                const float sum = scattered_sums<4>(gf, lane);
-                if ((lane & 7) == 0 && sum != 0.f)
-                    atomicAdd(reinterpret_cast<float *>(d.grad_fill + it.w) + (lane >> 3), sum);
-                ra = next_ra;
+                const float sum = scattered_sums<8>(lk, lane);
+                if ((lane & 3) == 0) reinterpret_cast<float *>(d.run_sum + 2 * (size_t)p)[lane >> 2] = sum;
             }
-            if (base == cell.beg) break;
+            float gf[4] = {0.f, 0.f, 0.f, 0.f};
+            float J[SPT];
+#pragma unroll
+            for (int k = 0; k < SPT; ++k) {
+                const float4 l = lam[k];
+                J[k] = l.x * av * (f.x - cb[k].x) + l.y * av * (f.y - cb[k].y) + l.z * av * (f.z - cb[k].z) +
+                       l.w * av * (av - cb[k].w);
+                if ((m >> (sub + 8 * k)) & 1u) {
+                    gf[0] += l.x * av;
+                    gf[1] += l.y * av;
+                    gf[2] += l.z * av;
+                    gf[3] += l.x * (f.x - cb[k].x) + l.y * (f.y - cb[k].y) + l.z * (f.z - cb[k].z) +
+                            l.w * (2.f * av - cb[k].w);
+                    lam[k] = make_float4(l.x * om, l.y * om, l.z * om, l.w * om);
+                }
+            }
+            group_adjoint<S>(a, d, (int64_t)it.y, head, a.fill_rule[it.w], J, lane);
+            const float sum = scattered_sums<4>(gf, lane);
+            if ((lane & 7) == 0 && sum != 0.f)
+                atomicAdd(reinterpret_cast<float *>(d.grad_fill + it.w) + (lane >> 3), sum);
+            ra = next_ra;
+            if (p == cell.first) break;
+            p = prev;
         }
         if (ra >= 0.f) {  // the first run
             float s[4] = {0.f, 0.f, 0.f, 0.f};

@@ -299,12 +299,16 @@ struct DiffArgs {
     int64_t nf;
     // per resolve pair that is a fragment: the affine map of the spans before it
     // in its cell (c -> run_a c + run_b; run_a < 0: none) and, backward, the sums
-    // of the run after it (2 per pair)
+    // of the run after it (2 per pair); the pairs of its cell's next and
+    // (backward) previous fragments
     float *run_a;
     float4 *run_b, *run_sum;
+    uint32_t *run_next, *run_prev;
     // the cells with fragments (numbers bin * 32 + column), and per cell number
-    // the map of its last run (as run_a, run_b) and the adjoint sum of its first
+    // the map of its last run (as run_a, run_b), the adjoint sum of its first, and
+    // its first and last fragments' pairs
     uint32_t *cell;
+    uint2 *cell_ends;
     float *cell_a;
     float4 *cell_b, *cell_sum;
     // per warp: tape_depth x (samples per thread) x 32 sample states, and pi_depth
