@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_fragment(FrameArgs a, const flo
 }
 
 // --------------------------------------------- winding scan + marks --
-constexpr int kMarkThreads = 256;
+constexpr int kMarkThreads = 512;
 constexpr int kMarkItems = 8;
 constexpr int kMarkTile = kMarkThreads * kMarkItems;
 constexpr uint64_t kSegBit = 1ull << 32;  // winding look-back: a scene starts in the tile (batches)
@@ -676,23 +676,22 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     }
     return v;
 }
+// Exclusive scan over the block, one barrier: every warp scans the warps' totals
+// itself.  sw (one word per warp) is not used for anything else.
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *sw, uint32_t *total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int W = kMarkThreads / 32;
-    uint32_t inc = warp_incl_scan(v);
+    const uint32_t inc = warp_incl_scan(v);
     if (lane == 31) sw[warp] = inc;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t t = lane < W ? sw[lane] : 0u;
-        uint32_t ti = warp_incl_scan(t);
-        if (lane < W) sw[lane] = ti - t;
-        if (lane == W - 1) sw[W] = ti;
+    uint32_t t = lane < W ? sw[lane] : 0u;
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += n;
     }
-    __syncthreads();
-    uint32_t r = sw[warp] + inc - v;
-    *total = sw[W];
-    __syncthreads();
-    return r;
+    *total = __shfl_sync(0xffffffffu, t, W - 1);
+    return __shfl_sync(0xffffffffu, t, (warp + 31) & 31) * (warp ? 1u : 0u) + inc - v;
 }
 
 // Segmented sums: (s, f) where f = a segment starts inside; a then b.
@@ -714,23 +713,15 @@ __device__ __forceinline__ SegSum block_excl_segscan(SegSum v, uint32_t *ss, uin
     if (lane == 0) prev = SegSum{0u, 0u};
     if (lane == 31) ss[warp] = inc.s, sf[warp] = inc.f;
     __syncthreads();
-    if (warp == 0) {
-        SegSum t = lane < W ? SegSum{ss[lane], sf[lane]} : SegSum{0u, 0u};
+    SegSum t = lane < W ? SegSum{ss[lane], sf[lane]} : SegSum{0u, 0u};
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const SegSum up{__shfl_up_sync(0xffffffffu, t.s, o), __shfl_up_sync(0xffffffffu, t.f, o)};
-            if (lane >= o) t = seg_then(up, t);
-        }
-        SegSum ex{__shfl_up_sync(0xffffffffu, t.s, 1), __shfl_up_sync(0xffffffffu, t.f, 1)};
-        if (lane == 0) ex = SegSum{0u, 0u};
-        if (lane < W) ss[lane] = ex.s, sf[lane] = ex.f;
-        if (lane == W - 1) ss[W] = t.s, sf[W] = t.f;
+    for (int o = 1; o < W; o <<= 1) {
+        const SegSum up{__shfl_up_sync(0xffffffffu, t.s, o), __shfl_up_sync(0xffffffffu, t.f, o)};
+        if (lane >= o) t = seg_then(up, t);
     }
-    __syncthreads();
-    const SegSum r = seg_then(SegSum{ss[warp], sf[warp]}, prev);
-    *total = SegSum{ss[W], sf[W]};
-    __syncthreads();
-    return r;
+    *total = SegSum{__shfl_sync(0xffffffffu, t.s, W - 1), __shfl_sync(0xffffffffu, t.f, W - 1)};
+    const SegSum before{__shfl_sync(0xffffffffu, t.s, (warp + 31) & 31), __shfl_sync(0xffffffffu, t.f, (warp + 31) & 31)};
+    return warp ? seg_then(before, prev) : prev;
 }
 
 struct Mark {
@@ -769,26 +760,31 @@ __device__ __forceinline__ uint32_t count_bins(const FrameArgs &a, const int4 &i
     return a.alt_shift >= 0 ? (uint32_t)item_bins(it, dp.W, dp.H, a.alt_shift, 0u, &b0) : 0u;
 }
 
+// Column and row of a cell from its key within the path (the inverse of
+// local_sort_key; the out-of-range sentinel's row is far outside).
+__device__ __forceinline__ int local_x(uint64_t k) { return 2 * (int)((uint32_t)k & 0xFFFu) - 2; }
+__device__ __forceinline__ int local_y(uint64_t k, int nrows) {
+    const int rr = (int)(((uint32_t)k >> 12) & 0xFFFu);
+    return rr == nrows ? 0 : (rr == nrows - 1 ? 0x7FFF : 2 * (rr + 1));
+}
+
 // k_mark_merged_fragment_and_span (cu:462-535) on sorted position i with
-// keys k0 (position i - 1) and k1 (position i) and scanned winding w.
+// keys k0 (position i - 1) and k1 (position i) and scanned winding w.  Keys of
+// one path order and compare as its cells do, so the marks need the cell's
+// column and row only for the viewport test.
 __device__ __forceinline__ Mark mark_of(int64_t i, uint64_t k0, uint64_t k1, int8_t w, const FrameArgs &a) {
-    const Dim dm = dim_of(a, (uint32_t)(k1 >> 24));
-    const int W = dm.W, H = dm.H, nrows = (H + 1) / 2;
-    const uint32_t key1 = (uint32_t)key_from_local((uint32_t)(k1 & 0xFFFFFFu), nrows);
-    const int x1 = key_x(key1), y1 = key_y(key1);
-    const bool oob = x1 < 0 || y1 < 0 || x1 >= W || y1 >= H;
-    Mark m{0u, 0u};
-    if (i == 0) {
-        m.ff = oob ? 0u : 1u;
-        return m;
+    const uint32_t p1 = (uint32_t)(k1 >> 24);
+    const Dim dm = dim_of(a, p1);
+    const int x1 = local_x(k1), y1 = local_y(k1, (dm.H + 1) / 2);
+    const bool in = x1 >= 0 && x1 < dm.W && y1 < dm.H;
+    if (i == 0) return Mark{in ? 1u : 0u, 0u};
+    Mark m{in && k0 != k1 ? 1u : 0u, 0u};
+    // a span: the same row of the same path, with columns left out between
+    // (equal for two sentinels: none)
+    if ((k0 >> 12) == (k1 >> 12) && ((uint32_t)k0 & 0xFFFu) + 1u < ((uint32_t)k1 & 0xFFFu)) {
+        const uint8_t fr = a.fill_rule[p1];
+        m.sf = (fr == 0 && w != 0) || (fr == 1 && (w & 1)) ? 1u : 0u;
     }
-    const uint32_t p0 = (uint32_t)(k0 >> 24), p1 = (uint32_t)(k1 >> 24);
-    const uint32_t key0 = (uint32_t)key_from_local((uint32_t)(k0 & 0xFFFFFFu), nrows);
-    const int x0 = key_x(key0), y0 = key_y(key0);
-    m.ff = oob ? 0u : ((p0 != p1 || key0 != key1) ? 1u : 0u);
-    const uint8_t fr = a.fill_rule[p1];
-    const bool wf = (fr == 0 && w != 0) || (fr == 1 && (w & 1));
-    m.sf = (y0 == y1 && (x0 + 2) < x1 && p0 == p1 && wf) ? 1u : 0u;
     return m;
 }
 
@@ -801,7 +797,13 @@ __device__ __forceinline__ Mark mark_of(int64_t i, uint64_t k0, uint64_t k1, int
 // scene sees the scan a single-scene render gives it); then the merged and
 // span marks, scanned with a second look-back, and the draw items written.
 // The last tile writes the item counts.  Sorted keys are read 128 bits at a
-// time; each carries its fragment's scan winding in bits 60-63.
+// time; each carries its fragment's scan winding in bits 60-63.  Bound by the
+// wait for the two look-backs (40% of the stalls) and by issue: an entry makes
+// up to two draw items, so a warp lists its items and writes them 32 at a time.
+// With the two kinds written entry by entry (20 lanes active), 2048 entries to
+// a tile and three barriers to a scan, this took 373 us on 20,000 paths over
+// 2048 x 2048, 1230 on a batch of 48 scenes and 88 on 2,500 paths over 1917 x
+// 1079; here 307, 941 and 72 (tiles of 2048 entries: 321, 972, 78).
 __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const uint64_t *__restrict__ skey,
                                                             int8_t *__restrict__ wn_scan,
                                                             int4 *__restrict__ draw, uint32_t *__restrict__ heads,
@@ -810,9 +812,10 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
                                                             FrameCounters *__restrict__ ctr,
                                                             uint64_t *__restrict__ st_wn, uint64_t *__restrict__ st_fl,
                                                             uint32_t spin_cap) {
-    __shared__ uint32_t ss[kMarkThreads / 32 + 1], sf[kMarkThreads / 32 + 1];
+    __shared__ uint32_t ss[kMarkThreads / 32], sf[kMarkThreads / 32], sm[kMarkThreads / 32];
     __shared__ uint32_t s_tile;
-    __shared__ uint64_t s_pre;
+    __shared__ uint64_t s_pre, s_pre2;
+    __shared__ uint16_t s_item[kMarkThreads / 32][2 * 32 * kMarkItems];
     const int64_t nf = ctr->nf;
     const int64_t ntiles = (nf + kMarkTile - 1) / kMarkTile;
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctr->tiles[1], 1u);
@@ -881,12 +884,11 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
         run.s += (uint32_t)v[j];
     }
     if (cnt == kMarkItems) {
-        uint2 packed;
-        packed.x = (uint32_t)(uint8_t)ws[0] | ((uint32_t)(uint8_t)ws[1] << 8) | ((uint32_t)(uint8_t)ws[2] << 16) |
-                   ((uint32_t)(uint8_t)ws[3] << 24);
-        packed.y = (uint32_t)(uint8_t)ws[4] | ((uint32_t)(uint8_t)ws[5] << 8) | ((uint32_t)(uint8_t)ws[6] << 16) |
-                   ((uint32_t)(uint8_t)ws[7] << 24);
-        *reinterpret_cast<uint2 *>(wn_scan + base) = packed;
+        uint32_t packed[kMarkItems / 4] = {};
+#pragma unroll
+        for (int j = 0; j < kMarkItems; ++j) packed[j / 4] |= (uint32_t)(uint8_t)ws[j] << (8 * (j % 4));
+#pragma unroll
+        for (int j = 0; j < kMarkItems / 4; ++j) reinterpret_cast<uint32_t *>(wn_scan + base)[j] = packed[j];
     } else {
 #pragma unroll
         for (int j = 0; j < kMarkItems; ++j)
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
         fs += mk[j].ff | (mk[j].sf << 16);
     }
     uint32_t ftot;
-    const uint32_t fpre = block_excl_scan(fs, ss, &ftot);
+    const uint32_t fpre = block_excl_scan(fs, sm, &ftot);
     const uint64_t ftot_w = ((uint64_t)(ftot & 0xFFFFu) << 31) | (uint64_t)(ftot >> 16);
     if (threadIdx.x < 32) {
         uint64_t pre = 0;
@@ -911,7 +913,7 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
         }
         if (threadIdx.x == 0) {
             lb_store(st_fl + t, kLbInclusive | ((pre + ftot_w) & kLbPayload));
-            s_pre = pre;
+            s_pre2 = pre;
             if (t == ntiles - 1) {  // the frame's item counts
                 const uint64_t all = pre + ftot_w;
                 const uint32_t nm = (uint32_t)(all >> 31) & 0x7FFFFFFFu, ns = (uint32_t)all & 0x7FFFFFFFu;
@@ -922,50 +924,53 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
         }
     }
     __syncthreads();
-    uint32_t nfb = (uint32_t)(s_pre >> 31) + (fpre & 0xFFFFu);
-    uint32_t nsb = (uint32_t)(s_pre & 0x7FFFFFFFu) + (fpre >> 16);
-    uint32_t span_px = 0, pairs_alt = 0;  // this thread's span pixels and pairs in the other tile
+    // the warp's items listed (entry within the warp, a span's with bit 15 set),
+    // then written 32 at a time, whichever lane's entry they come from
+    const int lane = threadIdx.x & 31;
+    uint16_t *const item = s_item[threadIdx.x >> 5];
+    uint32_t nfb = (uint32_t)(s_pre2 >> 31) + (fpre & 0xFFFFu);
+    const uint32_t nsb = (uint32_t)(s_pre2 & 0x7FFFFFFFu) + (fpre >> 16);
+    const uint32_t first = __shfl_sync(0xffffffffu, nfb + nsb, 0);
+    uint32_t at = nfb + nsb - first;
 #pragma unroll
     for (int j = 0; j < kMarkItems; ++j) {
-        const uint32_t ff = mk[j].ff, sfl = mk[j].sf;
-        if (ff | sfl) {
-            const uint64_t k1 = k[j + 1];
+        if (mk[j].ff) item[at++] = (uint16_t)(lane * kMarkItems + j);
+        if (mk[j].sf) item[at++] = (uint16_t)(0x8000 | (lane * kMarkItems + j));
+    }
+    const uint32_t n = __shfl_sync(0xffffffffu, at, 31);
+    nfb = __shfl_sync(0xffffffffu, nfb, 0);
+    __syncwarp();
+    const int64_t warp_base = base - lane * kMarkItems;
+    uint32_t span_px = 0, pairs_alt = 0;  // this thread's span pixels and pairs in the other tile
+    for (uint32_t q0 = 0; q0 < n; q0 += 32) {
+        const uint32_t q = q0 + lane;
+        const bool live = q < n;
+        const uint32_t code = live ? item[q] : 0x8000u;
+        const bool span = (code & 0x8000u) != 0u;
+        const uint32_t frags = __ballot_sync(0xffffffffu, !span);
+        if (live) {
+            const int64_t i = warp_base + (code & 0x7FFFu);
+            const uint64_t k1 = skey[i] & kKeyMask;
             const uint32_t p = (uint32_t)(k1 >> 24);
-            const int32_t fill = (int32_t)a.fill_rgba[p];
             const Dim dp = dim_of(a, p);
-            const int nrows = (dp.H + 1) / 2;
-            const uint32_t key1 = (uint32_t)key_from_local((uint32_t)(k1 & 0xFFFFFFu), nrows);
-            if (item_scene != nullptr) {
-                const uint32_t sc = a.path_scene[p];
-                if (ff) item_scene[nfb + nsb] = sc;
-                if (sfl) item_scene[nfb + nsb + ff] = sc;
+            const int x1 = local_x(k1), y = local_y(k1, (dp.H + 1) / 2);
+            int4 it = make_int4((int32_t)(((uint32_t)y << 16) | (uint32_t)x1), 2, (int32_t)a.fill_rgba[p], 0);
+            if (span) {
+                const int x0 = local_x(skey[i - 1]) + 2;  // (columns start at -2)
+                it.x = (int32_t)(((uint32_t)y << 16) | (uint32_t)x0);
+                it.y = x1 - x0;
+                span_px += (uint32_t)(x1 - x0);
+            } else {
+                const uint32_t g = nfb + __popc(frags & ((1u << lane) - 1u));
+                it.w = (int)(g + 1);
+                heads[g] = (uint32_t)i;
             }
-            if (a.item_path != nullptr) {
-                if (ff) a.item_path[nfb + nsb] = p;
-                if (sfl) a.item_path[nfb + nsb + ff] = p;
-            }
-            if (ff) {
-                const int32_t pos = (int32_t)(((uint32_t)key_y(key1) << 16) | (uint32_t)key_x(key1));
-                const int4 it = make_int4(pos, 2, fill, (int)(nfb + 1));
-                draw[nfb + nsb] = it;
-                pairs_alt += count_bins(a, it, dp, p, bin_count);
-                heads[nfb] = (uint32_t)(base + j);
-            }
-            if (sfl) {
-                const uint32_t key0 = (uint32_t)key_from_local((uint32_t)(k[j] & 0xFFFFFFu), nrows);
-                const int y0 = key_y(key0);
-                int x0 = (int16_t)(key_x(key0) + 2);
-                const int x1 = key_x(key1);
-                x0 = max(0, x0);
-                const int32_t pos = (int32_t)(((uint32_t)y0 << 16) | (uint32_t)x0);
-                const int4 it = make_int4(pos, x1 - x0, fill, 0);
-                draw[nfb + nsb + ff] = it;
-                pairs_alt += count_bins(a, it, dp, p, bin_count);
-                span_px += (uint32_t)max(x1 - x0, 0);
-            }
+            draw[first + q] = it;
+            if (item_scene != nullptr) item_scene[first + q] = a.path_scene[p];
+            if (a.item_path != nullptr) a.item_path[first + q] = p;
+            pairs_alt += count_bins(a, it, dp, p, bin_count);
         }
-        nfb += ff;
-        nsb += sfl;
+        nfb += __popc(frags);
     }
     const uint32_t wpx = __reduce_add_sync(0xffffffffu, span_px);
     const uint32_t wpa = __reduce_add_sync(0xffffffffu, pairs_alt);
