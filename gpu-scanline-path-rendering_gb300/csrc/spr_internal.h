@@ -222,11 +222,11 @@ int64_t scan_mark_status_words(int64_t cap_nf);
 int launch_scan_mark(const FrameArgs &a, int64_t cap_nf, const uint64_t *skey, int8_t *wn_scan, int4 *draw,
                      uint32_t *heads, uint32_t *item_scene, uint32_t *bin_count, FrameCounters *counters,
                      uint64_t *tile_status, uint32_t spin_cap, cudaStream_t s);
-// Merged masks from the sorted keys and fragment indices (perm), which hold
-// at least 16 entries past cap_nf, and the fragments' masks.
-int launch_stencil(const FrameArgs &a, int64_t cap_nf, FrameCounters *ctr, const uint64_t *skey, const uint32_t *perm,
-                   const uint32_t *mask, const int8_t *wn_scan, const uint32_t *heads, uint32_t *merged_mask,
-                   uint32_t spin_cap, cudaStream_t s);
+// Merged masks from the sorted keys and fragment indices (perm) and the
+// fragments' masks.
+int launch_stencil(const FrameArgs &a, int64_t cap_nf, const FrameCounters *ctr, const uint64_t *skey,
+                   const uint32_t *perm, const uint32_t *mask, const int8_t *wn_scan, const uint32_t *heads,
+                   uint32_t *merged, cudaStream_t s);
 // The draw items of every resolve bin in draw order: bin b's are
 // pval[bin_off[b] .. bin_off[b + 1]) (bin_off: the exclusive scan of the
 // bin counts; bin_fill: n_bins words, zero before).

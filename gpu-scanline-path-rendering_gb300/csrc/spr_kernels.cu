@@ -984,115 +984,61 @@ __global__ void __launch_bounds__(kMarkThreads) k_scan_mark(FrameArgs a, const u
 // mask bit (the reference's packed counters), reduced to the 7-bit winding
 // number and tested against the fill rule.
 //
-// A block takes 256 consecutive merged fragments, whose groups are one
-// contiguous run of sorted positions [heads[g0], heads[g0 + 256]).  The run
-// (up to kStencilStage positions, from a 16-entry boundary) is staged into
-// shared memory by bulk copies (cp.async.bulk, completion on an mbarrier)
-// of the sorted keys (with the change signs in bits 60-63) and fragment
-// indices; positions past the staged run are read from global memory.  The
-// sample masks are read through the fragment indices.
-constexpr int kStencilStage = 1024;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-// Waits for phase 0 of mbarrier `bar`, at most `cap` polls; false if it
-// did not complete.
-__device__ __forceinline__ bool mbar_wait0(uint32_t bar, uint32_t cap) {
-    for (uint32_t it = 0; it < cap; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, "
-            "p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(0u)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-struct StencilStage {
-    uint64_t key[kStencilStage];
-    uint32_t perm[kStencilStage];
-    uint64_t bar;
-};
-
+// A thread per group: the group's head, then its first key, index and winding
+// together, then mask by mask with the next key and index on the way.  Bound by
+// the latency of these loads, one after the other.  With 256 groups' keys and
+// indices staged in shared memory by bulk copies, which every thread of the block
+// waited for, the stage took 346 us on 20,000 paths over 2048 x 2048, 846 on a
+// batch of 48 scenes and 57 on 2,500 paths over 1917 x 1079; here 293, 678 and 41
+// (with two threads a group at 32 samples 344 and 772; with 4 blocks to an SM at
+// 32 samples and 6 at fewer 303, 705 and 41).
 template <int S>
-__global__ void __launch_bounds__(kThreads, 5) k_stencil(FrameArgs a, FrameCounters *__restrict__ ctr,
+__global__ void __launch_bounds__(kThreads, S == 32 ? 5 : 8) k_stencil(FrameArgs a, const FrameCounters *__restrict__ ctr,
                                                       const uint64_t *__restrict__ skey,
                                                       const uint32_t *__restrict__ perm,
                                                       const uint32_t *__restrict__ mask,
                                                       const int8_t *__restrict__ wn_scan,
                                                       const uint32_t *__restrict__ heads,
-                                                      uint32_t *__restrict__ merged, uint32_t spin_cap) {
+                                                      uint32_t *__restrict__ merged) {
     constexpr int WORDS = S / 8;
-    __shared__ __align__(16) StencilStage st;
-    const int64_t nf = ctr->nf, nm = ctr->n_merged;
-    const int64_t g0 = (int64_t)blockIdx.x * blockDim.x;
-    if (g0 >= nm) return;
-    // the block's run of sorted positions, from a 16-entry boundary
-    const int64_t s16 = (int64_t)heads[g0] & ~(int64_t)15;
-    const int64_t e = g0 + (int64_t)blockDim.x < nm ? (int64_t)heads[g0 + blockDim.x] : nf;
-    const int64_t e16 = (e + 15) & ~(int64_t)15;
-    const int64_t n_st = min(e16 - s16, (int64_t)kStencilStage);  // a multiple of 16
-    const uint32_t bar = smem_addr(&st.bar);
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t bytes = (uint32_t)n_st * (8u + 4u);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-        bulk_g2s(st.key, skey + s16, (uint32_t)n_st * 8u, bar);
-        bulk_g2s(st.perm, perm + s16, (uint32_t)n_st * 4u, bar);
-    }
-    // this thread's group head and its scanned winding, while the copies run
-    const int64_t g = g0 + threadIdx.x;
-    const bool live = g < nm;
-    const int64_t h = live ? (int64_t)heads[g] : 0;
-    const int32_t w0 = live ? (int32_t)wn_scan[h] : 0;
-    if (!mbar_wait0(bar, spin_cap)) {
-        if (threadIdx.x == 0) atomicOr(&ctr->status, kStatusTimeout);
-        mbar_wait0(bar, spin_cap);  // the copies still in flight write this block's shared memory
-        return;
-    }
-    if (!live) return;
-    auto key_at = [&](int64_t j) { return j - s16 < n_st ? st.key[j - s16] : skey[j]; };
-    const uint64_t kh = key_at(h) & kKeyMask;
+    const uint32_t nf = ctr->nf, g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ctr->n_merged) return;
+    const uint32_t h = heads[g];
+    const int32_t w0 = (int32_t)__ldg(wn_scan + h);
+    const uint64_t k0 = __ldg(skey + h);
+    const uint32_t raw0 = __ldg(perm + h);
+    const uint64_t kh = k0 & kKeyMask;
     // the group's fragments with a winding change: fn(change sign, mask)
     auto walk = [&](auto &&fn) {
-        for (int64_t j = h; j < nf; ++j) {
-            const bool staged = j - s16 < n_st;
-            const uint64_t kj = staged ? st.key[j - s16] : skey[j];
-            if ((kj & kKeyMask) != kh) break;
+        uint64_t kj = k0;
+        uint32_t raw = raw0;
+        for (uint32_t j = h;;) {
+            // (the next position, asked for with this one's mask)
+            const uint32_t jn = j + 1;
+            const uint64_t kn = jn < nf ? __ldg(skey + jn) : ~0ull;
+            const uint32_t rn = jn < nf ? __ldg(perm + jn) : 0u;
             const int32_t chg = fw_chg((uint32_t)(kj >> kFwShift));
-            if (chg == 0) continue;
-            const uint32_t raw = staged ? st.perm[j - s16] : perm[j];
-            uint32_t m[WORDS];
-            if constexpr (WORDS == 1) {
-                m[0] = __ldg(mask + raw);
-            } else if constexpr (WORDS == 2) {
-                const uint2 v = __ldg(reinterpret_cast<const uint2 *>(mask) + raw);
-                m[0] = v.x;
-                m[1] = v.y;
-            } else {
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mask) + raw);
-                m[0] = v.x;
-                m[1] = v.y;
-                m[2] = v.z;
-                m[3] = v.w;
+            if (chg != 0) {
+                uint32_t m[WORDS];
+                if constexpr (WORDS == 1) {
+                    m[0] = __ldg(mask + raw);
+                } else if constexpr (WORDS == 2) {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(mask) + raw);
+                    m[0] = v.x;
+                    m[1] = v.y;
+                } else {
+                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(mask) + raw);
+                    m[0] = v.x;
+                    m[1] = v.y;
+                    m[2] = v.z;
+                    m[3] = v.w;
+                }
+                fn(chg, m);
             }
-            fn(chg, m);
+            if (jn >= nf || (kn & kKeyMask) != kh) break;
+            j = jn;
+            kj = kn;
+            raw = rn;
         }
     };
     const int fr = a.fill_rule[(uint32_t)(kh >> 24)];
@@ -1138,7 +1084,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_stencil(FrameArgs a, FrameCount
             // nonzero: any bit of the 7-bit winding; even-odd: its lowest bit
             const uint32_t ret = fr == 0 ? (pl[0][w] | pl[1][w] | pl[2][w] | pl[3][w] | pl[4][w] | pl[5][w] | pl[6][w])
                                          : pl[0][w];
-            merged[g * WORDS + w] = ret;
+            merged[(size_t)g * WORDS + w] = ret;
         }
         return;
     }
@@ -1171,7 +1117,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_stencil(FrameArgs a, FrameCount
             }
             ret |= (wv & 0x01010101u) << b;
         }
-        merged[g * WORDS + w] = ret;
+        merged[(size_t)g * WORDS + w] = ret;
     }
 }
 
@@ -2335,17 +2281,17 @@ int launch_scan_mark(const FrameArgs &a, int64_t cap_nf, const uint64_t *skey, i
     return 1;
 }
 
-int launch_stencil(const FrameArgs &a, int64_t cap_nf, FrameCounters *ctr, const uint64_t *skey, const uint32_t *perm,
-                   const uint32_t *mask, const int8_t *wn_scan, const uint32_t *heads, uint32_t *merged,
-                   uint32_t spin_cap, cudaStream_t s) {
+int launch_stencil(const FrameArgs &a, int64_t cap_nf, const FrameCounters *ctr, const uint64_t *skey,
+                   const uint32_t *perm, const uint32_t *mask, const int8_t *wn_scan, const uint32_t *heads,
+                   uint32_t *merged, cudaStream_t s) {
     if (cap_nf <= 0) return 0;
     const unsigned g = grid_for(cap_nf);
     if (a.S == 8)
-        k_stencil<8><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged, spin_cap);
+        k_stencil<8><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged);
     else if (a.S == 16)
-        k_stencil<16><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged, spin_cap);
+        k_stencil<16><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged);
     else
-        k_stencil<32><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged, spin_cap);
+        k_stencil<32><<<g, kThreads, 0, s>>>(a, ctr, skey, perm, mask, wn_scan, heads, merged);
     return 1;
 }
 

@@ -23,9 +23,9 @@ def lines(points):
                      [0xFF2040FF + 977 * k & 0xFFFFFFFF | 0x80000000 for k in range(len(points))])
 
 
-def check(scene, W, H):
-    ref = oracle.run(scene, W, H, samples=8)
-    with spr.VGRasterizer(W, H, samples=8) as r:
+def check(scene, W, H, samples=8):
+    ref = oracle.run(scene, W, H, samples=samples)
+    with spr.VGRasterizer(W, H, samples=samples) as r:
         r.add_vg(scene)
         r.rasterize()
         for st in ("SORT_PERM", "DRAW_LIST", "MERGED_MASK"):
@@ -53,3 +53,16 @@ def test_spans(W, H, rows):
     boxes += [[(x + .5, 3.5), (x + 5.5, 3.5), (x + 5.5, 2 * rows - 4.5), (x + .5, 2 * rows - 4.5)]
               for x in range(4, W - 8, max(W // 9, 8))]
     check(lines(boxes), W, H)
+
+
+@pytest.mark.parametrize("samples", [8, 16, 32])
+@pytest.mark.parametrize("n", [1, 2, 33, 127, 128, 200])
+def test_groups_of_many_fragments(n, samples):
+    # n nested triangles of one path in the last cell of the frame, and as many cells of one
+    poly = []
+    for k in range(n):
+        e = .8 * k / n
+        poly += [(62.1 + e, 62.2 + e), (63.9 - e / 9, 62.3 + e), (63 + e / 9, 63.9 - e / 9)]
+    one = [[(2 * (k % 30) + .2, 2 * (k // 30) + .3), (2 * (k % 30) + 1.7, 2 * (k // 30) + .6),
+            (2 * (k % 30) + .9, 2 * (k // 30) + 1.8)] for k in range(n)]
+    check(lines(one + [poly]), 64, 64, samples)
