@@ -6,9 +6,8 @@
 // Device memory: the scene lives in per-handle buffers written once by
 // spr_set_scene; every per-frame array is a grow-only buffer of the handle
 // (the role of the reference's 256 MB bump arena, cuda_cached_allocator.h),
-// so steady-state frames allocate nothing.  The frame reads back three
-// counts to size its work (fragments, merged fragments + spans, resolve
-// pairs); everything else stays on the device.
+// so steady-state frames allocate nothing.  A sized frame reads back its entry
+// count (with its longest path) and its counters; the others read nothing.
 
 #include <cuda_runtime.h>
 

@@ -8,10 +8,15 @@
 // (1 - a) (the same blend as the multisample resolve, without the 8-bit
 // sRGB storage), and a pixel is the mean of its samples.
 //
-// Backward, per sample: a tape of the state before every draw item that
-// touches the sample's cell is recorded in draw order and swept in reverse
-// with the adjoint lambda of the state (lambda *= 1 - a through every
-// covering item), giving the exact fill gradients.  Geometry is
+// Spans cover every sample of a cell, so the spans between two fragments of a
+// cell are one affine map: a first pass composes them, a lane per cell, and the
+// passes over samples go through the cells' fragments only.
+//
+// Backward, per sample: a tape of the state before every fragment of the
+// sample's cell is recorded in draw order and swept in reverse with the adjoint
+// lambda of the state (lambda *= 1 - a through every covering item), giving the
+// exact fill gradients (the spans' in a last pass, from two sums per run of
+// them).  Geometry is
 // differentiated by edge sampling: a pixel is taken as the mean over its S
 // sample rows of the row integral of the composite, so moving the crossing
 // x_c of a chord with sample row y_r by dx changes the pixel by
