@@ -1195,12 +1195,18 @@ __global__ void k_bin_count(FrameArgs a, const int4 *__restrict__ draw, const ui
 // (first | width << 16 | row << 29) and its merged sample mask (every sample
 // for a span), so that the resolve reads each bin's items and masks as one
 // contiguous run instead of gathering them.  (Widths stay below 2^13:
-// viewports are at most 4096 pixels wide.)  With the network in shared memory
-// (about 12,000 warp instructions for a bin of 528 items against 2,700) this
-// took 522 us on the 20,000-path 2048 x 2048 scene, 1690 on a batch of 48 scenes and
-// 68 on 64 paths over 512 x 512; here 264, 955 and 32.
+// viewports are at most 4096 pixels wide.)  Bound by the
+// records' gathers.  On the 20,000-path 2048 x 2048 scene this kernel took 522 us
+// with the network in shared memory (about 12,000 warp instructions for a bin of
+// 528 items against 2,700), 264 with it in registers, 228 with the records
+// gathered 4 x 32 at a time and 185 with one rolled body for the strides across
+// lanes (the unrolled bodies of the six list lengths did not fit the instruction
+// cache); all of the binning 695 -> 438 -> 398 -> 358, on a batch of 48 scenes
+// 2180 -> 1498 -> 1356 -> 1318.  (2 and 8 x 32 at a time: 410 and 399, 1396 and
+// 1383.)
 constexpr int kBinSortWarps = 4;
 constexpr int kBinSortRegs = 1024;
+constexpr int kBinGather = 4;
 
 template <int K>
 __device__ __forceinline__ void warp_sort(uint32_t (&k)[K], int lane) {
@@ -1209,37 +1215,44 @@ __device__ __forceinline__ void warp_sort(uint32_t (&k)[K], int lane) {
         x = lo;
         y = hi;
     };
+    // within the lane
 #pragma unroll
-    for (int size = 2; size <= 32 * K; size *= 2) {
-        if (size <= K) {  // mirror within the lane
+    for (int size = 2; size <= K; size *= 2) {
+#pragma unroll
+        for (int r = 0; r < K; ++r)
+            if ((r ^ (size - 1)) > r) order(k[r], k[r ^ (size - 1)]);
+#pragma unroll
+        for (int j = size / 4; j > 0; j /= 2)
 #pragma unroll
             for (int r = 0; r < K; ++r)
-                if ((r ^ (size - 1)) > r) order(k[r], k[r ^ (size - 1)]);
-        } else {  // with register K - 1 - r of the mirrored lane
-            const bool lo = (lane & (size / K / 2)) == 0;
+                if ((r ^ j) > r) order(k[r], k[r ^ j]);
+    }
+    // across 2, 4, .. 32 lanes (one body for all, which the instruction cache holds
+    // beside the other list lengths')
+#pragma unroll 1
+    for (int lanes = 2; lanes <= 32; lanes *= 2) {
+        const bool lo = (lane & (lanes / 2)) == 0;  // with register K - 1 - r of the mirrored lane
 #pragma unroll
-            for (int r = 0; r < (K + 1) / 2; ++r) {
-                const uint32_t u = __shfl_xor_sync(0xffffffffu, k[K - 1 - r], size / K - 1);
-                const uint32_t v = __shfl_xor_sync(0xffffffffu, k[r], size / K - 1);
-                k[r] = (k[r] < u) == lo ? k[r] : u;
-                if (K - 1 - r != r) k[K - 1 - r] = (k[K - 1 - r] < v) == lo ? k[K - 1 - r] : v;
+        for (int r = 0; r < (K + 1) / 2; ++r) {
+            const uint32_t u = __shfl_xor_sync(0xffffffffu, k[K - 1 - r], lanes - 1);
+            const uint32_t v = __shfl_xor_sync(0xffffffffu, k[r], lanes - 1);
+            k[r] = (k[r] < u) == lo ? k[r] : u;
+            if (K - 1 - r != r) k[K - 1 - r] = (k[K - 1 - r] < v) == lo ? k[K - 1 - r] : v;
+        }
+#pragma unroll 1
+        for (int j = lanes / 4; j > 0; j /= 2) {
+            const bool jlo = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const uint32_t u = __shfl_xor_sync(0xffffffffu, k[r], j);
+                k[r] = (k[r] < u) == jlo ? k[r] : u;
             }
         }
 #pragma unroll
-        for (int j = size / 4; j > 0; j /= 2) {
-            if (j < K) {
+        for (int j = K / 2; j > 0; j /= 2)
 #pragma unroll
-                for (int r = 0; r < K; ++r)
-                    if ((r ^ j) > r) order(k[r], k[r ^ j]);
-            } else {
-                const bool lo = (lane & (j / K)) == 0;
-#pragma unroll
-                for (int r = 0; r < K; ++r) {
-                    const uint32_t u = __shfl_xor_sync(0xffffffffu, k[r], j / K);
-                    k[r] = (k[r] < u) == lo ? k[r] : u;
-                }
-            }
-        }
+            for (int r = 0; r < K; ++r)
+                if ((r ^ j) > r) order(k[r], k[r ^ j]);
     }
 }
 
@@ -1328,13 +1341,30 @@ __global__ void __launch_bounds__(kBinSortWarps * 32)
     if (regs)
         for (uint32_t i = lane; i < n; i += 32) run[i] = st[bin_sort_at(i)];
     if (rec_a == nullptr) return;
-    for (uint32_t i = lane; i < n; i += 32) {
-        const uint32_t idx = regs ? st[bin_sort_at(i)] : run[i];
-        const int4 it = draw[idx];
-        const uint32_t ro = (uint32_t)(((it.x >> 16) / 2) & band_mask);  // the item's cell row within the band
-        rec_a[beg + i] = make_uint2((uint32_t)it.z,
-                                    ((uint32_t)it.x & 0xFFFFu) | ((uint32_t)it.y << 16) | (ro << 29));
-        rec_m[beg + i] = it.w != 0 ? reinterpret_cast<const MV *>(merged)[it.w - 1] : MaskVec<MW>::all();
+    // the records of kBinGather x 32 items at a time: all their items' loads, then
+    // all their masks', before the first is used
+    for (uint32_t i0 = lane; i0 < n + lane; i0 += 32 * kBinGather) {
+        int4 it[kBinGather];
+        MV m[kBinGather];
+#pragma unroll
+        for (int r = 0; r < kBinGather; ++r) {
+            const uint32_t i = min(i0 + 32 * r, n - 1);
+            it[r] = __ldg(draw + (regs ? st[bin_sort_at(i)] : run[i]));
+        }
+#pragma unroll
+        for (int r = 0; r < kBinGather; ++r) {
+            m[r] = MaskVec<MW>::all();
+            if (it[r].w != 0) m[r] = __ldg(reinterpret_cast<const MV *>(merged) + (it[r].w - 1));
+        }
+#pragma unroll
+        for (int r = 0; r < kBinGather; ++r) {
+            const uint32_t i = i0 + 32 * r;
+            if (i >= n) break;
+            const uint32_t ro = (uint32_t)(((it[r].x >> 16) / 2) & band_mask);  // the item's cell row within the band
+            rec_a[beg + i] = make_uint2((uint32_t)it[r].z,
+                                        ((uint32_t)it[r].x & 0xFFFFu) | ((uint32_t)it[r].y << 16) | (ro << 29));
+            rec_m[beg + i] = m[r];
+        }
     }
 }
 
