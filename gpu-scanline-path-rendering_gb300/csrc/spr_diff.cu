@@ -469,18 +469,22 @@ __device__ __forceinline__ void add_span(Affine &run, const float4 &f) {
                         f.w * f.w + run.b.w * om);
     run.a *= om;
 }
-constexpr float kNoSpans = -1.f;  // in place of a run's factor: the run holds no span
+// In place of a run's factor: the run holds no span.  Any value can be a factor
+// (alpha has no range: the product of 1 - alpha goes below zero past alpha 1), so
+// the mark is a NaN that no operation returns (theirs is 0x7FFFFFFF), told by its bits.
+constexpr uint32_t kNoSpans = 0xFFFFFFFFu;
+__device__ __forceinline__ bool no_spans(float ra) { return __float_as_uint(ra) == kNoSpans; }
 
 // First pass over a unit's items, a lane per cell (at column x).  A span covers
 // every sample of a cell, so the spans between two fragments of a cell are one
 // affine map of its samples' state: the map before each fragment goes to
 // d.run_b / d.run_a at the fragment's place (a fragment is in one cell), with
 // the places of the cell's next and (backward) previous fragments, the map after
-// the last one is returned (a = kNoSpans: no spans).  ends: the cell's first and
+// the last one is returned (no_spans(a): none).  ends: the cell's first and
 // last fragment, if it has n_frags > 0.
 __device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, int &n_frags,
                                             uint2 &ends) {
-    const Affine none{kNoSpans, make_float4(0.f, 0.f, 0.f, 0.f)};
+    const Affine none{__uint_as_float(kNoSpans), make_float4(0.f, 0.f, 0.f, 0.f)};
     const int lane = threadIdx.x & 31;
     Affine run = none;
     n_frags = 0;
@@ -496,7 +500,7 @@ __device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bo
             if (cols >> 16) {  // (uniform) a span
                 const float4 f = shfl_fill(my_fill, q);
                 if (touch) {
-                    if (run.a < 0.f) run.a = 1.f;
+                    if (no_spans(run.a)) run.a = 1.f;
                     add_span(run, f);
                 }
             } else if (touch) {
@@ -519,7 +523,7 @@ __device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bo
 
 template <int SPT>
 __device__ __forceinline__ void apply_run(float4 (&c)[SPT], float ra, const float4 &rb) {
-    if (ra < 0.f) return;  // (uniform: no spans)
+    if (no_spans(ra)) return;  // (uniform)
 #pragma unroll
     for (int k = 0; k < SPT; ++k)
         c[k] = make_float4(ra * c[k].x + rb.x, ra * c[k].y + rb.y, ra * c[k].z + rb.z, ra * c[k].w + rb.w);
@@ -728,7 +732,7 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
             float4 cb[SPT];
 #pragma unroll
             for (int k = 0; k < SPT; ++k) cb[k] = tape[((size_t)slot * SPT + k) * 32];
-            if (ra >= 0.f) {  // (uniform) the run of spans that follows starts where the fragment ends
+            if (!no_spans(ra)) {  // (uniform) the run of spans that follows starts where the fragment ends
 #pragma unroll
                 for (int k = 0; k < SPT; ++k) c[k] = cb[k];
                 apply_fragment<S>(c, f, m, sub);
@@ -772,7 +776,7 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
             if (p == cell.first) break;
             p = prev;
         }
-        if (ra >= 0.f) {  // the first run
+        if (!no_spans(ra)) {  // the first run
             float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int k = 0; k < SPT; ++k) {

@@ -298,7 +298,7 @@ struct DiffArgs {
     const float2 *tvert;
     int64_t nf;
     // per resolve pair that is a fragment: the affine map of the spans before it
-    // in its cell (c -> run_a c + run_b; run_a < 0: none) and, backward, the sums
+    // in its cell (c -> run_a c + run_b; run_a marked where there are none) and, backward, the sums
     // of the run after it (2 per pair); the pairs of its cell's next and
     // (backward) previous fragments
     float *run_a;
