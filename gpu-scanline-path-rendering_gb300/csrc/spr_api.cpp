@@ -126,7 +126,7 @@ struct spr_handle {
     // differentiable frames: per-fragment chords and left masks, per-item
     // paths, the per-block tapes, the transformed-vertex gradient and the
     // stored -> input vertex map
-    DevBuf chord, lmask, vmask, item_path, tape, run_pi, bruns, dcells, grad_tvert, vmap, bitems, chain, ekey[2], eval[2];
+    DevBuf chord, lmask, vmask, item_path, tape, run_pi, bruns, dcells, grad_tvert, vmap, bitems, chain, fill_sum, ekey[2], eval[2];
     // 256-sample frames: the pass being rendered, the passes' fixed-point
     // sample sums, and a pass's fill gradient / the summed vertex gradient
     int pass = 0;
@@ -220,7 +220,7 @@ std::vector<DevBuf *> handle_bufs(spr_handle *h) {
                       &h->rec_a,      &h->rec_m,   &h->bins,
                       &h->image,      &h->counters, &h->dump_tmp, &h->overflow, &h->scenes_d, &h->path_scene,
                       &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->run_pi, &h->bruns, &h->dcells,
-                      &h->grad_tvert, &h->vmap, &h->bitems, &h->vmask, &h->chain, &h->ekey[0], &h->ekey[1], &h->eval[0],
+                      &h->grad_tvert, &h->vmap, &h->bitems, &h->vmask, &h->chain, &h->fill_sum, &h->ekey[0], &h->ekey[1], &h->eval[0],
                       &h->eval[1], &h->sc_vpos, &h->sc_type, &h->sc_pid, &h->sc_w, &h->scene_flags,
                       &h->sums, &h->gfill_pass, &h->gtvert_total, &h->grad_table, &h->grad_ramp, &h->path_start, &h->seg_list,
                       &h->output, &h->lb_mark, &h->lb_pair};
@@ -707,7 +707,10 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
     }
     int st = ensure(h->grad_tvert, 8 * (size_t)std::max<uint32_t>(h->V, 1));
     if (st) return st;
-    if ((st = ensure(h->chain, 8 * (size_t)std::max<int64_t>(h->nf, 1)))) return st;
+    if ((st = ensure(h->chain, 8 * (size_t)std::max<int64_t>(h->nf, 1))) ||
+        (st = ensure(h->fill_sum, 32 * (size_t)std::max<uint32_t>(h->P, 1))))
+        return st;
+    d.fill_sum = h->fill_sum.as<double>();
     d.grad_tvert = h->grad_tvert.as<float2>();
     const bool multi = dc.passes > 1;  // the pass's gradients go to staging buffers first
     if (multi) {
@@ -727,7 +730,7 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.run_pi = h->run_pi.as<float>();
         d.tape_depth = h->tape_depth;
         d.pi_depth = h->pi_depth;
-        cudaMemsetAsync(d.grad_fill, 0, 16 * (size_t)h->P, s);
+        cudaMemsetAsync(d.fill_sum, 0, 32 * (size_t)h->P, s);
         cudaMemsetAsync(h->grad_tvert.p, 0, 8 * (size_t)h->V, s);
         cudaMemsetAsync(&ctr->diff_status, 0, 4, s);
         cudaMemsetAsync(d.chain, 0, 8 * (size_t)h->nf, s);

@@ -16,7 +16,10 @@
 // sample's cell is recorded in draw order and swept in reverse with the adjoint
 // lambda of the state (lambda *= 1 - a through every covering item), giving the
 // exact fill gradients (the spans' in a last pass, from two sums per run of
-// them).  Geometry is
+// them).  A path has up to millions of fragments and spans, whose shares of its fill
+// gradient are added to memory one by one: in 64 bits, where their order and number
+// do not show (in 32 bits the gradient of a path of 1,500 curves was off by 3e-6, ten
+// times its shares' own rounding).  Geometry is
 // differentiated by edge sampling: a pixel is taken as the mean over its S
 // sample rows of the row integral of the composite, so moving the crossing
 // x_c of a chord with sample row y_r by dx changes the pixel by
@@ -404,9 +407,11 @@ __global__ void k_diff_gather(DiffArgs d, int words) {
     d.bmm[p] = it.w != 0 ? load_merged(d.merged, words, (uint32_t)it.w - 1u) : make_uint4(0u, 0u, 0u, 0u);
 }
 
-// The crossing sums of every fragment chained to its curve's control points.
+// The crossing sums of every fragment chained to its curve's control points, and
+// the fill gradients from their sums.
 __global__ void k_diff_chain(FrameArgs a, DiffArgs d) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 4 * (int64_t)a.P) reinterpret_cast<float *>(d.grad_fill)[i] = (float)d.fill_sum[i];
     if (i >= d.nf) return;
     const float2 r = d.chain[i];
     if (r.x == 0.f && r.y == 0.f) return;
@@ -771,7 +776,7 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
             group_adjoint<S>(a, d, (int64_t)it.y, head, a.fill_rule[it.w], J, lane);
             const float sum = scattered_sums<4>(gf, lane);
             if ((lane & 7) == 0 && sum != 0.f)
-                atomicAdd(reinterpret_cast<float *>(d.grad_fill + it.w) + (lane >> 3), sum);
+                atomicAdd(d.fill_sum + 4 * (size_t)it.w + (lane >> 3), (double)sum);
             ra = next_ra;
             if (p == cell.first) break;
             p = prev;
@@ -888,7 +893,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
                 if (!__any_sync(0xffffffffu, any)) continue;
                 reduce_scatter<16, 16, 32>(v, lane);  // lane i: the sum of value i
                 const uint32_t path = __shfl_sync(0xffffffffu, my_it.w, min(q0 + (lane >> 2), 31));
-                if (v[0] != 0.f) atomicAdd(reinterpret_cast<float *>(d.grad_fill + path) + (lane & 3), v[0]);
+                if (v[0] != 0.f) atomicAdd(d.fill_sum + 4 * (size_t)path + (lane & 3), (double)v[0]);
             }
         }
     }
@@ -999,8 +1004,9 @@ int launch_diff(const FrameArgs &a, const DiffArgs &d, cudaStream_t s) {
         k_diff_spans<<<bin_grid, kDiffThreads, 0, s>>>(a, d);
         ++n;
     }
-    if (BWD && d.nf > 0) {
-        k_diff_chain<<<(unsigned)((d.nf + 255) / 256), 256, 0, s>>>(a, d);
+    const int64_t chain = std::max<int64_t>(d.nf, 4 * (int64_t)a.P);
+    if (BWD && chain > 0) {
+        k_diff_chain<<<(unsigned)((chain + 255) / 256), 256, 0, s>>>(a, d);
         ++n;
     }
     return n;

@@ -277,6 +277,7 @@ struct DiffArgs {
     const float4 *grad_image;  // backward input, dL/d(pixel), W x H
     float4 *image;             // forward output, W x H
     float4 *grad_fill;         // per path
+    double *fill_sum;          // 4 per path (zero before): the sums grad_fill is made from
     float2 *grad_tvert;        // per stored vertex, in transformed space
     const int4 *draw;
     const uint32_t *merged;
