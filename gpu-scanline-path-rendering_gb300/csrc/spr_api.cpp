@@ -720,16 +720,18 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.grad_fill = h->gfill_pass.as<float4>();
     }
     d.chain = h->chain.as<float2>();
+    // the depths grow until the frame fits, and the handle keeps those that served
+    // (a growth that is refused leaves it as it was)
+    d.tape_depth = h->tape_depth;
+    d.pi_depth = h->pi_depth;
     // (most bins hold fewer than four times the mean of items)
-    while (h->pi_depth < 4 * (d.npairs / std::max<int64_t>(a.n_bins, 1)) && h->pi_depth < (1 << 16)) h->pi_depth *= 2;
+    while (d.pi_depth < 4 * (d.npairs / std::max<int64_t>(a.n_bins, 1)) && d.pi_depth < (1 << 16)) d.pi_depth *= 2;
     for (;;) {
-        if ((st = ensure(h->tape, 16 * (size_t)diff_tape_words(a, h->tape_depth))) ||
-            (st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, h->pi_depth))))
+        if ((st = ensure(h->tape, 16 * (size_t)diff_tape_words(a, d.tape_depth))) ||
+            (st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, d.pi_depth))))
             return st;
         d.tape = h->tape.as<float4>();
         d.run_pi = h->run_pi.as<float>();
-        d.tape_depth = h->tape_depth;
-        d.pi_depth = h->pi_depth;
         cudaMemsetAsync(d.fill_sum, 0, 32 * (size_t)h->P, s);
         cudaMemsetAsync(h->grad_tvert.p, 0, 8 * (size_t)h->V, s);
         cudaMemsetAsync(&ctr->diff_status, 0, 4, s);
@@ -740,9 +742,11 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
         const uint32_t status = h->h_u32[0];
         if (status == 0u) break;
-        if ((status & 1u) && (h->tape_depth *= 2) > (1 << 17)) return SPR_ERR_CAPACITY_EXCEEDED;
-        if ((status & 2u) && (h->pi_depth *= 2) > (1 << 24)) return SPR_ERR_CAPACITY_EXCEEDED;
+        if ((status & 1u) && (d.tape_depth *= 2) > (1 << 17)) return SPR_ERR_CAPACITY_EXCEEDED;
+        if ((status & 2u) && (d.pi_depth *= 2) > (1 << 24)) return SPR_ERR_CAPACITY_EXCEEDED;
     }
+    h->tape_depth = d.tape_depth;
+    h->pi_depth = d.pi_depth;
     const float2 *gt = h->grad_tvert.as<float2>();
     if (multi) {
         *L += launch_accumulate(dc.grad_fill, reinterpret_cast<float *>(d.grad_fill), 4 * (int64_t)h->P, dc.pass == 0,
