@@ -152,7 +152,7 @@ struct spr_handle {
     // raw curve arrays of the device-side scene upload (kept for vertex updates)
     DevBuf sc_vpos, sc_type, sc_pid, sc_w, scene_flags;
     bool scene_on_device = false, scene_has_arcw = false;
-    int tape_depth = 64, pi_depth = 128;  // (grown by the backward as its frames need)
+    int tape_depth = 64;  // (grown by the backward as its frames need)
     // frame buffers
     DevBuf tvert, pvis, counts, offsets, scan_tmp, entries, key, pidw, wn, mask, skey[2], sval[2], sort_tmp,
         wn_scan, draw, heads, merged, pval, rec_a, rec_m, bins, image, counters, dump_tmp, overflow;
@@ -720,18 +720,14 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.grad_fill = h->gfill_pass.as<float4>();
     }
     d.chain = h->chain.as<float2>();
-    // the depths grow until the frame fits, and the handle keeps those that served
+    if ((st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, d.npairs)))) return st;
+    d.run_pi = h->run_pi.as<float>();
+    // the depth grows until the frame fits, and the handle keeps the one that served
     // (a growth that is refused leaves it as it was)
     d.tape_depth = h->tape_depth;
-    d.pi_depth = h->pi_depth;
-    // (most bins hold fewer than four times the mean of items)
-    while (d.pi_depth < 4 * (d.npairs / std::max<int64_t>(a.n_bins, 1)) && d.pi_depth < (1 << 16)) d.pi_depth *= 2;
     for (;;) {
-        if ((st = ensure(h->tape, 16 * (size_t)diff_tape_words(a, d.tape_depth))) ||
-            (st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, d.pi_depth))))
-            return st;
+        if ((st = ensure(h->tape, 16 * (size_t)diff_tape_words(a, d.tape_depth)))) return st;
         d.tape = h->tape.as<float4>();
-        d.run_pi = h->run_pi.as<float>();
         cudaMemsetAsync(d.fill_sum, 0, 32 * (size_t)h->P, s);
         cudaMemsetAsync(h->grad_tvert.p, 0, 8 * (size_t)h->V, s);
         cudaMemsetAsync(&ctr->diff_status, 0, 4, s);
@@ -740,13 +736,10 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         cudaMemcpyAsync(h->h_u32, &ctr->diff_status, 4, cudaMemcpyDeviceToHost, s);
         ++h->host_syncs;
         if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
-        const uint32_t status = h->h_u32[0];
-        if (status == 0u) break;
-        if ((status & 1u) && (d.tape_depth *= 2) > (1 << 17)) return SPR_ERR_CAPACITY_EXCEEDED;
-        if ((status & 2u) && (d.pi_depth *= 2) > (1 << 24)) return SPR_ERR_CAPACITY_EXCEEDED;
+        if (h->h_u32[0] == 0u) break;
+        if ((d.tape_depth *= 2) > (1 << 17)) return SPR_ERR_CAPACITY_EXCEEDED;
     }
     h->tape_depth = d.tape_depth;
-    h->pi_depth = d.pi_depth;
     const float2 *gt = h->grad_tvert.as<float2>();
     if (multi) {
         *L += launch_accumulate(dc.grad_fill, reinterpret_cast<float *>(d.grad_fill), 4 * (int64_t)h->P, dc.pass == 0,

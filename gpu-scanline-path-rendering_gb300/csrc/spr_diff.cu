@@ -801,22 +801,26 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
 // the run's later spans (found first, in reverse), so a span's gradient needs
 // only its run's sums (c before the span = ra * c_run + rb); it is summed over
 // the unit's cells before it goes to memory.
+// The factors pi of 32 items and 32 cells are held in shared memory.  The first
+// sweep, from the bin's end, leaves pi at the end of every 32 items in memory, and
+// the forward sweep finds those of its 32 items again from there: 4 bytes a pair,
+// where a factor for every item and cell took a buffer of the deepest bin's items
+// for every warp (2.5 GB for a bin of 4,096).
 __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffArgs d) {
     const int lane = threadIdx.x & 31;
-    const size_t wslot = (size_t)blockIdx.x * (kDiffThreads / 32) + (threadIdx.x >> 5);
-    float *const pis = d.run_pi + wslot * (size_t)d.pi_depth * 32 + lane;  // item i: [i * 32]
+    __shared__ float s_pi[kDiffThreads / 32][32][32];  // item, cell
+    float(*const pis)[32] = s_pi[threadIdx.x >> 5];
     Unit u;
     while (next_unit(a, d, lane, u)) {
         if (u.fin == u.beg) continue;
-        if (u.fin - u.beg > (uint32_t)d.pi_depth) {
-            if (lane == 0) atomicOr(d.status, 2u);
-            continue;
-        }
         const bool active = lane < u.cells;
         const int x = u.x0 + 2 * lane;
-        float pi = 1.f;
+        // pi at the end of the bin's items from base on, 32 at a time: [base - u.beg]
+        // (a bin's place: past the earlier bins' items and 32 for each of them)
+        float *const ends = d.run_pi + ((size_t)(u.beg & ~31u) + u.cell0 + lane);
         bool frags = false;
-        for (uint32_t base = u.beg + ((u.fin - u.beg - 1) & ~31u);; base -= 32) {
+        // pi before each of the 32 items from base on, given that after them
+        auto sweep = [&](uint32_t base, float pi) {
             const uint32_t mine = min(base + lane, u.fin - 1);
             const uint32_t my_cols = item_cols(__ldg(&d.bitem[mine]));
             const float my_a = __ldg(&d.bfill[mine].w);
@@ -828,12 +832,18 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
                     pi = 1.f;
                     frags = true;
                 } else {
-                    pis[(size_t)(base + q - u.beg) * 32] = pi;
+                    pis[q][lane] = pi;
                     pi *= om;
                 }
             }
-            if (base == u.beg) break;
+            return pi;
+        };
+        float pi = 1.f;
+        for (uint32_t base = u.beg + ((u.fin - u.beg - 1) & ~31u); base != u.beg; base -= 32) {
+            ends[base - u.beg] = pi;
+            pi = sweep(base, pi);
         }
+        sweep(u.beg, pi);
         // the sums of the cell's first run, whose samples start white (not
         // used if that run is empty); of a cell without fragments: the pixels'
         // adjoints
@@ -854,6 +864,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
         float4 Ks = Ls;
         Affine run{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
         for (uint32_t base = u.beg; base < u.fin; base += 32) {
+            if (base != u.beg) sweep(base, ends[base - u.beg]);
             const uint32_t mine = min(base + lane, u.fin - 1);
             const uint4 my_it = __ldg(&d.bitem[mine]);
             const uint32_t my_cols = item_cols(my_it);
@@ -880,7 +891,7 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
                     const float4 f = shfl_fill(my_fill, q);
                     if (touch) {
                         any = true;
-                        const float pl = pis[(p - u.beg) * 32], av = f.w;
+                        const float pl = pis[q][lane], av = f.w;
                         const float cx = run.a * Ks.x + run.b.x * Ls.x, cy = run.a * Ks.y + run.b.y * Ls.y;
                         const float cz = run.a * Ks.z + run.b.z * Ls.z, cw = run.a * Ks.w + run.b.w * Ls.w;
                         v[4 * j] = pl * av * Ls.x;
@@ -1024,7 +1035,7 @@ int64_t diff_tape_words(const FrameArgs &a, int depth) {
     return diff_blocks(a) * (int64_t)depth * (a.S / 8) * kDiffThreads;
 }
 
-int64_t diff_pi_words(const FrameArgs &a, int depth) { return diff_blocks(a) * (int64_t)depth * kDiffThreads; }
+int64_t diff_pi_words(const FrameArgs &a, int64_t npairs) { return npairs + a.n_bins * (kTileW / 2); }
 
 __global__ void k_accumulate(float *__restrict__ dst, const float *__restrict__ src, int64_t n, int first) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

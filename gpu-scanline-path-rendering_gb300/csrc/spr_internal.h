@@ -312,14 +312,13 @@ struct DiffArgs {
     uint2 *cell_ends;
     float *cell_a;
     float4 *cell_b, *cell_sum;
-    // per warp: tape_depth x (samples per thread) x 32 sample states, and pi_depth
-    // x 32 span factors (backward)
+    // per warp: tape_depth x (samples per thread) x 32 sample states (backward)
     float4 *tape;
-    float *run_pi;
-    int tape_depth, pi_depth;
+    int tape_depth;
+    float *run_pi;  // per bin, 32 of its items and cell: the spans' factor at their end (backward)
     uint32_t *queue;     // unit queue; then the cell list's length and its queue (zeroed by the launchers)
     uint32_t *n_cells, *cell_queue;
-    uint32_t *status;    // bit 0: a cell has more fragments than tape_depth, bit 1: a bin more items than pi_depth (rerun with more)
+    uint32_t *status;    // bit 0: a cell has more fragments than tape_depth (rerun with more)
     // pixel = out_scale * (mean of the samples), added to the image when
     // accumulate (the passes of a 256-sample frame: 1/8 each); the backward
     // takes out_scale * dL/d(pixel) likewise
@@ -328,7 +327,7 @@ struct DiffArgs {
 };
 int64_t diff_blocks(const FrameArgs &a);
 int64_t diff_tape_words(const FrameArgs &a, int depth);      // float4 count of the sample-state tape
-int64_t diff_pi_words(const FrameArgs &a, int depth);        // float count of the span factors
+int64_t diff_pi_words(const FrameArgs &a, int64_t npairs);   // float count of the span factors
 int launch_diff_forward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 int launch_diff_backward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 // dL/d(stored vertex in transformed space) -> dL/d(input vertex), dL/d(path affine).

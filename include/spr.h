@@ -396,8 +396,7 @@ int spr_diff_render(spr_handle *h, const float *fill_rgba, float *image, void *s
  * step timing off) the backward reuses that frame's coverage stages and runs
  * the adjoint kernels only; otherwise every stage is recomputed.  256-sample
  * frames always recompute their 8 passes.  The tape of the cells'
- * fragments and the span factors grow by themselves (one extra readback per
- * doubling). */
+ * fragments grows by itself (one extra readback per doubling). */
 int spr_diff_backward(spr_handle *h, const float *fill_rgba, const float *grad_image, float *grad_fill,
                       float *grad_vertex, float *grad_affine, void *stream);
 /* New positions of the scene's vertices (2 floats per vertex, in the scene's

@@ -62,3 +62,61 @@ def test_a_refused_growth_does_not_stick():
             deep.render(r)
             deep.backward(r)
             deep.check()
+
+
+def marks(n, x0, y0, w, rng):
+    """n small quadrilaterals in the band of rows y0, y0 + 1: curves and paths."""
+    pts, pid = [], []
+    for p in range(n):
+        cx, cy = x0 + rng.uniform(0.2, w - 0.2), y0 + rng.uniform(0.2, 1.8)
+        q = [(cx - .15, cy - .15), (cx + .15, cy - .1), (cx + .1, cy + .15), (cx - .1, cy + .1)]
+        for k in range(4):
+            pts += [q[k], q[(k + 1) % 4]]
+            pid.append(p)
+    return pts, pid
+
+
+def line_scene(pts, pid):
+    m, n = len(pid), pid[-1] + 1
+    return spr.Scene(np.asarray(pts, np.float32), np.repeat(pid, 2), 2 * np.arange(m), np.full(m, spr.CURVE_LINEAR), pid,
+                     np.zeros(m), np.zeros(n), np.full(n, 0xFF808080))
+
+
+def test_one_crowded_bin_under_a_limit():
+    """4,096 paths in one bin of 8,192, some 130 to a cell: buffers by the items
+    there are, not by the deepest bin for every warp.  (Under this limit the
+    tape, 64 -> 256 fragments deep, is the largest: 800 MB.)"""
+    W = H = 1024
+    fit = Fit(line_scene(*marks(4096, 64, 100, 62, np.random.default_rng(0))), W, H, 8)
+    with spr.VGRasterizer(W, H, samples=8) as r:
+        r.set_memory_limit(1200 << 20)
+        for _ in range(2):
+            fit.render(r)
+            fit.backward(r)
+            fit.check()
+
+
+@pytest.mark.parametrize("samples", [8, 32])
+def test_crowded_band_among_empty_ones(samples):
+    """500 slanted boxes along one band of a tall viewport, and 80 marks in one of
+    its cells: bins of ten to twenty times the mean of items, and a tape that grows."""
+    W, H = 192, 512
+    rng = np.random.default_rng(4)
+    pts, pid = [], []
+    for p in range(500):
+        x0, x1 = rng.uniform(-5, W * 0.3), rng.uniform(W * 0.6, W + 5)
+        q = [(x0, 198), (x1, 198.5), (x1 - rng.uniform(0, 6), 204), (x0 + rng.uniform(0, 6), 204)]
+        for k in range(4):
+            pts += [q[k], q[(k + 1) % 4]]
+            pid.append(p)
+    pm, im = marks(80, 100, 200, 2, rng)
+    fit = Fit(line_scene(pts + pm, pid + [500 + p for p in im]), W, H, samples)
+    with spr.VGRasterizer(W, H, samples=samples) as r:
+        fit.render(r)
+        fit.backward(r)
+        assert r.frame_stats()["host_syncs"] > 1  # (more than 64 fragments in a cell)
+        fit.check()
+        fit.render(r)
+        fit.backward(r)
+        assert r.frame_stats()["host_syncs"] == 1
+        fit.check()
