@@ -126,7 +126,7 @@ struct spr_handle {
     // differentiable frames: per-fragment chords and left masks, per-item
     // paths, the per-block tapes, the transformed-vertex gradient and the
     // stored -> input vertex map
-    DevBuf chord, lmask, vmask, item_path, tape, run_pi, bruns, dcells, grad_tvert, vmap, bitems, chain, fill_sum, ekey[2], eval[2];
+    DevBuf chord, lmask, vmask, item_path, tape, bruns, dcells, dparts, grad_tvert, vmap, bitems, chain, fill_sum, ekey[2], eval[2];
     // 256-sample frames: the pass being rendered, the passes' fixed-point
     // sample sums, and a pass's fill gradient / the summed vertex gradient
     int pass = 0;
@@ -219,7 +219,7 @@ std::vector<DevBuf *> handle_bufs(spr_handle *h) {
                       &h->wn_scan,    &h->draw,    &h->heads,    &h->merged,  &h->pval,
                       &h->rec_a,      &h->rec_m,   &h->bins,
                       &h->image,      &h->counters, &h->dump_tmp, &h->overflow, &h->scenes_d, &h->path_scene,
-                      &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->run_pi, &h->bruns, &h->dcells,
+                      &h->item_scene, &h->chord,  &h->lmask,   &h->item_path, &h->tape,  &h->bruns, &h->dcells, &h->dparts,
                       &h->grad_tvert, &h->vmap, &h->bitems, &h->vmask, &h->chain, &h->fill_sum, &h->ekey[0], &h->ekey[1], &h->eval[0],
                       &h->eval[1], &h->sc_vpos, &h->sc_type, &h->sc_pid, &h->sc_w, &h->scene_flags,
                       &h->sums, &h->gfill_pass, &h->gtvert_total, &h->grad_table, &h->grad_ramp, &h->path_start, &h->seg_list,
@@ -687,6 +687,19 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
     d.queue = ctr->diff_queue;
     d.n_cells = d.queue + 1;
     d.cell_queue = d.queue + 2;
+    d.n_parts = d.queue + 3;
+    // per part of a bin with many items: 32 cells' runs, ends and (backward) factors, and the part itself; per bin: the parts done
+    const int64_t parts = diff_parts(d.npairs);
+    if (parts > 0) {
+        int st = ensure(h->dparts, (dc.backward ? 1032 : 904) * (size_t)parts + 4 * (size_t)a.n_bins);
+        if (st) return st;
+        d.part_b = h->dparts.as<float4>();
+        d.part_ends = reinterpret_cast<uint2 *>(d.part_b + 32 * parts);
+        d.part = d.part_ends + 32 * parts;
+        d.part_a = reinterpret_cast<float *>(d.part + parts);
+        d.part_pi = dc.backward ? d.part_a + 32 * parts : nullptr;
+        d.part_done = reinterpret_cast<uint32_t *>(d.part_a + (dc.backward ? 64 : 32) * parts);
+    }
     // per cell of the bins: its place in the list, the run map, the adjoint sum and the first and last fragments
     const int64_t cells = a.n_bins * 32;
     {
@@ -720,8 +733,6 @@ int diff_stage(spr_handle *h, const FrameArgs &a, const DiffCall &dc, const uint
         d.grad_fill = h->gfill_pass.as<float4>();
     }
     d.chain = h->chain.as<float2>();
-    if ((st = ensure(h->run_pi, 4 * (size_t)diff_pi_words(a, d.npairs)))) return st;
-    d.run_pi = h->run_pi.as<float>();
     // the depth grows until the frame fits, and the handle keeps the one that served
     // (a growth that is refused leaves it as it was)
     d.tape_depth = h->tape_depth;

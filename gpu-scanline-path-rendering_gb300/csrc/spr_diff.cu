@@ -45,6 +45,11 @@ namespace {
 
 constexpr int kDiffThreads = 256;    // 8 warps, each working on its own cells
 constexpr int kTileW = kBinW;  // columns of a resolve bin
+// Items that a warp takes of a bin, at most, in the passes with a lane per cell.
+// Forward and backward of 2,000 paths over 256 x 256, of 4,096 paths in one bin of
+// 1024 x 1024 and of a batch of 16 scenes, us: a warp to a bin 8793, 3784 and 4514;
+// 256 items 3902, 1634 and 4560; 128 items 3954, 1604 and 4507.
+constexpr uint32_t kPartItems = 128;
 
 __device__ __forceinline__ uint32_t pixel_mask(const uint4 &mm, int S, int k) {
     if (S == 32) return k == 0 ? mm.x : (k == 1 ? mm.y : (k == 2 ? mm.z : mm.w));
@@ -394,9 +399,18 @@ __device__ __forceinline__ BinScene bin_scene(const FrameArgs &a, uint32_t b) {
     return r;
 }
 
-// The items of the resolve pairs in bin order, one contiguous record each.
-__global__ void k_diff_gather(DiffArgs d, int words) {
+// The items of the resolve pairs in bin order, one contiguous record each, and the
+// parts of the bins that have more than kPartItems.
+__global__ void k_diff_gather(DiffArgs d, int words, int64_t n_bins) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n_bins) {
+        const uint32_t n = d.bend[p] - d.bstart[p];
+        if (n > kPartItems) {
+            const uint32_t parts = (n + kPartItems - 1) / kPartItems, at = atomicAdd(d.n_parts, parts);
+            d.part_done[p] = 0u;
+            for (uint32_t k = 0; k < parts; ++k) d.part[at + k] = make_uint2((uint32_t)p, k);
+        }
+    }
     if (p >= d.npairs) return;
     const uint32_t idx = d.pval[p];
     const int4 it = d.draw[idx];
@@ -419,20 +433,42 @@ __global__ void k_diff_chain(FrameArgs a, DiffArgs d) {
     fragment_chain(a, d, (uint32_t)i, (c.z - c.x) / (c.w - c.y), r.x, r.y);
 }
 
-// A bin of the passes with a lane per cell, taken by a warp from a queue.
+// A bin of the passes with a lane per cell, or kPartItems items of a bin that has
+// more, taken by a warp from a queue (the parts first).  Such a bin's parts are
+// worked on by different warps: 2,000 paths over 256 x 256 have 3,300 items a bin
+// and 512 bins, and a warp to each of them left most of the chip idle.
 struct Unit {
     BinScene bs;
-    uint32_t beg, fin;  // the bin's items
+    uint32_t bin, part, parts;  // part of parts (one: the whole bin)
+    uint32_t place;     // ... its place in the list of parts
+    uint32_t beg, fin;  // its items
     uint32_t cell0;     // the first cell's number (bin * cells of a bin + column)
     int x0, y0, cells;  // its pixel; cells within the viewport
 };
-__device__ __forceinline__ bool next_unit(const FrameArgs &a, const DiffArgs &d, int lane, Unit &u) {
-    uint32_t b = 0;
-    if (lane == 0) b = atomicAdd(d.queue, 1u);
-    b = __shfl_sync(0xffffffffu, b, 0);
-    if ((int64_t)b >= a.n_bins) return false;
-    u.beg = d.bstart[b];
-    u.fin = d.bend[b];
+__device__ __forceinline__ bool next_unit(const FrameArgs &a, const DiffArgs &d, uint32_t n_parts, int lane, Unit &u) {
+    uint32_t b, n;
+    for (;;) {
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(d.queue, 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        u.place = k;
+        u.part = 0u;
+        if (k < n_parts) {
+            const uint2 e = __ldg(&d.part[k]);
+            b = e.x;
+            u.part = e.y;
+        } else {
+            if ((int64_t)(k - n_parts) >= a.n_bins) return false;
+            b = k - n_parts;
+        }
+        u.beg = d.bstart[b];
+        n = d.bend[b] - u.beg;
+        if (k < n_parts || n <= kPartItems) break;
+    }
+    u.bin = b;
+    u.parts = max((n + kPartItems - 1) / kPartItems, 1u);
+    u.beg += u.part * kPartItems;
+    u.fin = u.beg + min(n - u.part * kPartItems, kPartItems);
     u.bs = bin_scene(a, b);
     const int ntx = (u.bs.W + kTileW - 1) / kTileW, tile = (int)(u.bs.lb % ntx);
     u.cell0 = b * (kTileW / 2);
@@ -479,6 +515,24 @@ __device__ __forceinline__ void add_span(Affine &run, const float4 &f) {
 // the mark is a NaN that no operation returns (theirs is 0x7FFFFFFF), told by its bits.
 constexpr uint32_t kNoSpans = 0xFFFFFFFFu;
 __device__ __forceinline__ bool no_spans(float ra) { return __float_as_uint(ra) == kNoSpans; }
+__device__ __forceinline__ Affine empty_run() {
+    return Affine{__uint_as_float(kNoSpans), make_float4(0.f, 0.f, 0.f, 0.f)};
+}
+// The run f, then the run g.
+__device__ __forceinline__ Affine run_then(const Affine &f, const Affine &g) {
+    if (no_spans(f.a)) return g;
+    if (no_spans(g.a)) return f;
+    return Affine{f.a * g.a, make_float4(g.a * f.b.x + g.b.x, g.a * f.b.y + g.b.y, g.a * f.b.z + g.b.z,
+                                         g.a * f.b.w + g.b.w)};
+}
+constexpr uint32_t kNoFragment = 0xFFFFFFFFu;  // in place of a fragment's place: there is none ...
+constexpr uint32_t kLaterFragment = 0xFFFFFFFEu;  // ... before, but the cell has some
+
+// Fragment p follows fragment prev in their cell.
+__device__ __forceinline__ void link(const DiffArgs &d, uint32_t prev, uint32_t p) {
+    d.run_next[prev] = p;
+    if (d.run_prev != nullptr) d.run_prev[p] = prev;
+}
 
 // First pass over a unit's items, a lane per cell (at column x).  A span covers
 // every sample of a cell, so the spans between two fragments of a cell are one
@@ -486,14 +540,11 @@ __device__ __forceinline__ bool no_spans(float ra) { return __float_as_uint(ra) 
 // d.run_b / d.run_a at the fragment's place (a fragment is in one cell), with
 // the places of the cell's next and (backward) previous fragments, the map after
 // the last one is returned (no_spans(a): none).  ends: the cell's first and
-// last fragment, if it has n_frags > 0.
-__device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, int &n_frags,
-                                            uint2 &ends) {
-    const Affine none{__uint_as_float(kNoSpans), make_float4(0.f, 0.f, 0.f, 0.f)};
+// last fragment, if it has any (kNoFragment otherwise).
+__device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bool active, int x, uint2 &ends) {
     const int lane = threadIdx.x & 31;
-    Affine run = none;
-    n_frags = 0;
-    ends = make_uint2(0u, 0u);
+    Affine run = empty_run();
+    ends = make_uint2(kNoFragment, kNoFragment);
     for (uint32_t base = u.beg; base < u.fin; base += 32) {
         const uint32_t mine = min(base + lane, u.fin - 1);
         const uint32_t my_cols = item_cols(__ldg(&d.bitem[mine]));
@@ -512,18 +563,73 @@ __device__ __forceinline__ Affine cell_runs(const DiffArgs &d, const Unit &u, bo
                 const uint32_t p = base + q;
                 d.run_b[p] = run.b;
                 d.run_a[p] = run.a;
-                if (n_frags++ == 0) {
-                    ends.x = p;
-                } else {
-                    d.run_next[ends.y] = p;
-                    if (d.run_prev != nullptr) d.run_prev[p] = ends.y;
-                }
+                if (ends.x == kNoFragment) ends.x = p;
+                else link(d, ends.y, p);
                 ends.y = p;
-                run = none;
+                run = empty_run();
             }
         }
     }
     return run;
+}
+
+// A part of a bin is done: its cells' runs after their last fragments (of the whole
+// part, where they have none) and their first and last fragments are left for the
+// warp that finishes the bin's last part, which joins the parts' runs and links
+// (true: as if it had gone through the whole bin; last, ends: the bin's).  For the
+// adjoint's third pass it leaves each part the state that it starts from: the run
+// and the last fragment before it, and the factor of the spans after it.
+__device__ __forceinline__ bool join_parts(const DiffArgs &d, const Unit &u, int lane, Affine &last, uint2 &ends) {
+    const size_t mine = (size_t)u.place * 32 + lane;
+    d.part_b[mine] = last.b;
+    d.part_a[mine] = last.a;
+    d.part_ends[mine] = ends;
+    __threadfence();
+    __syncwarp();
+    uint32_t done = 0;
+    if (lane == 0) done = atomicAdd(&d.part_done[u.bin], 1u);
+    if (__shfl_sync(0xffffffffu, done, 0) + 1u != u.parts) return false;
+    __threadfence();
+    // (written by other warps of this launch: read from L2)
+    const size_t first = (size_t)(u.place - u.part) * 32 + lane;
+    bool frags = false;
+    if (d.part_pi != nullptr) {
+        float pi = 1.f;
+        for (uint32_t k = u.parts; k-- > 0;) {
+            const size_t at = first + (size_t)k * 32;
+            const uint2 e = __ldcg(&d.part_ends[at]);
+            d.part_pi[at] = pi;
+            if (e.x != kNoFragment) pi = 1.f, frags = true;
+            const float f = e.x != kNoFragment ? __ldcg(&d.run_a[e.x]) : __ldcg(&d.part_a[at]);
+            if (!no_spans(f)) pi *= f;
+        }
+    }
+    last = empty_run();
+    ends = make_uint2(kNoFragment, kNoFragment);
+    for (uint32_t k = 0; k < u.parts; ++k) {
+        const size_t at = first + (size_t)k * 32;
+        const uint2 e = __ldcg(&d.part_ends[at]);
+        const Affine run{__ldcg(&d.part_a[at]), __ldcg(&d.part_b[at])};
+        if (d.part_pi != nullptr) {
+            d.part_b[at] = last.b;
+            d.part_a[at] = last.a;
+            d.part_ends[at].x = ends.y != kNoFragment ? ends.y : (frags ? kLaterFragment : kNoFragment);
+        }
+        if (e.x == kNoFragment) {
+            last = run_then(last, run);
+            continue;
+        }
+        if (!no_spans(last.a)) {
+            const Affine lead = run_then(last, Affine{__ldcg(&d.run_a[e.x]), __ldcg(&d.run_b[e.x])});
+            d.run_b[e.x] = lead.b;
+            d.run_a[e.x] = lead.a;
+        }
+        if (ends.x == kNoFragment) ends.x = e.x;
+        else link(d, ends.y, e.x);
+        ends.y = e.y;
+        last = run;
+    }
+    return true;
 }
 
 template <int SPT>
@@ -563,14 +669,16 @@ __device__ __forceinline__ void store_pixel(const DiffArgs &d, int64_t pix, floa
 template <bool FORWARD>
 __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArgs d) {
     const int lane = threadIdx.x & 31;
+    const uint32_t n_parts = *d.n_parts;
     Unit u;
-    while (next_unit(a, d, lane, u)) {
+    while (next_unit(a, d, n_parts, lane, u)) {
         const bool active = lane < u.cells;
         const int x = u.x0 + 2 * lane;
-        int n_frags;
         uint2 ends;
-        const Affine last = cell_runs(d, u, active, x, n_frags, ends);
-        if (FORWARD && active && n_frags == 0) {
+        Affine last = cell_runs(d, u, active, x, ends);
+        if (u.parts > 1u && !join_parts(d, u, lane, last, ends)) continue;
+        const bool frags = ends.x != kNoFragment;
+        if (FORWARD && active && !frags) {
             float4 c[1] = {make_float4(1.f, 1.f, 1.f, 1.f)};
             apply_run(c, last.a, last.b);
             const float s = d.out_scale;
@@ -581,11 +689,11 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_runs(FrameArgs a, DiffArg
                 if (X < u.bs.W && Y < u.bs.H) store_pixel(d, u.bs.image_off + (int64_t)Y * u.bs.W + X, v);
             }
         }
-        const uint32_t cells = __ballot_sync(0xffffffffu, n_frags > 0);
+        const uint32_t cells = __ballot_sync(0xffffffffu, frags);
         uint32_t base = 0;
         if (lane == 0 && cells) base = atomicAdd(d.n_cells, (uint32_t)__popc(cells));
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (n_frags > 0) {
+        if (frags) {
             d.cell[base + __popc(cells & ((1u << lane) - 1u))] = u.cell0 + lane;
             d.cell_ends[u.cell0 + lane] = ends;
             d.cell_b[u.cell0 + lane] = last.b;
@@ -801,24 +909,32 @@ __global__ void __launch_bounds__(kDiffThreads, 3) k_diff_backward(FrameArgs a, 
 // the run's later spans (found first, in reverse), so a span's gradient needs
 // only its run's sums (c before the span = ra * c_run + rb); it is summed over
 // the unit's cells before it goes to memory.
-// The factors pi of 32 items and 32 cells are held in shared memory.  The first
-// sweep, from the bin's end, leaves pi at the end of every 32 items in memory, and
-// the forward sweep finds those of its 32 items again from there: 4 bytes a pair,
-// where a factor for every item and cell took a buffer of the deepest bin's items
-// for every warp (2.5 GB for a bin of 4,096).
+// The factors pi of 32 items and 32 cells are held in shared memory, and the first
+// sweep, from the unit's end, leaves pi at the end of every 32 items there too: the
+// forward sweep finds those of its 32 items again from it.  (A factor for every item
+// and cell of the deepest bin, for every warp, took 2.5 GB for a bin of 4,096.)
 __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffArgs d) {
     const int lane = threadIdx.x & 31;
-    __shared__ float s_pi[kDiffThreads / 32][32][32];  // item, cell
-    float(*const pis)[32] = s_pi[threadIdx.x >> 5];
+    __shared__ float s_pi[kDiffThreads / 32][32][32];                // item, cell
+    __shared__ float s_ends[kDiffThreads / 32][kPartItems / 32][32];  // 32 items, cell
+    float(*const pis)[32] = s_pi[threadIdx.x >> 5], (*const pi_ends)[32] = s_ends[threadIdx.x >> 5];
+    const uint32_t n_parts = *d.n_parts;
     Unit u;
-    while (next_unit(a, d, lane, u)) {
+    while (next_unit(a, d, n_parts, lane, u)) {
         if (u.fin == u.beg) continue;
         const bool active = lane < u.cells;
         const int x = u.x0 + 2 * lane;
-        // pi at the end of the bin's items from base on, 32 at a time: [base - u.beg]
-        // (a bin's place: past the earlier bins' items and 32 for each of them)
-        float *const ends = d.run_pi + ((size_t)(u.beg & ~31u) + u.cell0 + lane);
-        bool frags = false;
+        // the state that a part of a bin starts from
+        uint32_t before = kNoFragment;  // the last fragment before it
+        Affine run = empty_run();       // the spans since
+        float pi = 1.f;
+        if (u.parts > 1u) {
+            const size_t at = (size_t)u.place * 32 + lane;
+            before = d.part_ends[at].x;
+            run = Affine{d.part_a[at], d.part_b[at]};
+            pi = d.part_pi[at];
+        }
+        bool frags = before != kNoFragment;
         // pi before each of the 32 items from base on, given that after them
         auto sweep = [&](uint32_t base, float pi) {
             const uint32_t mine = min(base + lane, u.fin - 1);
@@ -838,17 +954,20 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
             }
             return pi;
         };
-        float pi = 1.f;
         for (uint32_t base = u.beg + ((u.fin - u.beg - 1) & ~31u); base != u.beg; base -= 32) {
-            ends[base - u.beg] = pi;
+            pi_ends[(base - u.beg) / 32][lane] = pi;
             pi = sweep(base, pi);
         }
         sweep(u.beg, pi);
         // the sums of the cell's first run, whose samples start white (not
         // used if that run is empty); of a cell without fragments: the pixels'
         // adjoints
-        float4 Ls = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (frags) {
+        float4 Ls = make_float4(0.f, 0.f, 0.f, 0.f), Ks;
+        const bool inside = before < kLaterFragment;  // past a fragment: its run's sums
+        if (inside) {
+            Ls = d.run_sum[2 * (size_t)before];
+            Ks = d.run_sum[2 * (size_t)before + 1];
+        } else if (frags) {
             Ls = d.cell_sum[u.cell0 + lane];
         } else if (active) {
 #pragma unroll
@@ -861,10 +980,10 @@ __global__ void __launch_bounds__(kDiffThreads) k_diff_spans(FrameArgs a, DiffAr
                 }
             }
         }
-        float4 Ks = Ls;
-        Affine run{1.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+        if (!inside) Ks = Ls;
+        if (no_spans(run.a)) run.a = 1.f;
         for (uint32_t base = u.beg; base < u.fin; base += 32) {
-            if (base != u.beg) sweep(base, ends[base - u.beg]);
+            if (base != u.beg) sweep(base, pi_ends[(base - u.beg) / 32][lane]);
             const uint32_t mine = min(base + lane, u.fin - 1);
             const uint4 my_it = __ldg(&d.bitem[mine]);
             const uint32_t my_cols = item_cols(my_it);
@@ -992,14 +1111,16 @@ int diff_sm_count() {
 template <bool BWD>
 int launch_diff(const FrameArgs &a, const DiffArgs &d, cudaStream_t s) {
     if (a.n_bins <= 0) return 0;
-    cudaMemsetAsync(d.queue, 0, 3 * sizeof(uint32_t), s);  // (and the cell list's length and queue after it)
+    cudaMemsetAsync(d.queue, 0, 4 * sizeof(uint32_t), s);  // (and the lists' lengths and the cells' queue after it)
     const unsigned grid = (unsigned)diff_blocks(a);
     int n = 2;
     if (d.npairs > 0) {
-        k_diff_gather<<<(unsigned)((d.npairs + 255) / 256), 256, 0, s>>>(d, a.S / 8);
+        k_diff_gather<<<(unsigned)((std::max(d.npairs, a.n_bins) + 255) / 256), 256, 0, s>>>(d, a.S / 8, a.n_bins);
         ++n;
     }
-    const unsigned bin_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((a.n_bins + 7) / 8, grid));
+    // (a warp per bin, or part of one, as far as they are resident)
+    const int64_t units = a.n_bins + diff_parts(d.npairs);
+    const unsigned bin_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((units + 7) / 8, 8 * (int64_t)diff_sm_count()));
     k_diff_runs<!BWD><<<bin_grid, kDiffThreads, 0, s>>>(a, d);
     // (the forward has no tape of its own per warp: as many blocks as are resident)
     const unsigned fwd_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(a.n_bins * 4, 5 * (int64_t)diff_sm_count()));
@@ -1035,7 +1156,8 @@ int64_t diff_tape_words(const FrameArgs &a, int depth) {
     return diff_blocks(a) * (int64_t)depth * (a.S / 8) * kDiffThreads;
 }
 
-int64_t diff_pi_words(const FrameArgs &a, int64_t npairs) { return npairs + a.n_bins * (kTileW / 2); }
+// (a bin of n > kPartItems items has fewer than 2 n / kPartItems parts)
+int64_t diff_parts(int64_t npairs) { return npairs > kPartItems ? 2 * npairs / kPartItems : 0; }
 
 __global__ void k_accumulate(float *__restrict__ dst, const float *__restrict__ src, int64_t n, int first) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

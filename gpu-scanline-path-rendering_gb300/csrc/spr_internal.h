@@ -50,7 +50,7 @@ struct FrameCounters {
     uint32_t need_pairs;   // resolve pairs of the frame
     uint32_t n_items;      // n_merged + n_span
     uint32_t tiles[3];     // look-back tile counters: entry offsets, scan-mark, pair offsets
-    uint32_t diff_queue[3];  // differentiable frames: DiffArgs::queue
+    uint32_t diff_queue[4];  // differentiable frames: DiffArgs::queue
     uint32_t diff_status;  // differentiable frames: DiffArgs::status
     uint32_t n_seg[3], q_seg[3];  // segment sort: listed segments by size class, and those taken
     uint32_t longest;            // entries of the longest path (sized frames)
@@ -315,9 +315,16 @@ struct DiffArgs {
     // per warp: tape_depth x (samples per thread) x 32 sample states (backward)
     float4 *tape;
     int tape_depth;
-    float *run_pi;  // per bin, 32 of its items and cell: the spans' factor at their end (backward)
-    uint32_t *queue;     // unit queue; then the cell list's length and its queue (zeroed by the launchers)
-    uint32_t *n_cells, *cell_queue;
+    // the parts of the bins with many items (bin, part), the parts done of such a
+    // bin, and per part and cell: the run at its end and its first and last
+    // fragments, after that (backward) the state it starts from: the run and the last
+    // fragment before it and the factor of the spans after it
+    uint2 *part, *part_ends;
+    uint32_t *part_done;
+    float4 *part_b;
+    float *part_a, *part_pi;
+    uint32_t *queue;     // unit queue; then the cell list's length and its queue, the part list's length (zeroed by the launchers)
+    uint32_t *n_cells, *cell_queue, *n_parts;
     uint32_t *status;    // bit 0: a cell has more fragments than tape_depth (rerun with more)
     // pixel = out_scale * (mean of the samples), added to the image when
     // accumulate (the passes of a 256-sample frame: 1/8 each); the backward
@@ -327,7 +334,7 @@ struct DiffArgs {
 };
 int64_t diff_blocks(const FrameArgs &a);
 int64_t diff_tape_words(const FrameArgs &a, int depth);      // float4 count of the sample-state tape
-int64_t diff_pi_words(const FrameArgs &a, int64_t npairs);   // float count of the span factors
+int64_t diff_parts(int64_t npairs);                          // most parts of bins with many items
 int launch_diff_forward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 int launch_diff_backward(const FrameArgs &a, const DiffArgs &d, cudaStream_t s);
 // dL/d(stored vertex in transformed space) -> dL/d(input vertex), dL/d(path affine).

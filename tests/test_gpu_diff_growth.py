@@ -15,10 +15,10 @@ REL_TOL = 1e-3  # (as the reference-gradient tests)
 class Fit:
     """One scene's fill, gradient and outputs, and the oracle's."""
 
-    def __init__(self, scene, W, H, samples, seed=3):
+    def __init__(self, scene, W, H, samples, seed=3, alpha=(0.02, 0.6)):
         rng = np.random.default_rng(seed)
         self.scene = scene
-        fill = np.c_[rng.uniform(0, 1, (scene.n_paths, 3)), rng.uniform(0.02, 0.6, (scene.n_paths, 1))].astype(np.float32)
+        fill = np.c_[rng.uniform(0, 1, (scene.n_paths, 3)), rng.uniform(*alpha, (scene.n_paths, 1))].astype(np.float32)
         G = rng.normal(size=(H, W, 4)).astype(np.float32)
         self.ref_img, self.ref = oracle.diff(scene, W, H, fill, grad_image=G, samples=samples)
         self.fill, self.G = torch.tensor(fill, device="cuda"), torch.tensor(G, device="cuda")
@@ -36,7 +36,7 @@ class Fit:
         torch.cuda.synchronize()
         assert np.abs(self.img.cpu().numpy() - self.ref_img).max() < 1e-5
         for got, ref in ((self.gf, self.ref["fill"]), (self.gv, self.ref["vertex"])):
-            assert np.linalg.norm(got.cpu().numpy() - ref) / np.linalg.norm(ref) < REL_TOL
+            assert np.linalg.norm(got.cpu().numpy() - ref) / max(np.linalg.norm(ref), 1e-30) < REL_TOL
 
 
 def test_a_refused_growth_does_not_stick():
@@ -120,3 +120,39 @@ def test_crowded_band_among_empty_ones(samples):
         fit.backward(r)
         assert r.frame_stats()["host_syncs"] == 1
         fit.check()
+
+
+def covers(n, marked, W, H, rng):
+    """n paths over the whole viewport and past it (a span in every cell row, no
+    fragment), and after every `marked`-th of them a mark in some cell."""
+    pts, pid, k = [], [], 0
+
+    def add(q):
+        nonlocal k
+        for j in range(4):
+            pts.extend([q[j], q[(j + 1) % 4]])
+            pid.append(k)
+        k += 1
+
+    for p in range(n):
+        add([(-7, -5), (W + 7, -5), (W + 7, H + 5), (-7, H + 5)])
+        if marked and p % marked == marked - 1:
+            x, y = rng.uniform(0.2, W - 0.2), rng.uniform(0.2, H - 0.2)
+            add([(x - .15, y - .15), (x + .15, y - .1), (x + .1, y + .15), (x - .1, y + .1)])
+    return line_scene(pts, pid)
+
+
+@pytest.mark.parametrize("samples", [8, 16, 32])
+@pytest.mark.parametrize("marked", [0, 1, 40, 300])
+@pytest.mark.parametrize("n", [127, 128, 129, 256, 257, 513, 800])
+def test_bins_in_parts(n, marked, samples):
+    """Bins of up to 128 items and of two to thirteen times as many, which several
+    warps go through in parts: cells without fragments, with fragments in every
+    part, in some, in the last only.  (Alphas are small: the lowest layer counts.)"""
+    W, H = 70, 3
+    fit = Fit(covers(n, marked, W, H, np.random.default_rng(n)), W, H, samples, alpha=(0.001, 0.01))
+    with spr.VGRasterizer(W, H, samples=samples) as r:
+        for _ in range(2):
+            fit.render(r)
+            fit.backward(r)
+            fit.check()
