@@ -538,7 +538,7 @@ int set_scene_host(spr_handle *h, const spr_scene_view *v) {
     if ((st = upload(h->fill, v->path_fill_rgba, P))) return st;
     h->has_affine = v->path_affine != nullptr;
     if (h->has_affine && (st = upload(h->affine, v->path_affine, 6 * (size_t)P))) return st;
-    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), nullptr);
+    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), nullptr, nullptr);
     if (cudaStreamSynchronize(nullptr) != cudaSuccess) return cuda_status();
     h->P = P;
     h->C = C;
@@ -594,8 +594,7 @@ int spr_set_scene(spr_handle *h, const spr_scene_view *v) {
                          v->curve_arc_w ? h->sc_w.as<float>() : nullptr, C, V, P, h->vertex.as<float2>(),
                          h->vpid.as<uint32_t>(), h->vmap.as<uint32_t>(), h->curves.as<CurveDesc>(),
                          h->scene_flags.as<uint32_t>(), s);
-    // (of an invalid scene: entries past P are never written)
-    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), s);
+    launch_path_starts(h->curves.as<CurveDesc>(), C, P, h->path_start.as<uint32_t>(), h->scene_flags.as<uint32_t>(), s);
     cudaMemcpyAsync(h->h_u32, h->scene_flags.p, 4, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return cuda_status();
     if ((st = cuda_status())) return st;

@@ -139,9 +139,11 @@ __host__ __device__ __forceinline__ int fw_chg(uint32_t b) { return (int)(b << 2
 int launch_segment_sort(uint32_t P, int64_t cap_nf, const uint32_t *offsets, uint64_t *keys, uint32_t *vals,
                         uint64_t *keys_out, uint32_t *vals_out, const uint32_t *path_start, uint32_t *list,
                         FrameCounters *ctr, cudaStream_t s);
-// First curve of every path (P + 1 words; curves ascend by path), and the
-// entries of the longest path.
-int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, cudaStream_t s);
+// First curve of every path (P + 1 words; curves ascend by path; not written if bit
+// 0 of *invalid, a scene's flags on the device or null, is set), and the entries of
+// the longest path.
+int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, const uint32_t *invalid,
+                       cudaStream_t s);
 int launch_longest_path(const uint32_t *path_start, const uint32_t *offsets, uint32_t P, uint32_t *longest,
                         cudaStream_t s);
 int64_t radix_tmp_words(int64_t n);

@@ -293,10 +293,13 @@ __device__ __forceinline__ int digit_bits(int bits) {
     return passes > 0 ? (bits + passes - 1) / passes : 0;
 }
 
-// First curve of every path (curves ascending by path); start[P] = C.
-__global__ void k_path_starts(const CurveDesc *__restrict__ curves, uint32_t C, uint32_t P, uint32_t *__restrict__ start) {
+// First curve of every path (curves ascending by path); start[P] = C.  Nothing is
+// written for a scene found invalid (bit 0 of *invalid, if given): its curves may be
+// in any order, or not written, and every one of them would fill up to P entries.
+__global__ void k_path_starts(const CurveDesc *__restrict__ curves, uint32_t C, uint32_t P, uint32_t *__restrict__ start,
+                              const uint32_t *__restrict__ invalid) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > (int64_t)C) return;
+    if (c > (int64_t)C || (invalid != nullptr && (*invalid & 1u))) return;
     const uint32_t lo = c == 0 ? 0u : curves[c - 1].pid + 1u;
     const uint32_t hi = c == (int64_t)C ? P : curves[c].pid;
     for (uint32_t q = lo; q <= hi && q <= P; ++q) start[q] = (uint32_t)c;
@@ -642,8 +645,9 @@ int sort_sms() {
 
 }  // namespace
 
-int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, cudaStream_t s) {
-    k_path_starts<<<(unsigned)(((int64_t)C + 1 + 255) / 256), 256, 0, s>>>(curves, C, P, path_start);
+int launch_path_starts(const CurveDesc *curves, uint32_t C, uint32_t P, uint32_t *path_start, const uint32_t *invalid,
+                       cudaStream_t s) {
+    k_path_starts<<<(unsigned)(((int64_t)C + 1 + 255) / 256), 256, 0, s>>>(curves, C, P, path_start, invalid);
     return 1;
 }
 
