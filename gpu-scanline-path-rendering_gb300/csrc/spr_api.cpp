@@ -1047,8 +1047,10 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
                 if ((st = scene_bins(h, frame_bin_shift(h, false), s))) return st;
                 a = make_args(h, false);
                 nbins = a.n_bins;
+                // (more bins, for the resolve more warps too)
                 if ((st = ensure(h->bins, 4 * (size_t)bin_words(nbins))) ||
-                    (st = ensure(h->lb_pair, 8 * (size_t)lookback_words(nbins))))
+                    (st = ensure(h->lb_pair, 8 * (size_t)lookback_words(nbins))) ||
+                    (st = ensure(h->overflow, 4 * (size_t)std::max<int64_t>(resolve_overflow_words(a), 1))))
                     return st;
                 bin_off = h->bins.as<uint32_t>();
                 bin_count = bin_off + bin_stride(nbins);
