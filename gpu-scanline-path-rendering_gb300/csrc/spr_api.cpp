@@ -785,6 +785,14 @@ struct ZeroedWords {
     }
 };
 
+// Resolve bins of a frame in tiles of 1 << shift columns.
+int64_t frame_bins(const spr_handle *h, int shift) {
+    if (h->n_scenes == 0) return (int64_t)bin_cols(h->cfg.width, shift) * bin_rows(h->cfg.height, shift);
+    int64_t n = 0;
+    for (const SceneInfo &si : h->scenes_h) n += (int64_t)bin_cols(si.W, shift) * bin_rows(si.H, shift);
+    return n;
+}
+
 // The batch scene table for bin geometry `shift` (tiles of 1 << shift
 // columns): every scene's tile and band counts and first bin, uploaded when
 // the geometry differs from the table's.
@@ -909,7 +917,11 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
     // flags, look-back words of the entry-offset and pair-offset scans, pair
     // counts and fill counters of the bins
     const ZeroedWords z(h->P, h->C, nbins);
-    if ((st = ensure(h->counters, 4 * (size_t)z.total))) return st;
+    // (a frame that may change its tile leaves room for the next one's words: frames
+    // after a sized one allocate nothing, and a captured one cannot)
+    int64_t words = z.total;
+    if (a.alt_shift >= 0) words = std::max(words, ZeroedWords(h->P, h->C, frame_bins(h, a.alt_shift)).total);
+    if ((st = ensure(h->counters, 4 * (size_t)words))) return st;
     FrameCounters *ctr = h->counters.as<FrameCounters>();
     uint32_t *const zw = h->counters.as<uint32_t>();
     // stage 3: transform + visibility

@@ -36,3 +36,23 @@ def test_many_entries_in_every_bin(W, H, samples):
         for _ in range(2):
             r.rasterize()
             assert np.array_equal(r.read_image().reshape(-1), ref["IMAGE"])
+
+
+def test_next_frames_allocate_nothing():
+    """The frame after the change is captured, replayed, and runs under a memory
+    limit of what the first one took."""
+    W, H = 2048, 10
+    scene = marks(20, W, H, 6.0, 1)
+    ref = oracle.run(scene, W, H, samples=8, ms_output=False)
+    for graph in (True, False):
+        with spr.VGRasterizer(W, H, samples=8, ms_output=False) as r:
+            r.set_graph_replay(graph)
+            r.add_vg(scene)
+            r.rasterize()
+            held = r.frame_stats()["device_bytes"]
+            r.set_memory_limit(held)
+            for k in range(3):
+                r.rasterize()
+                assert r.frame_stats()["host_syncs"] == 0 and r.graph_replays() == (k + 1 if graph else 0)
+                assert np.array_equal(r.read_image().reshape(-1), ref["IMAGE"])
+            assert r.frame_stats()["device_bytes"] == held
