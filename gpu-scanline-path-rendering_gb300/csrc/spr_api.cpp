@@ -1346,7 +1346,8 @@ int spr_autotune(spr_handle *h, int32_t frames, void *stream, spr_tune *out) {
         if (t < best) best = t, best_emit = v;
     }
     h->tune_emit = best_emit;
-    for (int v = 2; v <= 3 && !st; ++v) {  // 4 is the default
+    const int resident = resolve_resident(make_args(h));
+    for (int v = 2; v < std::min(resident, 4) && !st; ++v) {  // (the default: as many as are resident)
         h->tune_bps = v;
         float t = 0.f;
         if ((st = time_frames(h, stream, frames, &t))) break;

@@ -196,7 +196,7 @@ struct FrameArgs {
     uint32_t n_grad;
     const uint32_t *grad_ramp;
     float rev[13];
-    int resolve_bps;  // resolve blocks per SM (1..4; 0 = the default 4)
+    int resolve_bps;  // resolve blocks per SM, at most (1..4; 0: as many as are resident)
 };
 
 // path_flags: P words, zero before.
@@ -250,6 +250,7 @@ int launch_bin_sort(const uint32_t *bin_off, int64_t nbins, uint32_t *pval, cons
 // resolve_overflow_words(a) words, the cell entries past the ones each warp
 // keeps in shared memory (multisample modes; unused otherwise).
 int64_t resolve_warps(const FrameArgs &a);
+int resolve_resident(const FrameArgs &a);  // its resident blocks per SM
 int64_t resolve_overflow_words(const FrameArgs &a);
 // RGBA8 image of a 256-sample frame from the sums its 8 passes accumulated.
 // Rows 0, 1 and 3 (columns 0, 1, 3) of the output transform's inverse.

@@ -2192,9 +2192,12 @@ int sm_count() {
 }
 
 // Shared memory of a resolve block: the tables and one cell state per warp.
+template <int S>
+size_t resolve_smem(bool ms) {
+    return sizeof(SmemTables) + (size_t)kResolveWarps * (ms ? sizeof(CellState<S / 8, kCellCap>) : sizeof(CellState<S / 8, 1>));
+}
 size_t resolve_smem(int S, bool ms) {
-    const int MW = S / 8, CAP = ms ? kCellCap : 1;
-    return sizeof(SmemTables) + (size_t)kResolveWarps * ((size_t)CAP * (MW + 1) * 32 * 4 + (size_t)(kWin + 1) * 32 * 4);
+    return S == 8 ? resolve_smem<8>(ms) : (S == 16 ? resolve_smem<16>(ms) : resolve_smem<32>(ms));
 }
 
 // Resolve blocks per SM: as many as fit in shared memory (at most 4), or
@@ -2209,32 +2212,24 @@ int64_t resolve_blocks(const FrameArgs &a) {
     return std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sm_count() * resolve_bps(a)));
 }
 
-template <int S, bool MS, bool SRGB, bool GRAD>
-void resolve_variant_g(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
-                     FrameCounters *ctr, cudaStream_t s) {
-    constexpr int CAP = MS ? kCellCap : 1;
-    const size_t smem = sizeof(SmemTables) + (size_t)kResolveWarps * sizeof(CellState<S / 8, CAP>);
-    auto kern = GRAD ? k_resolve_grad<S, MS, SRGB> : k_resolve<S, MS, SRGB>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // resident blocks per SM (registers or shared memory), so that every
-    // launched block runs at once; never more than resolve_blocks(a), which
-    // sized the overflow entry area
-    int fit = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kResolveWarps * 32, smem) != cudaSuccess || fit < 1)
-        fit = 1;
-    const int64_t blocks = std::min<int64_t>(resolve_blocks(a), (int64_t)sm_count() * fit);
-    kern<<<(unsigned)blocks, kResolveWarps * 32, smem, s>>>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr);
-}
-
-// Gradient paints get their own instantiations: the per-pixel paint costs
-// registers that plain frames should not pay for.
+// The frame's resolve kernel.  Gradient paints get their own instantiations: the
+// per-pixel paint costs registers that plain frames should not pay for.
+using ResolveKernel = void (*)(FrameArgs, const uint2 *, const uint32_t *, const uint32_t *, const uint32_t *,
+                               uint32_t *, uint32_t *, FrameCounters *);
 template <int S, bool MS, bool SRGB>
-void resolve_variant(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
-                     FrameCounters *ctr, cudaStream_t s) {
-    if (a.grad_table != nullptr)
-        resolve_variant_g<S, MS, SRGB, true>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr, s);
-    else
-        resolve_variant_g<S, MS, SRGB, false>(a, rec_a, rec_m, bstart, bend, image, overflow, ctr, s);
+ResolveKernel resolve_kernel(bool paints) {
+    return paints ? k_resolve_grad<S, MS, SRGB> : k_resolve<S, MS, SRGB>;
+}
+template <int S>
+ResolveKernel resolve_kernel(bool ms, bool srgb, bool paints) {
+    if (ms) return srgb ? resolve_kernel<S, true, true>(paints) : resolve_kernel<S, true, false>(paints);
+    return srgb ? resolve_kernel<S, false, true>(paints) : resolve_kernel<S, false, false>(paints);
+}
+ResolveKernel resolve_kernel(const FrameArgs &a) {
+    const bool ms = a.ms_output != 0, srgb = a.srgb != 0, paints = a.grad_table != nullptr;
+    if (a.S == 8) return resolve_kernel<8>(ms, srgb, paints);
+    if (a.S == 16) return resolve_kernel<16>(ms, srgb, paints);
+    return resolve_kernel<32>(ms, srgb, paints);
 }
 
 }  // namespace
@@ -2359,26 +2354,25 @@ int launch_bin_sort(const uint32_t *bin_off, int64_t nbins, uint32_t *pval, cons
 }
 
 
+// Resident resolve blocks per SM (registers or shared memory).
+int resolve_resident(const FrameArgs &a) {
+    const ResolveKernel kern = resolve_kernel(a);
+    const size_t smem = resolve_smem(a.S, a.ms_output != 0);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int fit = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kResolveWarps * 32, smem) != cudaSuccess || fit < 1)
+        fit = 1;
+    return fit;
+}
+
 int launch_resolve(const FrameArgs &a, const uint2 *rec_a, const uint32_t *rec_m, const uint32_t *bstart, const uint32_t *bend, uint32_t *image, uint32_t *overflow,
                     FrameCounters *counters, cudaStream_t s) {
     if (a.n_bins <= 0) return 0;
-    const bool ms = a.ms_output != 0, srgb = a.srgb != 0;
-    if (a.S == 8) {
-        if (ms && srgb) resolve_variant<8, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (ms) resolve_variant<8, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (srgb) resolve_variant<8, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else resolve_variant<8, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-    } else if (a.S == 16) {
-        if (ms && srgb) resolve_variant<16, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (ms) resolve_variant<16, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (srgb) resolve_variant<16, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else resolve_variant<16, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-    } else {
-        if (ms && srgb) resolve_variant<32, true, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (ms) resolve_variant<32, true, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else if (srgb) resolve_variant<32, false, true>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-        else resolve_variant<32, false, false>(a, rec_a, rec_m, bstart, bend, image, overflow, counters, s);
-    }
+    // every launched block runs at once; never more than resolve_blocks(a),
+    // which sized the overflow entry area
+    const int64_t blocks = std::min<int64_t>(resolve_blocks(a), (int64_t)sm_count() * resolve_resident(a));
+    resolve_kernel(a)<<<(unsigned)blocks, kResolveWarps * 32, resolve_smem(a.S, a.ms_output != 0), s>>>(
+        a, rec_a, rec_m, bstart, bend, image, overflow, counters);
     return 1;
 }
 
