@@ -994,7 +994,7 @@ int render_frame(spr_handle *h, void *stream, const DiffCall *dc) {
         order = ealt ? h->eval[1].as<uint32_t>() : h->eval[0].as<uint32_t>();
     }
     // (the sort's second value buffer, not yet in use, holds the crossings of
-    // the warps with more than fit in shared memory)
+    // the blocks with more than fit in shared memory)
     L += launch_curve_emit(a, h->tvert.as<float2>(), h->pvis.as<uint8_t>(), h->offsets.as<uint32_t>(), order,
                            h->sval[1].as<float>(), h->entries.as<int2>(), cap_nf, ctr, s);
     L += launch_fragment(a, h->tvert.as<float2>(), h->entries.as<int2>(), cap_nf, ctr, h->key.as<int32_t>(),

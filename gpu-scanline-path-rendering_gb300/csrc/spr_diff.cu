@@ -482,12 +482,6 @@ __device__ __forceinline__ bool next_unit(const FrameArgs &a, const DiffArgs &d,
 // stores to the runs' maps and factors between the loads would otherwise keep
 // them one after the other.)
 
-// Item `it` touches the cell at column x (a fragment covers one cell).
-__device__ __forceinline__ bool touches(const uint4 &it, int x) {
-    const int ix = (int)(it.x & 0xFFFFu);
-    return it.z != 0u ? ix == x : (x >= ix && x < ix + (int)it.y);
-}
-
 // 32 of a bin's items, one per lane, for the passes with a lane per cell, which
 // take them one by one through shuffles (a load at a time would leave a memory
 // latency between them).  Column | length << 16 (a fragment: 0).
@@ -498,6 +492,7 @@ __device__ __forceinline__ float4 shfl_fill(const float4 &f, int q) {
     return make_float4(__shfl_sync(0xffffffffu, f.x, q), __shfl_sync(0xffffffffu, f.y, q),
                        __shfl_sync(0xffffffffu, f.z, q), __shfl_sync(0xffffffffu, f.w, q));
 }
+// An item of columns `cols` touches the cell at column x.
 __device__ __forceinline__ bool touches(uint32_t cols, int x) {
     const int ix = (int)(cols & 0xFFFFu), len = (int)(cols >> 16);
     return len == 0 ? ix == x : (x >= ix && x < ix + len);

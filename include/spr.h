@@ -377,7 +377,7 @@ const char *spr_status_string(int32_t status);
  * replaced by a float composite: every sample is composited in linear RGBA
  * over opaque white in painter's order, c' = f.rgb * a + c.rgb * (1 - a),
  * c'.a = a * a + c.a * (1 - a), with the path colours f taken from
- * fill_rgba (4 floats per path) instead of path_fill_rgba, and a pixel is
+ * fill_rgba (4 floats per path, of any value) instead of path_fill_rgba, and a pixel is
  * the mean of its samples.  All pointers are device pointers.  The handle's
  * RGBA8 image is not written (batches: spr_batch_diff_render).
  */
